@@ -89,6 +89,26 @@ bool aligned16(const void* p) { return p == nullptr || (reinterpret_cast<uintptr
 
 int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
+// Channels a relaid-out pixel or a packed filter tap is stored with.  The kernels copy 128 bytes of channels at a time;
+// a pitch that leaves those pieces unaligned makes most of them straddle two cache lines, and the copies, which bound
+// long reductions, slow down accordingly, so that channels fill whole 128-byte lines (or an even share of one):
+// zeros are never computed with more often than before, since a block of 128 bytes was always multiplied whole.
+int padded_channels(int dtype, int c) {
+  const int es = elem_size(dtype);
+  for (int bytes = 16; bytes < 128; bytes *= 2)
+    if (c * es <= bytes) return bytes / es;
+  return round_up(c, 128 / es);
+}
+
+// The same for the relaid-out activations, except where only rows of 16-byte multiples keep them within the built-in
+// scratch of fdnn_conv2d_fwd_static_scratch: that call takes every problem whose tightest layout fits.
+int padded_x_channels(const fdnn_conv_desc* d) {
+  const int es = elem_size(d->dtype), wide = padded_channels(d->dtype, d->c), tight = round_up(d->c, 16 / es);
+  const long long per_channel = (long long)(d->dtype == FDNN_F32 ? 2 : 1) * d->n * d->h * d->w * es;
+  const bool fits = per_channel * tight <= FDNN_STATIC_SCRATCH_BYTES;
+  return fits && per_channel * wide > FDNN_STATIC_SCRATCH_BYTES ? tight : wide;
+}
+
 // Can the tensor-core path express this geometry?  Limits are those of the
 // im2col tensor map: box corners in [-128, 127], tap offsets <= 255,
 // traversal strides <= 8.
@@ -146,6 +166,37 @@ long long y_pixel_stride(const fdnn_conv_desc* d, int oh, int ow) {
 
 bool y_is_dense_nhwc(const fdnn_conv_desc* d, int oh, int ow, const void* y) {
   return y_pixel_stride(d, oh, ow) > 0 && aligned16(y);
+}
+
+// How the single-CTA kernel's epilogue writes a y that has no TMA map (see epilogue_store_strided): along channels
+// when they are contiguous, along pixels when every image's pixels are (NCHW), with the widest unit that every run's
+// start is a multiple of (and, along pixels, that no image boundary cuts); otherwise element by element.
+void choose_strided_store(const fdnn_conv_desc& d, int oh, int ow, const void* y, IgemmParams* p) {
+  const int es = elem_size(d.dtype);
+  const long long sn = d.y_strides[0], sk = d.y_strides[1], sh = d.y_strides[2], sw = d.y_strides[3];
+  const uintptr_t base = reinterpret_cast<uintptr_t>(y);
+  auto fits = [es](long long extent, long long stride, int unit) { return extent <= 1 || stride * es % unit == 0; };
+  p->y_mode = 0;
+  p->y_unit = es;
+  if (d.k > 1 && sk == 1) {
+    p->y_mode = 2;
+    for (int unit = 16; unit > es; unit /= 2) {
+      if (base % unit == 0 && fits(d.n, sn, unit) && fits(oh, sh, unit) && fits(ow, sw, unit)) {
+        p->y_unit = unit;
+        break;
+      }
+    }
+    return;
+  }
+  const bool pixels = ow > 1 ? (sw == 1 && (oh == 1 || sh == ow)) : (oh == 1 || sh == 1);
+  if (!pixels) return;
+  p->y_mode = 1;
+  for (int unit = 16; unit > es; unit /= 2) {
+    if ((long long)oh * ow * es % unit == 0 && base % unit == 0 && fits(d.n, sn, unit) && fits(d.k, sk, unit)) {
+      p->y_unit = unit;
+      break;
+    }
+  }
 }
 
 // Low-channel mode (C <= 4, e.g. the 7x7 stride-2 stem): four neighbouring
@@ -238,8 +289,7 @@ int choose_pixel_group(const fdnn_conv_desc* d, int oh, int ow, const void* y) {
 // The equivalent convolution of a pixel-grouped layer (filter strides describe the packed [Q*K][R][S'][Cpad]).
 fdnn_conv_desc grouped_desc(const fdnn_conv_desc* d, int q, int oh, int ow) {
   fdnn_conv_desc v = *d;
-  const int gran = 16 / elem_size(d->dtype);
-  const int c_pad = round_up(d->c, gran);
+  const int c_pad = padded_channels(d->dtype, d->c);
   v.k = q * d->k;
   v.s = d->s + (q - 1) * d->stride_w;
   v.stride_w = q * d->stride_w;
@@ -457,7 +507,7 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
         plan->flops = flops;
         plan->bytes = bytes;
         plan->w_packed = 1;
-        plan->packed_weight_bytes = (long long)v.k * v.r * v.s * round_up(d->c, 16 / es) * es;
+        plan->packed_weight_bytes = (long long)v.k * v.r * v.s * padded_channels(d->dtype, d->c) * es;
         return FDNN_OK;
       }
     }
@@ -478,12 +528,12 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
                          (d->r <= 1 || (d->s > 1 ? d->w_strides[2] == (long long)d->s * d->w_strides[3]
                                                  : d->w_strides[2] % gran == 0)) &&
                          aligned16(w);
-  const int c_pad = round_up(d->c, gran);
+  const int c_pad = padded_channels(d->dtype, d->c);
   plan->c_padded = c_pad;
   plan->x_repacked = x_inplace ? 0 : 1;
   plan->w_packed = w_inplace ? 0 : 1;
   const int planes = (d->dtype == FDNN_F32) ? 2 : 1;
-  if (!x_inplace) plan->workspace_bytes = (long long)planes * d->n * d->h * d->w * c_pad * es;
+  if (!x_inplace) plan->workspace_bytes = (long long)planes * d->n * d->h * d->w * padded_x_channels(d) * es;
   if (!w_inplace) plan->packed_weight_bytes = (long long)planes * d->k * d->r * d->s * c_pad * es;
   plan->tile_m = 128;
   plan->tile_k = 128 / es;
@@ -1284,15 +1334,16 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   int a_c = d.c;
   long long a_plane = 0;
   if (plan.x_repacked) {
-    a_plane = (long long)d.n * d.h * d.w * c_pad;
+    const int x_pad = padded_x_channels(&d);
+    a_plane = (long long)d.n * d.h * d.w * x_pad;
     e = launch_repack_x(d.dtype, x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w,
-                        c_pad, workspace, a_plane, stream);
+                        x_pad, workspace, a_plane, stream);
     if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
     a_base = workspace;
-    a_sw = c_pad;
-    a_sh = (long long)d.w * c_pad;
-    a_sn = (long long)d.h * d.w * c_pad;
-    a_c = c_pad;
+    a_sw = x_pad;
+    a_sh = (long long)d.w * x_pad;
+    a_sn = (long long)d.h * d.w * x_pad;
+    a_c = x_pad;
   }
   const void* b_base = w;
   long long b_stap = d.s > 1 ? d.w_strides[3] : (d.r > 1 ? d.w_strides[2] : any_stride);
@@ -1365,6 +1416,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
       tmY = tmA;
     }
   }
+  if (!p.tma_store && !out_f32) choose_strided_store(d, plan.oh, plan.ow, y, &p);
   alignas(64) CUtensorMap tmR = tmY;
   alignas(64) CUtensorMap tmRbox = tmY;
   if (residual != nullptr && p.tma_store) {

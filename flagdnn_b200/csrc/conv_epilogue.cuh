@@ -10,6 +10,7 @@
 
 #include <type_traits>
 
+#include "conv_convert.cuh"
 #include "sm100_ptx.cuh"
 #include "stream_k.cuh"
 
@@ -263,6 +264,279 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_row, int n0, int 
       // committed even when empty so that "all but the latest group" always means the other buffer
       if (st_rows > 0) tma_store_3d(st_rows >= 32 ? tm_full : tm_tail, buf, n0 + g * kPerStore, st_row, st_img);
       bulk_commit_group();
+    }
+  }
+}
+
+// Epilogue for a y the TMA unit cannot write (its strides or base are not multiples of 16 bytes, or its pixels and
+// not its channels are contiguous): the same arithmetic, and 32 rows x 128 bytes are staged in shared memory all the
+// same, but the warp then writes them itself, with lanes along whichever dimension of y is contiguous and `unit` bytes
+// per lane, the widest the alignment of y allows:
+//   kYPixels    NCHW: staged as [column][32 pixels]; a unit is 2 / 4 / 8 neighbouring pixels of one channel.  Units
+//               never straddle two images (the host picks a unit that divides OH * OW)
+//   kYChannels  channels-last rows of a pitch that is not a multiple of 16 bytes: staged as [pixel][64 columns]
+// Where 16-bit rows may start at odd elements (unit 2), each run is written as the 4-byte words it covers whole, plus a
+// 2-byte element at either end.
+// What this is bound by: the stores.  One 2-byte store per value straight from the registers, lanes along pixels,
+// as before, kept the L1-to-L2 request path 53-77 % busy with the tensor pipe at 10 % (24 x 45 x 37 pixels, 104 -> 150
+// channels bf16 3x3: 106 us), and NCHW y cost 20 us per 128 x 256 tile.
+constexpr int kYScattered = 0, kYPixels = 1, kYChannels = 2;
+struct StridedOut {
+  void* y;                 // element type of the operands
+  const void* res;         // residual with y's strides, or nullptr
+  long long y_off;         // this lane's pixel: element offset of channel 0
+  long long sn, sk;        // element strides between images and between channels
+  int mode, unit;          // kY*, bytes per lane and store
+  int m0, M, ohw;          // the warp's first GEMM row, rows overall, pixels per image
+  bool row_ok;             // this lane's row exists
+};
+
+template <typename U> __device__ __forceinline__ U lds_unit(uint32_t a);
+template <> __device__ __forceinline__ uint32_t lds_unit<uint32_t>(uint32_t a) { return lds_u32(a); }
+template <> __device__ __forceinline__ uint2 lds_unit<uint2>(uint32_t a) { return lds_v2(a); }
+template <> __device__ __forceinline__ uint4 lds_unit<uint4>(uint32_t a) { return lds_v4(a); }
+
+// The four writers of a staged group.  Each reads a batch of units from shared memory before it stores the first: with
+// load and store of one unit after another the warp waits a shared-memory round trip per store (21 k clocks per
+// 128 x 256 tile instead of the few thousand its stores take).
+//
+// [column][32 pixels] in shared memory, U units along pixels; `out`: column 0, this lane's unit.
+template <typename U, int COL_BYTES>
+__device__ __forceinline__ void strided_pixels(char* out, uint32_t sbuf, int lane, int nc, bool ok, long long col_bytes) {
+  constexpr int kLanes = COL_BYTES / int(sizeof(U)), kPer = 32 / kLanes, kBatch = 4;
+  const int unit = lane % kLanes;
+  for (int c0 = lane / kLanes; c0 < nc; c0 += kPer * kBatch) {
+    U v[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int c = c0 + i * kPer;
+      if (c < nc) v[i] = lds_unit<U>(sbuf + c * COL_BYTES + unit * int(sizeof(U)));
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int c = c0 + i * kPer;
+      if (ok && c < nc) *reinterpret_cast<U*>(out + c * col_bytes) = v[i];
+    }
+  }
+}
+
+// 16-bit pixels whose columns may start at odd elements: the words a column's run covers whole, and its two ends;
+// 16 lanes per column.  Rows that do not lie in one image go element by element.
+__device__ __forceinline__ void strided_odd_pixels(uint16_t* y, uint32_t sbuf, int lane, int nc, bool whole, bool row_ok,
+                                                   long long run_off, long long lane_off, long long sk) {
+  if (!whole) {
+    if (!row_ok) return;
+    for (int c0 = 0; c0 < nc; c0 += 8) {
+      uint16_t v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c0 + i < nc) v[i] = lds_u16(sbuf + (c0 + i) * 64 + lane * 2);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c0 + i < nc) y[lane_off + (c0 + i) * sk] = v[i];
+    }
+    return;
+  }
+  // word l of a column that starts on a word boundary; else the halves either side of the boundary after it, and lane
+  // 15, whose neighbour wraps to word 0, writes the first and the last element
+  const int l = lane & 15, cc = lane >> 4;
+  uint16_t* run = y + run_off + cc * sk;
+  const uint32_t src = sbuf + cc * 64;
+  const uint32_t par0 = uint32_t(reinterpret_cast<uintptr_t>(run) >> 1) & 1u;   // two columns further: the same parity
+#pragma unroll 2
+  for (int c0 = 0; c0 < nc; c0 += 8) {
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      lo[i] = lds_u32(src + (c0 + 2 * i) * 64 + l * 4);
+      hi[i] = lds_u32(src + (c0 + 2 * i) * 64 + ((l + 1) & 15) * 4);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (c0 + 2 * i + cc < nc) {
+        if (par0 == 0u) {
+          *reinterpret_cast<uint32_t*>(run + 2 * l) = lo[i];
+        } else if (l != 15) {
+          *reinterpret_cast<uint32_t*>(run + 2 * l + 1) = __byte_perm(lo[i], hi[i], 0x5432);
+        } else {
+          run[31] = uint16_t(lo[i] >> 16);
+          run[0] = uint16_t(hi[i]);
+        }
+      }
+      run += 2 * sk;
+    }
+  }
+}
+
+// [pixel][128 bytes of columns], swizzled, U units along columns; row r's element offset is lane r's y_off.
+template <typename U, int ES>
+__device__ __forceinline__ void strided_channels(char* out, uint32_t sbuf, int lane, int nc, uint32_t rows_ok, long long y_off) {
+  constexpr int kLanes = 128 / int(sizeof(U)), kPer = 32 / kLanes, kBatch = 8;
+  const int byte0 = (lane % kLanes) * int(sizeof(U));
+  const bool full = byte0 + int(sizeof(U)) <= nc * ES;
+#pragma unroll 1
+  for (int r0 = 0; r0 < 32; r0 += kPer * kBatch) {
+    U v[kBatch];
+    long long off[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int r = (r0 + i * kPer + lane / kLanes) & 31;
+      v[i] = lds_unit<U>(sbuf + r * 128 + ((((byte0 >> 4) ^ (r & 7)) << 4) | (byte0 & 15)));
+      off[i] = __shfl_sync(0xffffffffu, y_off, r);
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int r = r0 + i * kPer + lane / kLanes;
+      if (r >= 32 || !((rows_ok >> r) & 1u)) continue;
+      char* dst = out + off[i] * ES + byte0;
+      if (full) {
+        *reinterpret_cast<U*>(dst) = v[i];
+      } else {   // the last columns: element by element
+        for (int b = 0; byte0 + b < nc * ES; b += ES) {
+          const int byte = byte0 + b;
+          const uint32_t a = sbuf + r * 128 + ((((byte >> 4) ^ (r & 7)) << 4) | (byte & 15));
+          if constexpr (ES == 2) *reinterpret_cast<uint16_t*>(dst + b) = lds_u16(a);
+          else *reinterpret_cast<uint32_t*>(dst + b) = lds_u32(a);
+        }
+      }
+    }
+  }
+}
+
+// The same for 16-bit rows that may start at odd elements: one row per store, as whole words and two ends (as in
+// strided_odd_pixels).
+__device__ __forceinline__ void strided_odd_channels(char* out, uint32_t sbuf, int lane, int nc, uint32_t rows_ok, long long y_off) {
+  uint16_t* y = reinterpret_cast<uint16_t*>(out);
+  auto word = [&](int r, int w) { return sbuf + r * 128 + ((((w >> 2) ^ (r & 7)) << 4) | ((w & 3) << 2)); };
+#pragma unroll 1
+  for (int r0 = 0; r0 < 32; r0 += 8) {
+    uint32_t lo[8], hi[8];
+    long long off[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      off[i] = __shfl_sync(0xffffffffu, y_off, r0 + i);
+      lo[i] = lds_u32(word(r0 + i, lane));
+      hi[i] = lds_u32(word(r0 + i, (lane + 1) & 31));
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (!((rows_ok >> (r0 + i)) & 1u)) continue;
+      uint16_t* run = y + off[i];
+      const bool par = (reinterpret_cast<uintptr_t>(run) & 2u) != 0;
+      const int a = 2 * lane + (par ? 1 : 0);
+      const uint32_t v = par ? __byte_perm(lo[i], hi[i], 0x5432) : lo[i];
+      if (a + 1 < nc) *reinterpret_cast<uint32_t*>(run + a) = v;
+      else if (a < nc) run[a] = uint16_t(v);
+      if (par && lane == 31) run[0] = uint16_t(hi[i]);
+    }
+  }
+}
+
+template <typename T, int BN, bool RES>
+__device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, int kout, int act, const float* s_scale,
+                                                       const float* s_bias, uint8_t* my_out, int lane,
+                                                       const StridedOut& o, uint32_t& store_seq) {
+  constexpr int kEs = int(sizeof(T));
+  constexpr int kCols = 128 / kEs;                 // columns per group: 64 (16-bit) or 32 (fp32)
+  constexpr int kLoads = kCols / 32;
+  constexpr int kColBytes = 32 * kEs;              // one column's 32 pixels
+  int groups = (kout - n0 + kCols - 1) / kCols;
+  if (groups > BN / kCols) groups = BN / kCols;
+  if (groups <= 0) return;
+  char* y = static_cast<char*>(o.y);
+  const uint32_t rows_ok = __ballot_sync(0xffffffffu, o.row_ok);
+  // kYPixels: the unit of pixels this lane writes (the same one for every column)
+  const int unit_px = o.unit / kEs;
+  const int lanes_per_col = kColBytes / (o.unit >= 4 ? o.unit : 4);
+  const int my_unit = lane & (lanes_per_col - 1);
+  long long u_off = 0;
+  bool u_ok = false, whole = false;
+  if (o.mode == kYPixels) {
+    const int px = kEs == 2 && o.unit == 2 ? 0 : my_unit * unit_px;
+    const int m = o.m0 + px;
+    const int img = m / o.ohw;
+    u_ok = m < o.M;
+    u_off = img * o.sn + (m - img * o.ohw);
+    whole = rows_ok == 0xffffffffu && (o.m0 + 31) / o.ohw == o.m0 / o.ohw;   // 32 pixels of one image
+  }
+#pragma unroll 1
+  for (int g = 0; g < groups; ++g) {
+    uint32_t raw[kLoads][32];
+#pragma unroll
+    for (int l = 0; l < kLoads; ++l) tmem_ld_32x32b_x32(t_row + g * kCols + l * 32, raw[l]);
+    uint8_t* buf = my_out + (store_seq & 1u) * (32 * 128);
+    ++store_seq;
+    const int col0 = n0 + g * kCols;
+    const int nc = kout - col0 < kCols ? kout - col0 : kCols;    // columns of this group that exist
+    tmem_ld_wait();
+    uint32_t row[32];
+#pragma unroll
+    for (int l = 0; l < kLoads; ++l) {
+      float v[32];
+#pragma unroll
+      for (int j4 = 0; j4 < 8; ++j4) {
+        const float4 sc = reinterpret_cast<const float4*>(s_scale + g * kCols + l * 32)[j4];
+        const float4 bi = reinterpret_cast<const float4*>(s_bias + g * kCols + l * 32)[j4];
+        v[4 * j4 + 0] = fmaf(__uint_as_float(raw[l][4 * j4 + 0]), sc.x, bi.x);
+        v[4 * j4 + 1] = fmaf(__uint_as_float(raw[l][4 * j4 + 1]), sc.y, bi.y);
+        v[4 * j4 + 2] = fmaf(__uint_as_float(raw[l][4 * j4 + 2]), sc.z, bi.z);
+        v[4 * j4 + 3] = fmaf(__uint_as_float(raw[l][4 * j4 + 3]), sc.w, bi.w);
+      }
+      if constexpr (RES) {
+        if (o.res != nullptr && o.row_ok) {
+          const T* res = static_cast<const T*>(o.res) + o.y_off + (long long)(col0 + l * 32) * o.sk;
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (l * 32 + j < nc) v[j] += to_f32<T>(res[j * o.sk]);
+        }
+      }
+      if (act > 1) {   // uniform; kept apart so that the common paths do not fetch 32 copies of erf and tanh
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = apply_activation(v[j], act);
+      }
+      if constexpr (kEs == 4) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) row[j] = __float_as_uint(act == 1 ? relu_keep_nan(v[j]) : v[j]);
+      } else if (act == 1) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) row[l * 16 + j] = round_pack2_relu<T>(v[2 * j], v[2 * j + 1]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) row[l * 16 + j] = round_pack2<T>(v[2 * j], v[2 * j + 1]);
+      }
+    }
+    const uint32_t sbuf = smem_u32(buf);
+    if (o.mode == kYPixels) {
+      if constexpr (kEs == 4) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sts_u32(sbuf + j * 128 + lane * 4, row[j]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          sts_u16(sbuf + (2 * j) * 64 + lane * 2, uint16_t(row[j]));
+          sts_u16(sbuf + (2 * j + 1) * 64 + lane * 2, uint16_t(row[j] >> 16));
+        }
+      }
+      __syncwarp();
+      if (kEs == 2 && o.unit == 2) {
+        strided_odd_pixels(reinterpret_cast<uint16_t*>(y), sbuf, lane, nc, whole, o.row_ok, u_off + col0 * o.sk,
+                           o.y_off + col0 * o.sk, o.sk);
+      } else {
+        char* out = y + (u_off + col0 * o.sk) * kEs;
+        if (o.unit == 16) strided_pixels<uint4, kColBytes>(out, sbuf, lane, nc, u_ok, o.sk * kEs);
+        else if (o.unit == 8) strided_pixels<uint2, kColBytes>(out, sbuf, lane, nc, u_ok, o.sk * kEs);
+        else strided_pixels<uint32_t, kColBytes>(out, sbuf, lane, nc, u_ok, o.sk * kEs);
+      }
+    } else {   // kYChannels
+#pragma unroll
+      for (int q = 0; q < 8; ++q)   // 16-byte pieces swizzled by row, as for the TMA store
+        sts_v4(sbuf + lane * 128 + ((q ^ (lane & 7)) << 4), make_uint4(row[4 * q], row[4 * q + 1], row[4 * q + 2], row[4 * q + 3]));
+      __syncwarp();
+      char* out = y + (long long)col0 * kEs;
+      if (kEs == 2 && o.unit == 2) strided_odd_channels(out, sbuf, lane, nc, rows_ok, o.y_off);
+      else if (o.unit == 16) strided_channels<uint4, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
+      else if (o.unit == 8) strided_channels<uint2, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
+      else strided_channels<uint32_t, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
     }
   }
 }

@@ -121,7 +121,9 @@ __device__ __forceinline__ void store32_contig(T* dst, const float (&v)[32]) {
   }
 }
 
-template <typename T, int BN, bool RES>
+// DENSE: y goes through the TMA unit (p.tma_store); otherwise through the warps' own stores, whose registers would push
+// the dense path's loop state to local memory if both lived in one kernel.
+template <typename T, int BN, bool RES, bool DENSE>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
                   const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmB2,
@@ -168,7 +170,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     fence_barrier_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
-    if (p.tma_store) tma_prefetch_desc(&tmY);
+    if constexpr (DENSE) tma_prefetch_desc(&tmY);
     if constexpr (Cfg::kSplit) {
       tma_prefetch_desc(&tmA2);
       tma_prefetch_desc(&tmB2);
@@ -215,7 +217,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if constexpr (RES) {
         // the epilogue of this tile will read its 128 x BN residual values a whole main loop from now:
         // ask for them to be brought into L2 so that its loads are short and HBM reads are requested early
-        if (do_a && p.residual != nullptr && p.tma_store && !p.lowc) tma_prefetch_l2_3d(&tmR, n_tile * BN, m_tile * kBM, 0);
+        if (DENSE && do_a && p.residual != nullptr && !p.lowc) tma_prefetch_l2_3d(&tmR, n_tile * BN, m_tile * kBM, 0);
       }
       const uint32_t a_tx = (Cfg::kSplit ? 2u : 1u) * (p.lowc ? uint32_t(p.a_tx_bytes) : uint32_t(Cfg::kABytes));
       const uint32_t b_tx = (Cfg::kSplit ? 2u : 1u) * uint32_t(Cfg::kBBytes);
@@ -380,7 +382,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     uint32_t store_seq = 0;
     uint32_t res_phases = 0;
     ResidualFetch rf;
-    rf.tm = (g_res != nullptr && p.tma_store) ? &tmRbox : nullptr;
+    rf.tm = (DENSE && g_res != nullptr) ? &tmRbox : nullptr;
     rf.bars = res_bar + (warp - kFirstEpiWarp) * 2;
     rf.phases = &res_phases;
     rf.abort_flag = abort_flag;
@@ -436,12 +438,23 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         st_row = m_tile * kBM + ew * 32;
         st_rows = 32;
       }
-      if (p.tma_store) {
+      if constexpr (DENSE) {
         // a tile's last warp may own fewer than 32 valid rows: tmA2 then holds a second
         // output map whose box is exactly that short (low-channel mode, 16-bit only)
         epilogue_store_tile<T, WC, RES>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
                                    out_stage + (warp - kFirstEpiWarp) * 2 * 32 * kRowBytes, lane, &tmY, &tmA2, st_row,
                                    st_img, st_rows, store_seq, &rf, g_scale != nullptr);
+      } else if (p.y_mode != kYScattered) {
+        StridedOut so;
+        so.y = p.y;
+        so.res = g_res;
+        so.y_off = y_off;
+        so.sn = p.y_sn; so.sk = p.y_sk;
+        so.mode = p.y_mode; so.unit = p.y_unit;
+        so.m0 = m_tile * kBM + ew * 32; so.M = p.M; so.ohw = ohw;
+        so.row_ok = row_ok;
+        epilogue_store_strided<T, WC, RES>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
+                                           out_stage + (warp - kFirstEpiWarp) * 2 * 32 * kRowBytes, lane, so, store_seq);
       } else {
 #pragma unroll 1
       for (int chunk = 0; chunk < WC / 32; ++chunk) {
@@ -486,7 +499,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       tc_fence_before();
       mbar_arrive(&tmem_empty[buf]);
     }
-    if (p.tma_store && lane == 0) bulk_wait_group0();  // stores must be done before the CTA retires
+    if (DENSE && lane == 0) bulk_wait_group0();  // stores must be done before the CTA retires
     if (p.prof && blockIdx.x == 0 && threadIdx.x == 32 * kFirstEpiWarp) {  // first epilogue warp
       p.prof[8] = prof_ewait; p.prof[9] = clock64() - prof_t0;
     }
@@ -517,19 +530,23 @@ cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CU
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = launch_overlap_enabled() ? 1 : 0;
-  if (p.residual != nullptr)
-    return cudaLaunchKernelEx(&cfg, conv_igemm_kernel<T, BN, true>, tmA, tmA2, tmB, tmB2, tmY, tmR, tmRbox, p);
-  return cudaLaunchKernelEx(&cfg, conv_igemm_kernel<T, BN, false>, tmA, tmA2, tmB, tmB2, tmY, tmR, tmRbox, p);
+  const bool res = p.residual != nullptr, dense = p.tma_store != 0;
+  auto* kernel = res ? (dense ? conv_igemm_kernel<T, BN, true, true> : conv_igemm_kernel<T, BN, true, false>)
+                     : (dense ? conv_igemm_kernel<T, BN, false, true> : conv_igemm_kernel<T, BN, false, false>);
+  return cudaLaunchKernelEx(&cfg, kernel, tmA, tmA2, tmB, tmB2, tmY, tmR, tmRbox, p);
 }
 
 template <typename T, int BN>
 cudaError_t prepare_one() {
   using Cfg = TileCfg<T, BN>;
-  cudaError_t e = cudaFuncSetAttribute(conv_igemm_kernel<T, BN, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(conv_igemm_kernel<T, BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              Cfg::kSmemBytes);
+  auto opt_in = [](const void* kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+  };
+  cudaError_t e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, false, true>));
+  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, true, true>));
+  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, false, false>));
+  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, true, false>));
+  return e;
 }
 
 }  // namespace
