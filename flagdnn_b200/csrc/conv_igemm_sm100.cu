@@ -8,8 +8,7 @@
 //               128 pixels x 128 bytes of activations (padding arrives as the
 //               copy's zero fill) into a ring of shared-memory stages guarded
 //               by full/empty mbarriers;
-//               and one tiled copy of the filter slice (optionally issued by a
-//               second producer warp, FDNN_PRODUCERS=2);
+//               and one tiled copy of the filter slice;
 //   warp 1      MMA issuer: tcgen05.mma from shared-memory descriptors into one
 //               of two fp32 accumulators in tensor memory; tcgen05.commit frees
 //               the stage and, after the last reduction step, publishes the
@@ -48,15 +47,7 @@ constexpr int kRowBytes = 128;      // one swizzled shared-memory row
 #define FDNN_EPI_WARPS 8
 #endif
 constexpr int kEpiWarps = FDNN_EPI_WARPS;  // 8: two per tensor-memory lane quarter (4: one)
-#ifndef FDNN_PRODUCERS
-#define FDNN_PRODUCERS 1
-#endif
-// 2: activation and filter copies come from different warps.  Measured on B200: no faster on any layer
-// shape (a reduction step is bound by shared-memory bandwidth, operand reads of the MMAs plus the copies'
-// fills, not by the issuing thread), so one producer is the default.
-constexpr int kProducers = FDNN_PRODUCERS;
-constexpr int kFilterProducerWarp = 2;  // in the first warp group, beside the producer and the issuer
-// Warp group 0 holds the producer, the issuer (and the optional filter producer); the epilogue warps are
+// Warp group 0 holds the producer and the issuer; the epilogue warps are
 // whole warp groups after it, so that group 0 can hand most of its registers to them: the kernel starts
 // with 168 registers per thread (64 K / 384), group 0 keeps kRegsLean and each epilogue thread gets
 // kRegsEpilogue — the epilogue holds two 32-column accumulator slices, a finished row and, with a
@@ -155,7 +146,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   griddep_launch_dependents();  // all CTAs of this grid are resident: the next launch may queue behind them
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
-      mbar_init(&full_bar[i], kProducers);
+      mbar_init(&full_bar[i], 1);
       mbar_init(&empty_bar[i], 1);
     }
     mbar_init(&tmem_full[0], 1);
@@ -190,17 +181,24 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int k_iters = p.R * p.S * p.c_blocks;
   const int ohw = p.OH * p.OW;
 
-  // One elected thread issues copies; with two producers the activation and the filter copies of a
-  // stage come from different warps and each credits its own bytes to the stage's "full" barrier.
-  auto produce = [&](const bool do_a, const bool do_b, const bool record) {
-    uint32_t it = 0;
+  // How a reduction step's operands are copied.
+  constexpr int kIm2col = 0, kWindows = 1;
+  // The whole warp walks the steps and one elected lane issues (see the issuer): the copy-issuing role is as close to
+  // the critical path of narrow tiles as the MMA-issuing one.
+  auto produce = [&](auto mode_tag, auto prof_tag) {
+    constexpr int kMode = decltype(mode_tag)::value;
+    constexpr bool kProf = decltype(prof_tag)::value;
+    const bool lead = elect_one();
+    uint32_t it = 0, stage = 0, phase = 0;
     bool alive = true;
-    long long prof_wait = 0, prof_issue = 0, prof_t0 = p.prof ? clock64() : 0;
+    long long prof_wait = 0, prof_issue = 0, prof_t0 = kProf ? clock64() : 0;
+    const uint32_t tx = (Cfg::kSplit ? 2u : 1u) *
+                        ((kMode == kWindows ? uint32_t(p.a_tx_bytes) : uint32_t(Cfg::kABytes)) + uint32_t(Cfg::kBBytes));
     for (int tile = blockIdx.x; tile < total_tiles && alive; tile += gridDim.x) {
       const int m_tile = tile / p.n_tiles;
       const int n_tile = tile - m_tile * p.n_tiles;
       int img, w_base, h_base;
-      if (p.lowc) {
+      if constexpr (kMode == kWindows) {
         img = m_tile / p.tiles_per_image;
         const int ti = m_tile - img * p.tiles_per_image;
         w_base = 0;
@@ -214,63 +212,65 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         w_base = ow0 * p.stride_w - p.pad_left;
         h_base = oh0 * p.stride_h - p.pad_top;
       }
-      if constexpr (RES) {
+      if constexpr (RES && DENSE) {
         // the epilogue of this tile will read its 128 x BN residual values a whole main loop from now:
         // ask for them to be brought into L2 so that its loads are short and HBM reads are requested early
-        if (DENSE && do_a && p.residual != nullptr && !p.lowc) tma_prefetch_l2_3d(&tmR, n_tile * BN, m_tile * kBM, 0);
+        if (lead && p.residual != nullptr && !p.lowc) tma_prefetch_l2_3d(&tmR, n_tile * BN, m_tile * kBM, 0);
       }
-      const uint32_t a_tx = (Cfg::kSplit ? 2u : 1u) * (p.lowc ? uint32_t(p.a_tx_bytes) : uint32_t(Cfg::kABytes));
-      const uint32_t b_tx = (Cfg::kSplit ? 2u : 1u) * uint32_t(Cfg::kBBytes);
-      const uint32_t my_tx = (do_a ? a_tx : 0u) + (do_b ? b_tx : 0u);
-      for (int r = 0; r < p.R && alive; ++r) {
-        for (int s = 0; s < p.S && alive; ++s) {
-          const uint16_t off_w = static_cast<uint16_t>(s * p.dil_w);
-          const uint16_t off_h = static_cast<uint16_t>(r * p.dil_h);
-          const int tap = r * p.S + s;
-          for (int cb = 0; cb < p.c_blocks; ++cb, ++it) {
-            const uint32_t stage = it % kStages;
-            const uint32_t phase = (it / kStages) & 1u;
-            const long long pt0 = p.prof ? clock64() : 0;
-            if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, abort_flag, p.status,
-                                   kIncidentProducerWait, p.wait_limit)) {
-              alive = false;
-              break;
-            }
-            const long long pt1 = p.prof ? clock64() : 0;
-            prof_wait += pt1 - pt0;
-            uint8_t* st = stage_base + stage * Cfg::kStageBytes;
-            mbar_arrive_expect_tx(&full_bar[stage], my_tx);
-            const int c0 = cb * Cfg::kKB;
-            if (do_a) {
-              if (p.lowc) {
-                // window copy: (64 elements, all quads of a row, `ohs` rows at the conv stride, image)
-                tma_load_4d(st, &tmA, &full_bar[stage], 0, 0, h_base + r * p.dil_h, img);
-              } else {
-                tma_load_im2col_4d(st, &tmA, &full_bar[stage], c0, w_base, h_base, img, off_w, off_h);
-              }
-              if constexpr (Cfg::kSplit) {
-                tma_load_im2col_4d(st + Cfg::kABytes, &tmA2, &full_bar[stage], c0, w_base, h_base,
-                                   img, off_w, off_h);
-              }
-            }
-            if (do_b) {
-              if constexpr (Cfg::kSplit) {
-                tma_load_3d(st + 2 * Cfg::kABytes, &tmB, &full_bar[stage], c0, tap, n_tile * BN);
-                tma_load_3d(st + 2 * Cfg::kABytes + Cfg::kBBytes, &tmB2, &full_bar[stage], c0, tap,
-                            n_tile * BN);
-              } else {
-                tma_load_3d(st + Cfg::kABytes, &tmB, &full_bar[stage], c0, tap, n_tile * BN);
-              }
-            }
-            if (p.prof) prof_issue += clock64() - pt1;
+      int r = 0, s = 0, cb = 0;
+      for (int kit = 0; kit < k_iters; ++kit, ++it) {
+        long long pt0 = 0, pt1 = 0;
+        if constexpr (kProf) pt0 = clock64();
+        if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, kIncidentProducerWait, p.wait_limit)) {
+          alive = false;
+          break;
+        }
+        if constexpr (kProf) {
+          pt1 = clock64();
+          prof_wait += pt1 - pt0;
+        }
+        if (lead) {
+          uint8_t* st = stage_base + stage * Cfg::kStageBytes;
+          uint64_t* bar = &full_bar[stage];
+          mbar_arrive_expect_tx(bar, tx);
+          const int c0 = cb * Cfg::kKB;
+          if constexpr (kMode == kWindows) {
+            // window copy: (64 elements, all quads of a row, `ohs` rows at the conv stride, image)
+            tma_load_4d(st, &tmA, bar, 0, 0, h_base + r * p.dil_h, img);
+          } else {
+            const uint16_t off_w = static_cast<uint16_t>(s * p.dil_w), off_h = static_cast<uint16_t>(r * p.dil_h);
+            tma_load_im2col_4d(st, &tmA, bar, c0, w_base, h_base, img, off_w, off_h);
+            if constexpr (Cfg::kSplit)
+              tma_load_im2col_4d(st + Cfg::kABytes, &tmA2, bar, c0, w_base, h_base, img, off_w, off_h);
+          }
+          if constexpr (Cfg::kSplit) {
+            tma_load_3d(st + 2 * Cfg::kABytes, &tmB, bar, c0, r * p.S + s, n_tile * BN);
+            tma_load_3d(st + 2 * Cfg::kABytes + Cfg::kBBytes, &tmB2, bar, c0, r * p.S + s, n_tile * BN);
+          } else {
+            tma_load_3d(st + Cfg::kABytes, &tmB, bar, c0, r * p.S + s, n_tile * BN);
+          }
+        }
+        __syncwarp();
+        if constexpr (kProf) prof_issue += clock64() - pt1;
+        if (++stage == uint32_t(kStages)) {
+          stage = 0;
+          phase ^= 1u;
+        }
+        if (++cb == p.c_blocks) {
+          cb = 0;
+          if (++s == p.S) {
+            s = 0;
+            ++r;
           }
         }
       }
     }
-    if (record && p.prof && blockIdx.x == 0) {
-      p.prof[0] = prof_wait; p.prof[1] = prof_issue; p.prof[2] = clock64() - prof_t0; p.prof[3] = it;
+    if constexpr (kProf) {
+      if (lead && blockIdx.x == 0) {
+        p.prof[0] = prof_wait; p.prof[1] = prof_issue; p.prof[2] = clock64() - prof_t0; p.prof[3] = it;
+      }
     }
-    if (!alive || *abort_flag) {
+    if (lead && (!alive || *abort_flag)) {
       // Teardown after an incident: let the copies already issued land before
       // the CTA gives its shared memory back.
       const uint32_t first = it > uint32_t(kStages) ? it - kStages : 0u;
@@ -280,6 +280,11 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                           kIncidentDrainWait, kWaitLimitCycles / 16);
       }
     }
+    __syncwarp();
+  };
+  auto produce_any = [&](auto mode_tag) {
+    if (p.prof == nullptr) produce(mode_tag, std::false_type{});
+    else produce(mode_tag, std::true_type{});
   };
 
   if (warp < kFirstEpiWarp) {
@@ -288,80 +293,90 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #endif
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0 && !p.skip_copies) produce(true, kProducers == 1, true);
-  } else if (kProducers == 2 && warp == kFilterProducerWarp) {
-    // ---------------------------------------------- producer of the filter copies
-    if (lane == 0 && !p.skip_copies) produce(false, true, false);
+    if (!p.skip_copies) {
+      if (p.lowc) produce_any(std::integral_constant<int, kWindows>{});
+      else produce_any(std::integral_constant<int, kIm2col>{});
+    }
   } else if (warp == 1) {
     // -------------------------------------------------------------- issuer
-    if (lane == 0) {
-      uint32_t it = 0;
-      uint32_t tcount = 0;
-      bool alive = true;
-      long long prof_wfull = 0, prof_wtmem = 0, prof_t0 = p.prof ? clock64() : 0;
-      for (int tile = blockIdx.x; tile < total_tiles && alive; tile += gridDim.x, ++tcount) {
-        const uint32_t buf = tcount & 1u;
-        const uint32_t bphase = (tcount >> 1) & 1u;
-        const long long mt0 = p.prof ? clock64() : 0;
-        if (!mbar_wait_bounded(&tmem_empty[buf], bphase ^ 1u, abort_flag, p.status,
-                               kIncidentMmaWaitTmem, p.wait_limit)) {
-          alive = false;
-          break;
-        }
-        if (p.prof) prof_wtmem += clock64() - mt0;
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * BN;
-        // the reduction loop holds the wait, the MMAs and the commit and nothing else: the issuing thread is on
-        // the critical path of every step (cycle counters are compiled into a second copy of the loop)
-        auto reduce = [&](auto prof_tag) {
-          constexpr bool kProf = decltype(prof_tag)::value;
-          for (int kit = 0; kit < k_iters; ++kit, ++it) {
-            const uint32_t stage = it % kStages;
-            const uint32_t phase = (it / kStages) & 1u;
-            long long mt1 = 0;
-            if constexpr (kProf) mt1 = clock64();
-            if (!mbar_wait_bounded(&full_bar[stage], phase, abort_flag, p.status,
-                                   kIncidentMmaWaitFull, p.wait_limit)) {
-              alive = false;
-              break;
-            }
-            if constexpr (kProf) prof_wfull += clock64() - mt1;
-            tc_fence_after();
-            const uint32_t st = smem_u32(stage_base + stage * Cfg::kStageBytes);
+    // The whole warp walks the loop and one elected lane issues, so that descriptors and addresses are uniform values:
+    // what the issuing thread does between two MMAs bounds the reduction step of tiles up to 128 columns.  A lane that
+    // walks alone, building each descriptor anew and waiting with the suspend-time hint, needs 433 clocks per step of
+    // four MMAs (64 clocks of issue each, 45 for the commit, 135 for the wait); this loop needs 254 (64 columns), 268
+    // (128) and 513 (256, where the MMAs themselves are the limit).
+    const bool lead = elect_one();
+    uint32_t stage = 0, phase = 0;
+    uint32_t tcount = 0;
+    bool alive = true;
+    long long prof_wfull = 0, prof_wtmem = 0, prof_t0 = p.prof ? clock64() : 0;
+    const uint32_t ring = smem_u32(stage_base);
+    for (int tile = blockIdx.x; tile < total_tiles && alive; tile += gridDim.x, ++tcount) {
+      const uint32_t buf = tcount & 1u;
+      const uint32_t bphase = (tcount >> 1) & 1u;
+      const long long mt0 = p.prof ? clock64() : 0;
+      if (!mbar_wait_warp(&tmem_empty[buf], bphase ^ 1u, abort_flag, p.status, kIncidentMmaWaitTmem, p.wait_limit)) {
+        alive = false;
+        break;
+      }
+      if (p.prof) prof_wtmem += clock64() - mt0;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + buf * BN;
+      // the reduction loop holds the wait, the MMAs and the commit and nothing else (cycle counters are compiled into a
+      // second copy of the loop)
+      auto reduce = [&](auto prof_tag) {
+        constexpr bool kProf = decltype(prof_tag)::value;
+        for (int kit = 0; kit < k_iters; ++kit) {
+          long long mt1 = 0;
+          if constexpr (kProf) mt1 = clock64();
+          if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, kIncidentMmaWaitFull, p.wait_limit)) {
+            alive = false;
+            break;
+          }
+          if constexpr (kProf) prof_wfull += clock64() - mt1;
+          tc_fence_after();
+          if (lead) {
+            const uint32_t st = ring + stage * Cfg::kStageBytes;
+            const uint64_t a0 = make_sw128_kmajor_desc(st);
+            const uint64_t b0 = make_sw128_kmajor_desc(st + (Cfg::kSplit ? 2 : 1) * Cfg::kABytes);
 #pragma unroll
             for (int k = 0; k < Cfg::kKB / Cfg::kUK; ++k) {
+              // 32 bytes of reduction elements further (the address field counts 16-byte units)
+              const uint64_t a = a0 + uint64_t(k * 2);
+              const uint64_t b = b0 + uint64_t(k * 2);
               const uint32_t acc = (kit > 0 || k > 0) ? 1u : 0u;
               if constexpr (Cfg::kSplit) {
-                const uint64_t a_hi = make_sw128_kmajor_desc(st + k * 32);
-                const uint64_t a_lo = make_sw128_kmajor_desc(st + Cfg::kABytes + k * 32);
-                const uint64_t b_hi = make_sw128_kmajor_desc(st + 2 * Cfg::kABytes + k * 32);
-                const uint64_t b_lo =
-                    make_sw128_kmajor_desc(st + 2 * Cfg::kABytes + Cfg::kBBytes + k * 32);
-                mma_tf32(d_tmem, a_lo, b_hi, kIdesc, acc);
-                mma_tf32(d_tmem, a_hi, b_lo, kIdesc, 1u);
-                mma_tf32(d_tmem, a_hi, b_hi, kIdesc, 1u);
+                const uint64_t a_lo = a + uint64_t(Cfg::kABytes / 16), b_lo = b + uint64_t(Cfg::kBBytes / 16);
+                mma_tf32(d_tmem, a_lo, b, kIdesc, acc);
+                mma_tf32(d_tmem, a, b_lo, kIdesc, 1u);
+                mma_tf32(d_tmem, a, b, kIdesc, 1u);
               } else {
-                const uint64_t a = make_sw128_kmajor_desc(st + k * 32);
-                const uint64_t b = make_sw128_kmajor_desc(st + Cfg::kABytes + k * 32);
                 mma_f16(d_tmem, a, b, kIdesc, acc);
               }
             }
             tc_commit(&empty_bar[stage]);
           }
-        };
-        if (p.prof == nullptr) reduce(std::false_type{}); else reduce(std::true_type{});
-        if (alive) tc_commit(&tmem_full[buf]);
-      }
-      if (p.prof && blockIdx.x == 0) {
-        p.prof[4] = prof_wfull; p.prof[5] = prof_wtmem; p.prof[6] = clock64() - prof_t0; p.prof[7] = tcount;
-      }
-      if (!alive || *abort_flag) {
-        // Make sure no MMA is still writing tensor memory before it is freed.
-        volatile uint32_t never = 0;
-        tc_commit(drain_bar);
-        mbar_wait_bounded(drain_bar, 0u, &never, p.status, kIncidentDrainWait, kWaitLimitCycles / 16);
-      }
+          __syncwarp();
+          if (++stage == uint32_t(kStages)) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      };
+      if (p.prof == nullptr) reduce(std::false_type{});
+      else reduce(std::true_type{});
+      if (alive && lead) tc_commit(&tmem_full[buf]);
+      __syncwarp();
     }
+    if (p.prof && blockIdx.x == 0 && lead) {
+      p.prof[4] = prof_wfull; p.prof[5] = prof_wtmem; p.prof[6] = clock64() - prof_t0; p.prof[7] = tcount;
+    }
+    if (lead && (!alive || *abort_flag)) {
+      // Make sure no MMA is still writing tensor memory before it is freed.
+      volatile uint32_t never = 0;
+      tc_commit(drain_bar);
+      mbar_wait_bounded(drain_bar, 0u, &never, p.status, kIncidentDrainWait, kWaitLimitCycles / 16);
+    }
+    __syncwarp();
   }
   } else {
 #ifndef FDNN_NO_REG_REALLOC

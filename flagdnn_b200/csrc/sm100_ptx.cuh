@@ -119,6 +119,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The same without the suspend-time hint: for a role on the critical path that expects the phase to be complete (the
+// hint costs some 30 clocks even then).
+__device__ __forceinline__ bool mbar_try_wait_now(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t"
+      "}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait.  Gives up after `limit_cycles` SM clocks (about 2 s by
 // default) or as soon as another role raised `*abort_flag`; on giving up it
 // records `incident` in the device status word and raises the flag itself, so
@@ -144,6 +160,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
       }
     }
   }
+}
+
+// The wait of a whole warp: every lane gets the same answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
+                                               uint32_t* status_word, uint32_t incident, long long limit_cycles) {
+  if (__all_sync(0xffffffffu, mbar_try_wait_now(bar, parity))) return true;
+  const bool ok = mbar_wait_bounded(bar, parity, abort_flag, status_word, incident, limit_cycles);
+  return __all_sync(0xffffffffu, ok);
 }
 
 // ------------------------------------------- programmatic dependent launch
