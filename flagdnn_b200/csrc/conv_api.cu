@@ -305,6 +305,19 @@ fdnn_conv_desc grouped_desc(const fdnn_conv_desc* d, int q, int oh, int ow) {
   return v;
 }
 
+// A one-tap filter whose K dimension is contiguous (mm's second operand, [C][K] row-major with rows of 16-byte
+// multiples) can be read in place, since the tensor core takes an MN-major operand as well.  It saves the transposing
+// copy of every call (2 us and the filter moved twice) but the product itself runs some 20 % slower (8192 rows x 4096 x
+// 4096 bf16: 210 us against 184 us after a 13.5 us copy), so that it pays up to a few thousand rows
+// (654 x 208 @ 208 x 112: 7.5 -> 5.3 us).
+bool filter_mn_major(const fdnn_conv_desc* d, const void* w) {
+  if (elem_size(d->dtype) != 2 || d->r * d->s != 1 || d->k <= 1 || d->c <= 1 || d->w_strides[0] != 1 ||
+      d->w_strides[1] % 8 != 0 || d->w_strides[1] < d->k || !aligned16(w))
+    return false;
+  const double filter = double(d->c) * d->k, products = filter * d->n * d->h * d->w;
+  return 2.9e-10 * products < 2.0 + 0.8e-6 * filter;   // both sides in microseconds
+}
+
 // Reduction splitting on CTA pairs: T tiles of K reduction steps on P pairs.  Whole tiles cost
 // ceil(T / P) * K steps on the busiest pair, an even split ceil(T * K / P) plus the exchange of one partial
 // tile (about three steps' worth of time).  Ranges shorter than 12 steps are not split (boundaries snap to
@@ -531,10 +544,11 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
   const int c_pad = padded_channels(d->dtype, d->c);
   plan->c_padded = c_pad;
   plan->x_repacked = x_inplace ? 0 : 1;
-  plan->w_packed = w_inplace ? 0 : 1;
+  const bool w_direct = w_inplace || filter_mn_major(d, w);
+  plan->w_packed = w_direct ? 0 : 1;
   const int planes = (d->dtype == FDNN_F32) ? 2 : 1;
   if (!x_inplace) plan->workspace_bytes = (long long)planes * d->n * d->h * d->w * padded_x_channels(d) * es;
-  if (!w_inplace) plan->packed_weight_bytes = (long long)planes * d->k * d->r * d->s * c_pad * es;
+  if (!w_direct) plan->packed_weight_bytes = (long long)planes * d->k * d->r * d->s * c_pad * es;
   plan->tile_m = 128;
   plan->tile_k = 128 / es;
   const int m_tiles = int(((long long)m + 127) / 128);
@@ -1345,6 +1359,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     a_sn = (long long)d.h * d.w * x_pad;
     a_c = x_pad;
   }
+  const bool b_mn = !plan.w_packed && filter_mn_major(&d, w);
   const void* b_base = w;
   long long b_stap = d.s > 1 ? d.w_strides[3] : (d.r > 1 ? d.w_strides[2] : any_stride);
   long long b_sk = d.k > 1 ? d.w_strides[0] : any_stride;
@@ -1362,7 +1377,15 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   st = encode_activation_map(&tmA, d.dtype, a_base, a_c, d.w, d.h, d.n, a_sw, a_sh, a_sn, &d);
   if (st != FDNN_OK) return st;
   const int b_box_rows = plan.algo == FDNN_ALGO_IGEMM_PAIR ? 128 : plan.tile_n;  // each CTA of a pair stages half
-  st = encode_filter_map(&tmB, d.dtype, b_base, b_c, d.r * d.s, d.k, b_stap, b_sk, b_box_rows);
+  if (b_mn) {
+    cuuint64_t dims[3] = {cuuint64_t(d.k), cuuint64_t(d.c), 1};
+    cuuint64_t strides[2] = {cuuint64_t(d.w_strides[1]) * es, cuuint64_t(d.w_strides[1]) * es * cuuint64_t(d.c)};
+    cuuint32_t box[3] = {64, 64, 1};   // kMnBoxElems filters x one reduction step
+    cuuint32_t estr[3] = {1, 1, 1};
+    st = encode_tiled(&tmB, d.dtype, b_base, 3, dims, strides, box, estr, "filter, K contiguous");
+  } else {
+    st = encode_filter_map(&tmB, d.dtype, b_base, b_c, d.r * d.s, d.k, b_stap, b_sk, b_box_rows);
+  }
   if (st != FDNN_OK) return st;
   if (d.dtype == FDNN_F32) {
     st = encode_activation_map(&tmA2, d.dtype, static_cast<const char*>(a_base) + a_plane * es, a_c, d.w,
@@ -1394,6 +1417,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   p.bias = bias; p.scale = scale; p.y = y;
   p.residual = residual;
   p.act = activation;
+  p.b_mn = b_mn ? 1 : 0;
   const bool out_f32 = (d.algo & FDNN_ALGO_FLAG_OUT_F32) != 0;
   if (out_f32 && residual != nullptr) return fail(FDNN_NOT_SUPPORTED, "no residual with a float32 output from 16-bit operands");
   p.out_f32 = out_f32 ? 1 : 0;
@@ -1433,7 +1457,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   if (p.status == nullptr) return fail(FDNN_CUDA_ERROR, "status word address unavailable");
   if (plan.algo == FDNN_ALGO_IGEMM_PAIR) {
     if (!p.tma_store) return fail(FDNN_NOT_SUPPORTED, "the CTA-pair kernel needs a dense channels-last output");
-    p.b_resident = (d.k <= 256 && d.r * d.s * p.c_blocks <= igemm_pair_max_resident_steps()) ? 1 : 0;
+    p.b_resident = (!b_mn && d.k <= 256 && d.r * d.s * p.c_blocks <= igemm_pair_max_resident_steps()) ? 1 : 0;
     // reduction splitting when the caller brought the scratch for it
     if (plan.stream_k && !p.b_resident && sk_scratch != nullptr && sk_bytes >= plan.streamk_bytes &&
         (reinterpret_cast<uintptr_t>(sk_scratch) & 255u) == 0) {

@@ -267,7 +267,12 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
               tma_load_im2col_4d_pair(st, &tmA, bar, c0, w_base, h_base, img, static_cast<uint16_t>(s_ * p.dil_w),
                                       static_cast<uint16_t>(r * p.dil_h));
             }
-            if (!b_resident) tma_load_3d_pair(st + kABytes, &tmB, bar, c0, r * p.S + s_, b_row0);
+            if (p.b_mn) {   // filter with K contiguous: two boxes of 64 filters x 64 channels
+              tma_load_3d_pair(st + kABytes, &tmB, bar, b_row0, c0, 0);
+              tma_load_3d_pair(st + kABytes + kMnBoxBytes, &tmB, bar, b_row0 + int(kMnBoxElems), c0, 0);
+            } else if (!b_resident) {
+              tma_load_3d_pair(st + kABytes, &tmB, bar, c0, r * p.S + s_, b_row0);
+            }
             if constexpr (kProf) prof_issue += clock64() - pt1;
             if (++stage == uint32_t(n_stages)) {
               stage = 0;
@@ -309,6 +314,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       const uint32_t tfull_own = smem_u32(&tmem_full[0]);
       const uint32_t tfull_peer = map_to_cta(tfull_own, 1);
       const uint32_t raw_empty_peer = map_to_cta(smem_u32(&raw_empty[0]), 1);
+      const bool mn = p.b_mn != 0;     // the filter lies MN-major in its stages
       const int k16 = p.k16_per_step;  // 16-element reduction slices per step that hold data (4, or 3)
       TileWalk walk;
       walk_init(walk, split, pair_id, num_pairs, total_tiles, k_iters, p.sk_min_frag);
@@ -326,7 +332,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         const uint32_t d_tmem = tmem_base + buf * kPairN;
         // The reduction loop is the hot path of every layer and is sensitive to anything beside the wait, the
         // MMAs and the commits (a conditional barrier arrive in it cost 17 % on the 3x3 256-channel layer):
-        // it exists once with four MMAs per step and once with a runtime count for the 3-channel mode.
+        // it exists once with four MMAs per step and once with a runtime count and filter layout (the 3-channel
+        // mode, filters read MN-major).
         auto reduce = [&](auto four_tag, auto prof_tag) {
           constexpr bool kFour = decltype(four_tag)::value;
           constexpr bool kProf = decltype(prof_tag)::value;
@@ -351,8 +358,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             } else {
               for (int k = 0; k < k16; ++k) {
                 const uint64_t a = make_sw128_kmajor_desc(st + k * 32);
-                const uint64_t b = make_sw128_kmajor_desc(bt + k * 32);
-                mma_f16_pair(d_tmem, a, b, kIdesc, (kit > walk.kb || k > 0) ? 1u : 0u);
+                const uint64_t b = mn ? make_sw128_mnmajor_desc(bt + k * kMnStepBytes) : make_sw128_kmajor_desc(bt + k * 32);
+                mma_f16_pair(d_tmem, a, b, mn ? (kIdesc | kIdescBMnMajor) : kIdesc, (kit > walk.kb || k > 0) ? 1u : 0u);
               }
             }
             tc_commit_pair(empty_own + stage * 8);
@@ -363,7 +370,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             }
           }
         };
-        if (k16 != kKB / 16) {
+        if (k16 != kKB / 16 || mn) {
           reduce(std::false_type{}, std::false_type{});
         } else if (p.prof == nullptr) {
           reduce(std::true_type{}, std::false_type{});

@@ -182,7 +182,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int ohw = p.OH * p.OW;
 
   // How a reduction step's operands are copied.
-  constexpr int kIm2col = 0, kWindows = 1;
+  constexpr int kIm2col = 0, kWindows = 1, kFilterMn = 2;
   // The whole warp walks the steps and one elected lane issues (see the issuer): the copy-issuing role is as close to
   // the critical path of narrow tiles as the MMA-issuing one.
   auto produce = [&](auto mode_tag, auto prof_tag) {
@@ -246,6 +246,10 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           if constexpr (Cfg::kSplit) {
             tma_load_3d(st + 2 * Cfg::kABytes, &tmB, bar, c0, r * p.S + s, n_tile * BN);
             tma_load_3d(st + 2 * Cfg::kABytes + Cfg::kBBytes, &tmB2, bar, c0, r * p.S + s, n_tile * BN);
+          } else if constexpr (kMode == kFilterMn) {   // filter with K contiguous: boxes of 64 filters x 64 channels
+#pragma unroll
+            for (int j = 0; j < BN / int(kMnBoxElems); ++j)
+              tma_load_3d(st + Cfg::kABytes + j * kMnBoxBytes, &tmB, bar, n_tile * BN + j * int(kMnBoxElems), c0, 0);
           } else {
             tma_load_3d(st + Cfg::kABytes, &tmB, bar, c0, r * p.S + s, n_tile * BN);
           }
@@ -295,6 +299,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // ------------------------------------------------------------ producer
     if (!p.skip_copies) {
       if (p.lowc) produce_any(std::integral_constant<int, kWindows>{});
+      else if (p.b_mn) produce_any(std::integral_constant<int, kFilterMn>{});
       else produce_any(std::integral_constant<int, kIm2col>{});
     }
   } else if (warp == 1) {
@@ -323,8 +328,9 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const uint32_t d_tmem = tmem_base + buf * BN;
       // the reduction loop holds the wait, the MMAs and the commit and nothing else (cycle counters are compiled into a
       // second copy of the loop)
-      auto reduce = [&](auto prof_tag) {
+      auto reduce = [&](auto prof_tag, auto mn_tag) {
         constexpr bool kProf = decltype(prof_tag)::value;
+        constexpr bool kMn = decltype(mn_tag)::value;   // the filter lies MN-major in its stages (16-bit types)
         for (int kit = 0; kit < k_iters; ++kit) {
           long long mt1 = 0;
           if constexpr (kProf) mt1 = clock64();
@@ -337,12 +343,13 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           if (lead) {
             const uint32_t st = ring + stage * Cfg::kStageBytes;
             const uint64_t a0 = make_sw128_kmajor_desc(st);
-            const uint64_t b0 = make_sw128_kmajor_desc(st + (Cfg::kSplit ? 2 : 1) * Cfg::kABytes);
+            const uint64_t b0 = kMn ? make_sw128_mnmajor_desc(st + Cfg::kABytes)
+                                    : make_sw128_kmajor_desc(st + (Cfg::kSplit ? 2 : 1) * Cfg::kABytes);
 #pragma unroll
             for (int k = 0; k < Cfg::kKB / Cfg::kUK; ++k) {
               // 32 bytes of reduction elements further (the address field counts 16-byte units)
               const uint64_t a = a0 + uint64_t(k * 2);
-              const uint64_t b = b0 + uint64_t(k * 2);
+              const uint64_t b = b0 + uint64_t(k * (kMn ? int(kMnStepBytes / 16) : 2));
               const uint32_t acc = (kit > 0 || k > 0) ? 1u : 0u;
               if constexpr (Cfg::kSplit) {
                 const uint64_t a_lo = a + uint64_t(Cfg::kABytes / 16), b_lo = b + uint64_t(Cfg::kBBytes / 16);
@@ -350,7 +357,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 mma_tf32(d_tmem, a, b_lo, kIdesc, 1u);
                 mma_tf32(d_tmem, a, b, kIdesc, 1u);
               } else {
-                mma_f16(d_tmem, a, b, kIdesc, acc);
+                mma_f16(d_tmem, a, b, kMn ? (kIdesc | kIdescBMnMajor) : kIdesc, acc);
               }
             }
             tc_commit(&empty_bar[stage]);
@@ -362,8 +369,9 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           }
         }
       };
-      if (p.prof == nullptr) reduce(std::false_type{});
-      else reduce(std::true_type{});
+      if (p.b_mn) reduce(std::false_type{}, std::true_type{});
+      else if (p.prof == nullptr) reduce(std::false_type{}, std::false_type{});
+      else reduce(std::true_type{}, std::false_type{});
       if (alive && lead) tc_commit(&tmem_full[buf]);
       __syncwarp();
     }

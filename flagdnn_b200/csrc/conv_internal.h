@@ -42,6 +42,7 @@ struct IgemmParams {
   int tiles_per_image;   // low-channel mode: ceil(OH / ohs)
   int ohs;               // low-channel mode: output rows per tile
   int a_tx_bytes;        // bytes one activation copy delivers (rows_per_tile * 128 in low-channel mode)
+  int b_mn;              // 1: one tap, filter with K contiguous ([C][K]): read in place as an MN-major operand
   int b_resident;        // pair kernel: the filter half stays in shared memory for the whole launch
   // Low-channel mode on a dense 3-channel NHWC input (the stem), pair kernel only: no relayout pass.  Two warps
   // of each CTA copy the tile's input rows, shifted to a 16-byte boundary and zero-padded left and right,

@@ -487,6 +487,22 @@ __device__ __forceinline__ uint64_t make_sw128_kmajor_desc(uint32_t smem_addr) {
   return d;
 }
 
+// The same for an operand stored MN-major (its rows run along M or N, one reduction element each): boxes of 64 M/N
+// elements (128 bytes) x 64 reduction rows, 128-byte swizzle, one after another.  Eight reduction rows take 1024 bytes
+// (stride byte offset), the next 64 M/N elements are one 8192-byte box further (leading byte offset); an MMA's 16
+// reduction elements take 2048 bytes.  The instruction descriptor says so with kIdescBMnMajor.
+constexpr uint32_t kMnBoxElems = 64, kMnBoxBytes = 8192, kMnStepBytes = 2048;
+__device__ __forceinline__ uint64_t make_sw128_mnmajor_desc(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((smem_addr & 0x3ffff) >> 4);
+  d |= static_cast<uint64_t>(kMnBoxBytes >> 4) << 16;
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;
+  d |= static_cast<uint64_t>(1) << 46;
+  d |= static_cast<uint64_t>(2) << 61;
+  return d;
+}
+constexpr uint32_t kIdescBMnMajor = 1u << 16;
+
 // Instruction descriptor: fp32 accumulate, both operands K-major, dense.
 //   bits [4,6) D format (1 = f32); [7,10) A format; [10,13) B format
 //   (0 = f16, 1 = bf16, 2 = tf32); bit 15/16 A/B major (0 = K);
