@@ -848,6 +848,24 @@ uint32_t* g_status_ptr[64];  // device address of g_status_word, looked up once 
 
 }  // namespace
 
+int current_sm_count() { return sm_count(); }
+
+// x of a depthwise layer as (channel, column, row, image), boxes of `chunk` channels x `span` pixels x `rows` rows; what lies outside
+// arrives as zeros, which is the padding.
+bool encode_depthwise_map(CUtensorMap* tm, int dtype, const DirectParams& p, int chunk, int span, int rows) {
+  const int es = elem_size(dtype);
+  // a stride over an extent of one says nothing: any multiple of 16 bytes will do
+  const long long any = (long long)(p.C * es + 15) / 16 * 16;
+  const long long sw = p.W > 1 ? p.x_s[3] * es : any, sh = p.H > 1 ? p.x_s[2] * es : any, sn = p.N > 1 ? p.x_s[0] * es : any;
+  cuuint64_t dims[4] = {cuuint64_t(p.C), cuuint64_t(p.W), cuuint64_t(p.H), cuuint64_t(p.N)};
+  cuuint64_t strides[3] = {cuuint64_t(sw), cuuint64_t(sh), cuuint64_t(sn)};
+  cuuint32_t box[4] = {cuuint32_t(chunk), cuuint32_t(span), cuuint32_t(rows), 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return memo_encode_tiled(tm, tm_dtype(dtype), 4, const_cast<void*>(p.x), dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 uint32_t* device_status_word() {
   void* p = nullptr;
   if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) {
@@ -1209,6 +1227,28 @@ int fdnn_conv2d_fwd_ex(const fdnn_conv_desc* desc, const void* x, const void* w,
                   true, desc->k, streamk_scratch, streamk_bytes);
 }
 
+// One-time set-up of the current device for kernels that use tensor maps and bounded waits.
+static int prepare_device(int* device) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return fail_cuda("cudaGetDevice", e);
+  if (dev < 0 || dev >= 64) return fail(FDNN_BAD_PARAM, "device ordinal out of range");
+  std::call_once(g_prepare_once[dev], [dev]() {
+    int major = 0;
+    cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
+    g_prepare_result[dev] = (major == 10) ? igemm_prepare_device() : cudaErrorNoKernelImageForDevice;
+    if (g_prepare_result[dev] == cudaSuccess) g_prepare_result[dev] = igemm_pair_prepare_device();
+    g_status_ptr[dev] = device_status_word();
+  });
+  if (g_prepare_result[dev] == cudaErrorNoKernelImageForDevice)
+    return fail(FDNN_ARCH_MISMATCH, "the implicit-GEMM kernels are built for sm_100a only");
+  if (g_prepare_result[dev] != cudaSuccess) return fail_cuda("kernel attribute setup", g_prepare_result[dev]);
+  std::call_once(g_driver_once, load_driver_entry_points);
+  if (!g_driver_ok) return fail(FDNN_CUDA_ERROR, "driver entry points for tensor maps not found");
+  *device = dev;
+  return FDNN_OK;
+}
+
 // k_real: length of bias / scale (differs from desc->k only for the equivalent convolution of a
 // pixel-grouped layer, whose GEMM column j uses entry j % k_real).
 static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, const void* w_packed,
@@ -1276,7 +1316,18 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     }
     p.x = x; p.w = w; p.bias = bias; p.scale = scale; p.residual = residual; p.y = y;
     p.act = activation;
-    const int dw = (d.algo & 0xff) == FDNN_ALGO_AUTO ? depthwise_kind(d.dtype, p) : 0;  // a forced "direct" stays direct
+    int dw = (d.algo & 0xff) == FDNN_ALGO_AUTO ? depthwise_kind(d.dtype, p) : 0;  // a forced "direct" stays direct
+    if (dw == 6) {
+      int dev = 0;
+      if (prepare_device(&dev) == FDNN_OK && g_status_ptr[dev] != nullptr) {
+        const long long limit = g_wait_limit.load(std::memory_order_relaxed);
+        cudaError_t e = launch_depthwise_tma(d.dtype, p, g_status_ptr[dev], limit > 0 ? limit : default_wait_limit_cycles(), stream);
+        if (e == cudaSuccess) return FDNN_OK;
+        if (e != cudaErrorInvalidValue) return fail_cuda("depthwise launch", e);
+        cudaGetLastError();
+      }
+      dw = 1;   // no tensor map over this x: the kernel that reads it with plain loads
+    }
     cudaError_t e = dw != 0 ? launch_depthwise(d.dtype, p, dw, stream) : launch_direct(d.dtype, p, stream);
     if (e != cudaSuccess) return fail_cuda("direct conv launch", e);
     return FDNN_OK;
@@ -1284,21 +1335,9 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
 
   // ---- tensor-core path
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return fail_cuda("cudaGetDevice", e);
-  if (dev < 0 || dev >= 64) return fail(FDNN_BAD_PARAM, "device ordinal out of range");
-  std::call_once(g_prepare_once[dev], [dev]() {
-    int major = 0;
-    cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
-    g_prepare_result[dev] = (major == 10) ? igemm_prepare_device() : cudaErrorNoKernelImageForDevice;
-    if (g_prepare_result[dev] == cudaSuccess) g_prepare_result[dev] = igemm_pair_prepare_device();
-    g_status_ptr[dev] = device_status_word();
-  });
-  if (g_prepare_result[dev] == cudaErrorNoKernelImageForDevice)
-    return fail(FDNN_ARCH_MISMATCH, "the implicit-GEMM kernels are built for sm_100a only");
-  if (g_prepare_result[dev] != cudaSuccess) return fail_cuda("kernel attribute setup", g_prepare_result[dev]);
-  std::call_once(g_driver_once, load_driver_entry_points);
-  if (!g_driver_ok) return fail(FDNN_CUDA_ERROR, "driver entry points for tensor maps not found");
+  st = prepare_device(&dev);
+  if (st != FDNN_OK) return st;
+  cudaError_t e = cudaSuccess;
 
   if (plan.w_packed && w_packed == nullptr)
     return fail(FDNN_BAD_PARAM, "this problem needs a packed filter (fdnn_conv2d_pack_weight); w_packed is NULL");

@@ -26,6 +26,7 @@
 #include "conv_convert.cuh"
 #include "conv_epilogue.cuh"
 #include "conv_internal.h"
+#include "f32x2.cuh"
 
 namespace fdnn {
 namespace {
@@ -33,18 +34,6 @@ namespace {
 constexpr int kDwThreads = 256;
 constexpr int kDwMaxSmemFloats = 12288;  // 48 KB of taps at most
 constexpr int kDwRounds = 6;              // units a resident thread group should get at least (load balance)
-
-// SM count of the current device, looked up once per device ordinal.
-inline int sm_count_dw() {
-  static std::atomic<int> cached[64];
-  int dev = 0, v = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  v = cached[dev].load(std::memory_order_relaxed);
-  if (v > 0) return v;
-  if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) return 148;
-  cached[dev].store(v, std::memory_order_relaxed);
-  return v;
-}
 
 template <typename T>
 __device__ __forceinline__ void unpack_vec(const uint4& q, float (&v)[16 / sizeof(T)]) {
@@ -112,23 +101,6 @@ __device__ __forceinline__ void store_words_streaming(void* ptr, const Words<VB>
   } else {
     __stcs(static_cast<uint32_t*>(ptr), r.w[0]);
   }
-}
-// Two fp32 values of neighbouring channels in one 64-bit register, the operand form of fma.rn.f32x2 (two
-// independent, correctly rounded fp32 FMAs per instruction).  They are kept as 64-bit integers so that the
-// compiler carries each pair through branches and loops as one value instead of splitting and re-joining it.
-using F2 = unsigned long long;
-__device__ __forceinline__ F2 f2_make(uint32_t lo_bits, uint32_t hi_bits) {
-  F2 d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo_bits), "r"(hi_bits));
-  return d;
-}
-__device__ __forceinline__ void f2_split(F2 v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
 }
 // The words as fp32 pairs of neighbouring channels (one pair per word for 16-bit types, per two words for fp32).
 template <typename T, int VB>
@@ -430,6 +402,114 @@ depthwise_plane_kernel(const DirectParams p) {
   }
 }
 
+// ------------------------------------------------- NCHW, several small planes per block
+// Dense planes of any size (rows that start on no vector boundary: 7 x 7, 13 x 13, 33 x 33 ...).  A block copies
+// `group` whole planes, which lie one after another in memory, to shared memory in 16-byte pieces (the copy keeps the
+// address modulo 16, so that both sides are aligned; the ends go element by element), computes from there, stages its
+// outputs beside them and writes those back the same way.  A work item is four neighbouring outputs of a row.
+// What bounds it: one block per plane (depthwise_plane_kernel) leaves most of a block idle on small planes and loads and
+// stores single elements; 128 x 1024 planes of 7 x 7 took 269 us, 95 GB/s.
+template <typename T>
+__device__ __forceinline__ void copy_elements(T* dst, const T* src, int count) {   // equal addresses modulo 16
+  const int head = min(count, int((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / int(sizeof(T)));
+  const int vecs = (count - head) / (16 / int(sizeof(T)));
+  const int tail0 = head + vecs * (16 / int(sizeof(T)));
+  for (int i = threadIdx.x; i < vecs; i += blockDim.x)
+    reinterpret_cast<uint4*>(dst + head)[i] = reinterpret_cast<const uint4*>(src + head)[i];
+  for (int i = threadIdx.x; i < head; i += blockDim.x) dst[i] = src[i];
+  for (int i = tail0 + threadIdx.x; i < count; i += blockDim.x) dst[i] = src[i];
+}
+
+template <typename T, int KR, int KS, int KSTRIDE>
+__global__ void __launch_bounds__(kDwThreads)
+depthwise_planes_kernel(const DirectParams p, int group) {
+  constexpr int PW = 4;
+  constexpr int kSpan = (PW - 1) * KSTRIDE + KS;
+  extern __shared__ __align__(16) uint8_t s_planes[];
+  const int hw = p.H * p.W, ohw = p.OH * p.OW;
+  const int plane0 = blockIdx.x * group;
+  const int planes = min(group, p.N * p.C - plane0);
+  const T* x = static_cast<const T*>(p.x) + (long long)plane0 * hw;
+  T* y = static_cast<T*>(p.y) + (long long)plane0 * ohw;
+  const T* res = p.residual != nullptr ? static_cast<const T*>(p.residual) + (long long)plane0 * ohw : nullptr;
+  T* sx = reinterpret_cast<T*>(s_planes + (reinterpret_cast<uintptr_t>(x) & 15));
+  uint8_t* s_out = s_planes + (size_t(group) * hw * sizeof(T) + 31) / 16 * 16;
+  T* sy = reinterpret_cast<T*>(s_out + (reinterpret_cast<uintptr_t>(y) & 15));
+  copy_elements(sx, x, planes * hw);
+  __syncthreads();
+  const int owg = (p.OW + PW - 1) / PW, per_plane = p.OH * owg;
+  for (int i = threadIdx.x; i < planes * per_plane; i += kDwThreads) {
+    const int pl = i / per_plane, rest = i - pl * per_plane;
+    const int oh = rest / owg, ow0 = (rest - oh * owg) * PW;
+    const int c = (plane0 + pl) % p.C;
+    const T* w = static_cast<const T*>(p.w) + c * p.w_s[0];
+    const T* in = sx + pl * hw;
+    const int iw0 = ow0 * KSTRIDE - p.pad_left;
+    float acc[PW];
+#pragma unroll
+    for (int q = 0; q < PW; ++q) acc[q] = 0.0f;
+#pragma unroll
+    for (int r = 0; r < KR; ++r) {
+      const int ih = oh * KSTRIDE + r - p.pad_top;
+      if (ih < 0 || ih >= p.H) continue;
+      float wt[KS];
+#pragma unroll
+      for (int s = 0; s < KS; ++s) wt[s] = to_f32<T>(__ldg(w + r * p.w_s[2] + s * p.w_s[3]));
+      const T* row = in + ih * p.W + iw0;
+#pragma unroll
+      for (int j = 0; j < kSpan; ++j) {
+        const float xv = (iw0 + j >= 0 && iw0 + j < p.W) ? to_f32<T>(row[j]) : 0.0f;
+#pragma unroll
+        for (int q = 0; q < PW; ++q) {
+          const int s = j - q * KSTRIDE;
+          if (s >= 0 && s < KS) acc[q] = fmaf(xv, wt[s], acc[q]);
+        }
+      }
+    }
+    const float sc = p.scale != nullptr ? to_f32<T>(static_cast<const T*>(p.scale)[c]) : 1.0f;
+    const float bi = p.bias != nullptr ? to_f32<T>(static_cast<const T*>(p.bias)[c]) : 0.0f;
+    const int o = pl * ohw + oh * p.OW + ow0;
+#pragma unroll
+    for (int q = 0; q < PW; ++q) {
+      if (ow0 + q < p.OW) {
+        float a = fmaf(acc[q], sc, bi);
+        if (res != nullptr) a += to_f32<T>(res[o + q]);
+        sy[o + q] = from_f32<T>(p.act == 1 ? relu_keep_nan(a) : (p.act ? apply_activation(a, p.act) : a));
+      }
+    }
+  }
+  __syncthreads();
+  copy_elements(y, sy, planes * ohw);
+}
+
+// Planes per block: about two work items per thread, as many as 40 KB hold; 0: not a case (planes too large, or not
+// dense).
+inline int planes_per_block(const DirectParams& p, int es) {
+  const long long hw = (long long)p.H * p.W, ohw = (long long)p.OH * p.OW;
+  auto dense = [&](const long long (&s)[4], long long w, long long plane) {
+    return (w <= 1 || s[3] == 1) && (plane == w || s[2] == w) && (p.C <= 1 || s[1] == plane) &&
+           (p.N <= 1 || s[0] == p.C * plane);
+  };
+  if (!dense(p.x_s, p.W, hw) || !dense(p.y_s, p.OW, ohw)) return 0;
+  const long long bytes = (hw + ohw) * es, items = (long long)p.OH * ((p.OW + 3) / 4);
+  if (bytes > 40 * 1024) return 0;
+  long long g = (2 * kDwThreads + items - 1) / items;
+  if (g > 40 * 1024 / bytes) g = 40 * 1024 / bytes;
+  const long long spread = ((long long)p.N * p.C + 2 * 148 - 1) / (2 * 148);   // leave every SM a couple of blocks
+  if (g > spread) g = spread;
+  return int(g < 1 ? 1 : g);
+}
+
+template <typename T, int KR, int KS, int KSTRIDE>
+cudaError_t launch_planes(const DirectParams& p, cudaStream_t stream) {
+  const int group = planes_per_block(p, int(sizeof(T)));
+  if (group < 1) return cudaErrorInvalidValue;
+  const size_t smem = size_t(group) * (size_t(p.H) * p.W + size_t(p.OH) * p.OW) * sizeof(T) + 96;
+  const unsigned blocks = unsigned((p.N * p.C + group - 1) / group);
+  depthwise_planes_kernel<T, KR, KS, KSTRIDE><<<blocks, kDwThreads, smem, stream>>>(p, group);
+  return cudaGetLastError();
+}
+
 // ------------------------------------------------- NCHW, rows read as 16- or 8-byte vectors
 // W-contiguous planes whose rows start on VB-byte boundaries, "same" padding (pad_left == KS / 2), no dilation:
 // a thread owns V = VB / sizeof(T) neighbouring outputs of a row.  The input columns they need are KSTRIDE
@@ -604,7 +684,7 @@ cudaError_t launch_cl(Kernel kernel, const DirectParams& p, int V, int PW, int b
     cached.store(c, std::memory_order_relaxed);
   }
   const int chunks = (cv + g.tcx - 1) / g.tcx;
-  const long long resident = (long long)sm_count_dw() * (c & 255);
+  const long long resident = (long long)current_sm_count() * (c & 255);
   const long long groups = resident / chunks > 0 ? resident / chunks * g.tpy : g.tpy;   // units in flight
   // rows per unit: `band_max` while every resident thread group still gets kDwRounds units, fewer otherwise
   g.band_rows = band_max;
@@ -626,6 +706,7 @@ cudaError_t go_static(const DirectParams& p, int kind, cudaStream_t stream) {
   if constexpr (KR != 0) {
     if (kind == 3) return launch_rowvec<T, KR, KS, KSTRIDE, 16>(p, stream);
     if (kind == 4) return launch_rowvec<T, KR, KS, KSTRIDE, 8>(p, stream);
+    if (kind == 7) return launch_planes<T, KR, KS, KSTRIDE>(p, stream);
     if constexpr (sizeof(T) == 2) {
       if (kind == 5) return launch_rowvec<T, KR, KS, KSTRIDE, 4>(p, stream);
     }
@@ -655,7 +736,8 @@ cudaError_t go(const DirectParams& p, int channels_last, cudaStream_t stream) { 
 }  // namespace
 
 // 0: not a case for these kernels (the caller uses the direct kernel); 1: channels-last kernel; 2: plane kernel;
-// 3 / 4 / 5: row-vector kernel (NCHW) on 16- / 8- / 4-byte vectors.
+// 3 / 4 / 5: row-vector kernel (NCHW) on 16- / 8- / 4-byte vectors; 6: a case of kernel 1 that the staged kernel
+// (conv_depthwise_tma.cu) takes; 7: several dense planes per block.
 int depthwise_kind(int dtype, const DirectParams& p) {
   if (p.groups != p.C || p.K != p.C || p.C < 1) return 0;
   if (dtype != FDNN_F16 && dtype != FDNN_BF16 && dtype != FDNN_F32) return 0;
@@ -669,7 +751,7 @@ int depthwise_kind(int dtype, const DirectParams& p) {
                   mult(p.N, p.x_s[0]) && mult(p.H, p.x_s[2]) && mult(p.W, p.x_s[3]) && mult(p.N, p.y_s[0]) &&
                   mult(p.OH, p.y_s[2]) && mult(p.OW, p.y_s[3]) && (long long)(p.R * p.S + 2) * v <= kDwMaxSmemFloats &&
                   p.C > 1 && (long long)p.N * p.OH * p.OW < 2147483647LL && p.C / v < 65536LL * 8;
-  if (cl) return 1;
+  if (cl) return depthwise_tma_ok(p) ? 6 : 1;
   // W-contiguous planes with vector-aligned rows and "same" padding of an unrolled filter: the row-vector kernel
   // on the widest vectors the rows are aligned for (16 bytes; 8 for rows of 28 16-bit values; 4 for rows of 14)
   const bool unrolled = p.dil_h == 1 && p.dil_w == 1 && p.stride_h == p.stride_w && p.R == p.S &&
@@ -686,6 +768,8 @@ int depthwise_kind(int dtype, const DirectParams& p) {
         return vb == 16 ? 3 : (vb == 8 ? 4 : 5);
     }
   }
+  // (planes whose rows are vector-aligned stay with the row-vector kernel: 58 us against 109 us on 64 x 512 x 28 x 28)
+  if (unrolled && planes_per_block(p, es) > 0 && (long long)p.N * p.C < 2147483647LL) return 7;
   if ((long long)p.N * p.C < 2147483647LL && p.R * p.S <= kDwMaxSmemFloats) return 2;
   return 0;
 }

@@ -127,6 +127,12 @@ cudaError_t launch_direct(int dtype, const DirectParams& p, cudaStream_t stream)
 // of channels per thread), 2 for the kernel that gives every (image, channel) plane a block, 3 / 4 / 5 for the
 // NCHW kernel that reads rows as 16- / 8- / 4-byte vectors.
 int depthwise_kind(int dtype, const DirectParams& p);
+// 6: channels-last cases of the kernel that stages input rows through the TMA unit (conv_depthwise_tma.cu).
+bool depthwise_tma_ok(const DirectParams& p);
+cudaError_t launch_depthwise_tma(int dtype, const DirectParams& p, uint32_t* status, long long wait_limit, cudaStream_t stream);
+// Tensor map over a channels-last x for it: boxes of `chunk` channels x `span` pixels x `rows` rows.  False: not encodable.
+bool encode_depthwise_map(CUtensorMap* tm, int dtype, const DirectParams& p, int chunk, int span, int rows);
+int current_sm_count();   // of the current device (148 when none is visible)
 cudaError_t launch_depthwise(int dtype, const DirectParams& p, int kind, cudaStream_t stream);
 
 // Pooling (pool.cu): element strides of x and y in (n, c, h, w) order; idx (max pooling only) may be null.

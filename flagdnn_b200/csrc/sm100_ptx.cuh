@@ -17,7 +17,8 @@ enum : uint32_t {
   kIncidentEpilogueWait = 4,   // epilogue: accumulator never completed
   kIncidentDrainWait = 5,      // teardown: outstanding copies never landed
   kIncidentPartialWait = 6,    // epilogue of a split tile: another pair's partial sums never arrived
-  kIncidentResidualWait = 7    // epilogue: the residual box never landed in the staging buffer
+  kIncidentResidualWait = 7,   // epilogue: the residual box never landed in the staging buffer
+  kIncidentDepthwiseWait = 8   // depthwise: an input row never landed in its ring slot
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
