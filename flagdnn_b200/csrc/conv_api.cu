@@ -318,6 +318,17 @@ bool filter_mn_major(const fdnn_conv_desc* d, const void* w) {
   return 2.9e-10 * products < 2.0 + 0.8e-6 * filter;   // both sides in microseconds
 }
 
+// Below kSmallFlops a 16-bit layer still runs on the tensor-core kernel when its reduction is more than a few dozen
+// products long: the direct kernel walks it serially (one 64 x 14 x 14 image, 64 filters 3x3, f16: 26.6 us against
+// 5 us), and both round an fp32 sum once.  fp32 layers stay on exact products there.  Such a call needs what the
+// tensor-core plan asks for (packed filter, scratch); without it, fwd_impl runs the direct kernel as before, and the
+// scratch stays within the built-in one of fdnn_conv2d_fwd_static_scratch.
+constexpr double kSmallFlops = 2.0e7;
+bool small_on_tensor_cores(const fdnn_conv_desc* d, double flops) {
+  return elem_size(d->dtype) == 2 && d->c * d->r * d->s >= 64 && flops >= 2.0e5 &&
+         (long long)d->n * d->h * d->w * padded_x_channels(d) * 2 <= FDNN_STATIC_SCRATCH_BYTES;
+}
+
 // Reduction splitting on CTA pairs: T tiles of K reduction steps on P pairs.  Whole tiles cost
 // ceil(T / P) * K steps on the busiest pair, an even split ceil(T * K / P) plus the exchange of one partial
 // tile (about three steps' worth of time).  Ranges shorter than 12 steps are not split (boundaries snap to
@@ -374,6 +385,12 @@ fdnn_conv_desc dense_group_desc(const fdnn_conv_desc* d) {
   return v;
 }
 
+// Unless a tensor-core kernel was asked for, a grouped layer takes one of those routes only if the dense layer it turns
+// into is not a small one.
+bool worth_grouping(const fdnn_conv_desc* d, const fdnn_conv_plan& inner) {
+  return (d->algo & 0xff) != FDNN_ALGO_AUTO || inner.flops >= kSmallFlops;
+}
+
 fdnn_conv_desc one_group_desc(const fdnn_conv_desc* d) {
   fdnn_conv_desc sub = *d;
   sub.c = d->c / d->groups;
@@ -403,7 +420,7 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
     const fdnn_conv_desc v = dense_group_desc(d);
     fdnn_conv_plan pv;
     // the dense filter will sit 256-byte aligned at the front of the packed buffer: plan it as readable in place
-    if (make_plan(&v, x, nullptr, y, &pv, allow_group) == FDNN_OK && pv.algo != FDNN_ALGO_DIRECT) {
+    if (make_plan(&v, x, nullptr, y, &pv, allow_group) == FDNN_OK && pv.algo != FDNN_ALGO_DIRECT && worth_grouping(d, pv)) {
       const double flops = plan->flops, bytes = plan->bytes;
       *plan = pv;
       plan->flops = flops;   // the layer's own work, not the block-diagonal GEMM's
@@ -416,7 +433,7 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
   if (group_loop_ok(d)) {
     const fdnn_conv_desc sub = one_group_desc(d);
     fdnn_conv_plan ps;
-    if (make_plan(&sub, x, w, y, &ps, allow_group) == FDNN_OK && ps.algo != FDNN_ALGO_DIRECT) {
+    if (make_plan(&sub, x, w, y, &ps, allow_group) == FDNN_OK && ps.algo != FDNN_ALGO_DIRECT && worth_grouping(d, ps)) {
       const double flops = plan->flops, bytes = plan->bytes;
       *plan = ps;              // every group runs this plan; scratch is shared, the packed filters are not
       plan->flops = flops;
@@ -441,7 +458,7 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
   if ((algo == FDNN_ALGO_IGEMM || algo == FDNN_ALGO_IGEMM_PAIR) && !geom_ok)
     return fail(FDNN_NOT_SUPPORTED, "implicit-GEMM path does not support this problem");
   const bool want_auto = algo == FDNN_ALGO_AUTO;
-  if (want_auto) algo = (geom_ok && plan->flops >= 2.0e7) ? FDNN_ALGO_IGEMM : FDNN_ALGO_DIRECT;
+  if (want_auto) algo = (geom_ok && (plan->flops >= kSmallFlops || small_on_tensor_cores(d, plan->flops))) ? FDNN_ALGO_IGEMM : FDNN_ALGO_DIRECT;
   if (algo != FDNN_ALGO_IGEMM && algo != FDNN_ALGO_DIRECT && algo != FDNN_ALGO_IGEMM_PAIR)
     return fail(FDNN_BAD_PARAM, "unknown algo");
   plan->algo = algo;
@@ -1263,6 +1280,14 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   if (st != FDNN_OK) return st;
   if (activation < FDNN_ACT_NONE || activation > FDNN_ACT_GELU_TANH)
     return fail(FDNN_BAD_PARAM, "unknown activation");
+  if ((desc->algo & 0xff) == FDNN_ALGO_AUTO && desc->groups == 1 && plan.algo != FDNN_ALGO_DIRECT &&
+      plan.flops < kSmallFlops && allow_group && w != nullptr &&
+      ((plan.w_packed && w_packed == nullptr) || (plan.workspace_bytes > 0 && (workspace == nullptr || workspace_bytes < plan.workspace_bytes)))) {
+    // a small layer whose caller brought neither packed filter nor scratch (see small_on_tensor_cores)
+    fdnn_conv_desc direct = *desc;
+    direct.algo = FDNN_ALGO_DIRECT;
+    return fwd_impl(&direct, x, w, nullptr, bias, scale, residual, activation, y, nullptr, 0, stream_v, allow_group, k_real);
+  }
   const fdnn_conv_desc& d = *desc;
   if (d.n == 0 || plan.oh == 0 || plan.ow == 0) return FDNN_OK;  // empty output: nothing to launch
   if (x == nullptr || y == nullptr || (w == nullptr && w_packed == nullptr))
