@@ -15,6 +15,8 @@ from pathlib import Path
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libflagdnn_b200.so"
+HOST_SOURCE = CSRC / "host" / "fastcall.cpp"
+HOST_PATH = PKG_DIR / "_fastcall.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -39,7 +41,7 @@ def _stale() -> bool:
     if not LIB_PATH.exists():
         return True
     built = LIB_PATH.stat().st_mtime
-    deps = list(CSRC.glob("*")) + [PKG_DIR.parent / "include" / "flagdnn_b200.h"]
+    deps = [p for p in CSRC.glob("*") if p.is_file()] + [PKG_DIR.parent / "include" / "flagdnn_b200.h"]
     return any(p.stat().st_mtime > built for p in deps if p.exists())
 
 
@@ -61,6 +63,32 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     return LIB_PATH
 
 
+def build_host(force: bool = False, verbose: bool = False) -> Path:
+    """Compile the native host path of the eager operators (csrc/host/fastcall.cpp) against the installed torch."""
+    header = PKG_DIR.parent / "include" / "flagdnn_b200.h"
+    if not force and HOST_PATH.exists() and all(p.stat().st_mtime <= HOST_PATH.stat().st_mtime for p in (HOST_SOURCE, header)):
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{root / 'include'}", f"-I{root / 'include' / 'torch' / 'csrc' / 'api' / 'include'}",
+           f"-I{sysconfig.get_paths()['include']}", f"-I{cuda / 'include'}",
+           "-o", str(HOST_PATH), str(HOST_SOURCE), f"-L{root / 'lib'}",
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", f"-Wl,-rpath,{root / 'lib'}"]
+    if verbose:
+        print(" ".join(cmd), file=sys.stderr)
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"g++ failed ({proc.returncode}):\n{proc.stdout}\n{proc.stderr}")
+    return HOST_PATH
+
+
 if __name__ == "__main__":
+    build_host(force="--force" in sys.argv, verbose=True)
     build(force="--force" in sys.argv, verbose=True, ptxas_info="--ptxas-info" in sys.argv)
     print(LIB_PATH)

@@ -241,6 +241,44 @@ def _packed_weight(weight: torch.Tensor, d: nat.ConvDesc, plan: nat.ConvPlan, st
     return packed
 
 
+# ------------------------------------------------------------- native host path
+# csrc/host/fastcall.cpp reads the tensors' metadata, looks the plan up and calls the C ABI in one native call; it answers
+# None for everything it does not take, and the Python code below then does the call (or raises).
+_fast: Any = None
+
+
+def _packed_for_native(weight, desc_address: int, plan_address: int, stream: int, y_ptr: int) -> torch.Tensor:
+    return _packed_weight(weight, nat.ConvDesc.from_address(desc_address), nat.ConvPlan.from_address(plan_address),
+                          stream, y_ptr)
+
+
+def _load_fast() -> Any:
+    global _fast
+    if _fast is None:
+        try:
+            from . import _fastcall
+        except ImportError:      # not built: every call takes the Python code
+            _fast = False
+            return _fast
+        lib = nat.load()
+        address = [ctypes.cast(f, ctypes.c_void_p).value for f in
+                   (lib.fdnn_conv2d_query, lib.fdnn_conv2d_pack_weight, lib.fdnn_conv2d_fwd_ex)]
+        _fastcall.bind(*address, _packed_for_native)
+        _fast = _fastcall
+    return _fast
+
+
+def fast_conv(input, weight, bias, scale, residual, stride, padding, dilation, groups, act) -> Optional[torch.Tensor]:
+    """The convolution through the native host path, or None if that does not take the call."""
+    fast = _fast if _fast is not None else _load_fast()
+    if not fast or _STREAM_K:
+        return None
+    y = fast.conv(input, weight, bias, scale, residual, stride, padding, dilation, groups, _FORCED_ALGO, act)
+    if y.__class__ is int:
+        nat.check(y)
+    return y
+
+
 def conv2d_plan(input, weight, stride=1, padding=0, dilation=1, groups=1, algo=None) -> dict:
     """What the library would do for this call (kernel family, tile, scratch sizes)."""
     stride = _pair(stride)
@@ -354,6 +392,10 @@ def conv2d(
 ) -> torch.Tensor:
     """Drop-in for ``flag_dnn.ops.conv2d`` (src/flag_dnn/ops/conv2d.py:3575).  ``out`` (not in the
     reference) receives the result: any strides, the output's shape and the input's dtype."""
+    if out is None:
+        y = fast_conv(input, weight, bias, None, None, stride, padding, dilation, groups, nat.ACT_NONE)
+        if y is not None:
+            return y
     stride = _pair(stride)
     dilation = _pair(dilation)
     padding4 = _normalize_padding(weight, stride, padding, dilation)
@@ -385,6 +427,10 @@ def fused_conv2d_bias_relu(
     "none", "gelu" or "gelu_tanh").
     """
     del config
+    if out is None and groups == 1 and bias is not None and activation in _ACTIVATIONS:
+        y = fast_conv(input, weight, bias, scale, None, stride, padding, dilation, 1, _ACTIVATIONS[activation])
+        if y is not None:
+            return y
     if not (isinstance(input, torch.Tensor) and input.is_cuda):
         raise NotImplementedError("fused_conv2d_bias_relu requires runtime device input")
     if groups != 1:
@@ -436,6 +482,11 @@ def conv2d_bias_act(
     that fall outside ``fused_conv2d_bias_relu``'s contract and for a block's last
     convolution with its shortcut add (``residual`` has the output's shape; when it
     also has the output's strides the add happens in the kernel's epilogue)."""
+    if out is None and (activation is None or activation in _ACTIVATIONS):
+        act = _ACTIVATIONS[activation] if activation is not None else (nat.ACT_RELU if relu else nat.ACT_NONE)
+        y = fast_conv(input, weight, bias, scale, residual, stride, padding, dilation, groups, act)
+        if y is not None:
+            return y
     stride = _pair(stride)
     dilation = _pair(dilation)
     padding4 = _normalize_padding(weight, stride, padding, dilation)
@@ -465,6 +516,14 @@ def conv1d(
     """Drop-in for ``flag_dnn.ops.conv1d`` (src/flag_dnn/ops/conv1d.py:416): a convolution over
     [N, C, L] (or unbatched [C, L]) is the 2-D path with H = R = 1, so it runs on the same kernels.
     Checks and messages follow src/flag_dnn/ops/conv1d.py:21-66, 90-150, 436-446."""
+    fast = _load_fast()
+    if fast and not _STREAM_K:
+        y = fast.conv1d(input, weight, bias, stride, padding, dilation, groups, _FORCED_ALGO)
+        if y.__class__ is int:
+            nat.check(y)
+        if y is not None:
+            return y
+
     def single(v, name):
         if isinstance(v, int):
             return int(v)
@@ -555,6 +614,13 @@ def mm(
     on the same kernels (fp64 on the direct one).  Checks and messages follow src/flag_dnn/ops/mm.py:100-140,
     the ``out`` handling src/flag_dnn/ops/mm.py:153-181.  ``out_dtype=torch.float32`` with fp16 / bf16 operands
     stores the fp32 accumulators unrounded.  Complex tensors are not implemented on this path."""
+    fast = _load_fast()
+    if fast and not _STREAM_K and out is None and (out_dtype is None or out_dtype == input.dtype):
+        y = fast.mm(input, mat2, _FORCED_ALGO)
+        if y.__class__ is int:
+            nat.check(y)
+        if y is not None:
+            return y
     if input.dim() != 2:
         raise RuntimeError("self must be a matrix")
     if mat2.dim() != 2:

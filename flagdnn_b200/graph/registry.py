@@ -139,6 +139,11 @@ def _run_conv2d(inputs: list, attrs: dict) -> torch.Tensor:
 def _run_fused_conv2d_bias_relu(inputs: list, attrs: dict) -> torch.Tensor:
     from .. import conv_host as native
 
+    if len(inputs) == 3 and attrs.get("_out") is None:
+        y = native.fast_conv(inputs[0], inputs[1], inputs[2], None, None, attrs.get("stride", 1), attrs.get("padding", 0),
+                             attrs.get("dilation", 1), attrs.get("groups", 1), native.nat.ACT_RELU)
+        if y is not None:
+            return y
     _require_device(inputs, "fused_conv2d_bias_relu")
     a = _public(attrs)
     scale = inputs[3].reshape(-1) if len(inputs) > 3 else None  # captured as (K,1,1) or (1,K,1,1)
