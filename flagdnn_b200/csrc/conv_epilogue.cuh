@@ -284,7 +284,8 @@ constexpr int kYScattered = 0, kYPixels = 1, kYChannels = 2;
 struct StridedOut {
   void* y;                 // element type of the operands
   const void* res;         // residual with y's strides, or nullptr
-  long long y_off;         // this lane's pixel: element offset of channel 0
+  long long y_off;         // this lane's pixel: element offset of the (group's) first channel
+  long long k_off;         // element offset of the group's first channel alone
   long long sn, sk;        // element strides between images and between channels
   int mode, unit;          // kY*, bytes per lane and store
   int m0, M, ohw;          // the warp's first GEMM row, rows overall, pixels per image
@@ -456,7 +457,7 @@ __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, i
     const int m = o.m0 + px;
     const int img = m / o.ohw;
     u_ok = m < o.M;
-    u_off = img * o.sn + (m - img * o.ohw);
+    u_off = img * o.sn + (m - img * o.ohw) + o.k_off;
     whole = rows_ok == 0xffffffffu && (o.m0 + 31) / o.ohw == o.m0 / o.ohw;   // 32 pixels of one image
   }
 #pragma unroll 1

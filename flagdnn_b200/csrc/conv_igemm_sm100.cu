@@ -182,7 +182,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int ohw = p.OH * p.OW;
 
   // How a reduction step's operands are copied.
-  constexpr int kIm2col = 0, kWindows = 1, kFilterMn = 2;
+  constexpr int kIm2col = 0, kWindows = 1, kFilterMn = 2, kGroups = 3;
   // The whole warp walks the steps and one elected lane issues (see the issuer): the copy-issuing role is as close to
   // the critical path of narrow tiles as the MMA-issuing one.
   auto produce = [&](auto mode_tag, auto prof_tag) {
@@ -212,10 +212,13 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         w_base = ow0 * p.stride_w - p.pad_left;
         h_base = oh0 * p.stride_h - p.pad_top;
       }
+      const int group = kMode == kGroups ? n_tile / p.group_n_tiles : 0;
+      const int col0 = (n_tile - group * p.group_n_tiles) * BN;      // first column of the tile, within its group
+      const int b_row0 = group * p.Kout + col0;                      // and its filter
       if constexpr (RES && DENSE) {
         // the epilogue of this tile will read its 128 x BN residual values a whole main loop from now:
         // ask for them to be brought into L2 so that its loads are short and HBM reads are requested early
-        if (lead && p.residual != nullptr && !p.lowc) tma_prefetch_l2_3d(&tmR, n_tile * BN, m_tile * kBM, 0);
+        if (lead && p.residual != nullptr && !p.lowc) tma_prefetch_l2_3d(&tmR, col0, m_tile * kBM, group);
       }
       int r = 0, s = 0, cb = 0;
       for (int kit = 0; kit < k_iters; ++kit, ++it) {
@@ -239,19 +242,25 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             tma_load_4d(st, &tmA, bar, 0, 0, h_base + r * p.dil_h, img);
           } else {
             const uint16_t off_w = static_cast<uint16_t>(s * p.dil_w), off_h = static_cast<uint16_t>(r * p.dil_h);
-            tma_load_im2col_4d(st, &tmA, bar, c0, w_base, h_base, img, off_w, off_h);
-            if constexpr (Cfg::kSplit)
-              tma_load_im2col_4d(st + Cfg::kABytes, &tmA2, bar, c0, w_base, h_base, img, off_w, off_h);
+            if constexpr (kMode == kGroups) {
+              tma_load_im2col_5d(st, &tmA, bar, c0, w_base, h_base, img, group, off_w, off_h);
+              if constexpr (Cfg::kSplit)
+                tma_load_im2col_5d(st + Cfg::kABytes, &tmA2, bar, c0, w_base, h_base, img, group, off_w, off_h);
+            } else {
+              tma_load_im2col_4d(st, &tmA, bar, c0, w_base, h_base, img, off_w, off_h);
+              if constexpr (Cfg::kSplit)
+                tma_load_im2col_4d(st + Cfg::kABytes, &tmA2, bar, c0, w_base, h_base, img, off_w, off_h);
+            }
           }
           if constexpr (Cfg::kSplit) {
-            tma_load_3d(st + 2 * Cfg::kABytes, &tmB, bar, c0, r * p.S + s, n_tile * BN);
-            tma_load_3d(st + 2 * Cfg::kABytes + Cfg::kBBytes, &tmB2, bar, c0, r * p.S + s, n_tile * BN);
+            tma_load_3d(st + 2 * Cfg::kABytes, &tmB, bar, c0, r * p.S + s, b_row0);
+            tma_load_3d(st + 2 * Cfg::kABytes + Cfg::kBBytes, &tmB2, bar, c0, r * p.S + s, b_row0);
           } else if constexpr (kMode == kFilterMn) {   // filter with K contiguous: boxes of 64 filters x 64 channels
 #pragma unroll
             for (int j = 0; j < BN / int(kMnBoxElems); ++j)
-              tma_load_3d(st + Cfg::kABytes + j * kMnBoxBytes, &tmB, bar, n_tile * BN + j * int(kMnBoxElems), c0, 0);
+              tma_load_3d(st + Cfg::kABytes + j * kMnBoxBytes, &tmB, bar, b_row0 + j * int(kMnBoxElems), c0, 0);
           } else {
-            tma_load_3d(st + Cfg::kABytes, &tmB, bar, c0, r * p.S + s, n_tile * BN);
+            tma_load_3d(st + Cfg::kABytes, &tmB, bar, c0, r * p.S + s, b_row0);
           }
         }
         __syncwarp();
@@ -300,6 +309,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     if (!p.skip_copies) {
       if (p.lowc) produce_any(std::integral_constant<int, kWindows>{});
       else if (p.b_mn) produce_any(std::integral_constant<int, kFilterMn>{});
+      else if (p.groups > 1) produce_any(std::integral_constant<int, kGroups>{});
       else produce_any(std::integral_constant<int, kIm2col>{});
     }
   } else if (warp == 1) {
@@ -416,7 +426,9 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++tcount) {
       const int m_tile = tile / p.n_tiles;
       const int n_tile = tile - m_tile * p.n_tiles;
-      const int n0 = n_tile * BN + chalf * WC;  // first column this warp owns
+      const int group = p.groups > 1 ? n_tile / p.group_n_tiles : 0;
+      const int n0 = (n_tile - group * p.group_n_tiles) * BN + chalf * WC;  // first column (of the group) this warp owns
+      const int k0 = group * p.Kout;                                        // the group's first output channel
       const uint32_t buf = tcount & 1u;
       const uint32_t bphase = (tcount >> 1) & 1u;
 
@@ -424,8 +436,8 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         __syncwarp();
         for (int j = lane; j < WC; j += 32) {
           const int col = n0 + j;
-          s_scale[j] = (g_scale != nullptr && col < p.Kout) ? to_f32<T>(g_scale[col % p.k_real]) : 1.0f;
-          s_bias[j] = (g_bias != nullptr && col < p.Kout) ? to_f32<T>(g_bias[col % p.k_real]) : 0.0f;
+          s_scale[j] = (g_scale != nullptr && col < p.Kout) ? to_f32<T>(g_scale[k0 + col % p.k_real]) : 1.0f;
+          s_bias[j] = (g_bias != nullptr && col < p.Kout) ? to_f32<T>(g_bias[k0 + col % p.k_real]) : 0.0f;
         }
         __syncwarp();
         staged_n_tile = n_tile;
@@ -439,7 +451,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         const int rem = m - img * ohw;
         const int oh = rem / p.OW;
         const int ow = rem - oh * p.OW;
-        y_off = img * p.y_sn + oh * p.y_sh + ow * p.y_sw;
+        y_off = img * p.y_sn + oh * p.y_sh + ow * p.y_sw + k0 * p.y_sk;
       }
       const long long et0 = p.prof ? clock64() : 0;
       bool ok = mbar_wait_bounded(&tmem_full[buf], bphase, abort_flag, p.status, kIncidentEpilogueWait, p.wait_limit);
@@ -457,7 +469,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         st_row = (m_tile - st_img * p.tiles_per_image) * p.rows_per_tile + ew * 32;
         st_rows = p.rows_per_tile - ew * 32;
       } else {
-        st_img = 0;
+        st_img = group;   // the output map's third dimension: the group's channels
         st_row = m_tile * kBM + ew * 32;
         st_rows = 32;
       }
@@ -470,6 +482,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       } else if (p.y_mode != kYScattered) {
         StridedOut so;
         so.y = p.y;
+        so.k_off = k0 * p.y_sk;
         so.res = g_res;
         so.y_off = y_off;
         so.sn = p.y_sn; so.sk = p.y_sk;

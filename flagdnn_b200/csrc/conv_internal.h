@@ -42,6 +42,10 @@ struct IgemmParams {
   int tiles_per_image;   // low-channel mode: ceil(OH / ohs)
   int ohs;               // low-channel mode: output rows per tile
   int a_tx_bytes;        // bytes one activation copy delivers (rows_per_tile * 128 in low-channel mode)
+  // Grouped layers in one launch (single-CTA kernel): column tiles count through the groups; Kout and the maps over the
+  // filter, y and the residual are one group's, the activation map has the group as its fifth dimension.
+  int groups;            // 1: not grouped
+  int group_n_tiles;     // column tiles of one group (n_tiles = groups * group_n_tiles)
   int b_mn;              // 1: one tap, filter with K contiguous ([C][K]): read in place as an MN-major operand
   int b_resident;        // pair kernel: the filter half stays in shared memory for the whole launch
   // Low-channel mode on a dense 3-channel NHWC input (the stem), pair kernel only: no relayout pass.  Two warps

@@ -250,6 +250,20 @@ __device__ __forceinline__ void tma_load_im2col_4d(void* smem_dst, const CUtenso
       : "memory");
 }
 
+// The same over five dimensions (C, W, H, D, N), for grouped layers: D holds the images (the walk of pixelsPerColumn
+// pixels goes through W, H, D), N the group.
+__device__ __forceinline__ void tma_load_im2col_5d(void* smem_dst, const CUtensorMap* tm, uint64_t* bar, int32_t c,
+                                                   int32_t w, int32_t h, int32_t d, int32_t n, uint16_t off_w,
+                                                   uint16_t off_h) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2], {%8, %9, %10};"
+      :
+      : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tm)), "r"(smem_u32(bar)), "r"(c),
+        "r"(w), "r"(h), "r"(d), "r"(n), "h"(off_w), "h"(off_h), "h"(static_cast<uint16_t>(0))
+      : "memory");
+}
+
 // Tiled 2-D tensor store shared -> global (bulk-group completion).  Rows or
 // columns of the box that fall outside the tensor are not written.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tm, const void* smem_src, int32_t c0,

@@ -103,7 +103,7 @@ typedef struct fdnn_conv_plan {
   int32_t w_packed;             /* 1: fwd needs a packed filter from fdnn_conv2d_pack_weight */
   int32_t c_padded;             /* channel count the igemm kernel iterates over */
   int32_t grid, block;          /* launch shape of the main kernel */
-  int32_t launches;             /* kernels one fwd call launches (main + repack; per-group launches of a
+  int32_t launches;             /* kernels one fwd call launches at most (main + repack; per-group launches of a
                                    grouped layer all counted) */
   int32_t low_channel;          /* 1: C <= 4 path (pixel quads as GEMM rows, 16-pixel input windows) */
   int32_t pixel_group;          /* > 1: that many neighbouring output pixels form one GEMM row (narrow layers) */
