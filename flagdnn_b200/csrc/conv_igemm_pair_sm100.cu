@@ -178,10 +178,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 #endif
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    // The whole warp walks the steps and one elected lane issues, here and in the issuer: addresses, coordinates and
-    // descriptors are then uniform values (see conv_igemm_sm100.cu for what that is worth per step).
-    if (!p.skip_copies) {
-      const bool lead = elect_one();
+    if (lane == 0 && !p.skip_copies) {
       uint32_t stage = 0, phase = 0;
       bool alive = true;
       long long prof_wait = 0, prof_issue = 0, prof_iters = 0, prof_t0 = p.prof ? clock64() : 0;
@@ -189,12 +186,12 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       if (b_resident && pair_id < total_tiles) {
         // this CTA's 128 filter rows for every reduction step, once (n_tiles == 1 in this mode)
         const uint32_t bres = map_to_cta(smem_u32(bres_bar), 0);
-        if (lead && rank == 0) mbar_arrive_expect_tx(bres_bar, uint32_t(2 * k_iters * kBBytes));
+        if (rank == 0) mbar_arrive_expect_tx(bres_bar, uint32_t(2 * k_iters * kBBytes));
         int kit = 0;
         for (int r = 0; r < p.R; ++r)
           for (int s = 0; s < p.S; ++s)
             for (int cb = 0; cb < p.c_blocks; ++cb, ++kit)
-              if (lead) tma_load_3d_pair(b_res + kit * kBBytes, &tmB, bres, cb * kKB, r * p.S + s, int(rank) * kHalfN);
+              tma_load_3d_pair(b_res + kit * kBBytes, &tmB, bres, cb * kKB, r * p.S + s, int(rank) * kHalfN);
       }
       TileWalk walk;
       walk_init(walk, split, pair_id, num_pairs, total_tiles, k_iters, p.sk_min_frag);
@@ -222,7 +219,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         if constexpr (RES) {
           // this CTA's 128 x 256 residual values of the tile, asked into L2 a whole main loop before the
           // epilogue reads them (only the pair that finishes the tile reads them)
-          if (lead && p.residual != nullptr && !p.lowc && walk.ke == k_iters)
+          if (p.residual != nullptr && !p.lowc && walk.ke == k_iters)
             tma_prefetch_l2_3d(&tmR, n_tile * kPairN, m_tile * kRows, 0);
         }
         const uint32_t a_tx = p.lowc ? uint32_t(p.a_tx_bytes) : uint32_t(kABytes);
@@ -231,8 +228,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         if (p.fused3) {
           // the converter warps have written this tile's input rows into slot (tiles_done & 1)
           const uint32_t b_ = tiles_done & 1u;
-          if (!mbar_wait_warp(&raw_full[b_], (tiles_done >> 1) & 1u, abort_flag, p.status, kIncidentProducerWait,
-                              p.wait_limit)) {
+          if (!mbar_wait_bounded(&raw_full[b_], (tiles_done >> 1) & 1u, abort_flag, p.status, kIncidentProducerWait,
+                                 p.wait_limit)) {
             alive = false;
             break;
           }
@@ -250,7 +247,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           for (int kit = walk.kb; kit < walk.ke; ++kit) {
             long long pt0 = 0, pt1 = 0;
             if constexpr (kProf) pt0 = clock64();
-            if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, kIncidentProducerWait, p.wait_limit)) {
+            if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, abort_flag, p.status,
+                                   kIncidentProducerWait, p.wait_limit)) {
               alive = false;
               break;
             }
@@ -259,25 +257,17 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
               prof_wait += pt1 - pt0;
               ++prof_iters;
             }
-            if (lead) {
-              uint8_t* st = stage_base + stage * stage_stride;
-              if (rank == 0) mbar_arrive_expect_tx(&full_bar[stage], pair_tx);
-              const uint32_t bar = full0 + stage * 8;
-              const int c0 = cb * kKB;
-              if (p.lowc) {
-                tma_load_4d_pair(st, &tmA, bar, 0, 0, h_base + r * p.dil_h, img);
-              } else {
-                tma_load_im2col_4d_pair(st, &tmA, bar, c0, w_base, h_base, img, static_cast<uint16_t>(s_ * p.dil_w),
-                                        static_cast<uint16_t>(r * p.dil_h));
-              }
-              if (p.b_mn) {   // filter with K contiguous: two boxes of 64 filters x 64 channels
-                tma_load_3d_pair(st + kABytes, &tmB, bar, b_row0, c0, 0);
-                tma_load_3d_pair(st + kABytes + kMnBoxBytes, &tmB, bar, b_row0 + int(kMnBoxElems), c0, 0);
-              } else if (!b_resident) {
-                tma_load_3d_pair(st + kABytes, &tmB, bar, c0, r * p.S + s_, b_row0);
-              }
+            uint8_t* st = stage_base + stage * stage_stride;
+            if (rank == 0) mbar_arrive_expect_tx(&full_bar[stage], pair_tx);
+            const uint32_t bar = full0 + stage * 8;
+            const int c0 = cb * kKB;
+            if (p.lowc) {
+              tma_load_4d_pair(st, &tmA, bar, 0, 0, h_base + r * p.dil_h, img);
+            } else {
+              tma_load_im2col_4d_pair(st, &tmA, bar, c0, w_base, h_base, img, static_cast<uint16_t>(s_ * p.dil_w),
+                                      static_cast<uint16_t>(r * p.dil_h));
             }
-            __syncwarp();
+            if (!b_resident) tma_load_3d_pair(st + kABytes, &tmB, bar, c0, r * p.S + s_, b_row0);
             if constexpr (kProf) prof_issue += clock64() - pt1;
             if (++stage == uint32_t(n_stages)) {
               stage = 0;
@@ -294,7 +284,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         };
         if (p.prof == nullptr) copy_steps(std::false_type{}); else copy_steps(std::true_type{});
       }
-      if (p.prof && blockIdx.x == 0 && lead) {
+      if (p.prof && blockIdx.x == 0) {
         p.prof[0] = prof_wait; p.prof[1] = prof_issue; p.prof[2] = clock64() - prof_t0; p.prof[3] = prof_iters;
       }
       if (!alive || *abort_flag) {
@@ -306,28 +296,28 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------- issuer (leader only)
-    if (rank == 0) {
-      const bool lead = elect_one();
+    if (rank == 0 && lane == 0) {
       uint32_t stage = 0, phase = 0;
       uint32_t tcount = 0;
       bool alive = true;
       long long prof_wfull = 0, prof_wtmem = 0, prof_t0 = p.prof ? clock64() : 0;
       if (b_resident && pair_id < total_tiles) {
-        alive = mbar_wait_warp(bres_bar, 0u, abort_flag, p.status, kIncidentMmaWaitFull, p.wait_limit);
+        alive = mbar_wait_bounded(bres_bar, 0u, abort_flag, p.status, kIncidentMmaWaitFull, p.wait_limit);
       }
       const uint32_t empty_own = smem_u32(&empty_bar[0]);
       const uint32_t empty_peer = map_to_cta(empty_own, 1);
       const uint32_t tfull_own = smem_u32(&tmem_full[0]);
       const uint32_t tfull_peer = map_to_cta(tfull_own, 1);
       const uint32_t raw_empty_peer = map_to_cta(smem_u32(&raw_empty[0]), 1);
-      const uint32_t ring = smem_u32(stage_base), b_res0 = smem_u32(b_res);
+      const int k16 = p.k16_per_step;  // 16-element reduction slices per step that hold data (4, or 3)
       TileWalk walk;
       walk_init(walk, split, pair_id, num_pairs, total_tiles, k_iters, p.sk_min_frag);
       for (; alive && walk_next(walk); ++tcount) {
         const uint32_t buf = tcount & 1u;
         const uint32_t bphase = (tcount >> 1) & 1u;
         const long long mt0 = p.prof ? clock64() : 0;
-        if (!mbar_wait_warp(&tmem_empty[buf], bphase ^ 1u, abort_flag, p.status, kIncidentMmaWaitTmem, p.wait_limit)) {
+        if (!mbar_wait_bounded(&tmem_empty[buf], bphase ^ 1u, abort_flag, p.status,
+                               kIncidentMmaWaitTmem, p.wait_limit)) {
           alive = false;
           break;
         }
@@ -336,53 +326,51 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         const uint32_t d_tmem = tmem_base + buf * kPairN;
         // The reduction loop is the hot path of every layer and is sensitive to anything beside the wait, the
         // MMAs and the commits (a conditional barrier arrive in it cost 17 % on the 3x3 256-channel layer):
-        // it exists once with four MMAs per step, once with three (the 3-channel mode, 48 of a window's 64 elements
-        // hold data) and once for filters read MN-major.
-        auto reduce = [&](auto count_tag, auto mn_tag, auto prof_tag) {
-          constexpr int kCount = decltype(count_tag)::value;
-          constexpr bool kMn = decltype(mn_tag)::value;
+        // it exists once with four MMAs per step and once with a runtime count for the 3-channel mode.
+        auto reduce = [&](auto four_tag, auto prof_tag) {
+          constexpr bool kFour = decltype(four_tag)::value;
           constexpr bool kProf = decltype(prof_tag)::value;
           for (int kit = walk.kb; kit < walk.ke; ++kit) {
             long long mt1 = 0;
             if constexpr (kProf) mt1 = clock64();
-            if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, kIncidentMmaWaitFull, p.wait_limit)) {
+            if (!mbar_wait_bounded(&full_bar[stage], phase, abort_flag, p.status, kIncidentMmaWaitFull, p.wait_limit)) {
               alive = false;
               break;
             }
             if constexpr (kProf) prof_wfull += clock64() - mt1;
             tc_fence_after();
-            if (lead) {
-              const uint32_t st = ring + stage * stage_stride;
-              const uint32_t bt = b_resident ? b_res0 + kit * kBBytes : st + kABytes;
-              const uint64_t a0 = make_sw128_kmajor_desc(st);
-              const uint64_t b0 = kMn ? make_sw128_mnmajor_desc(bt) : make_sw128_kmajor_desc(bt);
+            const uint32_t st = smem_u32(stage_base + stage * stage_stride);
+            const uint32_t bt = b_resident ? smem_u32(b_res + kit * kBBytes) : st + kABytes;
+            if constexpr (kFour) {
 #pragma unroll
-              for (int k = 0; k < kCount; ++k)
-                mma_f16_pair(d_tmem, a0 + uint64_t(2 * k), b0 + uint64_t(k * (kMn ? int(kMnStepBytes / 16) : 2)),
-                             kMn ? (kIdesc | kIdescBMnMajor) : kIdesc, (kit > walk.kb || k > 0) ? 1u : 0u);
-              tc_commit_pair(empty_own + stage * 8);
-              tc_commit_pair(empty_peer + stage * 8);
+              for (int k = 0; k < kKB / 16; ++k) {
+                const uint64_t a = make_sw128_kmajor_desc(st + k * 32);
+                const uint64_t b = make_sw128_kmajor_desc(bt + k * 32);
+                mma_f16_pair(d_tmem, a, b, kIdesc, (kit > walk.kb || k > 0) ? 1u : 0u);
+              }
+            } else {
+              for (int k = 0; k < k16; ++k) {
+                const uint64_t a = make_sw128_kmajor_desc(st + k * 32);
+                const uint64_t b = make_sw128_kmajor_desc(bt + k * 32);
+                mma_f16_pair(d_tmem, a, b, kIdesc, (kit > walk.kb || k > 0) ? 1u : 0u);
+              }
             }
-            __syncwarp();
+            tc_commit_pair(empty_own + stage * 8);
+            tc_commit_pair(empty_peer + stage * 8);
             if (++stage == uint32_t(n_stages)) {
               stage = 0;
               phase ^= 1u;
             }
           }
         };
-        using Three = std::integral_constant<int, 3>;
-        using Four = std::integral_constant<int, kKB / 16>;
-        if (p.k16_per_step == 3) {
-          if (p.prof == nullptr) reduce(Three{}, std::false_type{}, std::false_type{});
-          else reduce(Three{}, std::false_type{}, std::true_type{});
-        } else if (p.b_mn) {
-          reduce(Four{}, std::true_type{}, std::false_type{});
+        if (k16 != kKB / 16) {
+          reduce(std::false_type{}, std::false_type{});
         } else if (p.prof == nullptr) {
-          reduce(Four{}, std::false_type{}, std::false_type{});
+          reduce(std::true_type{}, std::false_type{});
         } else {
-          reduce(Four{}, std::false_type{}, std::true_type{});   // cycle counters of the role (development aid)
+          reduce(std::true_type{}, std::true_type{});   // cycle counters of the role (development aid)
         }
-        if (alive && lead) {
+        if (alive) {
           tc_commit_pair(tfull_own + buf * 8);
           tc_commit_pair(tfull_peer + buf * 8);
           if (p.fused3) {
@@ -393,10 +381,10 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           }
         }
       }
-      if (p.prof && blockIdx.x == 0 && lead) {
+      if (p.prof && blockIdx.x == 0) {
         p.prof[4] = prof_wfull; p.prof[5] = prof_wtmem; p.prof[6] = clock64() - prof_t0; p.prof[7] = tcount;
       }
-      if (lead && (!alive || *abort_flag)) {
+      if (!alive || *abort_flag) {
         volatile uint32_t never = 0;
         tc_commit_pair(smem_u32(drain_bar));
         mbar_wait_bounded(drain_bar, 0u, &never, p.status, kIncidentDrainWait, kWaitLimitCycles / 16);
