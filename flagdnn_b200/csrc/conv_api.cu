@@ -257,6 +257,38 @@ LowChannel low_channel_geometry(const fdnn_conv_desc* d, int oh, int ow, const v
   return g;
 }
 
+// Window mode for other layers of fewer than 8 channels (a stem on NCHW tensors, or with an output width that is no
+// multiple of four): one GEMM row is one output pixel, its operand for a filter row the S x 8 stored values its taps
+// read, 16 * S contiguous bytes of the input relaid out as [N][H][w_pad][8] with the padding stored.  Windows of
+// neighbouring pixels overlap (a tiled map whose window stride is smaller than its length), the packed filter
+// [K, R, S, 8] is read as [K, R, S * 8], and a reduction takes R steps instead of R * S copies of 16-byte rows, each of
+// which costs the TMA unit as much as a 128-byte one (12 x 170 x 170 x 3 -> 32, 7x7 stride 2, NCHW bf16: 155 us).
+// Elements past S * 8 are out of the map's bounds and arrive as zeros.
+struct PixelWindows {
+  bool ok;
+  int ohs, rows_per_tile, tiles_per_image, w_pad;
+  long long scratch;
+};
+PixelWindows pixel_windows(const fdnn_conv_desc* d, int oh, int ow) {
+  PixelWindows g = {};
+  if (elem_size(d->dtype) != 2 || d->groups != 1 || d->c >= 8 || d->dil_w != 1 || d->s < 3 || d->s > 8) return g;
+  if (oh < 1 || ow < 1 || ow > 128 || d->stride_h > 8 || d->pad_top > 127 || (d->algo & FDNN_ALGO_FLAG_OUT_F32) != 0) return g;
+  g.ohs = 128 / ow;
+  if (g.ohs > oh) g.ohs = oh;
+  if (g.ohs * d->stride_h > 256) g.ohs = 256 / d->stride_h;
+  g.rows_per_tile = g.ohs * ow;
+  g.tiles_per_image = (oh + g.ohs - 1) / g.ohs;
+  if ((long long)d->n * g.tiles_per_image * 128 > 2000000000LL || (long long)d->n * d->h > 2000000000LL) return g;
+  const int need = d->stride_w * (ow - 1) + 8;
+  g.w_pad = need > d->pad_left + d->w ? need : d->pad_left + d->w;
+  g.scratch = (long long)d->n * d->h * g.w_pad * 16;
+  // half-empty tiles (few pixels per image, or rows just over 64 pixels) still take R steps instead of R * S; a call
+  // that fits the built-in scratch the other way keeps fitting it
+  const long long tight = (long long)d->n * d->h * d->w * 16;
+  g.ok = g.rows_per_tile * d->s >= 128 * 2 && !(g.scratch > FDNN_STATIC_SCRATCH_BYTES && tight <= FDNN_STATIC_SCRATCH_BYTES);
+  return g;
+}
+
 // Output-pixel grouping for narrow layers.  An MMA of 128 rows occupies the tensor
 // pipe for the same time whatever its column count, so a layer with K <= 128
 // output channels uses at most K/256 of the machine.  Grouping Q neighbouring
@@ -605,6 +637,21 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
   plan->grid = int(tiles < sms ? tiles : sms);
   plan->block = igemm_threads();
   plan->launches = 1 + plan->x_repacked;
+
+  if (plan->x_repacked && algo == FDNN_ALGO_IGEMM) {
+    const PixelWindows pw = pixel_windows(d, oh, ow);
+    if (pw.ok) {
+      const long long window_tiles = (long long)d->n * pw.tiles_per_image;
+      plan->workspace_bytes = pw.scratch;
+      plan->tile_n = choose_tile_n(d->dtype, int(window_tiles), d->k, sms);
+      if (forced_tile_n(d) != 0) plan->tile_n = forced_tile_n(d);
+      plan->stages = igemm_stages(d->dtype, plan->tile_n);
+      plan->smem_bytes = igemm_smem_bytes(d->dtype, plan->tile_n);
+      const long long all = window_tiles * ((d->k + plan->tile_n - 1) / plan->tile_n);
+      plan->grid = int(all < sms ? all : sms);
+      return FDNN_OK;
+    }
+  }
 
   // CTA pairs: 16-bit types writing a dense NHWC y.  Worth it when the layer is
   // wide enough for 256-channel tiles and has at least one full wave of pairs.
@@ -1541,7 +1588,15 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   const int k_group = d.k / groups;
   int a_c = d.c / groups;
   long long a_plane = 0;
-  if (plan.x_repacked) {
+  PixelWindows windows = {};
+  if (plan.algo == FDNN_ALGO_IGEMM && plan.x_repacked && plan.w_packed && residual == nullptr && batch == nullptr)
+    windows = pixel_windows(&d, plan.oh, plan.ow);
+  if (windows.ok) {
+    e = launch_repack_x_windows(x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w, d.pad_left,
+                                windows.w_pad, workspace, stream);
+    if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
+    a_base = workspace;
+  } else if (plan.x_repacked) {
     const int x_pad = batch != nullptr ? d.c : padded_x_channels(&d);   // groups side by side, 16-byte multiples each
     a_plane = (long long)d.n * d.h * d.w * x_pad;
     e = launch_repack_x(d.dtype, x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w,
@@ -1568,7 +1623,15 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   }
 
   alignas(64) CUtensorMap tmA, tmA2, tmB, tmB2;
-  st = encode_activation_map(&tmA, d.dtype, a_base, a_c, d.w, d.h, d.n, a_sw, a_sh, a_sn, &d, groups);
+  if (windows.ok) {
+    cuuint64_t dims[4] = {cuuint64_t(d.s) * 8, cuuint64_t(plan.ow), cuuint64_t(d.h), cuuint64_t(d.n)};
+    cuuint64_t strides[3] = {cuuint64_t(d.stride_w) * 16, cuuint64_t(windows.w_pad) * 16, cuuint64_t(d.h) * windows.w_pad * 16};
+    cuuint32_t box[4] = {64, cuuint32_t(plan.ow), cuuint32_t(windows.ohs * d.stride_h), 1};
+    cuuint32_t estr[4] = {1, 1, cuuint32_t(d.stride_h), 1};
+    st = encode_tiled(&tmA, d.dtype, a_base, 4, dims, strides, box, estr, "pixel windows");
+  } else {
+    st = encode_activation_map(&tmA, d.dtype, a_base, a_c, d.w, d.h, d.n, a_sw, a_sh, a_sn, &d, groups);
+  }
   if (st != FDNN_OK) return st;
   const int b_box_rows = plan.algo == FDNN_ALGO_IGEMM_PAIR ? 128 : plan.tile_n;  // each CTA of a pair stages half
   if (b_mn) {
@@ -1577,6 +1640,8 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     cuuint32_t box[3] = {64, 64, 1};   // kMnBoxElems filters x one reduction step
     cuuint32_t estr[3] = {1, 1, 1};
     st = encode_tiled(&tmB, d.dtype, b_base, 3, dims, strides, box, estr, "filter, K contiguous");
+  } else if (windows.ok) {
+    st = encode_filter_map(&tmB, d.dtype, b_base, d.s * 8, d.r, d.k, (long long)d.s * 8, b_sk, b_box_rows);
   } else {
     st = encode_filter_map(&tmB, d.dtype, b_base, b_c, d.r * d.s, d.k, b_stap, b_sk, b_box_rows);
   }
@@ -1607,6 +1672,16 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   p.R = d.r; p.S = d.s;
   p.c_blocks = (c_pad + plan.tile_k - 1) / plan.tile_k;
   p.m_tiles = (p.M + 127) / 128;
+  if (windows.ok) {
+    p.lowc = 1;
+    p.S = 1;
+    p.c_blocks = 1;
+    p.rows_per_tile = windows.rows_per_tile;
+    p.tiles_per_image = windows.tiles_per_image;
+    p.ohs = windows.ohs;
+    p.a_tx_bytes = windows.rows_per_tile * 128;
+    p.m_tiles = d.n * windows.tiles_per_image;
+  }
   p.group_n_tiles = (k_group + plan.tile_n - 1) / plan.tile_n;
   p.n_tiles = groups * p.group_n_tiles;
   if (batch != nullptr) {
@@ -1632,7 +1707,20 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   {
     const long long row = out_f32 ? 0 : y_pixel_stride(&d, plan.oh, plan.ow);
     if (row > 0 && (reinterpret_cast<uintptr_t>(y) & 15u) == 0) {
-      st = encode_output_map(&tmY, d.dtype, y, k_group, p.M, row, groups);
+      if (windows.ok) {
+        // (channel, pixel of the image, image), and the box of a tile's last rows in the unused slot of the fp32 map
+        cuuint64_t dims[3] = {cuuint64_t(d.k), cuuint64_t(plan.oh) * plan.ow, cuuint64_t(d.n)};
+        cuuint64_t strides[2] = {cuuint64_t(row) * es, cuuint64_t(row) * es * plan.oh * plan.ow};
+        cuuint32_t estr[3] = {1, 1, 1};
+        cuuint32_t box[3] = {64, 32, 1};
+        st = encode_tiled(&tmY, d.dtype, y, 3, dims, strides, box, estr, "window output");
+        if (st != FDNN_OK) return st;
+        const int tail = windows.rows_per_tile % 32;
+        box[1] = cuuint32_t(tail > 0 ? tail : 32);
+        st = encode_tiled(&tmA2, d.dtype, y, 3, dims, strides, box, estr, "window output tail");
+      } else {
+        st = encode_output_map(&tmY, d.dtype, y, k_group, p.M, row, groups);
+      }
       if (st != FDNN_OK) return st;
       p.tma_store = 1;
       p.y_row = row;
@@ -1640,7 +1728,11 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
       tmY = tmA;
     }
   }
-  if (!p.tma_store && !out_f32) choose_strided_store(d, plan.oh, plan.ow, y, &p);
+  if (!p.tma_store && !out_f32) {
+    choose_strided_store(d, plan.oh, plan.ow, y, &p);
+    // a tile of windows starts at a row of the image, so that units along pixels have to divide rows as well
+    while (windows.ok && p.y_mode == 1 && p.y_unit > es && plan.ow * es % p.y_unit != 0) p.y_unit /= 2;
+  }
   alignas(64) CUtensorMap tmR = tmY;
   alignas(64) CUtensorMap tmRbox = tmY;
   if (residual != nullptr && p.tma_store) {

@@ -443,8 +443,25 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         staged_n_tile = n_tile;
       }
 
-      const int m = m_tile * kBM + ew * 32 + lane;
-      const bool row_ok = m < p.M;
+      // Where this warp's 32 rows go in y seen as (channel, row, image): outside the window modes the whole output is one
+      // "image" (or, with several groups, the third dimension is the group)
+      int st_row, st_img, st_rows, m, m_end;
+      if (p.lowc) {
+        st_img = m_tile / p.tiles_per_image;
+        st_row = (m_tile - st_img * p.tiles_per_image) * p.rows_per_tile + ew * 32;
+        st_rows = p.rows_per_tile - ew * 32;
+        m = st_img * ohw + st_row;
+        m_end = m + (st_rows < ohw - st_row ? st_rows : ohw - st_row);   // a tile never crosses an image
+      } else {
+        st_img = group;
+        st_row = m_tile * kBM + ew * 32;
+        st_rows = 32;
+        m = st_row;
+        m_end = p.M;
+      }
+      const int m0 = m;
+      m += lane;
+      const bool row_ok = !(DENSE && p.lowc) && m < m_end;   // per-lane addresses: not needed for quads
       long long y_off = 0;
       if (row_ok) {
         const int img = m / ohw;
@@ -461,18 +478,6 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       tc_fence_after();
 
       const uint32_t t_row = tmem_base + (uint32_t(ew * 32) << 16) + buf * BN + chalf * WC;
-      // Where this warp's 32 rows go in y seen as (channel, row, image): the whole
-      // output is one "image" outside low-channel mode.
-      int st_row, st_img, st_rows;
-      if (p.lowc) {
-        st_img = m_tile / p.tiles_per_image;
-        st_row = (m_tile - st_img * p.tiles_per_image) * p.rows_per_tile + ew * 32;
-        st_rows = p.rows_per_tile - ew * 32;
-      } else {
-        st_img = group;   // the output map's third dimension: the group's channels
-        st_row = m_tile * kBM + ew * 32;
-        st_rows = 32;
-      }
       if constexpr (DENSE) {
         // a tile's last warp may own fewer than 32 valid rows: tmA2 then holds a second
         // output map whose box is exactly that short (low-channel mode, 16-bit only)
@@ -487,7 +492,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         so.y_off = y_off;
         so.sn = p.y_sn; so.sk = p.y_sk;
         so.mode = p.y_mode; so.unit = p.y_unit;
-        so.m0 = m_tile * kBM + ew * 32; so.M = p.M; so.ohw = ohw;
+        so.m0 = m0; so.M = m_end; so.ohw = ohw;
         so.row_ok = row_ok;
         epilogue_store_strided<T, WC, RES>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
                                            out_stage + (warp - kFirstEpiWarp) * 2 * 32 * kRowBytes, lane, so, store_seq);

@@ -162,6 +162,9 @@ cudaError_t launch_repack_x(int dtype, const void* x, const long long x_s[4], in
 // x -> [N][H][w_pad][4]: `pad_left` zero pixels, the image row, zeros up to w_pad; channel 4 is zero.
 cudaError_t launch_repack_x_lowc(int dtype, const void* x, const long long x_s[4], int N, int C, int H,
                                  int W, int pad_left, int w_pad, void* dst, cudaStream_t stream);
+// x of fewer than 8 channels (16-bit) -> [N][H][w_pad][8], padded with zero pixels left and right.
+cudaError_t launch_repack_x_windows(const void* x, const long long x_s[4], int N, int C, int H, int W, int pad_left,
+                                    int w_pad, void* dst, cudaStream_t stream);
 // w -> [4*K][R][64]: row (q, k) holds filter k shifted to the q-th output pixel of a quad: with `chans`
 // stored channels per pixel (4, or 3 for the fused 3-channel mode), element
 // shift_elems + chans * (stride_w * q + t) + c of tap row r is w[k][c][r][t]; everything else is zero.

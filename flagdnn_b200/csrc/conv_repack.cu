@@ -321,6 +321,27 @@ repack_x_lowc_c3_kernel(const uint16_t* __restrict__ x, long long sn, long long 
   }
 }
 
+// Few-channel input relayout for pixel windows: [N][H][w_pad][8], `pad_left` zero pixels, the image row, zeros to the end;
+// channels beyond C are zero.  One lane per stored pixel: 16-byte stores, reads coalesced along W (NCHW) or C * W (NHWC).
+__global__ void __launch_bounds__(256)
+repack_x_windows_kernel(const uint16_t* __restrict__ x, long long sn, long long sc, long long sh, long long sw, unsigned rows,
+                        int C, int H, int W, int pad_left, int w_pad, uint4* __restrict__ dst) {
+  const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= unsigned(w_pad)) return;
+  const int w = int(j) - pad_left;
+  for (unsigned row = blockIdx.y; row < rows; row += gridDim.y) {
+    uint32_t v[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+    if (w >= 0 && w < W) {
+      const unsigned n = row / unsigned(H), h = row - n * unsigned(H);
+      const uint16_t* src = x + n * sn + h * sh + w * sw;
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (c < C) v[c] = __ldg(src + c * sc);
+    }
+    dst[(long long)row * w_pad + j] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 pack_w_lowc_kernel(const T* __restrict__ w, long long sk, long long sc, long long sr, long long ss, int K,
@@ -483,6 +504,16 @@ cudaError_t launch_repack_x_lowc(int dtype, const void* x, const long long x_s[4
   } else {
     return cudaErrorInvalidValue;
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_repack_x_windows(const void* x, const long long x_s[4], int N, int C, int H, int W, int pad_left,
+                                    int w_pad, void* dst, cudaStream_t stream) {
+  const int threads = w_pad >= 256 ? 256 : (w_pad + 31) / 32 * 32;
+  const long long rows = (long long)N * H;
+  const dim3 grid(unsigned((w_pad + threads - 1) / threads), unsigned(rows < 32768 ? rows : 32768));
+  repack_x_windows_kernel<<<grid, threads, 0, stream>>>(static_cast<const uint16_t*>(x), x_s[0], x_s[1], x_s[2], x_s[3],
+                                                        unsigned(rows), C, H, W, pad_left, w_pad, static_cast<uint4*>(dst));
   return cudaGetLastError();
 }
 
