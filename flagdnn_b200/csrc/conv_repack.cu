@@ -13,9 +13,31 @@
 #include <type_traits>
 
 #include "conv_internal.h"
+#include "sm100_ptx.cuh"
 
 namespace fdnn {
 namespace {
+
+// First statement of every kernel here: the next launch of the stream may be set up as soon as all blocks of this one
+// run, and nothing of this one touches memory before the launch in front of it is complete (programmatic dependent
+// launch, as in the tensor-core kernels: relayout and main kernel are a few microseconds each on small layers).
+__device__ __forceinline__ void chain_launches() {
+  griddep_launch_dependents();
+  griddep_wait();
+}
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = launch_overlap_enabled() ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // fp32 -> (hi, lo) with hi = x rounded to TF32 and lo = (x - hi) rounded to
 // TF32; hi + lo carries about 21 mantissa bits of x.
@@ -45,6 +67,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 repack_x_generic(const T* __restrict__ x, long long sn, long long sc, long long sh, long long sw,
                  int N, int C, int H, int W, int c_pad, T* __restrict__ dst, long long plane) {
+  chain_launches();
   const long long total = (long long)N * H * W * c_pad;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -74,6 +97,7 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 transpose_repack(const T* __restrict__ x, long long mat_stride, long long mat_stride2, int mats2, long long sc, int mats,
                  int C, int P, int c_pad, T* __restrict__ dst, long long plane) {
+  chain_launches();
   constexpr int kCh = 128 / int(sizeof(T));   // channels per tile: 64 or 32
   constexpr int kVec = 16 / int(sizeof(T));   // elements per 16 bytes
   __shared__ uint32_t tile[64][33];
@@ -182,6 +206,7 @@ template <typename T, int UNIT>
 __global__ void __launch_bounds__(256)
 repack_rows(const T* __restrict__ x, long long sw, long long pixels, int C, int c_pad, T* __restrict__ dst,
             long long plane) {
+  chain_launches();
   constexpr int kVec = 16 / int(sizeof(T));
   const unsigned vecs = unsigned(c_pad / kVec);
   const long long total = pixels * vecs;
@@ -241,6 +266,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 pack_w_kernel(const T* __restrict__ w, long long sk, long long sc, long long sr, long long ss, int K,
               int C, int R, int S, int c_pad, T* __restrict__ dst, long long plane) {
+  chain_launches();
   const long long total = (long long)K * R * S * c_pad;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -259,6 +285,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 repack_x_lowc_kernel(const T* __restrict__ x, long long sn, long long sc, long long sh, long long sw,
                      int N, int C, int H, int W, int pad_left, int w_pad, T* __restrict__ dst) {
+  chain_launches();
   const long long total = (long long)N * H * w_pad;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -285,6 +312,7 @@ repack_x_lowc_kernel(const T* __restrict__ x, long long sn, long long sc, long l
 __global__ void __launch_bounds__(256)
 repack_x_lowc_c3_kernel(const uint16_t* __restrict__ x, long long sn, long long sh, int N, int H, int W,
                         int pad_left, int w_pad, uint16_t* __restrict__ dst) {
+  chain_launches();
   const int w8s = W / 8;
   const long long total = (long long)N * H * w8s;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -326,6 +354,7 @@ repack_x_lowc_c3_kernel(const uint16_t* __restrict__ x, long long sn, long long 
 __global__ void __launch_bounds__(256)
 repack_x_windows_kernel(const uint16_t* __restrict__ x, long long sn, long long sc, long long sh, long long sw, unsigned rows,
                         int C, int H, int W, int pad_left, int w_pad, uint4* __restrict__ dst) {
+  chain_launches();
   const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= unsigned(w_pad)) return;
   const int w = int(j) - pad_left;
@@ -346,6 +375,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 pack_w_lowc_kernel(const T* __restrict__ w, long long sk, long long sc, long long sr, long long ss, int K,
                    int C, int R, int S, int stride_w, int chans, int shift_elems, T* __restrict__ dst) {
+  chain_launches();
   const long long total = 4LL * K * R * 64;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -368,6 +398,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 pack_w_grouped_kernel(const T* __restrict__ w, long long sk, long long sc, long long sr, long long ss, int K,
                       int C, int R, int S, int stride_w, int q, int c_pad, T* __restrict__ dst) {
+  chain_launches();
   const int sv = S + (q - 1) * stride_w;
   const long long total = (long long)q * K * R * sv * c_pad;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -402,9 +433,11 @@ cudaError_t transpose_t(const T* x, long long ms, long long ms2, int mats2, long
                    mult(mats2, ms2);
   const long long tiles = (long long)mats * ((P + 63) / 64) * ((c_pad + 128 / int(sizeof(T)) - 1) / (128 / int(sizeof(T))));
   if (vec)
-    transpose_repack<T, true><<<grid_for(tiles, 1), 256, 0, stream>>>(x, ms, ms2, mats2, sc, mats, C, P, c_pad, dst, plane);
+    launch_chained(transpose_repack<T, true>, dim3(grid_for(tiles, 1)), 256, stream,
+        x, ms, ms2, mats2, sc, mats, C, P, c_pad, dst, plane);
   else
-    transpose_repack<T, false><<<grid_for(tiles, 1), 256, 0, stream>>>(x, ms, ms2, mats2, sc, mats, C, P, c_pad, dst, plane);
+    launch_chained(transpose_repack<T, false>, dim3(grid_for(tiles, 1)), 256, stream,
+        x, ms, ms2, mats2, sc, mats, C, P, c_pad, dst, plane);
   return cudaGetLastError();
 }
 
@@ -414,10 +447,11 @@ cudaError_t rows_t(const T* x, long long sw, long long pixels, int C, int c_pad,
                    cudaStream_t stream) {
   const int grid = grid_for(pixels * (c_pad / (16 / int(sizeof(T)))), 256);
   const uintptr_t a = reinterpret_cast<uintptr_t>(x) | (pixels > 1 ? uintptr_t(sw) * sizeof(T) : uintptr_t(0));
-  if (a % 16 == 0) repack_rows<T, 16><<<grid, 256, 0, stream>>>(x, sw, pixels, C, c_pad, dst, plane);
-  else if (a % 8 == 0) repack_rows<T, 8><<<grid, 256, 0, stream>>>(x, sw, pixels, C, c_pad, dst, plane);
-  else if (a % 4 == 0) repack_rows<T, 4><<<grid, 256, 0, stream>>>(x, sw, pixels, C, c_pad, dst, plane);
-  else if constexpr (sizeof(T) == 2) repack_rows<T, 2><<<grid, 256, 0, stream>>>(x, sw, pixels, C, c_pad, dst, plane);
+  if (a % 16 == 0) launch_chained(repack_rows<T, 16>, dim3(grid), 256, stream, x, sw, pixels, C, c_pad, dst, plane);
+  else if (a % 8 == 0) launch_chained(repack_rows<T, 8>, dim3(grid), 256, stream, x, sw, pixels, C, c_pad, dst, plane);
+  else if (a % 4 == 0) launch_chained(repack_rows<T, 4>, dim3(grid), 256, stream, x, sw, pixels, C, c_pad, dst, plane);
+  else if constexpr (sizeof(T) == 2) launch_chained(repack_rows<T, 2>, dim3(grid), 256, stream,
+      x, sw, pixels, C, c_pad, dst, plane);
   else return cudaErrorInvalidValue;   // fp32 elements are 4-byte aligned
   return cudaGetLastError();
 }
@@ -448,7 +482,8 @@ cudaError_t repack_x_t(const void* x, const long long x_s[4], int N, int C, int 
     if (even) return rows_t<T>(src, sw, (long long)N * H * W, C, c_pad, out, plane, stream);
   }
   const long long total = (long long)N * H * W * c_pad;
-  repack_x_generic<T><<<grid_for(total, 256), 256, 0, stream>>>(src, s[0], s[1], s[2], s[3], N, C, H, W, c_pad, out, plane);
+  launch_chained(repack_x_generic<T>, dim3(grid_for(total, 256)), 256, stream,
+      src, s[0], s[1], s[2], s[3], N, C, H, W, c_pad, out, plane);
   return cudaGetLastError();
 }
 
@@ -462,7 +497,7 @@ cudaError_t pack_w_t(const void* w, const long long s[4], int K, int C, int R, i
   if (R * S == 1 && s[0] == 1 && K > 1 && s[1] != 1)
     return transpose_t<T>(src, 0, 0, 1, s[1], 1, C, K, c_pad, out, plane, stream);
   const long long total = (long long)K * R * S * c_pad;
-  pack_w_kernel<T><<<grid_for(total, 256), 256, 0, stream>>>(
+  launch_chained(pack_w_kernel<T>, dim3(grid_for(total, 256)), 256, stream,
       src, s[0], s[1], s[2], s[3], K, C, R, S, c_pad, out, plane);
   return cudaGetLastError();
 }
@@ -487,18 +522,18 @@ cudaError_t launch_repack_x_lowc(int dtype, const void* x, const long long x_s[4
                     (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
   if (fast) {
     const long long items = (long long)N * H * (W / 8);
-    repack_x_lowc_c3_kernel<<<grid_for(items, 256), 256, 0, stream>>>(
+    launch_chained(repack_x_lowc_c3_kernel, dim3(grid_for(items, 256)), 256, stream,
         static_cast<const uint16_t*>(x), x_s[0], x_s[2], N, H, W, pad_left, w_pad, static_cast<uint16_t*>(dst));
     return cudaGetLastError();
   }
   const long long total = (long long)N * H * w_pad;
   const int grid = grid_for(total, 256);
   if (dtype == FDNN_F16) {
-    repack_x_lowc_kernel<__half><<<grid, 256, 0, stream>>>(static_cast<const __half*>(x), x_s[0], x_s[1], x_s[2],
-                                                           x_s[3], N, C, H, W, pad_left, w_pad,
-                                                           static_cast<__half*>(dst));
+    launch_chained(repack_x_lowc_kernel<__half>, dim3(grid), 256, stream,
+        static_cast<const __half*>(x), x_s[0], x_s[1], x_s[2], x_s[3], N, C, H, W, pad_left, w_pad,
+        static_cast<__half*>(dst));
   } else if (dtype == FDNN_BF16) {
-    repack_x_lowc_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
+    launch_chained(repack_x_lowc_kernel<__nv_bfloat16>, dim3(grid), 256, stream,
         static_cast<const __nv_bfloat16*>(x), x_s[0], x_s[1], x_s[2], x_s[3], N, C, H, W, pad_left, w_pad,
         static_cast<__nv_bfloat16*>(dst));
   } else {
@@ -512,8 +547,9 @@ cudaError_t launch_repack_x_windows(const void* x, const long long x_s[4], int N
   const int threads = w_pad >= 256 ? 256 : (w_pad + 31) / 32 * 32;
   const long long rows = (long long)N * H;
   const dim3 grid(unsigned((w_pad + threads - 1) / threads), unsigned(rows < 32768 ? rows : 32768));
-  repack_x_windows_kernel<<<grid, threads, 0, stream>>>(static_cast<const uint16_t*>(x), x_s[0], x_s[1], x_s[2], x_s[3],
-                                                        unsigned(rows), C, H, W, pad_left, w_pad, static_cast<uint4*>(dst));
+  launch_chained(repack_x_windows_kernel, grid, threads, stream,
+      static_cast<const uint16_t*>(x), x_s[0], x_s[1], x_s[2], x_s[3], unsigned(rows), C, H, W, pad_left, w_pad,
+      static_cast<uint4*>(dst));
   return cudaGetLastError();
 }
 
@@ -522,12 +558,13 @@ cudaError_t launch_pack_w_lowc(int dtype, const void* w, const long long w_s[4],
   const long long total = 4LL * K * R * 64;
   const int grid = grid_for(total, 256);
   if (dtype == FDNN_F16) {
-    pack_w_lowc_kernel<__half><<<grid, 256, 0, stream>>>(static_cast<const __half*>(w), w_s[0], w_s[1], w_s[2],
-                                                         w_s[3], K, C, R, S, stride_w, chans, shift_elems, static_cast<__half*>(dst));
+    launch_chained(pack_w_lowc_kernel<__half>, dim3(grid), 256, stream,
+        static_cast<const __half*>(w), w_s[0], w_s[1], w_s[2], w_s[3], K, C, R, S, stride_w, chans, shift_elems,
+        static_cast<__half*>(dst));
   } else if (dtype == FDNN_BF16) {
-    pack_w_lowc_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(w), w_s[0], w_s[1], w_s[2], w_s[3], K, C, R, S, stride_w, chans, shift_elems,
-        static_cast<__nv_bfloat16*>(dst));
+    launch_chained(pack_w_lowc_kernel<__nv_bfloat16>, dim3(grid), 256, stream,
+        static_cast<const __nv_bfloat16*>(w), w_s[0], w_s[1], w_s[2], w_s[3], K, C, R, S, stride_w, chans,
+        shift_elems, static_cast<__nv_bfloat16*>(dst));
   } else {
     return cudaErrorInvalidValue;
   }
@@ -539,11 +576,11 @@ cudaError_t launch_pack_w_grouped(int dtype, const void* w, const long long w_s[
   const long long total = (long long)q * K * R * (S + (q - 1) * stride_w) * c_pad;
   const int grid = grid_for(total, 256);
   if (dtype == FDNN_F16) {
-    pack_w_grouped_kernel<__half><<<grid, 256, 0, stream>>>(static_cast<const __half*>(w), w_s[0], w_s[1],
-                                                            w_s[2], w_s[3], K, C, R, S, stride_w, q, c_pad,
-                                                            static_cast<__half*>(dst));
+    launch_chained(pack_w_grouped_kernel<__half>, dim3(grid), 256, stream,
+        static_cast<const __half*>(w), w_s[0], w_s[1], w_s[2], w_s[3], K, C, R, S, stride_w, q, c_pad,
+        static_cast<__half*>(dst));
   } else if (dtype == FDNN_BF16) {
-    pack_w_grouped_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
+    launch_chained(pack_w_grouped_kernel<__nv_bfloat16>, dim3(grid), 256, stream,
         static_cast<const __nv_bfloat16*>(w), w_s[0], w_s[1], w_s[2], w_s[3], K, C, R, S, stride_w, q, c_pad,
         static_cast<__nv_bfloat16*>(dst));
   } else {
@@ -558,6 +595,7 @@ cudaError_t launch_pack_w_grouped(int dtype, const void* w, const long long w_s[
 template <typename T>
 __global__ void densify_w_kernel(const T* __restrict__ w, long long s0, long long s1, long long s2, long long s3, int K,
                                  int C, int R, int S, int groups, T* __restrict__ dense) {
+  chain_launches();
   const long long total = (long long)K * R * S * C;
   const int cg = C / groups, kg = K / groups;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -581,8 +619,8 @@ cudaError_t densify_w_t(const void* w, const long long w_s[4], int K, int C, int
   long long blocks = (total + 255) / 256;
   if (blocks > 148LL * 16) blocks = 148LL * 16;
   if (blocks < 1) blocks = 1;
-  densify_w_kernel<T><<<int(blocks), 256, 0, stream>>>(static_cast<const T*>(w), w_s[0], w_s[1], w_s[2], w_s[3], K, C, R,
-                                                       S, groups, static_cast<T*>(dense));
+  launch_chained(densify_w_kernel<T>, dim3(int(blocks)), 256, stream,
+      static_cast<const T*>(w), w_s[0], w_s[1], w_s[2], w_s[3], K, C, R, S, groups, static_cast<T*>(dense));
   return cudaGetLastError();
 }
 
