@@ -168,6 +168,13 @@ bool y_is_dense_nhwc(const fdnn_conv_desc* d, int oh, int ow, const void* y) {
   return y_pixel_stride(d, oh, ow) > 0 && aligned16(y);
 }
 
+// The least scratch a relayout of x works with: rows of 16-byte multiples.  Callers that size their buffer so (it was the
+// only layout once) get that one instead of the line-sized rows or the window mode the plan asks scratch for.
+long long tight_x_bytes(const fdnn_conv_desc* d) {
+  const int es = elem_size(d->dtype);
+  return (long long)(d->dtype == FDNN_F32 ? 2 : 1) * d->n * d->h * d->w * round_up(d->c, 16 / es) * es;
+}
+
 // How the single-CTA kernel's epilogue writes a y that has no TMA map (see epilogue_store_strided): along channels
 // when they are contiguous, along pixels when every image's pixels are (NCHW), with the widest unit that every run's
 // start is a multiple of (and, along pixels, that no image boundary cuts); otherwise element by element.
@@ -1542,7 +1549,8 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   if (plan.w_packed && w_packed == nullptr)
     return fail(FDNN_BAD_PARAM, "this problem needs a packed filter (fdnn_conv2d_pack_weight); w_packed is NULL");
   if (plan.workspace_bytes > 0 && batch == nullptr) {
-    if (workspace == nullptr || workspace_bytes < plan.workspace_bytes)
+    const long long least = plan.x_repacked && !plan.low_channel ? tight_x_bytes(&d) : plan.workspace_bytes;
+    if (workspace == nullptr || workspace_bytes < (least < plan.workspace_bytes ? least : plan.workspace_bytes))
       return fail(FDNN_WORKSPACE_TOO_SMALL, "workspace smaller than plan.workspace_bytes");
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
       return fail(FDNN_BAD_PARAM, "workspace must be 256-byte aligned");
@@ -1591,13 +1599,16 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   PixelWindows windows = {};
   if (plan.algo == FDNN_ALGO_IGEMM && plan.x_repacked && plan.w_packed && residual == nullptr && batch == nullptr)
     windows = pixel_windows(&d, plan.oh, plan.ow);
+  if (windows.scratch > workspace_bytes) windows.ok = false;
   if (windows.ok) {
     e = launch_repack_x_windows(x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w, d.pad_left,
                                 windows.w_pad, workspace, stream);
     if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
     a_base = workspace;
   } else if (plan.x_repacked) {
-    const int x_pad = batch != nullptr ? d.c : padded_x_channels(&d);   // groups side by side, 16-byte multiples each
+    int x_pad = batch != nullptr ? d.c : padded_x_channels(&d);   // groups side by side, 16-byte multiples each
+    if (batch == nullptr && (long long)(d.dtype == FDNN_F32 ? 2 : 1) * d.n * d.h * d.w * x_pad * es > workspace_bytes)
+      x_pad = round_up(d.c, 16 / es);
     a_plane = (long long)d.n * d.h * d.w * x_pad;
     e = launch_repack_x(d.dtype, x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w,
                         x_pad, workspace, a_plane, stream);

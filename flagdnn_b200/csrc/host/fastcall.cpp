@@ -61,7 +61,8 @@ std::unordered_map<PlanKey, fdnn_conv_plan, PlanHash>& plans() {   // used with 
 const at::Tensor* plain(PyObject* o) {
   if (!THPVariable_CheckExact(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
-  if (!t.defined() || !t.is_cuda() || t.layout() != at::kStrided || t.is_conj() || t.is_neg()) return nullptr;
+  if (!t.defined() || !t.is_cuda() || t.layout() != at::kStrided || !t.has_storage() || t.is_conj() || t.is_neg())
+    return nullptr;   // (tensors without storage: wrappers of function transforms)
   return &t;
 }
 

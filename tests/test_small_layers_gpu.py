@@ -85,3 +85,38 @@ def test_small_layer_without_packed_filter_and_scratch(native_lib):
     nat.check(native_lib.fdnn_conv2d_fwd(ctypes.byref(d), x.data_ptr(), w.data_ptr(), None, None, None, nat.ACT_NONE,
                                          y.data_ptr(), None, 0, stream))
     _check(y, x, w, None, 1, 1, 1)
+
+
+@pytest.mark.parametrize("c, dtype, code", [(136, torch.bfloat16, nat.BF16), (3, torch.float16, nat.F16), (20, torch.float32, nat.F32)])
+def test_scratch_of_the_tightest_layout_is_enough(native_lib, c, dtype, code):
+    """The plan asks scratch for line-sized rows (or windows); rows of 16-byte multiples are still accepted, less is not."""
+    n, h, w_, k = 4, 40, 46, 64
+    x = torch.randn(n, c, h, w_, device="cuda").to(dtype)
+    w = (torch.randn(k, c, 3, 3, device="cuda") / (3 * c ** 0.5)).to(dtype)
+    y = torch.empty(n, k, h, w_, device="cuda", dtype=dtype)
+    d = nat.ConvDesc()
+    d.dtype, d.n, d.c, d.h, d.w, d.k, d.r, d.s = code, n, c, h, w_, k, 3, 3
+    d.stride_h = d.stride_w = d.dil_h = d.dil_w = d.groups = 1
+    d.pad_top = d.pad_bottom = d.pad_left = d.pad_right = 1
+    d.algo = nat.ALGO_IGEMM
+    for i in range(4):
+        d.x_strides[i], d.w_strides[i], d.y_strides[i] = x.stride(i), w.stride(i), y.stride(i)
+    plan = nat.ConvPlan()
+    nat.check(native_lib.fdnn_conv2d_query(ctypes.byref(d), x.data_ptr(), w.data_ptr(), y.data_ptr(), ctypes.byref(plan)))
+    stream = torch.cuda.current_stream().cuda_stream
+    packed = torch.empty(plan.packed_weight_bytes, dtype=torch.uint8, device="cuda")
+    nat.check(native_lib.fdnn_conv2d_pack_weight(ctypes.byref(d), w.data_ptr(), y.data_ptr(), packed.data_ptr(),
+                                                 packed.numel(), stream))
+    es = x.element_size()
+    tight = (2 if dtype == torch.float32 else 1) * n * h * w_ * -(-c * es // 16) * 16
+    assert tight < plan.workspace_bytes
+    for nbytes in (plan.workspace_bytes, tight):
+        ws = torch.full((nbytes + 256,), 0x55, dtype=torch.uint8, device="cuda")
+        y.zero_()
+        nat.check(native_lib.fdnn_conv2d_fwd(ctypes.byref(d), x.data_ptr(), w.data_ptr(), packed.data_ptr(), None, None,
+                                             nat.ACT_NONE, y.data_ptr(), ws.data_ptr(), nbytes, stream))
+        _check(y, x, w, None, 1, 1, 1)
+        assert (ws[nbytes:] == 0x55).all(), "scratch written past its end"
+    status = native_lib.fdnn_conv2d_fwd(ctypes.byref(d), x.data_ptr(), w.data_ptr(), packed.data_ptr(), None, None,
+                                        nat.ACT_NONE, y.data_ptr(), ws.data_ptr(), tight - 16, stream)
+    assert status == nat.FDNN_WORKSPACE_TOO_SMALL
