@@ -296,9 +296,10 @@ PixelWindows pixel_windows(const fdnn_conv_desc* d, int oh, int ow) {
   return g;
 }
 
-// Output-pixel grouping for narrow layers.  An MMA of 128 rows occupies the tensor
-// pipe for the same time whatever its column count, so a layer with K <= 128
-// output channels uses at most K/256 of the machine.  Grouping Q neighbouring
+// Output-pixel grouping for narrow layers.  A reduction step of a narrow tile brings
+// almost as many operand bytes as one of a wide tile (24 / 32 / 48 KB for 64 / 128 / 256
+// columns), and an MMA of 64 columns runs at two thirds of the full rate, so a layer with
+// K <= 128 output channels uses a fraction of the machine.  Grouping Q neighbouring
 // output pixels of a row into one GEMM row turns the layer into an equivalent
 // convolution with Q*K output channels, a filter widened to S + (Q-1)*stride_w
 // taps (zero where a pixel does not reach) and a W-stride of Q*stride_w.  Its y,
@@ -733,7 +734,9 @@ GroupBatch group_batch(const fdnn_conv_desc* d, const void* x, const void* w, co
     const long long nt = ((long long)q * d->k + plan.tile_n - 1) / plan.tile_n;
     const double whole = double((mt * nt * (plan.tile_m / 128) + sms - 1) / sms) * d->r * (d->s + (q - 1) * d->stride_w) *
                          ((d->c + 63) / 64) * (plan.tile_n + 384);
-    if (batch > 0.8 * whole) return g;
+    // groups whose channels do not start on 64-byte boundaries pay more per copy (86 x 21 x 21, 80 channels in two groups of
+    // 40: 22 us dense, 31 us in one launch at 0.73 of its cost)
+    if (batch > ((sub.c * elem_size(d->dtype)) % 64 == 0 ? 0.7 : 0.5) * whole) return g;
   }
   g.tile_n = bn;
   return g;

@@ -660,6 +660,83 @@ cudaError_t launch_rowvec(const DirectParams& p, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
+// ------------------------------------------- channels-last, any channel count and alignment
+// Channels-last tensors whose channels do not come in 16-byte pieces (C = 109, 617 ...): a thread owns one channel of
+// PW neighbouring output columns of a band of rows, neighbouring lanes neighbouring channels, so that every access is
+// one run of a warp's channels; the taps stay in registers over the band.  The plane kernel, which these layers took,
+// reads one element per cache line: 437 -> 41 us on 197 x 617 x 13 x 13 f16, 3x3 stride 2; 352 -> 78 us on
+// 123 x 109 x 60 x 60 bf16.  Bound by the number of two-byte accesses.
+template <typename T, int KR, int KS, int KSTRIDE>
+__global__ void __launch_bounds__(kDwThreads)
+depthwise_cl_scalar_kernel(const DirectParams p, const DwRowTiling g) {
+  constexpr int PW = 4;
+  constexpr int kSpan = (PW - 1) * KSTRIDE + KS;
+  const long long unit = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (unit >= g.units) return;
+  const int c = int(unit % p.C);
+  long long rest = unit / p.C;
+  const int ow0 = int(rest % g.owg) * PW;
+  rest /= g.owg;
+  const int band = int(rest % g.bands);
+  const int n = int(rest / g.bands);
+  const int oh_begin = band * g.band_rows, oh_end = min(p.OH, oh_begin + g.band_rows);
+  const int iw0 = ow0 * KSTRIDE - p.pad_left;
+  const T* w = static_cast<const T*>(p.w) + c * p.w_s[0];
+  float wt[KR * KS];
+#pragma unroll
+  for (int r = 0; r < KR; ++r)
+#pragma unroll
+    for (int s = 0; s < KS; ++s) wt[r * KS + s] = to_f32<T>(__ldg(w + r * p.w_s[2] + s * p.w_s[3]));
+  const float sc = p.scale != nullptr ? to_f32<T>(static_cast<const T*>(p.scale)[c]) : 1.0f;
+  const float bi = p.bias != nullptr ? to_f32<T>(static_cast<const T*>(p.bias)[c]) : 0.0f;
+  const T* x = static_cast<const T*>(p.x) + n * p.x_s[0] + c;
+  const long long y0 = n * p.y_s[0] + c;
+  for (int oh = oh_begin; oh < oh_end; ++oh) {
+    float acc[PW];
+#pragma unroll
+    for (int q = 0; q < PW; ++q) acc[q] = 0.0f;
+#pragma unroll
+    for (int r = 0; r < KR; ++r) {
+      const int ih = oh * KSTRIDE + r - p.pad_top;
+      if (ih < 0 || ih >= p.H) continue;
+      const T* row = x + ih * p.x_s[2];
+      float xv[kSpan];
+#pragma unroll
+      for (int j = 0; j < kSpan; ++j)
+        xv[j] = iw0 + j >= 0 && iw0 + j < p.W ? to_f32<T>(__ldg(row + (iw0 + j) * p.x_s[3])) : 0.0f;
+#pragma unroll
+      for (int j = 0; j < kSpan; ++j)
+#pragma unroll
+        for (int q = 0; q < PW; ++q) {
+          const int s = j - q * KSTRIDE;
+          if (s >= 0 && s < KS) acc[q] = fmaf(xv[j], wt[r * KS + s], acc[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < PW; ++q) {
+      if (ow0 + q >= p.OW) continue;
+      const long long at = y0 + oh * p.y_s[2] + (ow0 + q) * p.y_s[3];
+      float a = fmaf(acc[q], sc, bi);
+      if (p.residual != nullptr) a += to_f32<T>(static_cast<const T*>(p.residual)[at]);
+      static_cast<T*>(p.y)[at] = from_f32<T>(apply_activation(a, p.act));
+    }
+  }
+}
+
+template <typename T, int KR, int KS, int KSTRIDE>
+cudaError_t launch_cl_scalar(const DirectParams& p, cudaStream_t stream) {
+  DwRowTiling g;
+  g.owg = (p.OW + 3) / 4;
+  g.band_rows = 8;   // fewer where that leaves under half a wave of threads
+  while (g.band_rows > 1 && (long long)p.N * p.C * ((p.OH + g.band_rows - 1) / g.band_rows) * g.owg < 148LL * 1024)
+    g.band_rows /= 2;
+  g.bands = (p.OH + g.band_rows - 1) / g.band_rows;
+  g.units = (long long)p.N * p.C * g.bands * g.owg;
+  depthwise_cl_scalar_kernel<T, KR, KS, KSTRIDE>
+      <<<unsigned((g.units + kDwThreads - 1) / kDwThreads), kDwThreads, 0, stream>>>(p, g);
+  return cudaGetLastError();
+}
+
 // Launch of a channels-last kernel: V channels per thread, PW output columns per unit, at most `band_max` rows.
 // The grid is the blocks the device keeps resident (asked of the runtime once per kernel and shared-memory
 // size), so that a block fills its shared memory once and then walks units.
@@ -707,6 +784,7 @@ cudaError_t go_static(const DirectParams& p, int kind, cudaStream_t stream) {
     if (kind == 3) return launch_rowvec<T, KR, KS, KSTRIDE, 16>(p, stream);
     if (kind == 4) return launch_rowvec<T, KR, KS, KSTRIDE, 8>(p, stream);
     if (kind == 7) return launch_planes<T, KR, KS, KSTRIDE>(p, stream);
+    if (kind == 8) return launch_cl_scalar<T, KR, KS, KSTRIDE>(p, stream);
     if constexpr (sizeof(T) == 2) {
       if (kind == 5) return launch_rowvec<T, KR, KS, KSTRIDE, 4>(p, stream);
     }
@@ -737,7 +815,7 @@ cudaError_t go(const DirectParams& p, int channels_last, cudaStream_t stream) { 
 
 // 0: not a case for these kernels (the caller uses the direct kernel); 1: channels-last kernel; 2: plane kernel;
 // 3 / 4 / 5: row-vector kernel (NCHW) on 16- / 8- / 4-byte vectors; 6: a case of kernel 1 that the staged kernel
-// (conv_depthwise_tma.cu) takes; 7: several dense planes per block.
+// (conv_depthwise_tma.cu) takes; 7: several dense planes per block; 8: channels-last, channel by channel.
 int depthwise_kind(int dtype, const DirectParams& p) {
   if (p.groups != p.C || p.K != p.C || p.C < 1) return 0;
   if (dtype != FDNN_F16 && dtype != FDNN_BF16 && dtype != FDNN_F32) return 0;
@@ -756,6 +834,9 @@ int depthwise_kind(int dtype, const DirectParams& p) {
   // on the widest vectors the rows are aligned for (16 bytes; 8 for rows of 28 16-bit values; 4 for rows of 14)
   const bool unrolled = p.dil_h == 1 && p.dil_w == 1 && p.stride_h == p.stride_w && p.R == p.S &&
                         (p.R == 3 || p.R == 5) && (p.stride_w == 1 || p.stride_w == 2);
+  if (unrolled && p.C >= 8 && p.x_s[1] == 1 && p.y_s[1] == 1 && p.x_s[3] != 1 &&
+      (long long)p.N * p.C * p.OH * ((p.OW + 3) / 4) < 2147483647LL * 128)
+    return 8;
   if (unrolled && p.pad_left == p.S / 2 && p.x_s[3] == 1 && p.y_s[3] == 1) {
     for (int vb = 16; vb >= 4; vb /= 2) {
       const int vv = vb / es;

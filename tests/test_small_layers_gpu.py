@@ -49,7 +49,7 @@ def test_small_layers_match_fp64(fd, case, dtype, layout):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("case", [(1, 64, 7, 7, 3, 1), (3, 104, 9, 17, 3, 1), (2, 64, 8, 8, 3, 2), (5, 200, 13, 5, 3, 2),
                                   (2, 96, 11, 10, 5, 1), (3, 64, 15, 9, 5, 2), (2, 130, 1, 1, 3, 1), (300, 128, 3, 2, 3, 1),
-                                  (2, 7, 33, 31, 3, 1), (1, 50, 111, 109, 3, 1), (40, 99, 7, 5, 5, 2)])
+                                  (2, 7, 33, 31, 3, 1), (3, 109, 14, 15, 3, 2), (2, 37, 9, 8, 5, 1), (1, 50, 111, 109, 3, 1), (40, 99, 7, 5, 5, 2)])
 def test_depthwise_tiles_match_fp64(fd, case, dtype, layout):
     n, c, h, w, r, stride = case
     g = torch.Generator().manual_seed(c + h)
