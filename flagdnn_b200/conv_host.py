@@ -213,16 +213,23 @@ def _plan_for(input, weight, out, stride, padding4, dilation, groups, algo):
     return d, plan
 
 
-def _packed_weight(weight: torch.Tensor, d: nat.ConvDesc, plan: nat.ConvPlan, stream: int, y_ptr: int) -> torch.Tensor:
-    version = int(getattr(weight, "_version", 0))
-    # the packed layout depends on the plan: generic [K,R,S,Cpad] or the low-channel quad layout
+def _packed_layout(d: nat.ConvDesc, plan: nat.ConvPlan) -> tuple:
+    """What a packed filter of this call holds, beside the filter's own values and shape: the geometry of the plan
+    (generic [K,R,S,Cpad], pixel-grouped or low-channel quads) and the group count.  A filter [K,C/G,R,S] serves
+    layers of any G that divides K, and what is packed for it depends on G: a block-diagonal dense filter has G * C/G
+    channels, padded to the same c_padded for several G."""
     if plan.pixel_group > 1:
         layout = ("grouped", plan.pixel_group, d.stride_w)
     elif plan.low_channel:
-        layout = ("lowc", plan.low_channel, d.stride_w)
+        layout = ("lowc", plan.low_channel, d.stride_w, d.pad_left)
     else:
-        layout = ("krsc", plan.c_padded)
-    key = (layout, id(weight), weight.data_ptr(), tuple(weight.shape), tuple(weight.stride()),
+        layout = ("krsc",)
+    return layout + (plan.c_padded, d.groups, plan.packed_weight_bytes)
+
+
+def _packed_weight(weight: torch.Tensor, d: nat.ConvDesc, plan: nat.ConvPlan, stream: int, y_ptr: int) -> torch.Tensor:
+    version = int(getattr(weight, "_version", 0))
+    key = (_packed_layout(d, plan), id(weight), weight.data_ptr(), tuple(weight.shape), tuple(weight.stride()),
            str(weight.dtype), weight.device.type, weight.device.index, version)
     entry = _PACKED_WEIGHT_CACHE.get(key)
     if entry is not None:
