@@ -18,6 +18,7 @@
 
 #include "conv_convert.cuh"
 #include "conv_internal.h"
+#include "pool_stretch.h"
 
 namespace fdnn {
 namespace {
@@ -251,7 +252,8 @@ adaptive_avg_pool2d_nhwc8_split_kernel(const PoolParams p) {
   const long long total = (long long)p.N * p.OH * p.OW * c8;
   const long long i = blockIdx.x * 32LL + lane;
   float sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int n = 0, oh = 0, ow = 0, cv = 0, count = 1;
+  int n = 0, oh = 0, ow = 0, cv = 0;
+  long long count = 1;                 // a window can have more pixels than an int counts
   if (i < total) {
     long long t = i;
     cv = int(t % c8); t /= c8;
@@ -261,11 +263,17 @@ adaptive_avg_pool2d_nhwc8_split_kernel(const PoolParams p) {
     const int h0 = win_start(oh, p.H, p.OH), h1 = win_end(oh, p.H, p.OH);
     const int w0 = win_start(ow, p.W, p.OW), w1 = win_end(ow, p.W, p.OW);
     const int ww = w1 - w0;
-    count = (h1 - h0) * ww;
+    count = (long long)(h1 - h0) * ww;
+    const long long k0 = stretch_begin(count, slice, 8), k1 = stretch_begin(count, slice + 1, 8);
+    int ih = h0 + int(k0 / ww), iw = w0 + int(k0 % ww);
     const T* xc = static_cast<const T*>(p.x) + n * p.x_s[0] + cv * 8;
 #pragma unroll 4
-    for (int k = count * slice / 8; k < count * (slice + 1) / 8; ++k) {
-      const uint4 q = __ldg(reinterpret_cast<const uint4*>(xc + (h0 + k / ww) * p.x_s[2] + (w0 + k % ww) * p.x_s[3]));
+    for (long long k = k0; k < k1; ++k) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(xc + ih * p.x_s[2] + iw * p.x_s[3]));
+      if (++iw == w1) {
+        iw = w0;
+        ++ih;
+      }
       const T* e = reinterpret_cast<const T*>(&q);
 #pragma unroll
       for (int j = 0; j < 8; ++j) sum[j] += to_f32<T>(e[j]);
