@@ -1457,6 +1457,9 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     if (own.tile_n != 0 && own.one.x_repacked) run = workspace != nullptr && per_group > 0 ? workspace_bytes / per_group : 0;
     if (run > d.groups) run = d.groups;
     if (own.tile_n != 0 && run > 1 && !(from_packed && (dense || w_packed == nullptr))) {
+      // what a launch per group checks for each of them: here once, before the first relayout writes to the scratch
+      if (own.one.x_repacked && (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
+        return fail(FDNN_BAD_PARAM, "workspace must be 256-byte aligned");
       fdnn_conv_desc part = d;
       const long long cg = d.c / d.groups, kg = d.k / d.groups;
       const long long filter_bytes = kg * d.r * d.s * own.one.c_padded * es;
