@@ -1229,6 +1229,34 @@ bool find_packed(const void* ptr, int dev, PackedLayout* out) {
   return false;
 }
 
+// The first record that contradicts `want` among `count` buffers of `stride` bytes laid one after another from `ptr` (the
+// packed filters of a layer's groups); false if none does.
+bool find_other_layout(const void* ptr, long long stride, int count, int dev, const PackedLayout& want, PackedLayout* have) {
+  const uintptr_t base = reinterpret_cast<uintptr_t>(ptr);
+  std::lock_guard<std::mutex> lock(g_packed_mutex);
+  for (int i = 0; i < kPackedRecords; ++i) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(g_packed[i].ptr);
+    if (at < base || g_packed[i].dev != dev || (at - base) % uintptr_t(stride) != 0 || (at - base) / uintptr_t(stride) >= uintptr_t(count))
+      continue;
+    if (!(g_packed[i].layout == want)) {
+      *have = g_packed[i].layout;
+      return true;
+    }
+  }
+  return false;
+}
+
+int fail_layout(const PackedLayout& have, const PackedLayout& want) {
+  char buf[320];
+  std::snprintf(buf, sizeof buf,
+                "the packed filter holds the %s of a %dx%dx%dx%d filter, this call reads the %s of a "
+                "%dx%dx%dx%d filter (other descriptor, or a y whose 16-byte alignment differs from the one "
+                "given to fdnn_conv2d_pack_weight): pack again for this call",
+                packed_layout_name(have.kind), have.k, have.c, have.r, have.s, packed_layout_name(want.kind),
+                want.k, want.c, want.r, want.s);
+  return fail(FDNN_BAD_PARAM, buf);
+}
+
 int current_device_or_minus1() {
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess) {
@@ -1463,6 +1491,12 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
       fdnn_conv_desc part = d;
       const long long cg = d.c / d.groups, kg = d.k / d.groups;
       const long long filter_bytes = kg * d.r * d.s * own.one.c_padded * es;
+      if (from_packed) {
+        PackedLayout have;
+        const PackedLayout want = packed_layout_of(one_group_desc(&d), own.one);
+        if (find_other_layout(w_packed, filter_bytes, d.groups, current_device_or_minus1(), want, &have))
+          return fail_layout(have, want);
+      }
       auto at = [es](const void* base, long long elems) -> const void* {
         return base == nullptr ? nullptr : static_cast<const char*>(base) + elems * es;
       };
@@ -1568,16 +1602,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     // a pixel-grouped layer, whose buffer was checked by the outer one)
     PackedLayout have;
     const PackedLayout want = packed_layout_of(d, plan);
-    if (find_packed(w_packed, dev, &have) && !(have == want)) {
-      char buf[320];
-      std::snprintf(buf, sizeof buf,
-                    "the packed filter holds the %s of a %dx%dx%dx%d filter, this call reads the %s of a "
-                    "%dx%dx%dx%d filter (other descriptor, or a y whose 16-byte alignment differs from the one "
-                    "given to fdnn_conv2d_pack_weight): pack again for this call",
-                    packed_layout_name(have.kind), have.k, have.c, have.r, have.s, packed_layout_name(want.kind),
-                    want.k, want.c, want.r, want.s);
-      return fail(FDNN_BAD_PARAM, buf);
-    }
+    if (find_packed(w_packed, dev, &have) && !(have == want)) return fail_layout(have, want);
   }
 
   if (plan.pixel_group > 1) {

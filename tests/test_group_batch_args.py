@@ -35,3 +35,39 @@ def test_scratch_off_256_bytes_is_refused(native_lib, offset):
                                         scratch + offset, plan.workspace_bytes, None)
     assert status == nat.FDNN_BAD_PARAM
     assert b"workspace must be 256-byte aligned" in native_lib.fdnn_last_error()
+
+
+@pytest.mark.gpu
+def test_filters_packed_for_another_layer_are_refused(native_lib):
+    """Two layers whose packed filters take the same bytes per group (24 and 32 channels are both padded to 32): each
+    call takes its own buffer and refuses the other's."""
+    groups, k, n, hw = 32, 48 * 32, 3, 21
+    g = torch.Generator().manual_seed(3)
+    layers = []
+    for cg in (24, 32):
+        x = torch.randn((n, cg * groups, hw, hw), generator=g).to(torch.bfloat16).cuda()
+        w = (torch.randn((k, cg, 3, 3), generator=g) * (cg * 9) ** -0.5).to(torch.bfloat16).cuda()      # NCHW: needs packing
+        y = torch.full((n, k, hw, hw), -7.0, dtype=torch.bfloat16, device="cuda")
+        d, plan = _desc(n, cg * groups, hw, hw, k, groups, x.stride(), w.stride(), y.stride()), nat.ConvPlan()
+        nat.check(native_lib.fdnn_conv2d_query(ctypes.byref(d), x.data_ptr(), w.data_ptr(), y.data_ptr(), ctypes.byref(plan)))
+        assert plan.w_packed == 1
+        packed = torch.empty(plan.packed_weight_bytes, dtype=torch.uint8, device="cuda")
+        nat.check(native_lib.fdnn_conv2d_pack_weight(ctypes.byref(d), w.data_ptr(), y.data_ptr(), packed.data_ptr(), packed.numel(), None))
+        layers.append((d, plan, x, w, y, packed))
+    assert layers[0][5].numel() == layers[1][5].numel()
+    scratch = torch.empty(max(l[1].workspace_bytes for l in layers), dtype=torch.uint8, device="cuda")
+
+    def run(i, packed):
+        d, plan, x, w, y, _ = layers[i]
+        return native_lib.fdnn_conv2d_fwd(ctypes.byref(d), x.data_ptr(), w.data_ptr(), packed.data_ptr(), None, None, nat.ACT_NONE,
+                                          y.data_ptr(), scratch.data_ptr(), scratch.numel(), None)
+
+    for i in (0, 1):
+        assert run(i, layers[1 - i][5]) == nat.FDNN_BAD_PARAM
+        assert b"pack again" in native_lib.fdnn_last_error()
+        torch.cuda.synchronize()
+        assert bool((layers[i][4] == -7.0).all()), "a refused call must not write"
+    for i in (0, 1):
+        nat.check(run(i, layers[i][5]))
+        want = torch.nn.functional.conv2d(layers[i][2].double(), layers[i][3].double(), None, 1, 1, 1, groups)
+        torch.testing.assert_close(layers[i][4].double(), want, rtol=2.0 ** -8, atol=2.0 ** -8 * want.abs().max().item())
