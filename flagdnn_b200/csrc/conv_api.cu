@@ -459,6 +459,13 @@ fdnn_conv_desc one_group_desc(const fdnn_conv_desc* d) {
   return sub;
 }
 
+struct GroupBatch {    // see group_batch below
+  int tile_n;          // 0: does not apply
+  fdnn_conv_plan one;
+};
+GroupBatch group_batch(const fdnn_conv_desc* d, const void* x, const void* w, const void* y, const fdnn_conv_plan& plan,
+                       bool dense);
+
 int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void* y,
               fdnn_conv_plan* plan, bool allow_group = true) {
   int st = validate(d);
@@ -487,6 +494,16 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
       plan->bytes = bytes;
       plan->w_packed = 1;
       plan->packed_weight_bytes = dense_filter_bytes(d) + pv.packed_weight_bytes;
+      if (allow_group && w != nullptr) {
+        // The forward call will run all groups in one launch on w itself: no filter to pack, which for this route is G
+        // times the size of w.  (With a NULL w the caller's filter is not known, and a packed one serves any.)
+        const GroupBatch own = group_batch(d, x, w, y, *plan, true);
+        const long long per_group = (long long)d->n * d->h * d->w * cg * es;
+        if (own.tile_n != 0 && !own.one.w_packed && (!own.one.x_repacked || plan->workspace_bytes >= 2 * per_group)) {
+          plan->w_packed = 0;
+          plan->packed_weight_bytes = 0;
+        }
+      }
       return FDNN_OK;
     }
   }
@@ -703,10 +720,6 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
 //     16 x 56 x 56: 44.9 -> 28.2 us; 64 -> 128 in two groups on 256 x 56 x 56 stays dense: 125 us).
 // Every group's channels start on 16 bytes in x, w and y, as for one launch per group, and the taps fit a
 // five-dimensional im2col map.
-struct GroupBatch {
-  int tile_n;          // 0: does not apply
-  fdnn_conv_plan one;
-};
 GroupBatch group_batch(const fdnn_conv_desc* d, const void* x, const void* w, const void* y, const fdnn_conv_plan& plan,
                        bool dense) {
   GroupBatch g;
@@ -1905,7 +1918,7 @@ struct HostArena {
 static int host_arena_layout(const fdnn_conv_desc* d, HostArena* a) {
   fdnn_conv_desc q = *d;
   // Device copies start 256-byte aligned, so alignment never forces a repack.
-  int st = make_plan(&q, nullptr, nullptr, nullptr, &a->plan);
+  int st = make_plan(&q, nullptr, reinterpret_cast<const void*>(uintptr_t(256)), nullptr, &a->plan);
   if (st != FDNN_OK) return st;
   const int es = elem_size(d->dtype);
   a->x_bytes = span_elems(d->x_strides, d->n, d->c, d->h, d->w) * es;

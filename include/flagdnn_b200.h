@@ -100,7 +100,8 @@ typedef struct fdnn_conv_plan {
   int32_t oh, ow;               /* output size, rule of src/flag_dnn/ops/conv2d.py:52-62 */
   int32_t tile_m, tile_n, tile_k, stages; /* igemm tile; 0 for direct */
   int32_t x_repacked;           /* 1: x is first rewritten into the workspace as NHWC, C padded */
-  int32_t w_packed;             /* 1: fwd needs a packed filter from fdnn_conv2d_pack_weight */
+  int32_t w_packed;             /* 1: fwd needs a packed filter from fdnn_conv2d_pack_weight (for some grouped layers only
+                                   when queried without w: given w's address, fwd may read all groups in place) */
   int32_t c_padded;             /* channel count the igemm kernel iterates over */
   int32_t grid, block;          /* launch shape of the main kernel */
   int32_t launches;             /* kernels one fwd call launches at most (main + repack; per-group launches of a

@@ -71,3 +71,34 @@ def test_filters_packed_for_another_layer_are_refused(native_lib):
         nat.check(run(i, layers[i][5]))
         want = torch.nn.functional.conv2d(layers[i][2].double(), layers[i][3].double(), None, 1, 1, 1, groups)
         torch.testing.assert_close(layers[i][4].double(), want, rtol=2.0 ** -8, atol=2.0 ** -8 * want.abs().max().item())
+
+
+def test_a_filter_read_in_place_is_not_asked_for_packed(native_lib):
+    """Eight groups of 64 channels: planned as one dense layer, run as one launch over the groups that reads w itself."""
+    c = k = 512
+    d = _desc(16, c, 28, 28, k, 8, (c * 784, 1, 28 * c, c), (64 * 9, 1, 192, 64), (k * 784, 1, 28 * k, k))
+    plan = nat.ConvPlan()
+    for w, packed in ((0x1000, 0), (None, 1), (0x1002, 1)):     # in place; not known yet; off 16 bytes
+        nat.check(native_lib.fdnn_conv2d_query(ctypes.byref(d), 0x100000, w, 0x2000000, ctypes.byref(plan)))
+        assert plan.w_packed == packed and (plan.packed_weight_bytes > 0) == bool(packed)
+    # two groups of 32 channels stay one dense layer, and [K, C, R, S] filters are packed for it
+    d = _desc(256, 64, 56, 56, 128, 2, (64 * 3136, 1, 56 * 64, 64), (32 * 9, 1, 96, 32), (128 * 3136, 1, 56 * 128, 128))
+    nat.check(native_lib.fdnn_conv2d_query(ctypes.byref(d), 0x100000, 0x1000, 0x2000000, ctypes.byref(plan)))
+    assert plan.w_packed == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("groups", [4, 8])
+def test_layers_in_one_launch_leave_no_packed_filter_behind(native_lib, groups):
+    import flagdnn_b200 as fd
+
+    g = torch.Generator().manual_seed(groups)
+    fmt = torch.channels_last
+    x = torch.randn((4, 64 * groups, 28, 28), generator=g).to(torch.bfloat16).cuda().contiguous(memory_format=fmt)
+    w = (torch.randn((64 * groups, 64, 3, 3), generator=g) / 24).to(torch.bfloat16).cuda().contiguous(memory_format=fmt)
+    before = set(fd.conv_host._PACKED_WEIGHT_CACHE)
+    y = fd.conv2d(x, w, None, 1, 1, 1, groups)
+    assert fd.conv_host.conv2d_plan(x, w, 1, 1, 1, groups)["w_packed"] == 0
+    assert set(fd.conv_host._PACKED_WEIGHT_CACHE) <= before
+    want = torch.nn.functional.conv2d(x.double(), w.double(), None, 1, 1, 1, groups)
+    torch.testing.assert_close(y.double(), want, rtol=2.0 ** -8, atol=2.0 ** -8 * want.abs().max().item())
