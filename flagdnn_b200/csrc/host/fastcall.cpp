@@ -15,6 +15,7 @@
 #include <ATen/ATen.h>
 #include <c10/core/DeviceGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <array>
@@ -189,8 +190,8 @@ PyObject* finish(int status, at::Tensor&& y) {
 
 // conv(input, weight, bias, scale, residual, stride, padding, dilation, groups, algo, activation)
 PyObject* fast_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS   // C++ exceptions leave as the Python types torch gives them (torch.OutOfMemoryError among them)
   if (n != 11 || g_fwd == nullptr) return none();
-  try {
     const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
     if (x == nullptr || w == nullptr || x->dim() != 4 || w->dim() != 4) return none();
     const int dtype = dtype_code(x->scalar_type());
@@ -247,16 +248,13 @@ PyObject* fast_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     const int st = launch(d, *x, *w, a[1], bias, scale, residual, int(act), y);
     return finish(st, std::move(y));
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  END_HANDLE_TH_ERRORS
 }
 
 // conv1d(input [N, C, L], weight, bias, stride, padding, dilation, groups, algo): the 2-D call with H = R = 1
 PyObject* fast_conv1d(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS   // C++ exceptions leave as the Python types torch gives them (torch.OutOfMemoryError among them)
   if (n != 8 || g_fwd == nullptr) return none();
-  try {
     const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
     if (x == nullptr || w == nullptr || x->dim() != 3 || w->dim() != 3) return none();
     const int dtype = dtype_code(x->scalar_type());
@@ -311,16 +309,13 @@ PyObject* fast_conv1d(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     const int st = launch(d, *x, *w, nullptr, bias, nullptr, nullptr, FDNN_ACT_NONE, y);
     return finish(st, std::move(y));
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  END_HANDLE_TH_ERRORS
 }
 
 // mm(a [M, K], b [K, N], algo): a 1x1 convolution over one row of M pixels whose filter is b transposed
 PyObject* fast_mm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS   // C++ exceptions leave as the Python types torch gives them (torch.OutOfMemoryError among them)
   if (n != 3 || g_fwd == nullptr) return none();
-  try {
     const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
     if (x == nullptr || w == nullptr || x->dim() != 2 || w->dim() != 2) return none();
     const int dtype = dtype_code(x->scalar_type());
@@ -353,10 +348,7 @@ PyObject* fast_mm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     d.y_strides[3] = nn;
     const int st = launch(d, *x, *w, nullptr, nullptr, nullptr, nullptr, FDNN_ACT_NONE, y);
     return finish(st, std::move(y));
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  END_HANDLE_TH_ERRORS
 }
 
 // bind(query, pack, fwd: addresses of the C ABI's functions, packed_weight: callback)
