@@ -63,10 +63,27 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     return LIB_PATH
 
 
+def host_tag() -> str:
+    """What the host path must have been compiled against; the module carries it as ``built_for``."""
+    import torch
+
+    return f"flagdnn host path for torch {torch.__version__}"
+
+
+def _host_stale() -> bool:
+    """Missing, older than its source or the C ABI's header, or compiled against another torch."""
+    header = PKG_DIR.parent / "include" / "flagdnn_b200.h"
+    if not HOST_PATH.exists():
+        return True
+    built = HOST_PATH.stat().st_mtime
+    if any(p.stat().st_mtime > built for p in (HOST_SOURCE, header) if p.exists()):
+        return True
+    return (host_tag() + "\0").encode() not in HOST_PATH.read_bytes()
+
+
 def build_host(force: bool = False, verbose: bool = False) -> Path:
     """Compile the native host path of the eager operators (csrc/host/fastcall.cpp) against the installed torch."""
-    header = PKG_DIR.parent / "include" / "flagdnn_b200.h"
-    if not force and HOST_PATH.exists() and all(p.stat().st_mtime <= HOST_PATH.stat().st_mtime for p in (HOST_SOURCE, header)):
+    if not force and not _host_stale():
         return HOST_PATH
     import sysconfig
 
@@ -74,8 +91,11 @@ def build_host(force: bool = False, verbose: bool = False) -> Path:
 
     root = Path(torch.__file__).resolve().parent
     cuda = Path(_nvcc()).resolve().parent.parent
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    cxx = os.environ.get("CXX", "g++")
+    if shutil.which(cxx) is None:
+        raise RuntimeError(f"{cxx} not found; set CXX or put it on PATH")
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DFDNN_HOST_TAG="{host_tag()}"',
            f"-I{root / 'include'}", f"-I{root / 'include' / 'torch' / 'csrc' / 'api' / 'include'}",
            f"-I{sysconfig.get_paths()['include']}", f"-I{cuda / 'include'}",
            "-o", str(HOST_PATH), str(HOST_SOURCE), f"-L{root / 'lib'}",
@@ -84,11 +104,11 @@ def build_host(force: bool = False, verbose: bool = False) -> Path:
         print(" ".join(cmd), file=sys.stderr)
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
-        raise RuntimeError(f"g++ failed ({proc.returncode}):\n{proc.stdout}\n{proc.stderr}")
+        raise RuntimeError(f"{cxx} failed ({proc.returncode}):\n{proc.stdout}\n{proc.stderr}")
     return HOST_PATH
 
 
 if __name__ == "__main__":
-    build_host(force="--force" in sys.argv, verbose=True)
     build(force="--force" in sys.argv, verbose=True, ptxas_info="--ptxas-info" in sys.argv)
+    build_host(force="--force" in sys.argv, verbose=True)   # the kernels do not wait for a host compiler
     print(LIB_PATH)

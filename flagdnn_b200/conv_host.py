@@ -8,6 +8,7 @@ with the Triton launches replaced by calls into the C ABI
 from __future__ import annotations
 
 import ctypes
+import warnings
 import weakref
 from collections import OrderedDict
 from typing import Any, Optional, Sequence, Tuple, Union
@@ -260,18 +261,25 @@ def _packed_for_native(weight, desc_address: int, plan_address: int, stream: int
 
 
 def _load_fast() -> Any:
+    """The native host path, bound to the kernel library; False where it cannot be used (once, with a warning)."""
     global _fast
     if _fast is None:
+        from . import build
+
         try:
             from . import _fastcall
-        except ImportError:      # not built: every call takes the Python code
+            if _fastcall.built_for != build.host_tag():
+                raise ImportError(f"it is the {_fastcall.built_for}, this is torch {torch.__version__}")
+            lib = nat.load()
+            address = [ctypes.cast(f, ctypes.c_void_p).value for f in
+                       (lib.fdnn_conv2d_query, lib.fdnn_conv2d_pack_weight, lib.fdnn_conv2d_fwd_ex)]
+            _fastcall.bind(*address, _packed_for_native, lib.fdnn_abi_version(), ctypes.sizeof(nat.ConvDesc),
+                           ctypes.sizeof(nat.ConvPlan))
+            _fast = _fastcall
+        except (ImportError, AttributeError, TypeError) as exc:   # not built, or built against something else
+            warnings.warn(f"flagdnn_b200: the native host path is not used, calls take some 15 us longer ({exc}); "
+                          "build it with `python -m flagdnn_b200.build`", RuntimeWarning, stacklevel=3)
             _fast = False
-            return _fast
-        lib = nat.load()
-        address = [ctypes.cast(f, ctypes.c_void_p).value for f in
-                   (lib.fdnn_conv2d_query, lib.fdnn_conv2d_pack_weight, lib.fdnn_conv2d_fwd_ex)]
-        _fastcall.bind(*address, _packed_for_native)
-        _fast = _fastcall
     return _fast
 
 

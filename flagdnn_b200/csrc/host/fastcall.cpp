@@ -351,11 +351,18 @@ PyObject* fast_mm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(query, pack, fwd: addresses of the C ABI's functions, packed_weight: callback)
+// bind(query, pack, fwd: addresses of the C ABI's functions, packed_weight: callback, version of the loaded library and the
+// sizes of the two structures as the caller knows them): refuses a library or caller of another ABI than this file's.
 PyObject* bind(PyObject*, PyObject* args) {
-  unsigned long long q, p, f;
+  unsigned long long q, p, f, desc_bytes, plan_bytes;
+  int version;
   PyObject* cb;
-  if (!PyArg_ParseTuple(args, "KKKO", &q, &p, &f, &cb)) return nullptr;
+  if (!PyArg_ParseTuple(args, "KKKOiKK", &q, &p, &f, &cb, &version, &desc_bytes, &plan_bytes)) return nullptr;
+  if (version != FDNN_ABI_VERSION || desc_bytes != sizeof(fdnn_conv_desc) || plan_bytes != sizeof(fdnn_conv_plan)) {
+    PyErr_Format(PyExc_ImportError, "compiled for version %d of the C ABI (structures of %zu and %zu bytes), given %d (%llu and %llu)",
+                 FDNN_ABI_VERSION, sizeof(fdnn_conv_desc), sizeof(fdnn_conv_plan), version, desc_bytes, plan_bytes);
+    return nullptr;
+  }
   Py_INCREF(cb);
   Py_XDECREF(g_packed_weight);
   g_packed_weight = cb;
@@ -375,4 +382,12 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_fastcall", nullptr, -1, kMethods
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__fastcall() { return PyModule_Create(&kModule); }
+// `built_for`: the torch this was compiled against (the build compares it with the installed one, and the loader too).
+PyMODINIT_FUNC PyInit__fastcall() {
+  PyObject* m = PyModule_Create(&kModule);
+  if (m != nullptr && PyModule_AddStringConstant(m, "built_for", FDNN_HOST_TAG) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

@@ -14,10 +14,11 @@ def pytest_configure(config):
 
 @pytest.fixture(scope="session")
 def native_lib():
-    """The built C-ABI library (compiled on demand; nvcc needs no GPU)."""
+    """The built C-ABI library and the native host path (compiled on demand; nvcc needs no GPU)."""
     from flagdnn_b200 import _native, build
 
     build.build()
+    build.build_host()
     return _native.load()
 
 
