@@ -361,13 +361,16 @@ bool filter_mn_major(const fdnn_conv_desc* d, const void* w) {
 }
 
 // Below kSmallFlops a 16-bit layer still runs on the tensor-core kernel when its reduction is more than a few dozen
-// products long: the direct kernel walks it serially (one 64 x 14 x 14 image, 64 filters 3x3, f16: 26.6 us against
-// 5 us), and both round an fp32 sum once.  fp32 layers stay on exact products there.  Such a call needs what the
-// tensor-core plan asks for (packed filter, scratch); without it, fwd_impl runs the direct kernel as before, and the
-// scratch stays within the built-in one of fdnn_conv2d_fwd_static_scratch.
+// products long: the direct kernel walks it serially (kernels of one 64 x 14 x 14 image, 64 filters 3x3, bf16: NCHW
+// 25.9 -> 8.2 us, channels-last 83.2 -> 4.9), and both round an fp32 sum once.  fp32 layers stay on exact products there.
+// Such a call needs what the tensor-core plan asks for (packed filter, scratch); without it, fwd_impl runs the direct
+// kernel as before, and the scratch stays within the built-in one of fdnn_conv2d_fwd_static_scratch.
+// Fewer than eight channels only in window mode (see pixel_windows): without it a reduction takes R * S copies of 16-byte
+// rows (3 -> 16 channels 11x11 on 32 x 32 NCHW: 35 us against the direct kernel's 20).
 constexpr double kSmallFlops = 2.0e7;
-bool small_on_tensor_cores(const fdnn_conv_desc* d, double flops) {
+bool small_on_tensor_cores(const fdnn_conv_desc* d, int oh, int ow, double flops) {
   return elem_size(d->dtype) == 2 && d->c * d->r * d->s >= 64 && flops >= 2.0e5 &&
+         (d->c >= 8 || pixel_windows(d, oh, ow).ok) &&
          (long long)d->n * d->h * d->w * padded_x_channels(d) * 2 <= FDNN_STATIC_SCRATCH_BYTES;
 }
 
@@ -542,7 +545,7 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
   if ((algo == FDNN_ALGO_IGEMM || algo == FDNN_ALGO_IGEMM_PAIR) && !geom_ok)
     return fail(FDNN_NOT_SUPPORTED, "implicit-GEMM path does not support this problem");
   const bool want_auto = algo == FDNN_ALGO_AUTO;
-  if (want_auto) algo = (geom_ok && (plan->flops >= kSmallFlops || small_on_tensor_cores(d, plan->flops))) ? FDNN_ALGO_IGEMM : FDNN_ALGO_DIRECT;
+  if (want_auto) algo = (geom_ok && (plan->flops >= kSmallFlops || small_on_tensor_cores(d, oh, ow, plan->flops))) ? FDNN_ALGO_IGEMM : FDNN_ALGO_DIRECT;
   if (algo != FDNN_ALGO_IGEMM && algo != FDNN_ALGO_DIRECT && algo != FDNN_ALGO_IGEMM_PAIR)
     return fail(FDNN_BAD_PARAM, "unknown algo");
   plan->algo = algo;
@@ -560,6 +563,11 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
 
   LowChannel lc = low_channel_geometry(d, oh, ow, y);
   if (out_f32) lc.ok = false;   // quads and pixel groups rely on y's 16-bit layout
+  // A quad multiplies each pixel's window by the zeros its neighbours' taps leave, so that an infinite pixel turns outputs
+  // that do not read it into NaN.  Small layers, which the direct kernel computes tap by tap, keep that apart, as pixel
+  // windows do (3 -> 16 channels 5x5 on 32 x 32: quads 5.8 us, windows 5.9, direct 11.9; 11x11, too wide for windows: 6.9
+  // against 19.9 on the direct kernel).
+  if (want_auto && plan->flops < kSmallFlops) lc.ok = false;
   if (lc.ok) {
     const int sms_lc = sm_count();
     const int m_tiles_lc = d->n * lc.tiles_per_image;
