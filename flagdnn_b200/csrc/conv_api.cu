@@ -1539,6 +1539,8 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   }
   if (batch == nullptr && d.groups > 1 && plan.algo != FDNN_ALGO_DIRECT && group_dense_ok(&d)) {
     // one dense convolution with the block-diagonal filter the pack step left at the front of w_packed
+    if (w_packed == nullptr && !plan.w_packed)   // planned as one launch on w; only the scratch can have kept it from that
+      return fail(FDNN_WORKSPACE_TOO_SMALL, "workspace smaller than plan.workspace_bytes");
     if (w_packed == nullptr)
       return fail(FDNN_BAD_PARAM, "a grouped layer on the dense route needs its packed filter; w_packed is NULL");
     const fdnn_conv_desc v = dense_group_desc(&d);

@@ -102,3 +102,17 @@ def test_layers_in_one_launch_leave_no_packed_filter_behind(native_lib, groups):
     assert set(fd.conv_host._PACKED_WEIGHT_CACHE) <= before
     want = torch.nn.functional.conv2d(x.double(), w.double(), None, 1, 1, 1, groups)
     torch.testing.assert_close(y.double(), want, rtol=2.0 ** -8, atol=2.0 ** -8 * want.abs().max().item())
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the addresses are made up; without a device nothing can use them")
+@pytest.mark.parametrize("scratch_bytes", [0, 256, 64 * 784 * 2])
+def test_too_little_scratch_is_called_that(native_lib, scratch_bytes):
+    """Eight groups of 64 channels in NCHW, filter read in place: scratch for less than two relaid-out groups."""
+    c = k = 512
+    d, plan = _desc(1, c, 28, 28, k, 8, (c * 784, 784, 28, 1), (64 * 9, 1, 192, 64), (k * 784, 784, 28, 1)), nat.ConvPlan()
+    x, w, y, scratch = 0x100000, 0x1000000, 0x2000000, 0x3000000
+    nat.check(native_lib.fdnn_conv2d_query(ctypes.byref(d), x, w, y, ctypes.byref(plan)))
+    assert plan.x_repacked == 1 and plan.w_packed == 0 and plan.workspace_bytes >= 8 * 64 * 784 * 2
+    status = native_lib.fdnn_conv2d_fwd(ctypes.byref(d), x, w, None, None, None, nat.ACT_NONE, y,
+                                        scratch if scratch_bytes else None, scratch_bytes, None)
+    assert status == nat.FDNN_WORKSPACE_TOO_SMALL
