@@ -1761,9 +1761,8 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   const bool out_f32 = (d.algo & FDNN_ALGO_FLAG_OUT_F32) != 0;
   if (out_f32 && residual != nullptr) return fail(FDNN_NOT_SUPPORTED, "no residual with a float32 output from 16-bit operands");
   p.out_f32 = out_f32 ? 1 : 0;
-  const int gran = out_f32 ? 4 : 16 / es;   // output elements per 16 bytes
-  p.vec_store = (d.y_strides[1] == 1 && d.y_strides[0] % gran == 0 && d.y_strides[2] % gran == 0 &&
-                 d.y_strides[3] % gran == 0 && (reinterpret_cast<uintptr_t>(y) & 15u) == 0)
+  p.vec_store = (out_f32 && d.y_strides[1] == 1 && d.y_strides[0] % 4 == 0 && d.y_strides[2] % 4 == 0 &&
+                 d.y_strides[3] % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15u) == 0)
                     ? 1
                     : 0;
   // y as one [M, K] matrix: consecutive output pixels are row_stride apart

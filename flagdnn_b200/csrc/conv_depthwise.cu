@@ -2,17 +2,21 @@
 //
 // A depthwise layer does 2*R*S flops per output element against two bytes read and two written: it is
 // bound by memory traffic, not arithmetic, so the job is to touch x and y once each with wide, coalesced
-// accesses and to keep the R*S taps out of global memory.  Two kernels, chosen by layout (the reference
-// has one Triton kernel per layout as well: src/flag_dnn/ops/conv2d.py:2613-2800 for NCHW,
+// accesses and to keep the R*S taps out of global memory.  The kernel follows from the layout, the alignment and the
+// filter (depthwise_kind; the reference has one Triton kernel per layout: src/flag_dnn/ops/conv2d.py:2613-2800 for NCHW,
 // src/flag_dnn/ops/conv2d.py:3089-3190 for channels-last):
 //
-//   channels-last  one thread owns 16 bytes of channels (8 x 16-bit or 4 x fp32) of four (two in the run-time
-//                  variant) neighbouring output pixels of a row; every input pixel it needs is one 16-byte
-//                  load that serves all of them; the filter sits in shared memory as fp32 [R*S][C];
-//   NCHW           one block owns one (image, channel) plane: its taps sit in registers (shared memory in the
-//                  run-time variant), its threads walk the plane's output pixels four (two) at a time along
-//                  W, and the plane's input stays in L1.
-// 3x3 and 5x5 filters at stride 1 and 2 without dilation have fully unrolled instantiations of both.
+//   channels-last  3x3 / 5x5 at stride 1 / 2 with chunks of 64 channels mostly full: conv_depthwise_tma.cu.  Otherwise
+//                  (depthwise_cl_kernel) one thread owns 16 bytes of channels (8 x 16-bit or 4 x fp32) of four (two in
+//                  the run-time variant) neighbouring output pixels of a row; every input pixel it needs is one 16-byte
+//                  load that serves all of them; the filter sits in shared memory as fp32 [R*S][C].  Channel counts
+//                  and pitches that fill no 16-byte pieces: depthwise_cl_scalar_kernel, a channel per thread;
+//   NCHW           rows on vector boundaries and "same" padding: depthwise_rowvec_kernel, a vector of neighbouring
+//                  outputs per thread.  Small dense planes whose rows start anywhere: depthwise_planes_kernel, several
+//                  whole planes per block in shared memory.  Otherwise (depthwise_plane_kernel) one block owns one
+//                  (image, channel) plane: its taps sit in registers (shared memory in the run-time variant), its threads
+//                  walk the plane's output pixels four (two) at a time along W, and the plane's input stays in L1.
+// 3x3 and 5x5 filters at stride 1 and 2 without dilation have fully unrolled instantiations.
 //
 // Arithmetic as everywhere in this library: fp32 accumulate (fp64 is left to the direct kernel), scale,
 // bias and residual in fp32, activation, one rounding.  Index arithmetic follows

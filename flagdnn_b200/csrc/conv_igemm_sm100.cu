@@ -90,26 +90,11 @@ struct TileCfg {
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 };
 
-// 32 finished values of one output pixel -> 32 consecutive channels of y.
-template <typename T>
-__device__ __forceinline__ void store32_contig(T* dst, const float (&v)[32]) {
-  if constexpr (std::is_same<T, float>::value) {
+// 32 finished values of one output pixel -> 32 consecutive channels of a float32 y.
+__device__ __forceinline__ void store32_contig(float* dst, const float (&v)[32]) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float4 q = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-      reinterpret_cast<float4*>(dst)[i] = q;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint4 q;
-      q.x = pack2(from_f32<T>(v[8 * i + 0]), from_f32<T>(v[8 * i + 1]));
-      q.y = pack2(from_f32<T>(v[8 * i + 2]), from_f32<T>(v[8 * i + 3]));
-      q.z = pack2(from_f32<T>(v[8 * i + 4]), from_f32<T>(v[8 * i + 5]));
-      q.w = pack2(from_f32<T>(v[8 * i + 6]), from_f32<T>(v[8 * i + 7]));
-      reinterpret_cast<uint4*>(dst)[i] = q;
-    }
-  }
+  for (int i = 0; i < 8; ++i)
+    reinterpret_cast<float4*>(dst)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
 }
 
 // DENSE: y goes through the TMA unit (p.tma_store); otherwise through the warps' own stores, whose registers would push
@@ -244,8 +229,6 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             const uint16_t off_w = static_cast<uint16_t>(s * p.dil_w), off_h = static_cast<uint16_t>(r * p.dil_h);
             if constexpr (kMode == kGroups) {
               tma_load_im2col_5d(st, &tmA, bar, c0, w_base, h_base, img, group, off_w, off_h);
-              if constexpr (Cfg::kSplit)
-                tma_load_im2col_5d(st + Cfg::kABytes, &tmA2, bar, c0, w_base, h_base, img, group, off_w, off_h);
             } else {
               tma_load_im2col_4d(st, &tmA, bar, c0, w_base, h_base, img, off_w, off_h);
               if constexpr (Cfg::kSplit)
@@ -307,10 +290,14 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (!p.skip_copies) {
-      if (p.lowc) produce_any(std::integral_constant<int, kWindows>{});
-      else if (p.b_mn) produce_any(std::integral_constant<int, kFilterMn>{});
-      else if (p.groups > 1) produce_any(std::integral_constant<int, kGroups>{});
-      else produce_any(std::integral_constant<int, kIm2col>{});
+      if constexpr (Cfg::kSplit) {   // the other modes are for 16-bit types
+        produce_any(std::integral_constant<int, kIm2col>{});
+      } else {
+        if (p.lowc) produce_any(std::integral_constant<int, kWindows>{});
+        else if (p.b_mn) produce_any(std::integral_constant<int, kFilterMn>{});
+        else if (p.groups > 1) produce_any(std::integral_constant<int, kGroups>{});
+        else produce_any(std::integral_constant<int, kIm2col>{});
+      }
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- issuer
@@ -518,7 +505,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           // 16-bit operands, float32 result: the finished values are stored as they are
           float* yf = static_cast<float*>(p.y);
           if (p.vec_store && col0 + 32 <= p.Kout) {
-            store32_contig<float>(yf + y_off + col0, v);
+            store32_contig(yf + y_off + col0, v);
           } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
@@ -526,13 +513,9 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             }
           }
         } else if (row_ok) {
-          if (p.vec_store && col0 + 32 <= p.Kout) {
-            store32_contig<T>(y + y_off + col0, v);
-          } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (col0 + j < p.Kout) y[y_off + (long long)(col0 + j) * p.y_sk] = from_f32<T>(v[j]);
-            }
+          for (int j = 0; j < 32; ++j) {   // channels apart: contiguous ones go through epilogue_store_strided
+            if (col0 + j < p.Kout) y[y_off + (long long)(col0 + j) * p.y_sk] = from_f32<T>(v[j]);
           }
         }
       }

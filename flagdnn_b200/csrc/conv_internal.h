@@ -29,15 +29,16 @@ struct IgemmParams {
   void* y;
   const void* residual;  // tensor with y's dtype and strides added before the activation, or nullptr
   int act;               // FDNN_ACT_* applied after scale, bias and residual
-  int vec_store;         // 1: y is channel-contiguous and 16-byte aligned per pixel
+  int vec_store;         // with out_f32, 1: y is channel-contiguous and 16-byte aligned per pixel
   int tma_store;         // 1: y is dense NHWC; the epilogue writes it through the tmY tensor map
   int y_mode;            // without tma_store: how the epilogue writes y (kY* of conv_epilogue.cuh)
   int y_unit;            // bytes per lane and store in those modes (16, 8, 4 or 2)
   int out_f32;           // 1: y is float32 although the operands are 16-bit (per-thread store path only)
-  // Low-channel mode (C <= 4): one GEMM row is a quad of 4 output pixels of one
+  // Window modes.  Low-channel (C <= 4): one GEMM row is a quad of 4 output pixels of one
   // image row, its reduction operand a 16-pixel window of the repacked input;
-  // a tile is `ohs` output rows x OW/4 quads and never crosses an image.
-  int lowc;              // 1: low-channel mode
+  // a tile is `ohs` output rows x OW/4 quads and never crosses an image.  Pixel windows (C < 8): one
+  // GEMM row is one output pixel, its operand the S x 8 stored values of its taps; tiles of `ohs` rows too.
+  int lowc;              // 1: one of these modes
   int rows_per_tile;     // valid GEMM rows per tile (128 outside low-channel mode)
   int tiles_per_image;   // low-channel mode: ceil(OH / ohs)
   int ohs;               // low-channel mode: output rows per tile
@@ -126,12 +127,16 @@ struct DirectParams {
   int act;  // FDNN_ACT_*
 };
 cudaError_t launch_direct(int dtype, const DirectParams& p, cudaStream_t stream);
-// Depthwise layers (groups == C == K) in f16 / bf16 / f32 (conv_depthwise.cu): `depthwise_kind` answers 0 when
-// the problem is not one of its cases (the direct kernel then runs), 1 for the channels-last kernel (16 bytes
-// of channels per thread), 2 for the kernel that gives every (image, channel) plane a block, 3 / 4 / 5 for the
-// NCHW kernel that reads rows as 16- / 8- / 4-byte vectors.
+// Depthwise layers (groups == C == K) in f16 / bf16 / f32: which kernel takes the problem.
+//   0  none of them (the direct kernel runs)
+//   1  channels-last, 16 bytes of channels per thread, plain loads
+//   2  one block per (image, channel) plane
+//   3, 4, 5  NCHW, rows read as 16- / 8- / 4-byte vectors
+//   6  channels-last, input rows staged by the TMA unit (conv_depthwise_tma.cu); 1 where no map can be made of x
+//   7  NCHW, several whole planes per block
+//   8  channels-last, one channel per thread (channel counts and pitches that fill no 16-byte pieces)
 int depthwise_kind(int dtype, const DirectParams& p);
-// 6: channels-last cases of the kernel that stages input rows through the TMA unit (conv_depthwise_tma.cu).
+// Whether a problem of kind 1 is one of kind 6.
 bool depthwise_tma_ok(const DirectParams& p);
 cudaError_t launch_depthwise_tma(int dtype, const DirectParams& p, uint32_t* status, long long wait_limit, cudaStream_t stream);
 // Tensor map over a channels-last x for it: boxes of `chunk` channels x `span` pixels x `rows` rows.  False: not encodable.
