@@ -1377,6 +1377,9 @@ int fdnn_conv2d_pack_weight(const fdnn_conv_desc* desc, const void* w, const voi
     st = make_plan(&d, nullptr, reinterpret_cast<const void*>(uintptr_t(1)), y, &plan);
   }
   if (st != FDNN_OK) return st;
+  // a grouped filter [K, C / groups, R, S] is packed group by group or made dense above, never as one of C channels
+  if (d.groups > 1 && d.algo != desc->algo) return fdnn_conv2d_pack_weight(&d, w, y, packed, packed_bytes, stream);
+  if (d.groups > 1) return fail(FDNN_NOT_SUPPORTED, "no packed layout for this grouped filter");
   if (w == nullptr || packed == nullptr) return fail(FDNN_BAD_PARAM, "w and packed must not be NULL");
   if (packed_bytes < plan.packed_weight_bytes)
     return fail(FDNN_WORKSPACE_TOO_SMALL, "packed filter buffer too small");

@@ -1,4 +1,6 @@
 """Packed filters kept between calls: one filter tensor used by layers of different group counts, padding or data."""
+import ctypes
+
 import pytest
 import torch
 
@@ -58,3 +60,32 @@ def test_one_filter_under_two_group_counts(native_lib, dtype, k, cg, r, hw, n, c
         y = fd.conv2d(x, w, None, 1, r // 2, 1, groups)
         want = torch.nn.functional.conv2d(x.double(), w.double(), None, 1, r // 2, 1, groups)
         torch.testing.assert_close(y.double(), want, rtol=eps, atol=eps * want.abs().max().item())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("c,k,groups", [(32, 32, 2), (96, 96, 12), (24, 40, 4)])
+def test_a_small_grouped_filter_is_packed_for_the_tensor_core_route(native_lib, dtype, c, k, groups):
+    """Planned as the direct kernel, which reads w itself; the packed form is that of the route a forced call takes, and
+    packing reads C / groups channels of each filter."""
+    nat = conv_host.nat
+    cg, hw, r = c // groups, 6, 3
+    g = torch.Generator().manual_seed(c + k)
+    fmt = torch.channels_last
+    x = torch.randn((1, c, hw, hw), generator=g).to(dtype).cuda().contiguous(memory_format=fmt)
+    w = (torch.randn((k, cg, r, r), generator=g) * (cg * r * r) ** -0.5).to(dtype).cuda()
+    y = torch.empty((1, k, hw, hw), dtype=dtype, device="cuda", memory_format=fmt)
+    args = (x, w, y, (1, 1), (1, 1, 1, 1), (1, 1), groups)
+    d, plan = conv_host._plan_for(*args, nat.ALGO_AUTO)
+    assert plan.algo == nat.ALGO_DIRECT
+    forced, want_plan = conv_host._plan_for(*args, nat.ALGO_IGEMM)
+    assert want_plan.w_packed
+    packed = torch.empty(want_plan.packed_weight_bytes, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    nat.check(native_lib.fdnn_conv2d_pack_weight(ctypes.byref(d), w.data_ptr(), y.data_ptr(), packed.data_ptr(), packed.numel(), stream))
+    scratch = torch.empty(max(want_plan.workspace_bytes, 256), dtype=torch.uint8, device="cuda")
+    nat.check(native_lib.fdnn_conv2d_fwd(ctypes.byref(forced), x.data_ptr(), w.data_ptr(), packed.data_ptr(), None, None, nat.ACT_NONE,
+                                         y.data_ptr(), scratch.data_ptr(), scratch.numel(), stream))
+    want = torch.nn.functional.conv2d(x.double(), w.double(), None, 1, 1, 1, groups)
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float32: 2e-5}[dtype]   # one rounding; split TF32
+    torch.testing.assert_close(y.double(), want, rtol=eps, atol=eps * want.abs().max().item())
