@@ -1486,8 +1486,10 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     return fail(FDNN_BAD_PARAM, "unknown activation");
   if ((desc->algo & 0xff) == FDNN_ALGO_AUTO && plan.algo != FDNN_ALGO_DIRECT && small_layer(desc, plan.flops) &&
       allow_group && batch == nullptr && w != nullptr &&
-      ((plan.w_packed && w_packed == nullptr) || (plan.workspace_bytes > 0 && (workspace == nullptr || workspace_bytes < plan.workspace_bytes)))) {
-    // a small layer whose caller brought neither packed filter nor scratch (see small_on_tensor_cores)
+      ((plan.w_packed && w_packed == nullptr) || (plan.workspace_bytes > 0 && (workspace == nullptr || workspace_bytes < plan.workspace_bytes)) ||
+       (desc->c < 8 && residual != nullptr))) {
+    // a small layer whose caller brought neither packed filter nor scratch, or one that was planned as pixel windows, which
+    // carry no residual (see small_on_tensor_cores)
     fdnn_conv_desc direct = *desc;
     direct.algo = FDNN_ALGO_DIRECT;
     return fwd_impl(&direct, x, w, nullptr, bias, scale, residual, activation, y, nullptr, 0, stream_v, allow_group, k_real);

@@ -63,3 +63,35 @@ def test_an_infinite_pixel_stays_in_its_windows(native_lib, case, layout):
     # one rounding of an fp32 sum
     size = want[finite].abs().max().item()
     torch.testing.assert_close(y.double()[finite], want[finite], rtol=2.0 ** -11, atol=2.0 ** -11 * size)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", [torch.channels_last, torch.contiguous_format])
+@pytest.mark.parametrize("case", SMALL)
+def test_residuals_are_taken(native_lib, case, layout):
+    """Through the C ABI, which refuses a residual where quads are planned."""
+    n, c, h, w, k, r, stride, pad = case
+    g = torch.Generator().manual_seed(k * r)
+    x = torch.randn((n, c, h, w), generator=g).half().cuda().contiguous(memory_format=layout)
+    wt = (torch.randn((k, c, r, r), generator=g) * (c * r * r) ** -0.5).half().cuda().contiguous(memory_format=layout)
+    want = torch.nn.functional.conv2d(x.double(), wt.double(), None, stride, pad)
+    res = torch.randn(want.shape, generator=g).half().cuda().contiguous(memory_format=layout)
+    y = torch.empty_like(res)
+    d, plan = nat.ConvDesc(), nat.ConvPlan()
+    d.dtype, d.groups, d.algo = nat.F16, 1, nat.ALGO_AUTO
+    d.n, d.c, d.h, d.w, d.k, d.r, d.s = n, c, h, w, k, r, r
+    d.stride_h = d.stride_w = stride
+    d.pad_top = d.pad_bottom = d.pad_left = d.pad_right = pad
+    d.dil_h = d.dil_w = 1
+    d.x_strides[:], d.w_strides[:], d.y_strides[:] = x.stride(), wt.stride(), y.stride()
+    nat.check(native_lib.fdnn_conv2d_query(ctypes.byref(d), x.data_ptr(), wt.data_ptr(), y.data_ptr(), ctypes.byref(plan)))
+    packed = torch.empty(max(plan.packed_weight_bytes, 1), dtype=torch.uint8, device="cuda")
+    scratch = torch.empty(max(plan.workspace_bytes, 1), dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    if plan.w_packed:
+        nat.check(native_lib.fdnn_conv2d_pack_weight(ctypes.byref(d), wt.data_ptr(), y.data_ptr(), packed.data_ptr(), packed.numel(), stream))
+    nat.check(native_lib.fdnn_conv2d_fwd_residual(
+        ctypes.byref(d), x.data_ptr(), wt.data_ptr(), packed.data_ptr() if plan.w_packed else None, None, None, res.data_ptr(),
+        nat.ACT_RELU, y.data_ptr(), scratch.data_ptr(), plan.workspace_bytes, stream))
+    want = torch.relu(want + res.double())
+    torch.testing.assert_close(y.double(), want, rtol=2.0 ** -11, atol=2.0 ** -11 * want.max().item())   # one rounding
