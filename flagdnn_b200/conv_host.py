@@ -230,8 +230,8 @@ def _packed_layout(d: nat.ConvDesc, plan: nat.ConvPlan) -> tuple:
 
 def _packed_weight(weight: torch.Tensor, d: nat.ConvDesc, plan: nat.ConvPlan, stream: int, y_ptr: int) -> torch.Tensor:
     version = int(getattr(weight, "_version", 0))
-    key = (_packed_layout(d, plan), id(weight), weight.data_ptr(), tuple(weight.shape), tuple(weight.stride()),
-           str(weight.dtype), weight.device.type, weight.device.index, version)
+    key = (_packed_layout(d, plan), id(weight), weight.data_ptr(), weight.shape, weight.stride(), weight.dtype,
+           weight.device, version)
     entry = _PACKED_WEIGHT_CACHE.get(key)
     if entry is not None:
         owner_ref, value = entry
