@@ -469,6 +469,17 @@ struct GroupBatch {    // see group_batch below
 GroupBatch group_batch(const fdnn_conv_desc* d, const void* x, const void* w, const void* y, const fdnn_conv_plan& plan,
                        bool dense);
 
+// w in place: [K, R, S, C]-like memory, taps evenly spaced.  A stride over an extent of one carries no information.
+bool filter_in_place(const fdnn_conv_desc* d, const void* w) {
+  const int es = elem_size(d->dtype), gran = 16 / es, cg = d->c / d->groups;
+  auto stride_ok = [gran](long long extent, long long stride) { return extent <= 1 || stride % gran == 0; };
+  return es == 2 && (cg == 1 || d->w_strides[1] == 1) && stride_ok(d->k, d->w_strides[0]) &&
+         stride_ok(d->s, d->w_strides[3]) && (d->s <= 1 || d->w_strides[3] >= cg) &&
+         (d->r <= 1 || (d->s > 1 ? d->w_strides[2] == (long long)d->s * d->w_strides[3]
+                                 : d->w_strides[2] % gran == 0)) &&
+         aligned16(w);
+}
+
 int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void* y,
               fdnn_conv_plan* plan, bool allow_group = true) {
   int st = validate(d);
@@ -644,12 +655,7 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
   const bool x_inplace = is16 && (d->c == 1 || d->x_strides[1] == 1) && stride_ok(d->n, d->x_strides[0]) &&
                          stride_ok(d->h, d->x_strides[2]) && stride_ok(d->w, d->x_strides[3]) &&
                          (d->w <= 1 || d->x_strides[3] >= d->c) && aligned16(x);
-  // w in place: [K, R, S, C]-like memory, taps evenly spaced
-  const bool w_inplace = is16 && (d->c == 1 || d->w_strides[1] == 1) && stride_ok(d->k, d->w_strides[0]) &&
-                         stride_ok(d->s, d->w_strides[3]) && (d->s <= 1 || d->w_strides[3] >= d->c) &&
-                         (d->r <= 1 || (d->s > 1 ? d->w_strides[2] == (long long)d->s * d->w_strides[3]
-                                                 : d->w_strides[2] % gran == 0)) &&
-                         aligned16(w);
+  const bool w_inplace = filter_in_place(d, w);
   const int c_pad = padded_channels(d->dtype, d->c);
   plan->c_padded = c_pad;
   plan->x_repacked = x_inplace ? 0 : 1;
@@ -716,6 +722,75 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
     }
   }
   return FDNN_OK;
+}
+
+// One activation copy per filter row (conv_rows_sm100.cu): whether a call that its plan sends to a tensor-core kernel runs
+// there instead, and on which tiles.  The layouts of x and of the packed filter stay those of the plan.  Measured kernels,
+// a copy per tap against this (bf16, channels-last, 3x3, microseconds): 256 -> 256 on 256 x 14 x 14 46.1 and 40.7, on
+// 128 images 31.1 and 22.7, on one 10.3 and 9.0; 64 -> 64 on 128 x 56 x 56 (four pixels per row before) 49.9 and 32.2;
+// 128 -> 128 on 128 x 28 x 28 34.7 and 25.1; 512 -> 512 on 128 x 7 x 7, an eighth of the walk rows no output, 30.5 and 27.6;
+// 104 -> 152 on 24 x 45 x 37 40.6 and 25.7; two groups 64 -> 128 on 256 x 56 x 56 (block-diagonal before) 122 and 72;
+// sixteen groups of 32 on 16 x 28 x 28 27.9 and 15.0.
+//   Where it lost: fewer pair tiles than pairs over one full channel block, nine steps in all (64 -> 128 on 8 x 28 x 28 5.5
+// and 5.9, on 16 x 28 x 28 6.4 and 7.0): those keep the smaller tiles of the single-CTA kernel.  With 32 channels or fewer
+// a copy per tap moves twice what it needs and this is ahead again (24 -> 24 on 112 x 112 10.4 and 7.0).
+//   Tiles: rounds of the pairs times what a step of a tile costs (172 / 257 / 513 clocks of MMAs for 64 / 128 / 256 columns).
+struct RowsMode {
+  int tile_n;          // 0: no
+  int pitch;           // walk rows per image row
+  int m_tiles, n_tiles, grid;
+  int blk_groups;      // groups per 64-channel block (1: not grouped)
+};
+// Every output pixel starts on a 32-byte boundary and its channels fill 32-byte pieces (16-bit types).
+bool sector_aligned(const fdnn_conv_desc& d, int oh, int ow, const void* y) {
+  return d.k % 16 == 0 && (reinterpret_cast<uintptr_t>(y) & 31u) == 0 && (d.n <= 1 || d.y_strides[0] % 16 == 0) &&
+         (oh <= 1 || d.y_strides[2] % 16 == 0) && (ow <= 1 || d.y_strides[3] % 16 == 0);
+}
+RowsMode rows_mode(const fdnn_conv_desc* d, int oh, int ow, const void* y) {
+  RowsMode g = {};
+  if (elem_size(d->dtype) != 2 || d->algo != FDNN_ALGO_AUTO || d->stride_w != 1 || d->s < 2 || (d->s - 1) * d->dil_w > kRowsCopy - 128)
+    return g;
+  fdnn_conv_desc one = *d;
+  one.groups = 1;
+  const int cg = d->c / d->groups, kg = d->k / d->groups;
+  if (!igemm_geometry_ok(&one) || oh < 1 || ow < 1 || cg < 8 || d->k < 8 || d->y_strides[1] != 1) return g;
+  g.pitch = d->w + (d->pad_left > d->pad_right ? d->pad_left : d->pad_right);
+  if (g.pitch - d->w - d->pad_left > 127 || ow > g.pitch) return g;
+  const long long walk = (long long)d->n * oh * g.pitch;
+  if (walk > 2000000000LL) return g;
+  const int sms = sm_count();
+  if (sms % 2 != 0) return g;
+  g.m_tiles = int((walk + 127) / 128);
+  g.blk_groups = 1;
+  if (d->groups > 1) {
+    if ((cg != 16 && cg != 32) || d->c % 64 != 0 || kg % 32 != 0 || !sector_aligned(*d, oh, ow, y)) return g;
+    g.blk_groups = 64 / cg;
+    const int bn = g.blk_groups * kg;
+    if (bn != 64 && bn != 128 && bn != 256) return g;
+    g.tile_n = bn;
+    g.n_tiles = d->c / 64;
+  } else {
+    int best = 0;
+    double best_cost = 1e300;
+    for (int bn = 64; bn <= 256; bn *= 2) {
+      if (bn > 64 && bn / 2 >= d->k) break;
+      const long long tiles = (long long)((g.m_tiles + 1) / 2) * ((d->k + bn - 1) / bn);
+      const double cost = double((tiles + sms / 2 - 1) / (sms / 2)) * (bn + 96);
+      if (cost <= best_cost) {
+        best_cost = cost;
+        best = bn;
+      }
+    }
+    g.tile_n = best;
+    g.n_tiles = (d->k + best - 1) / best;
+  }
+  const long long tiles = (long long)((g.m_tiles + 1) / 2) * g.n_tiles;
+  if (tiles < sms / 2 && d->c > 32 && d->c <= 64 && d->groups == 1) {
+    g.tile_n = 0;
+    return g;
+  }
+  g.grid = 2 * int(tiles < sms / 2 ? tiles : sms / 2);
+  return g;
 }
 
 // Several groups of a grouped 16-bit layer in one launch of the single-CTA kernel (see IgemmParams::groups), where that
@@ -889,17 +964,20 @@ CUtensorMapDataType tm_dtype(int dtype) {
 }
 
 // Activation map: NHWC tensor seen as (C, W, H, N); one copy brings 128 output
-// pixels x one 128-byte channel block for a single filter tap.
+// pixels x one 128-byte channel block for a single filter tap.  With a walk pitch (see conv_rows_sm100.cu) it walks
+// through rows of that many pixels, padding included, and brings kRowsCopy of them.
 int encode_activation_map(CUtensorMap* tm, int dtype, const void* base, int C, int W, int H, int N,
-                          long long sw, long long sh, long long sn, const fdnn_conv_desc* d, int groups = 1) {
+                          long long sw, long long sh, long long sn, const fdnn_conv_desc* d, int groups = 1,
+                          int walk_pitch = 0) {
   const int es = elem_size(dtype);
   cuuint64_t dims[4] = {cuuint64_t(C), cuuint64_t(W), cuuint64_t(H), cuuint64_t(N)};
   cuuint64_t strides[3] = {cuuint64_t(sw) * es, cuuint64_t(sh) * es, cuuint64_t(sn) * es};
   int lower[2] = {-d->pad_left, -d->pad_top};
   int upper[2] = {d->pad_right - (d->s - 1) * d->dil_w, d->pad_bottom - (d->r - 1) * d->dil_h};
+  if (walk_pitch > 0) upper[0] = walk_pitch - W - d->pad_left;   // the taps to the right are further rows of the copy
   cuuint32_t trav[4] = {1, cuuint32_t(d->stride_w), cuuint32_t(d->stride_h), 1};
   const cuuint32_t channels_per_pixel = 128 / es;
-  const cuuint32_t pixels_per_column = 128;
+  const cuuint32_t pixels_per_column = walk_pitch > 0 ? kRowsCopy : 128;
   // several groups in one launch: C channels per group, the images as the walk's third dimension, the groups behind them
   cuuint64_t dims5[5] = {cuuint64_t(C), cuuint64_t(W), cuuint64_t(H), cuuint64_t(N), cuuint64_t(groups)};
   cuuint64_t strides5[4] = {strides[0], strides[1], strides[2], cuuint64_t(C) * es};
@@ -1454,6 +1532,7 @@ static int prepare_device(int* device) {
     cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
     g_prepare_result[dev] = (major == 10) ? igemm_prepare_device() : cudaErrorNoKernelImageForDevice;
     if (g_prepare_result[dev] == cudaSuccess) g_prepare_result[dev] = igemm_pair_prepare_device();
+    if (g_prepare_result[dev] == cudaSuccess) g_prepare_result[dev] = rows_prepare_device();
     g_status_ptr[dev] = device_status_word();
   });
   if (g_prepare_result[dev] == cudaErrorNoKernelImageForDevice)
@@ -1462,6 +1541,110 @@ static int prepare_device(int* device) {
   std::call_once(g_driver_once, load_driver_entry_points);
   if (!g_driver_ok) return fail(FDNN_CUDA_ERROR, "driver entry points for tensor maps not found");
   *device = dev;
+  return FDNN_OK;
+}
+
+// Rewrites x into the scratch as dense NHWC where the plan says so, and says how the kernels see it.
+struct ActivationView {
+  const void* base;
+  int c;                       // channels that may be read
+  long long sw, sh, sn, plane; // element strides; offset of the second plane (fp32)
+};
+static int relayout_x(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, bool by_groups, const void* x, void* workspace,
+                      int64_t workspace_bytes, cudaStream_t stream, ActivationView* a) {
+  const int es = elem_size(d.dtype);
+  // Extent-one dimensions get a harmless aligned stride (theirs may be anything).
+  a->base = x;
+  a->c = by_groups ? d.c / d.groups : d.c;
+  a->sw = d.w > 1 ? d.x_strides[3] : plan.c_padded;
+  a->sh = d.h > 1 ? d.x_strides[2] : plan.c_padded;
+  a->sn = d.n > 1 ? d.x_strides[0] : plan.c_padded;
+  a->plane = 0;
+  if (!plan.x_repacked) return FDNN_OK;
+  int x_pad = by_groups ? d.c : padded_x_channels(&d);   // groups side by side, 16-byte multiples each
+  if (!by_groups && (long long)(d.dtype == FDNN_F32 ? 2 : 1) * d.n * d.h * d.w * x_pad * es > workspace_bytes)
+    x_pad = round_up(d.c, 16 / es);
+  a->plane = (long long)d.n * d.h * d.w * x_pad;
+  cudaError_t e = launch_repack_x(d.dtype, x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w, x_pad,
+                                  workspace, a->plane, stream);
+  if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
+  a->base = workspace;
+  a->sw = x_pad;
+  a->sh = (long long)d.w * x_pad;
+  a->sn = (long long)d.h * d.w * x_pad;
+  if (!by_groups) a->c = x_pad;
+  return FDNN_OK;
+}
+
+// The filter as the kernels of conv_rows_sm100.cu read it.
+struct FilterView {
+  const void* base;
+  int c, s_pitch, c_step;      // channels per tap, taps per filter row, first channel of group g: g * c_step
+  long long s_tap, s_k;
+};
+
+static int fwd_rows(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, const RowsMode& rows, int dev, const void* x,
+                    const FilterView& f, const void* bias, const void* scale, int activation, void* y, void* workspace,
+                    int64_t workspace_bytes, cudaStream_t stream) {
+  ActivationView a;
+  fdnn_conv_desc whole = d;    // a block of channels is copied whatever groups it holds
+  whole.groups = 1;
+  int st = relayout_x(whole, plan, false, x, workspace, workspace_bytes, stream, &a);
+  if (st != FDNN_OK) return st;
+  const int cg = d.c / d.groups, kg = d.k / d.groups;
+  alignas(64) CUtensorMap tmA, tmB;
+  st = encode_activation_map(&tmA, d.dtype, a.base, a.c, d.w, d.h, d.n, a.sw, a.sh, a.sn, &whole, 1, rows.pitch);
+  if (st != FDNN_OK) return st;
+  const bool blk = rows.blk_groups > 1;
+  RowsParams p = {};
+  p.M = d.n * plan.oh * rows.pitch;
+  p.Kout = d.k;
+  p.OH = plan.oh; p.OW = plan.ow;
+  p.P = rows.pitch;
+  p.stride_h = d.stride_h; p.pad_top = d.pad_top; p.pad_left = d.pad_left; p.dil_h = d.dil_h; p.dil_w = d.dil_w;
+  p.R = d.r; p.S = d.s;
+  p.s_pitch = f.s_pitch;
+  p.c_blocks = blk ? 1 : (d.c + 63) / 64;
+  p.m_tiles = rows.m_tiles;
+  p.n_tiles = rows.n_tiles;
+  p.blk_groups = rows.blk_groups;
+  p.cg = cg; p.kg = kg;
+  p.blk_c_step = f.c_step;
+  p.b_bytes = blk ? rows.blk_groups * (kg / 2) * cg * 2 : rows.tile_n / 2 * 128;
+  rows_stages(&p);
+  {
+    // (channel, filter, tap): one box per group (of a block of channels) and slot
+    cuuint64_t dims[3] = {cuuint64_t(f.c), cuuint64_t(d.k), cuuint64_t(d.r) * f.s_pitch};
+    cuuint64_t strides[2] = {cuuint64_t(f.s_k) * 2, cuuint64_t(f.s_tap) * 2};
+    cuuint32_t box[3] = {cuuint32_t(blk ? cg : 64), cuuint32_t(blk ? kg / 2 : rows.tile_n / 2), cuuint32_t(p.b_taps)};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = memo_encode_tiled(&tmB, tm_dtype(d.dtype), 3, const_cast<void*>(f.base), dims, strides, box, estr,
+                                   CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                   !blk ? CU_TENSOR_MAP_SWIZZLE_128B : cg == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(FDNN_CUDA_ERROR, "cuTensorMapEncodeTiled (filter rows) failed with CUresult " + std::to_string(int(r)));
+  }
+  p.y_sn = d.y_strides[0]; p.y_sk = 1; p.y_sh = d.y_strides[2]; p.y_sw = d.y_strides[3];
+  IgemmParams unit = {};
+  choose_strided_store(d, plan.oh, plan.ow, y, &unit);
+  p.y_unit = sector_aligned(d, plan.oh, plan.ow, y) ? 32 : unit.y_unit;
+  p.bias = bias; p.scale = scale; p.y = y;
+  p.act = activation;
+  IgemmParams dbg = {};
+  fill_debug_params(&dbg);
+  p.wait_limit = dbg.wait_limit;
+  p.skip_copies = dbg.skip_copies;
+  p.status = g_status_ptr[dev];
+  if (p.status == nullptr) return fail(FDNN_CUDA_ERROR, "status word address unavailable");
+  alignas(64) CUtensorMap tmY = tmA;
+  const long long row = y_pixel_stride(&d, plan.oh, plan.ow);
+  if (row > 0 && aligned16(y)) {
+    st = encode_output_map(&tmY, d.dtype, y, d.k, (long long)d.n * plan.oh * plan.ow, row);
+    if (st != FDNN_OK) return st;
+    p.y_rows = 1;
+  }
+  cudaError_t e = launch_rows(d.dtype, rows.tile_n, tmA, tmB, tmY, p, rows.grid, stream);
+  if (e != cudaSuccess) return fail_cuda("rows launch", e);
   return FDNN_OK;
 }
 
@@ -1500,6 +1683,23 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     return fail(FDNN_BAD_PARAM, "x, w and y must not be NULL");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
 
+  if (batch == nullptr && d.groups > 1 && plan.algo != FDNN_ALGO_DIRECT && allow_group && residual == nullptr) {
+    const RowsMode rows = rows_mode(&d, plan.oh, plan.ow, y);
+    const int cg = d.c / d.groups;
+    FilterView f = {w, cg, d.s, 0, d.s > 1 ? d.w_strides[3] : d.w_strides[2], d.w_strides[0]};
+    bool have = w != nullptr && filter_in_place(&d, w);
+    if (!have && group_dense_ok(&d) && w_packed != nullptr && aligned16(w_packed)) {
+      f = {w_packed, d.c, d.s, cg, d.c, (long long)d.r * d.s * d.c};   // the dense filter in front of the packed one
+      have = true;
+    }
+    if (rows.tile_n != 0 && have && (plan.x_repacked == 0 || (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 &&
+        workspace_bytes >= tight_x_bytes(&d)))) {
+      int dev = 0;
+      st = prepare_device(&dev);
+      if (st != FDNN_OK) return st;
+      return fwd_rows(d, plan, rows, dev, x, f, bias, scale, activation, y, workspace, workspace_bytes, stream);
+    }
+  }
   if (batch == nullptr && d.groups > 1 && plan.algo != FDNN_ALGO_DIRECT && allow_group) {
     const bool dense = group_dense_ok(&d);
     // where the filter of a group lies: in w itself, or (one launch per group) one after another in the packed buffer
@@ -1633,6 +1833,20 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     if (find_packed(w_packed, dev, &have) && !(have == want)) return fail_layout(have, want);
   }
 
+  if (batch == nullptr && residual == nullptr && allow_group && k_real == d.k && plan.low_channel == 0 &&
+      !(plan.x_repacked && d.c < 8)) {
+    const RowsMode rows = rows_mode(&d, plan.oh, plan.ow, y);
+    if (rows.tile_n != 0) {
+      const int c_pad = plan.c_padded;
+      FilterView f = {w, d.c, d.s, 0, d.s > 1 ? d.w_strides[3] : d.w_strides[2], d.k > 1 ? d.w_strides[0] : c_pad};
+      if (plan.w_packed) {
+        // a filter packed for Q grouped pixels starts with the filter of the first one, its taps in front of each row
+        const int s_pitch = plan.pixel_group > 1 ? d.s + (plan.pixel_group - 1) * d.stride_w : d.s;
+        f = {w_packed, c_pad, s_pitch, 0, c_pad, (long long)d.r * s_pitch * c_pad};
+      }
+      return fwd_rows(d, plan, rows, dev, x, f, bias, scale, activation, y, workspace, workspace_bytes, stream);
+    }
+  }
   if (plan.pixel_group > 1) {
     // run the equivalent convolution; its filter is the packed buffer, consumed in place
     const fdnn_conv_desc v = grouped_desc(&d, plan.pixel_group, plan.oh, plan.ow);
@@ -1645,38 +1859,22 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
 
   const int es = elem_size(d.dtype);
   const int c_pad = plan.c_padded;
-  const void* a_base = x;
-  // Extent-one dimensions get a harmless aligned stride (theirs may be anything).
   const long long any_stride = c_pad;
-  long long a_sw = d.w > 1 ? d.x_strides[3] : any_stride;
-  long long a_sh = d.h > 1 ? d.x_strides[2] : any_stride;
-  long long a_sn = d.n > 1 ? d.x_strides[0] : any_stride;
   const int groups = batch != nullptr ? d.groups : 1;
   const int k_group = d.k / groups;
-  int a_c = d.c / groups;
-  long long a_plane = 0;
   PixelWindows windows = {};
   if (plan.algo == FDNN_ALGO_IGEMM && plan.x_repacked && plan.w_packed && residual == nullptr && batch == nullptr)
     windows = pixel_windows(&d, plan.oh, plan.ow);
   if (windows.scratch > workspace_bytes) windows.ok = false;
+  ActivationView a = {};
   if (windows.ok) {
     e = launch_repack_x_windows(x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w, d.pad_left,
                                 windows.w_pad, workspace, stream);
     if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
-    a_base = workspace;
-  } else if (plan.x_repacked) {
-    int x_pad = batch != nullptr ? d.c : padded_x_channels(&d);   // groups side by side, 16-byte multiples each
-    if (batch == nullptr && (long long)(d.dtype == FDNN_F32 ? 2 : 1) * d.n * d.h * d.w * x_pad * es > workspace_bytes)
-      x_pad = round_up(d.c, 16 / es);
-    a_plane = (long long)d.n * d.h * d.w * x_pad;
-    e = launch_repack_x(d.dtype, x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w,
-                        x_pad, workspace, a_plane, stream);
-    if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
-    a_base = workspace;
-    a_sw = x_pad;
-    a_sh = (long long)d.w * x_pad;
-    a_sn = (long long)d.h * d.w * x_pad;
-    if (batch == nullptr) a_c = x_pad;
+    a.base = workspace;
+  } else {
+    st = relayout_x(d, plan, batch != nullptr, x, workspace, workspace_bytes, stream, &a);
+    if (st != FDNN_OK) return st;
   }
   const bool b_mn = !plan.w_packed && filter_mn_major(&d, w);
   const void* b_base = w;
@@ -1698,9 +1896,9 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     cuuint64_t strides[3] = {cuuint64_t(d.stride_w) * 16, cuuint64_t(windows.w_pad) * 16, cuuint64_t(d.h) * windows.w_pad * 16};
     cuuint32_t box[4] = {64, cuuint32_t(plan.ow), cuuint32_t(windows.ohs * d.stride_h), 1};
     cuuint32_t estr[4] = {1, 1, cuuint32_t(d.stride_h), 1};
-    st = encode_tiled(&tmA, d.dtype, a_base, 4, dims, strides, box, estr, "pixel windows");
+    st = encode_tiled(&tmA, d.dtype, a.base, 4, dims, strides, box, estr, "pixel windows");
   } else {
-    st = encode_activation_map(&tmA, d.dtype, a_base, a_c, d.w, d.h, d.n, a_sw, a_sh, a_sn, &d, groups);
+    st = encode_activation_map(&tmA, d.dtype, a.base, a.c, d.w, d.h, d.n, a.sw, a.sh, a.sn, &d, groups);
   }
   if (st != FDNN_OK) return st;
   const int b_box_rows = plan.algo == FDNN_ALGO_IGEMM_PAIR ? 128 : plan.tile_n;  // each CTA of a pair stages half
@@ -1717,8 +1915,8 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   }
   if (st != FDNN_OK) return st;
   if (d.dtype == FDNN_F32) {
-    st = encode_activation_map(&tmA2, d.dtype, static_cast<const char*>(a_base) + a_plane * es, a_c, d.w,
-                               d.h, d.n, a_sw, a_sh, a_sn, &d);
+    st = encode_activation_map(&tmA2, d.dtype, static_cast<const char*>(a.base) + a.plane * es, a.c, d.w,
+                               d.h, d.n, a.sw, a.sh, a.sn, &d);
     if (st != FDNN_OK) return st;
     st = encode_filter_map(&tmB2, d.dtype, static_cast<const char*>(b_base) + b_plane * es, b_c,
                            d.r * d.s, d.k, b_stap, b_sk, plan.tile_n);

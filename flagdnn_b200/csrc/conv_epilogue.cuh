@@ -433,7 +433,8 @@ __device__ __forceinline__ void strided_odd_channels(char* out, uint32_t sbuf, i
   }
 }
 
-template <typename T, int BN, bool RES>
+// NBUF staging buffers of 4 KB per warp.
+template <typename T, int BN, bool RES, int NBUF = 2>
 __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, int kout, int act, const float* s_scale,
                                                        const float* s_bias, uint8_t* my_out, int lane,
                                                        const StridedOut& o, uint32_t& store_seq) {
@@ -465,7 +466,7 @@ __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, i
     uint32_t raw[kLoads][32];
 #pragma unroll
     for (int l = 0; l < kLoads; ++l) tmem_ld_32x32b_x32(t_row + g * kCols + l * 32, raw[l]);
-    uint8_t* buf = my_out + (store_seq & 1u) * (32 * 128);
+    uint8_t* buf = my_out + (NBUF == 2 ? (store_seq & 1u) * (32 * 128) : 0u);
     ++store_seq;
     const int col0 = n0 + g * kCols;
     const int nc = kout - col0 < kCols ? kout - col0 : kCols;    // columns of this group that exist
@@ -507,6 +508,7 @@ __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, i
       }
     }
     const uint32_t sbuf = smem_u32(buf);
+    if constexpr (NBUF == 1) __syncwarp();   // the group before has been read
     if (o.mode == kYPixels) {
       if constexpr (kEs == 4) {
 #pragma unroll
@@ -538,6 +540,55 @@ __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, i
       else if (o.unit == 16) strided_channels<uint4, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
       else if (o.unit == 8) strided_channels<uint2, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
       else strided_channels<uint32_t, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
+    }
+  }
+}
+
+// Epilogue for 16-bit y along channels whose pixels start on 32-byte boundaries (a multiple of 16 channels, or views that
+// keep that): a lane writes its own pixel from the registers, 16 channels (one whole 32-byte sector) per store, without
+// staging.  y: the lane's pixel, first column of the warp's share; ok: the pixel exists.
+// read_done() is called once, when the accumulator has been read and before its last columns are stored.
+template <typename T, int WC, typename Done>
+__device__ __forceinline__ void epilogue_store_sectors(uint32_t t_row, int n0, int kout, int act, const float* s_scale,
+                                                       const float* s_bias, bool use_scale, T* y, bool ok, Done&& read_done) {
+  int chunks = (kout - n0 + 31) / 32;
+  if (chunks > WC / 32) chunks = WC / 32;
+  if (chunks <= 0) {
+    read_done();
+    return;
+  }
+  uint32_t raw[32];
+  tmem_ld_32x32b_x32(t_row, raw);
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    tmem_ld_wait();
+    float v[32];
+#pragma unroll
+    for (int j4 = 0; j4 < 8; ++j4) {
+      const float4 sc = use_scale ? reinterpret_cast<const float4*>(s_scale + c * 32)[j4] : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+      const float4 bi = reinterpret_cast<const float4*>(s_bias + c * 32)[j4];
+      v[4 * j4 + 0] = fmaf(__uint_as_float(raw[4 * j4 + 0]), sc.x, bi.x);
+      v[4 * j4 + 1] = fmaf(__uint_as_float(raw[4 * j4 + 1]), sc.y, bi.y);
+      v[4 * j4 + 2] = fmaf(__uint_as_float(raw[4 * j4 + 2]), sc.z, bi.z);
+      v[4 * j4 + 3] = fmaf(__uint_as_float(raw[4 * j4 + 3]), sc.w, bi.w);
+    }
+    if (c + 1 < chunks) tmem_ld_32x32b_x32(t_row + (c + 1) * 32, raw);   // travels while this chunk is rounded and stored
+    else read_done();
+    uint32_t row[16];
+    if (act == 1) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) row[j] = round_pack2_relu<T>(v[2 * j], v[2 * j + 1]);
+    } else {
+      if (act) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = apply_activation(v[j], act);
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) row[j] = round_pack2<T>(v[2 * j], v[2 * j + 1]);
+    }
+    if (ok) {
+      if (n0 + c * 32 + 16 <= kout) stg_v8(y + c * 32, row);
+      if (n0 + c * 32 + 32 <= kout) stg_v8(y + c * 32 + 16, row + 8);
     }
   }
 }

@@ -189,8 +189,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         if (rank == 0) mbar_arrive_expect_tx(bres_bar, uint32_t(2 * k_iters * kBBytes));
         int kit = 0;
         for (int r = 0; r < p.R; ++r)
-          for (int s = 0; s < p.S; ++s)
-            for (int cb = 0; cb < p.c_blocks; ++cb, ++kit)
+          for (int cb = 0; cb < p.c_blocks; ++cb)
+            for (int s = 0; s < p.S; ++s, ++kit)
               tma_load_3d_pair(b_res + kit * kBBytes, &tmB, bres, cb * kKB, r * p.S + s, int(rank) * kHalfN);
       }
       TileWalk walk;
@@ -237,11 +237,11 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           h_base = 0;
         }
         ++tiles_done;
-        // reduction step kit = (r * S + s) * c_blocks + cb
-        int tap = walk.kb / p.c_blocks;
-        int cb = walk.kb - tap * p.c_blocks;
-        int r = tap / p.S;
-        int s_ = tap - r * p.S;
+        // reduction step kit = (r * c_blocks + cb) * S + s, the order of conv_rows_sm100.cu (same fp32 sums, bit for bit)
+        const int row = walk.kb / p.S;
+        int s_ = walk.kb - row * p.S;
+        int r = row / p.c_blocks;
+        int cb = row - r * p.c_blocks;
         auto copy_steps = [&](auto prof_tag) {
           constexpr bool kProf = decltype(prof_tag)::value;
           for (int kit = walk.kb; kit < walk.ke; ++kit) {
@@ -273,10 +273,10 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
               stage = 0;
               phase ^= 1u;
             }
-            if (++cb == p.c_blocks) {
-              cb = 0;
-              if (++s_ == p.S) {
-                s_ = 0;
+            if (++s_ == p.S) {
+              s_ = 0;
+              if (++cb == p.c_blocks) {
+                cb = 0;
                 ++r;
               }
             }

@@ -252,10 +252,10 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           stage = 0;
           phase ^= 1u;
         }
-        if (++cb == p.c_blocks) {
-          cb = 0;
-          if (++s == p.S) {
-            s = 0;
+        if (++s == p.S) {   // the order of conv_rows_sm100.cu, so that the fp32 sums agree bit for bit
+          s = 0;
+          if (++cb == p.c_blocks) {
+            cb = 0;
             ++r;
           }
         }

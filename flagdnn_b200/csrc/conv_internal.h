@@ -113,6 +113,38 @@ int igemm_pair_stages();
 int igemm_pair_threads();
 int igemm_pair_max_resident_steps();  // reductions this short (and one channel tile) keep the filter resident
 
+// CTA pairs with one activation copy per filter row (conv_rows_sm100.cu): 16-bit types, W-stride 1, y along channels.
+constexpr int kRowsCopy = 136;   // walk rows of an activation copy: a tile's 128 and up to 8 for the taps to its right
+struct RowsParams {
+  int M;                 // N * OH * P walk rows
+  int Kout, OH, OW;
+  int P;                 // walk rows per image row
+  int stride_h, pad_top, pad_left, dil_h, dil_w;
+  int R, S;
+  int s_pitch;           // taps per filter row in memory (S, or more where the filter lies packed for grouped pixels)
+  int c_blocks;          // 64-channel blocks of a reduction (1 with blk_groups > 1)
+  int m_tiles, n_tiles;
+  int b_bytes;           // one CTA's filters of a tap and channel block
+  int a_stages, b_stages, b_resident, b_taps, b_slot;   // rings (rows_stages): copies, slots, whole filter, a slot's taps and bytes
+  int blk_groups;        // > 1: groups of a 64-channel block, of cg channels and kg filters each; column tiles are blocks
+  int cg, kg;
+  int blk_c_step;        // first channel of group g in the filter map: g * blk_c_step
+  long long y_sn, y_sk, y_sh, y_sw;
+  int y_unit;            // bytes per lane and store: 32 where every pixel starts on 32 bytes (grouped layers: always)
+  int y_rows;            // 1: y is one dense [pixels, K] matrix with a TMA map
+  const void* bias;
+  const void* scale;
+  void* y;
+  int act;
+  uint32_t* status;
+  long long wait_limit;
+  int skip_copies;
+};
+void rows_stages(RowsParams* p);
+cudaError_t launch_rows(int dtype, int tile_n, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY,
+                        const RowsParams& p, int grid, cudaStream_t stream);
+cudaError_t rows_prepare_device();
+
 // Direct convolution on CUDA cores (conv_direct.cu): any dtype, groups, strides.
 struct DirectParams {
   int N, C, H, W, K, R, S, OH, OW;

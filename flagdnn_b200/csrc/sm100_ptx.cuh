@@ -65,6 +65,12 @@ __device__ __forceinline__ void sts_u16(uint32_t a, uint16_t v) {
 __device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v) {
   asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
+// 32 bytes to global memory in one store (32-byte aligned).
+__device__ __forceinline__ void stg_v8(void* p, const uint32_t* v) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
 __device__ __forceinline__ void sts_v4(uint32_t a, uint4 v) {
   asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -414,6 +420,11 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// The same without ordering this thread's earlier global stores for the whole cluster: a release at cluster scope waits
+// until they are performed.  For hand-overs of tensor memory, which tcgen05 fences order.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 // Pair forms of the copies: data lands in THIS CTA's shared memory, the
 // completion bytes are credited to the mbarrier at `bar_cluster_addr`, which
 // may live in the partner CTA (the leader's "stage full" barrier).
@@ -471,6 +482,19 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster_addr) {
                    bar_cluster_addr)
                : "memory");
 }
+// High word of make_sw128_kmajor_desc; the low word is (address >> 4) | 1 << 16.
+constexpr uint32_t kSw128DescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+// ... and of K-major rows of 64 and 32 bytes in the swizzle of that width (eight rows take 512 and 256 bytes).
+constexpr uint32_t kSw64DescHi = (512u >> 4) | (1u << 14) | (4u << 29), kSw32DescHi = (256u >> 4) | (1u << 14) | (6u << 29);
+__device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t smem_addr) { return (smem_addr >> 4) | (1u << 16); }
+
+// The same arrival on the barrier at this offset in both CTAs of the pair.
+__device__ __forceinline__ void tc_commit_both(uint32_t bar_addr) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar_addr),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
+}
 __device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -481,6 +505,66 @@ __device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, u
       "}\n"
       :
       : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// Four of them over 64 reduction elements, from the low words of the two descriptors (the high word is the same for both):
+// `acc0` of the first, the others add; the operands advance by 2 and kBStep descriptor units.  What the issuing thread does
+// between two MMAs bounds narrow tiles, so that the descriptors are put together in place.
+#define FDNN_MMA4(GROUP)                                        \
+  asm volatile(                                                 \
+      "{\n\t"                                                   \
+      ".reg .pred p, q;\n\t"                                    \
+      ".reg .b64 a, b;\n\t"                                     \
+      ".reg .b32 x, y;\n\t"                                     \
+      "setp.ne.b32 p, %5, 0;\n\t"                               \
+      "setp.eq.b32 q, 0, 0;\n\t"                                \
+      "mov.b64 a, {%1, %3};\n\t"                                \
+      "mov.b64 b, {%2, %3};\n\t"                                \
+      "tcgen05.mma." GROUP ".kind::f16 [%0], a, b, %4, p;\n\t"  \
+      "add.u32 x, %1, 2;\n\t"                                   \
+      "add.u32 y, %2, %6;\n\t"                                  \
+      "mov.b64 a, {x, %3};\n\t"                                 \
+      "mov.b64 b, {y, %3};\n\t"                                 \
+      "tcgen05.mma." GROUP ".kind::f16 [%0], a, b, %4, q;\n\t"  \
+      "add.u32 x, %1, 4;\n\t"                                   \
+      "add.u32 y, %2, %7;\n\t"                                  \
+      "mov.b64 a, {x, %3};\n\t"                                 \
+      "mov.b64 b, {y, %3};\n\t"                                 \
+      "tcgen05.mma." GROUP ".kind::f16 [%0], a, b, %4, q;\n\t"  \
+      "add.u32 x, %1, 6;\n\t"                                   \
+      "add.u32 y, %2, %8;\n\t"                                  \
+      "mov.b64 a, {x, %3};\n\t"                                 \
+      "mov.b64 b, {y, %3};\n\t"                                 \
+      "tcgen05.mma." GROUP ".kind::f16 [%0], a, b, %4, q;\n\t"  \
+      "}\n"                                                     \
+      :                                                         \
+      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "n"(kSw128DescHi), "r"(idesc), "r"(acc0), "n"(kBStep), "n"(2 * kBStep), "n"(3 * kBStep) \
+      : "memory")
+template <int kBStep = 2>
+__device__ __forceinline__ void mma4_f16(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc0) {
+  FDNN_MMA4("cta_group::1");
+}
+template <int kBStep = 2>
+__device__ __forceinline__ void mma4_f16_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc0) {
+  FDNN_MMA4("cta_group::2");
+}
+#undef FDNN_MMA4
+
+// One of them from the low words of its descriptors and their constant high words.
+template <uint32_t kAHi, uint32_t kBHi>
+__device__ __forceinline__ void mma_f16_pair_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "mov.b64 a, {%1, %3};\n\t"
+      "mov.b64 b, {%2, %4};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %5, p;\n\t"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "n"(kAHi), "n"(kBHi), "r"(idesc), "r"(acc)
       : "memory");
 }
 
