@@ -124,7 +124,6 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();         // 0 = leader
-  const uint32_t peer = rank ^ 1u;
 
   griddep_launch_dependents();  // all CTAs of this grid are resident: the next launch may queue behind them
   if (threadIdx.x == 0) {
@@ -140,8 +139,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     mbar_init(&raw_empty[1], 1);
     mbar_init(&tmem_full[0], 1);
     mbar_init(&tmem_full[1], 1);
-    mbar_init(&tmem_empty[0], 2 * kEpiWarpsPair * 32);  // epilogue threads of both CTAs
-    mbar_init(&tmem_empty[1], 2 * kEpiWarpsPair * 32);
+    mbar_init(&tmem_empty[0], 2 * kEpiWarpsPair);  // epilogue warps of both CTAs
+    mbar_init(&tmem_empty[1], 2 * kEpiWarpsPair);
     mbar_init(drain_bar, 1);
     if constexpr (RES) {
       for (int i = 0; i < kEpiWarpsPair; ++i) mbar_init(&res_bar[i], 1);
@@ -305,9 +304,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         alive = mbar_wait_bounded(bres_bar, 0u, abort_flag, p.status, kIncidentMmaWaitFull, p.wait_limit);
       }
       const uint32_t empty_own = smem_u32(&empty_bar[0]);
-      const uint32_t empty_peer = map_to_cta(empty_own, 1);
       const uint32_t tfull_own = smem_u32(&tmem_full[0]);
-      const uint32_t tfull_peer = map_to_cta(tfull_own, 1);
+      const uint32_t ring_lo = sw128_desc_lo(smem_u32(stage_base)), b_res_lo = sw128_desc_lo(smem_u32(b_res));
       const uint32_t raw_empty_peer = map_to_cta(smem_u32(&raw_empty[0]), 1);
       const int k16 = p.k16_per_step;  // 16-element reduction slices per step that hold data (4, or 3)
       TileWalk walk;
@@ -325,7 +323,10 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * kPairN;
         // The reduction loop is the hot path of every layer and is sensitive to anything beside the wait, the
-        // MMAs and the commits (a conditional barrier arrive in it cost 17 % on the 3x3 256-channel layer):
+        // MMAs and the commits (a conditional barrier arrive in it cost 17 % on the 3x3 256-channel layer; descriptors
+        // put together in place, one commit for both CTAs, a first look at the barrier without the suspend-time hint and
+        // one hand-over of the accumulator per epilogue warp instead of per thread took 1024 -> 2048 1x1 stride 2 on
+        // 128 x 14 x 14 from 27.1 to 25.8 us, 32 x 1024 rows of a 4096 x 4096 product from 179.7 to 177.1):
         // it exists once with four MMAs per step and once with a runtime count for the 3-channel mode.
         auto reduce = [&](auto four_tag, auto prof_tag) {
           constexpr bool kFour = decltype(four_tag)::value;
@@ -333,30 +334,23 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           for (int kit = walk.kb; kit < walk.ke; ++kit) {
             long long mt1 = 0;
             if constexpr (kProf) mt1 = clock64();
-            if (!mbar_wait_bounded(&full_bar[stage], phase, abort_flag, p.status, kIncidentMmaWaitFull, p.wait_limit)) {
+            if (!mbar_try_wait_now(&full_bar[stage], phase) &&
+                !mbar_wait_bounded(&full_bar[stage], phase, abort_flag, p.status, kIncidentMmaWaitFull, p.wait_limit)) {
               alive = false;
               break;
             }
             if constexpr (kProf) prof_wfull += clock64() - mt1;
             tc_fence_after();
-            const uint32_t st = smem_u32(stage_base + stage * stage_stride);
-            const uint32_t bt = b_resident ? smem_u32(b_res + kit * kBBytes) : st + kABytes;
+            const uint32_t a_lo = ring_lo + stage * uint32_t(stage_stride / 16);
+            const uint32_t b_lo = b_resident ? b_res_lo + kit * (kBBytes / 16) : a_lo + kABytes / 16;
+            const uint32_t acc = kit > walk.kb ? 1u : 0u;
             if constexpr (kFour) {
-#pragma unroll
-              for (int k = 0; k < kKB / 16; ++k) {
-                const uint64_t a = make_sw128_kmajor_desc(st + k * 32);
-                const uint64_t b = make_sw128_kmajor_desc(bt + k * 32);
-                mma_f16_pair(d_tmem, a, b, kIdesc, (kit > walk.kb || k > 0) ? 1u : 0u);
-              }
+              mma4_f16_pair(d_tmem, a_lo, b_lo, kIdesc, acc);
             } else {
-              for (int k = 0; k < k16; ++k) {
-                const uint64_t a = make_sw128_kmajor_desc(st + k * 32);
-                const uint64_t b = make_sw128_kmajor_desc(bt + k * 32);
-                mma_f16_pair(d_tmem, a, b, kIdesc, (kit > walk.kb || k > 0) ? 1u : 0u);
-              }
+              for (uint32_t k = 0; k < uint32_t(k16); ++k)
+                mma_f16_pair_lo<kSw128DescHi, kSw128DescHi>(d_tmem, a_lo + 2 * k, b_lo + 2 * k, kIdesc, k == 0 ? acc : 1u);
             }
-            tc_commit_pair(empty_own + stage * 8);
-            tc_commit_pair(empty_peer + stage * 8);
+            tc_commit_both(empty_own + stage * 8);
             if (++stage == uint32_t(n_stages)) {
               stage = 0;
               phase ^= 1u;
@@ -371,8 +365,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           reduce(std::true_type{}, std::true_type{});   // cycle counters of the role (development aid)
         }
         if (alive) {
-          tc_commit_pair(tfull_own + buf * 8);
-          tc_commit_pair(tfull_peer + buf * 8);
+          tc_commit_both(tfull_own + buf * 8);
           if (p.fused3) {
             // every window copy of this tile has landed in both CTAs (all of its "stage full" barriers were
             // passed above): their converters may reuse the scratch slot
@@ -594,7 +587,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         __syncwarp();
         if (lane == 0) sk_flag_release(p.sk_flags + blockIdx.x * kSkFlagsPerCta + my_warp, 1u);
         tc_fence_before();
-        mbar_arrive_cluster(tempty_leader + buf * 8);
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(tempty_leader + buf * 8);
         continue;
       }
       int sk_count = 0;
@@ -645,7 +639,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             p.sk_flags[(2 * (pair_id - 1 - c) + int(rank)) * kSkFlagsPerCta + my_warp] = 0u;
       }
       tc_fence_before();
-      mbar_arrive_cluster(tempty_leader + buf * 8);
+      __syncwarp();
+      if (lane == 0) mbar_arrive_remote(tempty_leader + buf * 8);
     }
     if (lane == 0) bulk_wait_group0();
     if (p.prof && blockIdx.x == 0 && threadIdx.x == 32 * kFirstEpiWarpPair) {  // first epilogue warp of the first leader

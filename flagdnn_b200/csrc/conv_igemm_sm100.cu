@@ -136,8 +136,8 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     mbar_init(&tmem_full[0], 1);
     mbar_init(&tmem_full[1], 1);
-    mbar_init(&tmem_empty[0], Cfg::kActiveEpiWarps * 32);
-    mbar_init(&tmem_empty[1], Cfg::kActiveEpiWarps * 32);
+    mbar_init(&tmem_empty[0], Cfg::kActiveEpiWarps);
+    mbar_init(&tmem_empty[1], Cfg::kActiveEpiWarps);
     mbar_init(drain_bar, 1);
     if constexpr (RES) {
       for (int i = 0; i < 16; ++i) mbar_init(&res_bar[i], 1);
@@ -304,8 +304,9 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // The whole warp walks the loop and one elected lane issues, so that descriptors and addresses are uniform values:
     // what the issuing thread does between two MMAs bounds the reduction step of tiles up to 128 columns.  A lane that
     // walks alone, building each descriptor anew and waiting with the suspend-time hint, needs 433 clocks per step of
-    // four MMAs (64 clocks of issue each, 45 for the commit, 135 for the wait); this loop needs 254 (64 columns), 268
-    // (128) and 513 (256, where the MMAs themselves are the limit).
+    // four MMAs (64 clocks of issue each, 45 for the commit, 135 for the wait); as a whole warp 254 (64 columns), 268 (128)
+    // and 513 (256, where the MMAs themselves are the limit).  The four MMAs are one block with their descriptors put
+    // together in place: 227 and 257 clocks for 64 and 128 columns in a loop over 64-bit descriptors, 192 at best.
     const bool lead = elect_one();
     uint32_t stage = 0, phase = 0;
     uint32_t tcount = 0;
@@ -339,23 +340,21 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           tc_fence_after();
           if (lead) {
             const uint32_t st = ring + stage * Cfg::kStageBytes;
-            const uint64_t a0 = make_sw128_kmajor_desc(st);
-            const uint64_t b0 = kMn ? make_sw128_mnmajor_desc(st + Cfg::kABytes)
-                                    : make_sw128_kmajor_desc(st + (Cfg::kSplit ? 2 : 1) * Cfg::kABytes);
+            const uint32_t a_lo = sw128_desc_lo(st);
+            const uint32_t acc = kit > 0 ? 1u : 0u;
+            if constexpr (Cfg::kSplit) {
+              const uint32_t b_lo = sw128_desc_lo(st + 2 * Cfg::kABytes);
+              constexpr uint32_t kALow = Cfg::kABytes / 16, kBLow = Cfg::kBBytes / 16;   // from the high halves to the low ones
 #pragma unroll
-            for (int k = 0; k < Cfg::kKB / Cfg::kUK; ++k) {
-              // 32 bytes of reduction elements further (the address field counts 16-byte units)
-              const uint64_t a = a0 + uint64_t(k * 2);
-              const uint64_t b = b0 + uint64_t(k * (kMn ? int(kMnStepBytes / 16) : 2));
-              const uint32_t acc = (kit > 0 || k > 0) ? 1u : 0u;
-              if constexpr (Cfg::kSplit) {
-                const uint64_t a_lo = a + uint64_t(Cfg::kABytes / 16), b_lo = b + uint64_t(Cfg::kBBytes / 16);
-                mma_tf32(d_tmem, a_lo, b, kIdesc, acc);
-                mma_tf32(d_tmem, a, b_lo, kIdesc, 1u);
-                mma_tf32(d_tmem, a, b, kIdesc, 1u);
-              } else {
-                mma_f16(d_tmem, a, b, kMn ? (kIdesc | kIdescBMnMajor) : kIdesc, acc);
+              for (uint32_t k = 0; k < 8; k += 2) {   // 32 bytes of reduction elements further: two descriptor units
+                mma_tf32(d_tmem, a_lo + kALow + k, b_lo + k, kIdesc, k == 0 ? acc : 1u);
+                mma_tf32(d_tmem, a_lo + k, b_lo + kBLow + k, kIdesc, 1u);
+                mma_tf32(d_tmem, a_lo + k, b_lo + k, kIdesc, 1u);
               }
+            } else if constexpr (kMn) {
+              mma4_f16<int(kMnStepBytes / 16)>(d_tmem, a_lo, mnmajor_desc_lo(st + Cfg::kABytes), kIdesc | kIdescBMnMajor, acc);
+            } else {
+              mma4_f16(d_tmem, a_lo, sw128_desc_lo(st + Cfg::kABytes), kIdesc, acc);
             }
             tc_commit(&empty_bar[stage]);
           }
@@ -521,7 +520,8 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
       }
       tc_fence_before();
-      mbar_arrive(&tmem_empty[buf]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tmem_empty[buf]);   // one arrival per warp
     }
     if (DENSE && lane == 0) bulk_wait_group0();  // stores must be done before the CTA retires
     if (p.prof && blockIdx.x == 0 && threadIdx.x == 32 * kFirstEpiWarp) {  // first epilogue warp

@@ -326,6 +326,29 @@ __device__ __forceinline__ void fence_proxy_async_all() {
   asm volatile("fence.proxy.async;" ::: "memory");
 }
 
+// Shared-memory matrix descriptor for a K-major operand tile whose rows are
+// 128 bytes wide and stored with the 128-byte swizzle (what a TMA box with
+// CU_TENSOR_MAP_SWIZZLE_128B produces): 8-row groups are 1024 bytes apart.
+//   bits [0,14)  start address >> 4
+//   bits [16,30) leading byte offset >> 4 (unused for swizzled K-major; 1)
+//   bits [32,46) stride byte offset >> 4  (1024 >> 4 = 64)
+//   bits [46,48) descriptor version (1 on sm_100)
+//   bits [61,64) layout type (2 = SWIZZLE_128B)
+// The high word is a constant of the layout, the low word names the place.
+constexpr uint32_t kSw128DescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+// ... of K-major rows of 64 and 32 bytes in the swizzle of that width (eight rows take 512 and 256 bytes)
+constexpr uint32_t kSw64DescHi = (512u >> 4) | (1u << 14) | (4u << 29), kSw32DescHi = (256u >> 4) | (1u << 14) | (6u << 29);
+__device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t smem_addr) { return (smem_addr >> 4) | (1u << 16); }
+
+// The same for an operand stored MN-major (its rows run along M or N, one reduction element each): boxes of 64 M/N
+// elements (128 bytes) x 64 reduction rows, 128-byte swizzle, one after another.  Eight reduction rows take 1024 bytes
+// (stride byte offset), the next 64 M/N elements are one 8192-byte box further (leading byte offset); an MMA's 16
+// reduction elements take 2048 bytes.  The instruction descriptor says so with kIdescBMnMajor.
+// The high word of the descriptor is that of the K-major form.
+constexpr uint32_t kMnBoxElems = 64, kMnBoxBytes = 8192, kMnStepBytes = 2048;
+__device__ __forceinline__ uint32_t mnmajor_desc_lo(uint32_t smem_addr) { return (smem_addr >> 4) | (kMnBoxBytes >> 4) << 16; }
+constexpr uint32_t kIdescBMnMajor = 1u << 16;
+
 // ----------------------------------------------------------------- tcgen05
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -351,32 +374,6 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                    smem_u32(bar))
                : "memory");
-}
-
-// D[tmem] (+)= A[smem] * B[smem]; kind::f16 covers f16 and bf16 operands.
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                        uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                         uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 
 // 32 consecutive fp32 accumulator columns of this thread's TMEM lane.
@@ -482,12 +479,6 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster_addr) {
                    bar_cluster_addr)
                : "memory");
 }
-// High word of make_sw128_kmajor_desc; the low word is (address >> 4) | 1 << 16.
-constexpr uint32_t kSw128DescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
-// ... and of K-major rows of 64 and 32 bytes in the swizzle of that width (eight rows take 512 and 256 bytes).
-constexpr uint32_t kSw64DescHi = (512u >> 4) | (1u << 14) | (4u << 29), kSw32DescHi = (256u >> 4) | (1u << 14) | (6u << 29);
-__device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t smem_addr) { return (smem_addr >> 4) | (1u << 16); }
-
 // The same arrival on the barrier at this offset in both CTAs of the pair.
 __device__ __forceinline__ void tc_commit_both(uint32_t bar_addr) {
   asm volatile(
@@ -495,20 +486,7 @@ __device__ __forceinline__ void tc_commit_both(uint32_t bar_addr) {
       "h"(static_cast<uint16_t>(3))
       : "memory");
 }
-__device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                             uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Four of them over 64 reduction elements, from the low words of the two descriptors (the high word is the same for both):
+// Four MMAs D[tmem] (+)= A[smem] * B[smem] (kind::f16 covers f16 and bf16) over 64 reduction elements, from the low words of the two descriptors (the high word is the same for both):
 // `acc0` of the first, the others add; the operands advance by 2 and kBStep descriptor units.  What the issuing thread does
 // between two MMAs bounds narrow tiles, so that the descriptors are put together in place.
 #define FDNN_MMA4(GROUP)                                        \
@@ -551,7 +529,7 @@ __device__ __forceinline__ void mma4_f16_pair(uint32_t d_tmem, uint32_t a_lo, ui
 }
 #undef FDNN_MMA4
 
-// One of them from the low words of its descriptors and their constant high words.
+// One MMA of a CTA pair, from the low words of its descriptors and their constant high words.
 template <uint32_t kAHi, uint32_t kBHi>
 __device__ __forceinline__ void mma_f16_pair_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
   asm volatile(
@@ -568,39 +546,21 @@ __device__ __forceinline__ void mma_f16_pair_lo(uint32_t d_tmem, uint32_t a_lo, 
       : "memory");
 }
 
-// Shared-memory matrix descriptor for a K-major operand tile whose rows are
-// 128 bytes wide and stored with the 128-byte swizzle (what a TMA box with
-// CU_TENSOR_MAP_SWIZZLE_128B produces): 8-row groups are 1024 bytes apart.
-//   bits [0,14)  start address >> 4
-//   bits [16,30) leading byte offset >> 4 (unused for swizzled K-major; 1)
-//   bits [32,46) stride byte offset >> 4  (1024 >> 4 = 64)
-//   bits [46,48) descriptor version (1 on sm_100)
-//   bits [61,64) layout type (2 = SWIZZLE_128B)
-__device__ __forceinline__ uint64_t make_sw128_kmajor_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3ffff) >> 4);
-  d |= static_cast<uint64_t>(1) << 16;
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
+// fp32 operands as TF32 (one CTA): low descriptor words of K-major rows in the 128-byte swizzle.
+__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 a, {%1, %3};\n\t"
+      "mov.b64 b, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], a, b, %4, p;\n\t"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "n"(kSw128DescHi), "r"(idesc), "r"(acc)
+      : "memory");
 }
-
-// The same for an operand stored MN-major (its rows run along M or N, one reduction element each): boxes of 64 M/N
-// elements (128 bytes) x 64 reduction rows, 128-byte swizzle, one after another.  Eight reduction rows take 1024 bytes
-// (stride byte offset), the next 64 M/N elements are one 8192-byte box further (leading byte offset); an MMA's 16
-// reduction elements take 2048 bytes.  The instruction descriptor says so with kIdescBMnMajor.
-constexpr uint32_t kMnBoxElems = 64, kMnBoxBytes = 8192, kMnStepBytes = 2048;
-__device__ __forceinline__ uint64_t make_sw128_mnmajor_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3ffff) >> 4);
-  d |= static_cast<uint64_t>(kMnBoxBytes >> 4) << 16;
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
-constexpr uint32_t kIdescBMnMajor = 1u << 16;
 
 // Instruction descriptor: fp32 accumulate, both operands K-major, dense.
 //   bits [4,6) D format (1 = f32); [7,10) A format; [10,13) B format
