@@ -346,18 +346,13 @@ fdnn_conv_desc grouped_desc(const fdnn_conv_desc* d, int q, int oh, int ow) {
 }
 
 // A one-tap filter whose K dimension is contiguous (mm's second operand, [C][K] row-major with rows of 16-byte
-// multiples) can be read in place, since the tensor core takes an MN-major operand as well.  It saves the transposing
-// copy of every call (2 us and the filter moved twice), but the product itself runs some 10 to 20 % slower on large
-// problems (8192 rows x 4096 x 4096 bf16: 195 to 210 us against 184 us after a 13.5 us copy), which also have CTA pairs
-// to run on; the pair kernel takes K-major filters only.  654 x 208 @ 208 x 112: kernels 7.5 -> 4.8 us.
+// multiples) is read in place: the tensor core takes an MN-major operand as well.  It saves the transposing copy of every
+// call, the filter moved twice.  Calls with the copy and without, bf16: 8192 x 4096 @ 4096 x 4096 190.1 and 177.5 us,
+// 1024 x 4096 @ 4096 x 4096 42.1 and 29.8, 2048 cubed 23.8 and 18.8, 8192 x 512 @ 512 x 512 8.45 and 8.35.  (While the
+// thread that issues the MMAs was the bottleneck, large products ran 10 to 20 % slower on such an operand.)
 bool filter_mn_major(const fdnn_conv_desc* d, const void* w) {
-  if (elem_size(d->dtype) != 2 || d->r * d->s != 1 || d->k <= 1 || d->c <= 1 || d->w_strides[0] != 1 ||
-      d->w_strides[1] % 8 != 0 || d->w_strides[1] < d->k || !aligned16(w) || (d->algo & 0xff) == FDNN_ALGO_IGEMM_PAIR)
-    return false;
-  const double filter = double(d->c) * d->k, products = filter * d->n * d->h * d->w;
-  if (2.9e-10 * products >= 2.0 + 0.8e-6 * filter) return false;   // both sides in microseconds
-  const double pair_tiles = double(d->n) * d->h * d->w / 256 * ((d->k + 255) / 256);
-  return d->k < 256 || d->c < 1024 || pair_tiles < 32;             // too short or too small for pairs
+  return elem_size(d->dtype) == 2 && d->r * d->s == 1 && d->k > 1 && d->c > 1 && d->w_strides[0] == 1 &&
+         d->w_strides[1] % 8 == 0 && d->w_strides[1] >= d->k && aligned16(w) && (d->algo & 0xff) != FDNN_ALGO_IGEMM_PAIR;
 }
 
 // Below kSmallFlops a 16-bit layer still runs on the tensor-core kernel when its reduction is more than a few dozen
@@ -706,8 +701,7 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
   // whenever every pair has a tile; with 32 or more steps they still win with half the pairs idle (a pair reads
   // each operand byte from L2 once for two tiles: 512 -> 512 3x3 stride 2 at 128 images 38.5 -> 32.1 us).
   const bool pairs_fill = pair_tiles >= pairs_all || (k_steps >= 32 && 2 * pair_tiles >= pairs_all);
-  const bool mn = !plan->w_packed && filter_mn_major(d, w);
-  if (algo == FDNN_ALGO_IGEMM_PAIR || (want_auto && pair_ok && !mn && d->k >= 256 && k_steps >= 16 && (pairs_fill || sk_on))) {
+  if (algo == FDNN_ALGO_IGEMM_PAIR || (want_auto && pair_ok && d->k >= 256 && k_steps >= 16 && (pairs_fill || sk_on))) {
     plan->algo = FDNN_ALGO_IGEMM_PAIR;
     plan->tile_m = 256;
     plan->tile_n = 256;
@@ -2016,7 +2010,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   if (p.status == nullptr) return fail(FDNN_CUDA_ERROR, "status word address unavailable");
   if (plan.algo == FDNN_ALGO_IGEMM_PAIR) {
     if (!p.tma_store) return fail(FDNN_NOT_SUPPORTED, "the CTA-pair kernel needs a dense channels-last output");
-    p.b_resident = (d.k <= 256 && d.r * d.s * p.c_blocks <= igemm_pair_max_resident_steps()) ? 1 : 0;
+    p.b_resident = (d.k <= 256 && !b_mn && d.r * d.s * p.c_blocks <= igemm_pair_max_resident_steps()) ? 1 : 0;
     // reduction splitting when the caller brought the scratch for it
     if (plan.stream_k && !p.b_resident && sk_scratch != nullptr && sk_bytes >= plan.streamk_bytes &&
         (reinterpret_cast<uintptr_t>(sk_scratch) & 255u) == 0) {

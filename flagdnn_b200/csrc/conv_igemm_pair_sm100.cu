@@ -266,7 +266,12 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
               tma_load_im2col_4d_pair(st, &tmA, bar, c0, w_base, h_base, img, static_cast<uint16_t>(s_ * p.dil_w),
                                       static_cast<uint16_t>(r * p.dil_h));
             }
-            if (!b_resident) tma_load_3d_pair(st + kABytes, &tmB, bar, c0, r * p.S + s_, b_row0);
+            if (p.b_mn) {   // filter with K contiguous: boxes of 64 filters x 64 channels
+              tma_load_3d_pair(st + kABytes, &tmB, bar, b_row0, c0, 0);
+              tma_load_3d_pair(st + kABytes + kMnBoxBytes, &tmB, bar, b_row0 + int(kMnBoxElems), c0, 0);
+            } else if (!b_resident) {
+              tma_load_3d_pair(st + kABytes, &tmB, bar, c0, r * p.S + s_, b_row0);
+            }
             if constexpr (kProf) prof_issue += clock64() - pt1;
             if (++stage == uint32_t(n_stages)) {
               stage = 0;
@@ -306,6 +311,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       const uint32_t empty_own = smem_u32(&empty_bar[0]);
       const uint32_t tfull_own = smem_u32(&tmem_full[0]);
       const uint32_t ring_lo = sw128_desc_lo(smem_u32(stage_base)), b_res_lo = sw128_desc_lo(smem_u32(b_res));
+      const uint32_t mn_lo = mnmajor_desc_lo(smem_u32(stage_base) + kABytes);
       const uint32_t raw_empty_peer = map_to_cta(smem_u32(&raw_empty[0]), 1);
       const int k16 = p.k16_per_step;  // 16-element reduction slices per step that hold data (4, or 3)
       TileWalk walk;
@@ -328,7 +334,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         // one hand-over of the accumulator per epilogue warp instead of per thread took 1024 -> 2048 1x1 stride 2 on
         // 128 x 14 x 14 from 27.1 to 25.8 us, 32 x 1024 rows of a 4096 x 4096 product from 179.7 to 177.1):
         // it exists once with four MMAs per step and once with a runtime count for the 3-channel mode.
-        auto reduce = [&](auto four_tag, auto prof_tag) {
+        auto reduce = [&](auto four_tag, auto prof_tag, auto mn_tag) {
+          constexpr bool kMn = decltype(mn_tag)::value;   // the filter lies MN-major in its stages
           constexpr bool kFour = decltype(four_tag)::value;
           constexpr bool kProf = decltype(prof_tag)::value;
           for (int kit = walk.kb; kit < walk.ke; ++kit) {
@@ -344,7 +351,10 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             const uint32_t a_lo = ring_lo + stage * uint32_t(stage_stride / 16);
             const uint32_t b_lo = b_resident ? b_res_lo + kit * (kBBytes / 16) : a_lo + kABytes / 16;
             const uint32_t acc = kit > walk.kb ? 1u : 0u;
-            if constexpr (kFour) {
+            if constexpr (kMn) {
+              mma4_f16_pair<int(kMnStepBytes / 16)>(d_tmem, a_lo, mn_lo + (a_lo - ring_lo),
+                                                    kIdesc | kIdescBMnMajor, acc);
+            } else if constexpr (kFour) {
               mma4_f16_pair(d_tmem, a_lo, b_lo, kIdesc, acc);
             } else {
               for (uint32_t k = 0; k < uint32_t(k16); ++k)
@@ -357,12 +367,14 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             }
           }
         };
-        if (k16 != kKB / 16) {
-          reduce(std::false_type{}, std::false_type{});
+        if (p.b_mn) {
+          reduce(std::true_type{}, std::false_type{}, std::true_type{});
+        } else if (k16 != kKB / 16) {
+          reduce(std::false_type{}, std::false_type{}, std::false_type{});
         } else if (p.prof == nullptr) {
-          reduce(std::true_type{}, std::false_type{});
+          reduce(std::true_type{}, std::false_type{}, std::false_type{});
         } else {
-          reduce(std::true_type{}, std::true_type{});   // cycle counters of the role (development aid)
+          reduce(std::true_type{}, std::true_type{}, std::false_type{});   // cycle counters of the role (development aid)
         }
         if (alive) {
           tc_commit_both(tfull_own + buf * 8);
