@@ -723,12 +723,14 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
 // a copy per tap against this (bf16, channels-last, 3x3, microseconds): 256 -> 256 on 256 x 14 x 14 46.1 and 40.7, on
 // 128 images 31.1 and 22.7, on one 10.3 and 9.0; 64 -> 64 on 128 x 56 x 56 (four pixels per row before) 49.9 and 32.2;
 // 128 -> 128 on 128 x 28 x 28 34.7 and 25.1; 512 -> 512 on 128 x 7 x 7, an eighth of the walk rows no output, 30.5 and 27.6;
-// 104 -> 152 on 24 x 45 x 37 40.6 and 25.7; two groups 64 -> 128 on 256 x 56 x 56 (block-diagonal before) 122 and 72;
-// sixteen groups of 32 on 16 x 28 x 28 27.9 and 15.0.
-//   Where it lost: fewer pair tiles than pairs over one full channel block, nine steps in all (64 -> 128 on 8 x 28 x 28 5.5
-// and 5.9, on 16 x 28 x 28 6.4 and 7.0): those keep the smaller tiles of the single-CTA kernel.  With 32 channels or fewer
-// a copy per tap moves twice what it needs and this is ahead again (24 -> 24 on 112 x 112 10.4 and 7.0).
-//   Tiles: rounds of the pairs times what a step of a tile costs (172 / 257 / 513 clocks of MMAs for 64 / 128 / 256 columns).
+// 104 -> 152 on 24 x 45 x 37 40.6 and 25.7; NCHW 64 -> 64 on 128 x 56 x 56 60.1 and 38.0; two groups 64 -> 128 on
+// 256 x 56 x 56 (block-diagonal before) 122 and 72; sixteen groups of 32 on 16 x 28 x 28 27.9 and 15.0.
+//   Where it loses: fewer pair tiles than pairs and nine steps in all (64 -> 128 on 8 x 28 x 28 5.5 and 5.9: smaller tiles
+// start sooner), and where pair tiles fill a round and a bit (200 -> 200 5x5 on 20 x 31 x 29 NCHW: 141 tiles of 128 x 256
+// in one round against 152 in three, 42 and 50).  So both sides are counted in clocks of the busiest SM, with what a step
+// of four MMAs was measured to take: 380 / 520 / 780 for 64 / 128 / 256 columns and 640 on pairs with a copy per tap,
+// 230 / 310 / 570 here, 1500 more for a launch, and 1350 per copy where pixels straddle 128-byte lines (24 -> 24 on
+// 112 x 112 10.4 and 7.0).
 struct RowsMode {
   int tile_n;          // 0: no
   int pitch;           // walk rows per image row
@@ -740,14 +742,18 @@ bool sector_aligned(const fdnn_conv_desc& d, int oh, int ow, const void* y) {
   return d.k % 16 == 0 && (reinterpret_cast<uintptr_t>(y) & 31u) == 0 && (d.n <= 1 || d.y_strides[0] % 16 == 0) &&
          (oh <= 1 || d.y_strides[2] % 16 == 0) && (ow <= 1 || d.y_strides[3] % 16 == 0);
 }
-RowsMode rows_mode(const fdnn_conv_desc* d, int oh, int ow, const void* y) {
+RowsMode rows_mode(const fdnn_conv_desc* d, const fdnn_conv_plan& plan, const void* y) {
   RowsMode g = {};
+  const int oh = plan.oh, ow = plan.ow;
   if (elem_size(d->dtype) != 2 || d->algo != FDNN_ALGO_AUTO || d->stride_w != 1 || d->s < 2 || (d->s - 1) * d->dil_w > kRowsCopy - 128)
     return g;
   fdnn_conv_desc one = *d;
   one.groups = 1;
   const int cg = d->c / d->groups, kg = d->k / d->groups;
-  if (!igemm_geometry_ok(&one) || oh < 1 || ow < 1 || cg < 8 || d->k < 8 || d->y_strides[1] != 1) return g;
+  if (!igemm_geometry_ok(&one) || oh < 1 || ow < 1 || cg < 8 || d->k < 8) return g;
+  // y along channels, or along the pixels of every image
+  const bool pixels = (ow == 1 || d->y_strides[3] == 1) && (oh == 1 || d->y_strides[2] == ow);
+  if (d->y_strides[1] != 1 && !pixels) return g;
   g.pitch = d->w + (d->pad_left > d->pad_right ? d->pad_left : d->pad_right);
   if (g.pitch - d->w - d->pad_left > 127 || ow > g.pitch) return g;
   const long long walk = (long long)d->n * oh * g.pitch;
@@ -757,32 +763,41 @@ RowsMode rows_mode(const fdnn_conv_desc* d, int oh, int ow, const void* y) {
   g.m_tiles = int((walk + 127) / 128);
   g.blk_groups = 1;
   if (d->groups > 1) {
-    if ((cg != 16 && cg != 32) || d->c % 64 != 0 || kg % 32 != 0 || !sector_aligned(*d, oh, ow, y)) return g;
+    if ((cg != 16 && cg != 32) || d->c % 64 != 0 || kg % 32 != 0 || d->y_strides[1] != 1 || !sector_aligned(*d, oh, ow, y)) return g;
     g.blk_groups = 64 / cg;
     const int bn = g.blk_groups * kg;
     if (bn != 64 && bn != 128 && bn != 256) return g;
     g.tile_n = bn;
     g.n_tiles = d->c / 64;
   } else {
-    int best = 0;
-    double best_cost = 1e300;
+    // clocks of the busiest SM: rounds of tiles x steps x what a step takes
+    const long long pitch = 2 * d->x_strides[3];
+    const bool straddles = !plan.x_repacked && d->w > 1 && pitch % 128 != 0 && pitch != 16 && pitch != 32 && pitch != 64;
+    const double steps = double(d->r) * ((d->c + 63) / 64);
+    const int q = plan.pixel_group > 1 ? plan.pixel_group : 1;
+    const bool pair = plan.algo == FDNN_ALGO_IGEMM_PAIR;
+    const long long m_now = ((long long)d->n * oh * ow / q + plan.tile_m - 1) / plan.tile_m;
+    const long long tiles_now = m_now * (((long long)q * d->k + plan.tile_n - 1) / plan.tile_n);
+    const int units = pair ? sms / 2 : sms;
+    double step = pair ? 640 : plan.tile_n == 64 ? 380 : plan.tile_n == 128 ? 520 : 780;
+    if (straddles && step < 1350) step = 1350;
+    const double now = double((tiles_now + units - 1) / units) * steps * (d->s + (q - 1) * d->stride_w) * step;
+    double best_cost = now;
     for (int bn = 64; bn <= 256; bn *= 2) {
       if (bn > 64 && bn / 2 >= d->k) break;
       const long long tiles = (long long)((g.m_tiles + 1) / 2) * ((d->k + bn - 1) / bn);
-      const double cost = double((tiles + sms / 2 - 1) / (sms / 2)) * (bn + 96);
-      if (cost <= best_cost) {
+      double tap = bn == 64 ? 230 : bn == 128 ? 310 : 570;
+      if (straddles && tap * d->s < 1350) tap = 1350.0 / d->s;
+      const double cost = 1500 + double((tiles + sms / 2 - 1) / (sms / 2)) * steps * d->s * tap;
+      if (cost < best_cost) {
         best_cost = cost;
-        best = bn;
+        g.tile_n = bn;
       }
     }
-    g.tile_n = best;
-    g.n_tiles = (d->k + best - 1) / best;
+    if (g.tile_n == 0) return g;
+    g.n_tiles = (d->k + g.tile_n - 1) / g.tile_n;
   }
   const long long tiles = (long long)((g.m_tiles + 1) / 2) * g.n_tiles;
-  if (tiles < sms / 2 && d->c > 32 && d->c <= 64 && d->groups == 1) {
-    g.tile_n = 0;
-    return g;
-  }
   g.grid = 2 * int(tiles < sms / 2 ? tiles : sms / 2);
   return g;
 }
@@ -1618,10 +1633,10 @@ static int fwd_rows(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, const R
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(FDNN_CUDA_ERROR, "cuTensorMapEncodeTiled (filter rows) failed with CUresult " + std::to_string(int(r)));
   }
-  p.y_sn = d.y_strides[0]; p.y_sk = 1; p.y_sh = d.y_strides[2]; p.y_sw = d.y_strides[3];
+  p.y_sn = d.y_strides[0]; p.y_sk = d.y_strides[1]; p.y_sh = d.y_strides[2]; p.y_sw = d.y_strides[3];
   IgemmParams unit = {};
   choose_strided_store(d, plan.oh, plan.ow, y, &unit);
-  p.y_unit = sector_aligned(d, plan.oh, plan.ow, y) ? 32 : unit.y_unit;
+  p.y_unit = d.y_strides[1] == 1 && sector_aligned(d, plan.oh, plan.ow, y) ? 32 : unit.y_unit;
   p.bias = bias; p.scale = scale; p.y = y;
   p.act = activation;
   IgemmParams dbg = {};
@@ -1678,7 +1693,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
 
   if (batch == nullptr && d.groups > 1 && plan.algo != FDNN_ALGO_DIRECT && allow_group && residual == nullptr) {
-    const RowsMode rows = rows_mode(&d, plan.oh, plan.ow, y);
+    const RowsMode rows = rows_mode(&d, plan, y);
     const int cg = d.c / d.groups;
     FilterView f = {w, cg, d.s, 0, d.s > 1 ? d.w_strides[3] : d.w_strides[2], d.w_strides[0]};
     bool have = w != nullptr && filter_in_place(&d, w);
@@ -1829,7 +1844,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
 
   if (batch == nullptr && residual == nullptr && allow_group && k_real == d.k && plan.low_channel == 0 &&
       !(plan.x_repacked && d.c < 8)) {
-    const RowsMode rows = rows_mode(&d, plan.oh, plan.ow, y);
+    const RowsMode rows = rows_mode(&d, plan, y);
     if (rows.tile_n != 0) {
       const int c_pad = plan.c_padded;
       FilterView f = {w, d.c, d.s, 0, d.s > 1 ? d.w_strides[3] : d.w_strides[2], d.k > 1 ? d.w_strides[0] : c_pad};

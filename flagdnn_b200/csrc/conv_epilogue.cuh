@@ -593,6 +593,69 @@ __device__ __forceinline__ void epilogue_store_sectors(uint32_t t_row, int n0, i
   }
 }
 
+// Epilogue for 16-bit y along pixels (NCHW) when some of the warp's 32 rows are no output: a lane writes its own pixel of
+// one channel after another, neighbouring lanes neighbouring pixels, straight from the registers.
+//   y: the lane's pixel, first column of the warp's share; sk: elements between channels
+template <typename T, int WC, typename Done>
+__device__ __forceinline__ void epilogue_store_pixels(uint32_t t_row, int n0, int kout, int act, const float* s_scale,
+                                                      const float* s_bias, bool use_scale, uint16_t* y, long long sk, bool ok,
+                                                      Done&& read_done) {
+  int chunks = (kout - n0 + 31) / 32;
+  if (chunks > WC / 32) chunks = WC / 32;
+  if (chunks <= 0) {
+    read_done();
+    return;
+  }
+  uint32_t raw[32];
+  tmem_ld_32x32b_x32(t_row, raw);
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    tmem_ld_wait();
+    float v[32];
+#pragma unroll
+    for (int j4 = 0; j4 < 8; ++j4) {
+      const float4 sc = use_scale ? reinterpret_cast<const float4*>(s_scale + c * 32)[j4] : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+      const float4 bi = reinterpret_cast<const float4*>(s_bias + c * 32)[j4];
+      v[4 * j4 + 0] = fmaf(__uint_as_float(raw[4 * j4 + 0]), sc.x, bi.x);
+      v[4 * j4 + 1] = fmaf(__uint_as_float(raw[4 * j4 + 1]), sc.y, bi.y);
+      v[4 * j4 + 2] = fmaf(__uint_as_float(raw[4 * j4 + 2]), sc.z, bi.z);
+      v[4 * j4 + 3] = fmaf(__uint_as_float(raw[4 * j4 + 3]), sc.w, bi.w);
+    }
+    if (c + 1 < chunks) tmem_ld_32x32b_x32(t_row + (c + 1) * 32, raw);   // travels while this chunk is rounded and stored
+    else read_done();
+    uint32_t row[16];
+    if (act == 1) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) row[j] = round_pack2_relu<T>(v[2 * j], v[2 * j + 1]);
+    } else {
+      if (act) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = apply_activation(v[j], act);
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) row[j] = round_pack2<T>(v[2 * j], v[2 * j + 1]);
+    }
+    const int nc = kout - n0 - c * 32;
+    if (ok) {
+      if (nc >= 32) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          y[0] = uint16_t(row[j]);
+          y[sk] = uint16_t(row[j] >> 16);
+          y += 2 * sk;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (2 * j < nc) y[0] = uint16_t(row[j]);
+          if (2 * j + 1 < nc) y[sk] = uint16_t(row[j] >> 16);
+          y += 2 * sk;
+        }
+      }
+    }
+  }
+}
+
 // Contributor side of reduction splitting: this warp's 32 rows x WC raw fp32 accumulator columns go to the
 // CTA's slot (piece pc0 onwards, row `row`) instead of through the epilogue.
 template <int WC>

@@ -68,8 +68,11 @@ struct Cfg {
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
 };
 
-// BLK: groups per 64-channel block (1: not grouped).  SECTORS: y takes whole 32-byte sectors per lane.
-template <typename T, int BN, int BLK, bool SECTORS>
+// BLK: groups per 64-channel block (1: not grouped).  STORE: how y is written.
+constexpr int kStoreSectors = 0;    // along channels, whole 32-byte sectors per lane
+constexpr int kStoreChannels = 1;   // along channels, any alignment
+constexpr int kStorePixels = 2;     // along pixels
+template <typename T, int BN, int BLK, int STORE>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmY, const RowsParams p) {
@@ -373,15 +376,18 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(tempty_leader + buf * 8);
       };
-      if (SECTORS && p.y_rows && __all_sync(0xffffffffu, row_ok)) {
+      if (STORE == kStoreSectors && p.y_rows && __all_sync(0xffffffffu, row_ok)) {
         // 32 pixels one after another: boxes through the TMA unit
         const int pixel = __shfl_sync(0xffffffffu, real, 0);
         epilogue_store_tile<T, WC, false, 1>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY, pixel, 0, 32,
                                              store_seq, nullptr, g_scale != nullptr);
         read_done();
-      } else if constexpr (SECTORS) {
+      } else if constexpr (STORE == kStoreSectors) {
         epilogue_store_sectors<T, WC>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr,
                                       static_cast<T*>(p.y) + y_off + n0, row_ok, read_done);
+      } else if constexpr (STORE == kStorePixels) {
+        epilogue_store_pixels<T, WC>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr,
+                                     static_cast<uint16_t*>(p.y) + y_off + n0 * p.y_sk, p.y_sk, row_ok, read_done);
       } else {
         StridedOut so = {};
         so.y = p.y;
@@ -394,7 +400,7 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         read_done();
       }
     }
-    if (SECTORS && p.y_rows && lane == 0) bulk_wait_group0();   // stores must be done before the CTA retires
+    if (STORE == kStoreSectors && p.y_rows && lane == 0) bulk_wait_group0();   // stores must be done before the CTA retires
   }
   }
 
@@ -409,8 +415,8 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
-// The kernels a layer may run on: 32-byte stores for all of them, and a general store for layers that are not grouped.
-template <typename T, int BN, int BLK, bool SECTORS>
+// The kernels a layer may run on: 32-byte stores for all of them, the other stores for layers that are not grouped.
+template <typename T, int BN, int BLK, int STORE>
 cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
@@ -426,18 +432,20 @@ cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = launch_overlap_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, conv_rows_kernel<T, BN, BLK, SECTORS>, tmA, tmB, tmY, p);
+  return cudaLaunchKernelEx(&cfg, conv_rows_kernel<T, BN, BLK, STORE>, tmA, tmB, tmY, p);
 }
 
 template <typename T, int BN>
 cudaError_t launch_bn(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
-  const bool sectors = p.y_unit == 32;
-  if (p.blk_groups == 1)
-    return sectors ? launch_one<T, BN, 1, true>(tmA, tmB, tmY, p, grid, stream) : launch_one<T, BN, 1, false>(tmA, tmB, tmY, p, grid, stream);
-  if (!sectors) return cudaErrorInvalidValue;
-  if (p.blk_groups == 2) return launch_one<T, BN, 2, true>(tmA, tmB, tmY, p, grid, stream);
+  if (p.blk_groups == 1) {
+    if (p.y_sk != 1) return launch_one<T, BN, 1, kStorePixels>(tmA, tmB, tmY, p, grid, stream);
+    if (p.y_unit == 32) return launch_one<T, BN, 1, kStoreSectors>(tmA, tmB, tmY, p, grid, stream);
+    return launch_one<T, BN, 1, kStoreChannels>(tmA, tmB, tmY, p, grid, stream);
+  }
+  if (p.y_sk != 1 || p.y_unit != 32) return cudaErrorInvalidValue;
+  if (p.blk_groups == 2) return launch_one<T, BN, 2, kStoreSectors>(tmA, tmB, tmY, p, grid, stream);
   if constexpr (BN > 64) {   // four groups of 32 filters or more
-    if (p.blk_groups == 4) return launch_one<T, BN, 4, true>(tmA, tmB, tmY, p, grid, stream);
+    if (p.blk_groups == 4) return launch_one<T, BN, 4, kStoreSectors>(tmA, tmB, tmY, p, grid, stream);
   }
   return cudaErrorInvalidValue;
 }
@@ -447,11 +455,12 @@ cudaError_t prepare_bn() {
   auto opt_in = [](const void* kernel) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem);
   };
-  cudaError_t e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, true>));
-  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, false>));
-  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 2, true>));
+  cudaError_t e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, kStoreSectors>));
+  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, kStoreChannels>));
+  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, kStorePixels>));
+  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 2, kStoreSectors>));
   if constexpr (BN > 64) {
-    if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 4, true>));
+    if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 4, kStoreSectors>));
   }
   return e;
 }

@@ -7,30 +7,32 @@ import oracle
 
 pytestmark = pytest.mark.gpu
 
-# n, c, h, w, k, (r, s), padding, dilation, stride
+# n, c, h, w, k, (r, s), padding, dilation, stride; long reductions or many tiles, where this kernel is the one chosen
 LAYERS = {
-    "one_tile": (1, 64, 9, 13, 64, (3, 3), 1, 1, 1),
-    "two_tiles_by_one_row": (1, 64, 16, 15, 64, (3, 3), 1, 1, 1),          # 16 x 16 = 256 walk rows: one pair tile, full
-    "one_walk_row_more": (1, 64, 1, 256, 64, (1, 3), (0, 1), 1, 1),        # 257: the second pair holds one
-    "images_inside_a_tile": (37, 64, 5, 6, 64, (3, 3), 1, 1, 1),
-    "no_padding": (3, 64, 12, 20, 128, (3, 3), 0, 1, 1),
-    "wide_padding": (2, 64, 7, 9, 64, (3, 3), (3, 4), 1, 1),
-    "two_taps_same": (2, 64, 11, 18, 72, (2, 2), "same", 1, 1),            # right padding above left
-    "four_taps_same": (2, 40, 11, 18, 72, (4, 4), "same", 1, 1),
-    "dilation_4": (2, 64, 20, 21, 64, (3, 3), 4, 4, 1),
-    "nine_taps": (2, 32, 12, 30, 64, (1, 9), (0, 4), 1, 1),
-    "ten_taps": (2, 32, 12, 30, 64, (1, 10), (0, 4), 1, 1),                # one more than a copy holds: the other kernel
+    "one_tile": (1, 256, 9, 13, 64, (3, 3), 1, 1, 1),
+    "two_tiles_full": (1, 256, 16, 15, 64, (3, 3), 1, 1, 1),               # 16 x 16 = 256 walk rows: one pair tile, full
+    "one_walk_row_more": (1, 512, 1, 256, 64, (1, 3), (0, 1), 1, 1),       # 257: the second pair holds one
+    "images_inside_a_tile": (37, 256, 5, 6, 64, (3, 3), 1, 1, 1),
+    "no_padding": (3, 256, 12, 20, 128, (3, 3), 0, 1, 1),
+    "wide_padding": (2, 256, 7, 9, 64, (3, 3), (3, 4), 1, 1),
+    "two_taps_same": (2, 512, 11, 18, 72, (2, 2), "same", 1, 1),           # right padding above left
+    "four_taps_same": (2, 296, 11, 18, 72, (4, 4), "same", 1, 1),
+    "dilation_4": (2, 256, 20, 21, 64, (3, 3), 4, 4, 1),
+    "nine_taps": (2, 256, 12, 30, 64, (1, 9), (0, 4), 1, 1),
+    "ten_taps": (2, 256, 12, 30, 64, (1, 10), (0, 4), 1, 1),               # one more than a copy holds: the other kernel
     "five_by_five": (2, 104, 17, 19, 136, (5, 5), 2, 1, 1),
-    "stride_h": (3, 64, 21, 22, 64, (3, 3), 1, 1, (2, 1)),
-    "channels_8": (2, 8, 30, 30, 96, (3, 3), 1, 1, 1),
-    "channels_130": (2, 136, 13, 17, 128, (3, 3), 1, 1, 1),
-    "filters_150": (3, 72, 13, 17, 150, (3, 3), 1, 1, 1),                  # rows of 300 bytes
-    "filters_264": (3, 64, 14, 14, 264, (3, 3), 1, 1, 1),
-    "filters_272": (3, 64, 14, 14, 272, (3, 3), 1, 1, 1),                  # 16 columns of the last tile
-    "resident_128": (20, 64, 28, 28, 128, (3, 3), 1, 1, 1),                # several tiles per pair, whole filter kept
+    "stride_h": (3, 256, 21, 22, 64, (3, 3), 1, 1, (2, 1)),
+    "channels_8": (60, 8, 30, 30, 96, (3, 3), 1, 1, 1),
+    "channels_24": (1, 24, 112, 112, 24, (3, 3), 1, 1, 1),
+    "channels_264": (2, 264, 13, 17, 128, (3, 3), 1, 1, 1),
+    "filters_150": (3, 328, 13, 17, 150, (3, 3), 1, 1, 1),                 # rows of 300 bytes
+    "filters_264": (3, 320, 14, 14, 264, (3, 3), 1, 1, 1),
+    "filters_272": (3, 320, 14, 14, 272, (3, 3), 1, 1, 1),                 # 16 columns of the last tile
+    "resident_128": (20, 64, 56, 56, 128, (3, 3), 1, 1, 1),                # several tiles per pair, whole filter kept
     "streamed_128": (28, 128, 28, 28, 128, (3, 3), 1, 1, 1),
     "streamed_256": (60, 192, 28, 28, 256, (3, 3), 1, 1, 1),
     "grouped_pixels": (20, 64, 56, 56, 64, (3, 3), 1, 1, 1),               # the plan packs its filter for grouped pixels
+    "images_cut_by_warps": (9, 256, 7, 7, 96, (3, 3), 1, 1, 1),
 }
 
 
@@ -55,15 +57,19 @@ def _both(fd, call):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
 @pytest.mark.parametrize("filter_format", [torch.channels_last, torch.contiguous_format], ids=["krsc", "kcrs"])
+@pytest.mark.parametrize("layout", ["nhwc", "nchw"])
 @pytest.mark.parametrize("name", LAYERS)
-def test_bit_equal_to_a_copy_per_tap(native_lib, name, filter_format, dtype):
+def test_bit_equal_to_a_copy_per_tap(native_lib, name, layout, filter_format, dtype):
     import flagdnn_b200 as fd
 
     case = LAYERS[name]
     n, c, h, w, k, rs, pad, dil, stride = case
     x, wt, b, sc = _tensors(case, dtype, filter_format)
+    if layout == "nchw":
+        x = x.contiguous()
     got, per_tap = _both(fd, lambda: fd.conv2d(x, wt, b, stride=stride, padding=pad, dilation=dil))
     assert torch.equal(got, per_tap)
+    assert got.is_contiguous(memory_format=torch.channels_last if layout == "nhwc" else torch.contiguous_format) or 1 in got.shape
     if isinstance(pad, str):
         return
     pd, dl, st = ((v, v) if isinstance(v, int) else v for v in (pad, dil, stride))
