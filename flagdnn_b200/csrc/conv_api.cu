@@ -176,8 +176,8 @@ long long tight_x_bytes(const fdnn_conv_desc* d) {
 }
 
 // How the single-CTA kernel's epilogue writes a y that has no TMA map (see epilogue_store_strided): along channels
-// when they are contiguous, along pixels when every image's pixels are (NCHW), with the widest unit that every run's
-// start is a multiple of (and, along pixels, that no image boundary cuts); otherwise element by element.
+// when they are contiguous, with the widest unit that every pixel's start is a multiple of; along pixels when every image's
+// pixels are (NCHW); otherwise element by element.
 void choose_strided_store(const fdnn_conv_desc& d, int oh, int ow, const void* y, IgemmParams* p) {
   const int es = elem_size(d.dtype);
   const long long sn = d.y_strides[0], sk = d.y_strides[1], sh = d.y_strides[2], sw = d.y_strides[3];
@@ -196,14 +196,7 @@ void choose_strided_store(const fdnn_conv_desc& d, int oh, int ow, const void* y
     return;
   }
   const bool pixels = ow > 1 ? (sw == 1 && (oh == 1 || sh == ow)) : (oh == 1 || sh == 1);
-  if (!pixels) return;
-  p->y_mode = 1;
-  for (int unit = 16; unit > es; unit /= 2) {
-    if ((long long)oh * ow * es % unit == 0 && base % unit == 0 && fits(d.n, sn, unit) && fits(d.k, sk, unit)) {
-      p->y_unit = unit;
-      break;
-    }
-  }
+  if (pixels) p->y_mode = 1;
 }
 
 // Low-channel mode (C <= 4, e.g. the 7x7 stride-2 stem): four neighbouring
@@ -729,7 +722,7 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
 // start sooner), and where pair tiles fill a round and a bit (200 -> 200 5x5 on 20 x 31 x 29 NCHW: 141 tiles of 128 x 256
 // in one round against 152 in three, 42 and 50).  So both sides are counted in clocks of the busiest SM, with what a step
 // of four MMAs was measured to take: 380 / 520 / 780 for 64 / 128 / 256 columns and 640 on pairs with a copy per tap,
-// 230 / 310 / 570 here, 1500 more for a launch, and 1350 per copy where pixels straddle 128-byte lines (24 -> 24 on
+// 230 / 310 / 570 here (fp32, twelve MMAs: 800 / 1100 and 600 / 830), 1500 more for a launch, and 1350 per copy where pixels straddle 128-byte lines (24 -> 24 on
 // 112 x 112 10.4 and 7.0).
 struct RowsMode {
   int tile_n;          // 0: no
@@ -737,16 +730,17 @@ struct RowsMode {
   int m_tiles, n_tiles, grid;
   int blk_groups;      // groups per 64-channel block (1: not grouped)
 };
-// Every output pixel starts on a 32-byte boundary and its channels fill 32-byte pieces (16-bit types).
+// Every output pixel starts on a 32-byte boundary and its channels fill 32-byte pieces.
 bool sector_aligned(const fdnn_conv_desc& d, int oh, int ow, const void* y) {
-  return d.k % 16 == 0 && (reinterpret_cast<uintptr_t>(y) & 31u) == 0 && (d.n <= 1 || d.y_strides[0] % 16 == 0) &&
-         (oh <= 1 || d.y_strides[2] % 16 == 0) && (ow <= 1 || d.y_strides[3] % 16 == 0);
+  const int gran = 32 / elem_size(d.dtype);
+  return d.k % gran == 0 && (reinterpret_cast<uintptr_t>(y) & 31u) == 0 && (d.n <= 1 || d.y_strides[0] % gran == 0) &&
+         (oh <= 1 || d.y_strides[2] % gran == 0) && (ow <= 1 || d.y_strides[3] % gran == 0);
 }
 RowsMode rows_mode(const fdnn_conv_desc* d, const fdnn_conv_plan& plan, const void* y) {
   RowsMode g = {};
   const int oh = plan.oh, ow = plan.ow;
-  if (elem_size(d->dtype) != 2 || d->algo != FDNN_ALGO_AUTO || d->stride_w != 1 || d->s < 2 || (d->s - 1) * d->dil_w > kRowsCopy - 128)
-    return g;
+  const int es = elem_size(d->dtype);
+  if (es > 4 || d->algo != FDNN_ALGO_AUTO || d->stride_w != 1 || d->s < 2 || (d->s - 1) * d->dil_w > kRowsCopy - 128) return g;
   fdnn_conv_desc one = *d;
   one.groups = 1;
   const int cg = d->c / d->groups, kg = d->k / d->groups;
@@ -763,7 +757,7 @@ RowsMode rows_mode(const fdnn_conv_desc* d, const fdnn_conv_plan& plan, const vo
   g.m_tiles = int((walk + 127) / 128);
   g.blk_groups = 1;
   if (d->groups > 1) {
-    if ((cg != 16 && cg != 32) || d->c % 64 != 0 || kg % 32 != 0 || d->y_strides[1] != 1 || !sector_aligned(*d, oh, ow, y)) return g;
+    if (es != 2 || (cg != 16 && cg != 32) || d->c % 64 != 0 || kg % 32 != 0 || d->y_strides[1] != 1 || !sector_aligned(*d, oh, ow, y)) return g;
     g.blk_groups = 64 / cg;
     const int bn = g.blk_groups * kg;
     if (bn != 64 && bn != 128 && bn != 256) return g;
@@ -771,22 +765,23 @@ RowsMode rows_mode(const fdnn_conv_desc* d, const fdnn_conv_plan& plan, const vo
     g.n_tiles = d->c / 64;
   } else {
     // clocks of the busiest SM: rounds of tiles x steps x what a step takes
-    const long long pitch = 2 * d->x_strides[3];
+    const long long pitch = es * d->x_strides[3];
     const bool straddles = !plan.x_repacked && d->w > 1 && pitch % 128 != 0 && pitch != 16 && pitch != 32 && pitch != 64;
-    const double steps = double(d->r) * ((d->c + 63) / 64);
+    const double steps = double(d->r) * ((d->c * es + 127) / 128);
     const int q = plan.pixel_group > 1 ? plan.pixel_group : 1;
     const bool pair = plan.algo == FDNN_ALGO_IGEMM_PAIR;
     const long long m_now = ((long long)d->n * oh * ow / q + plan.tile_m - 1) / plan.tile_m;
     const long long tiles_now = m_now * (((long long)q * d->k + plan.tile_n - 1) / plan.tile_n);
     const int units = pair ? sms / 2 : sms;
     double step = pair ? 640 : plan.tile_n == 64 ? 380 : plan.tile_n == 128 ? 520 : 780;
+    if (es == 4) step = plan.tile_n == 64 ? 800 : 1100;   // twelve MMAs
     if (straddles && step < 1350) step = 1350;
     const double now = double((tiles_now + units - 1) / units) * steps * (d->s + (q - 1) * d->stride_w) * step;
     double best_cost = now;
-    for (int bn = 64; bn <= 256; bn *= 2) {
+    for (int bn = 64; bn <= (es == 2 ? 256 : 128); bn *= 2) {
       if (bn > 64 && bn / 2 >= d->k) break;
       const long long tiles = (long long)((g.m_tiles + 1) / 2) * ((d->k + bn - 1) / bn);
-      double tap = bn == 64 ? 230 : bn == 128 ? 310 : 570;
+      double tap = es == 4 ? (bn == 64 ? 600 : 830) : bn == 64 ? 230 : bn == 128 ? 310 : 570;
       if (straddles && tap * d->s < 1350) tap = 1350.0 / d->s;
       const double cost = 1500 + double((tiles + sms / 2 - 1) / (sms / 2)) * steps * d->s * tap;
       if (cost < best_cost) {
@@ -1600,10 +1595,16 @@ static int fwd_rows(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, const R
   whole.groups = 1;
   int st = relayout_x(whole, plan, false, x, workspace, workspace_bytes, stream, &a);
   if (st != FDNN_OK) return st;
-  const int cg = d.c / d.groups, kg = d.k / d.groups;
-  alignas(64) CUtensorMap tmA, tmB;
+  const int cg = d.c / d.groups, kg = d.k / d.groups, es = elem_size(d.dtype);
+  alignas(64) CUtensorMap tmA, tmA2, tmB;
   st = encode_activation_map(&tmA, d.dtype, a.base, a.c, d.w, d.h, d.n, a.sw, a.sh, a.sn, &whole, 1, rows.pitch);
   if (st != FDNN_OK) return st;
+  tmA2 = tmA;
+  if (es == 4) {
+    st = encode_activation_map(&tmA2, d.dtype, static_cast<const char*>(a.base) + a.plane * es, a.c, d.w, d.h, d.n, a.sw, a.sh,
+                               a.sn, &whole, 1, rows.pitch);
+    if (st != FDNN_OK) return st;
+  }
   const bool blk = rows.blk_groups > 1;
   RowsParams p = {};
   p.M = d.n * plan.oh * rows.pitch;
@@ -1613,21 +1614,22 @@ static int fwd_rows(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, const R
   p.stride_h = d.stride_h; p.pad_top = d.pad_top; p.pad_left = d.pad_left; p.dil_h = d.dil_h; p.dil_w = d.dil_w;
   p.R = d.r; p.S = d.s;
   p.s_pitch = f.s_pitch;
-  p.c_blocks = blk ? 1 : (d.c + 63) / 64;
+  p.halves = es == 4 ? 2 : 1;
+  p.c_blocks = blk ? 1 : (d.c * es + 127) / 128;
   p.m_tiles = rows.m_tiles;
   p.n_tiles = rows.n_tiles;
   p.blk_groups = rows.blk_groups;
   p.cg = cg; p.kg = kg;
   p.blk_c_step = f.c_step;
-  p.b_bytes = blk ? rows.blk_groups * (kg / 2) * cg * 2 : rows.tile_n / 2 * 128;
+  p.b_bytes = blk ? rows.blk_groups * (kg / 2) * cg * 2 : p.halves * (rows.tile_n / 2) * 128;
   rows_stages(&p);
   {
-    // (channel, filter, tap): one box per group (of a block of channels) and slot
-    cuuint64_t dims[3] = {cuuint64_t(f.c), cuuint64_t(d.k), cuuint64_t(d.r) * f.s_pitch};
-    cuuint64_t strides[2] = {cuuint64_t(f.s_k) * 2, cuuint64_t(f.s_tap) * 2};
-    cuuint32_t box[3] = {cuuint32_t(blk ? cg : 64), cuuint32_t(blk ? kg / 2 : rows.tile_n / 2), cuuint32_t(p.b_taps)};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = memo_encode_tiled(&tmB, tm_dtype(d.dtype), 3, const_cast<void*>(f.base), dims, strides, box, estr,
+    // (channel, filter, tap, half): one box per group (of a block of channels) and slot
+    cuuint64_t dims[4] = {cuuint64_t(f.c), cuuint64_t(d.k), cuuint64_t(d.r) * f.s_pitch, 2};
+    cuuint64_t strides[3] = {cuuint64_t(f.s_k) * es, cuuint64_t(f.s_tap) * es, cuuint64_t(d.k) * d.r * f.s_pitch * f.c * es};
+    cuuint32_t box[4] = {cuuint32_t(blk ? cg : 128 / es), cuuint32_t(blk ? kg / 2 : rows.tile_n / 2), cuuint32_t(p.b_taps), 2};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = memo_encode_tiled(&tmB, tm_dtype(d.dtype), es == 4 ? 4 : 3, const_cast<void*>(f.base), dims, strides, box, estr,
                                    CU_TENSOR_MAP_INTERLEAVE_NONE,
                                    !blk ? CU_TENSOR_MAP_SWIZZLE_128B : cg == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1652,7 +1654,7 @@ static int fwd_rows(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, const R
     if (st != FDNN_OK) return st;
     p.y_rows = 1;
   }
-  cudaError_t e = launch_rows(d.dtype, rows.tile_n, tmA, tmB, tmY, p, rows.grid, stream);
+  cudaError_t e = launch_rows(d.dtype, rows.tile_n, tmA, tmA2, tmB, tmY, p, rows.grid, stream);
   if (e != cudaSuccess) return fail_cuda("rows launch", e);
   return FDNN_OK;
 }
@@ -2004,11 +2006,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
       tmY = tmA;
     }
   }
-  if (!p.tma_store && !out_f32) {
-    choose_strided_store(d, plan.oh, plan.ow, y, &p);
-    // a tile of windows starts at a row of the image, so that units along pixels have to divide rows as well
-    while (windows.ok && p.y_mode == 1 && p.y_unit > es && plan.ow * es % p.y_unit != 0) p.y_unit /= 2;
-  }
+  if (!p.tma_store && !out_f32) choose_strided_store(d, plan.oh, plan.ow, y, &p);
   alignas(64) CUtensorMap tmR = tmY;
   alignas(64) CUtensorMap tmRbox = tmY;
   if (residual != nullptr && p.tma_store) {

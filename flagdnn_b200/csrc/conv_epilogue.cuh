@@ -268,27 +268,18 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_row, int n0, int 
   }
 }
 
-// Epilogue for a y the TMA unit cannot write (its strides or base are not multiples of 16 bytes, or its pixels and
-// not its channels are contiguous): the same arithmetic, and 32 rows x 128 bytes are staged in shared memory all the
-// same, but the warp then writes them itself, with lanes along whichever dimension of y is contiguous and `unit` bytes
-// per lane, the widest the alignment of y allows:
-//   kYPixels    NCHW: staged as [column][32 pixels]; a unit is 2 / 4 / 8 neighbouring pixels of one channel.  Units
-//               never straddle two images (the host picks a unit that divides OH * OW)
-//   kYChannels  channels-last rows of a pitch that is not a multiple of 16 bytes: staged as [pixel][64 columns]
+// Epilogue for a channels-last y the TMA unit cannot write (its strides or base are not multiples of 16 bytes): the same
+// arithmetic, and 32 rows x 128 bytes are staged in shared memory all the same, as [pixel][64 columns], but the warp then
+// writes them itself, with lanes along the channels and `unit` bytes per lane, the widest the alignment of y allows.
 // Where 16-bit rows may start at odd elements (unit 2), each run is written as the 4-byte words it covers whole, plus a
-// 2-byte element at either end.
-// What this is bound by: the stores.  One 2-byte store per value straight from the registers, lanes along pixels,
-// as before, kept the L1-to-L2 request path 53-77 % busy with the tensor pipe at 10 % (24 x 45 x 37 pixels, 104 -> 150
-// channels bf16 3x3: 106 us), and NCHW y cost 20 us per 128 x 256 tile.
-constexpr int kYScattered = 0, kYPixels = 1, kYChannels = 2;
+// 2-byte element at either end.  (One 2-byte store per value straight from the registers, each lane in a row of its own:
+// 24 x 45 x 37 pixels, 104 -> 150 channels bf16 3x3, 106 us.)
+constexpr int kYScattered = 0, kYPixels = 1, kYChannels = 2;   // how y is written: element by element, along pixels or channels
 struct StridedOut {
   void* y;                 // element type of the operands
   const void* res;         // residual with y's strides, or nullptr
   long long y_off;         // this lane's pixel: element offset of the (group's) first channel
-  long long k_off;         // element offset of the group's first channel alone
-  long long sn, sk;        // element strides between images and between channels
-  int mode, unit;          // kY*, bytes per lane and store
-  int m0, M, ohw;          // the warp's first GEMM row, rows overall, pixels per image
+  int unit;                // bytes per lane and store
   bool row_ok;             // this lane's row exists
 };
 
@@ -297,78 +288,10 @@ template <> __device__ __forceinline__ uint32_t lds_unit<uint32_t>(uint32_t a) {
 template <> __device__ __forceinline__ uint2 lds_unit<uint2>(uint32_t a) { return lds_v2(a); }
 template <> __device__ __forceinline__ uint4 lds_unit<uint4>(uint32_t a) { return lds_v4(a); }
 
-// The four writers of a staged group.  Each reads a batch of units from shared memory before it stores the first: with
-// load and store of one unit after another the warp waits a shared-memory round trip per store (21 k clocks per
-// 128 x 256 tile instead of the few thousand its stores take).
+// The writers of a staged group.  Each reads a batch of units from shared memory before it stores the first: with load
+// and store of one unit after another the warp waits a shared-memory round trip per store (21 k clocks per 128 x 256 tile
+// instead of the few thousand its stores take).
 //
-// [column][32 pixels] in shared memory, U units along pixels; `out`: column 0, this lane's unit.
-template <typename U, int COL_BYTES>
-__device__ __forceinline__ void strided_pixels(char* out, uint32_t sbuf, int lane, int nc, bool ok, long long col_bytes) {
-  constexpr int kLanes = COL_BYTES / int(sizeof(U)), kPer = 32 / kLanes, kBatch = 4;
-  const int unit = lane % kLanes;
-  for (int c0 = lane / kLanes; c0 < nc; c0 += kPer * kBatch) {
-    U v[kBatch];
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int c = c0 + i * kPer;
-      if (c < nc) v[i] = lds_unit<U>(sbuf + c * COL_BYTES + unit * int(sizeof(U)));
-    }
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int c = c0 + i * kPer;
-      if (ok && c < nc) *reinterpret_cast<U*>(out + c * col_bytes) = v[i];
-    }
-  }
-}
-
-// 16-bit pixels whose columns may start at odd elements: the words a column's run covers whole, and its two ends;
-// 16 lanes per column.  Rows that do not lie in one image go element by element.
-__device__ __forceinline__ void strided_odd_pixels(uint16_t* y, uint32_t sbuf, int lane, int nc, bool whole, bool row_ok,
-                                                   long long run_off, long long lane_off, long long sk) {
-  if (!whole) {
-    if (!row_ok) return;
-    for (int c0 = 0; c0 < nc; c0 += 8) {
-      uint16_t v[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (c0 + i < nc) v[i] = lds_u16(sbuf + (c0 + i) * 64 + lane * 2);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (c0 + i < nc) y[lane_off + (c0 + i) * sk] = v[i];
-    }
-    return;
-  }
-  // word l of a column that starts on a word boundary; else the halves either side of the boundary after it, and lane
-  // 15, whose neighbour wraps to word 0, writes the first and the last element
-  const int l = lane & 15, cc = lane >> 4;
-  uint16_t* run = y + run_off + cc * sk;
-  const uint32_t src = sbuf + cc * 64;
-  const uint32_t par0 = uint32_t(reinterpret_cast<uintptr_t>(run) >> 1) & 1u;   // two columns further: the same parity
-#pragma unroll 2
-  for (int c0 = 0; c0 < nc; c0 += 8) {
-    uint32_t lo[4], hi[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      lo[i] = lds_u32(src + (c0 + 2 * i) * 64 + l * 4);
-      hi[i] = lds_u32(src + (c0 + 2 * i) * 64 + ((l + 1) & 15) * 4);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (c0 + 2 * i + cc < nc) {
-        if (par0 == 0u) {
-          *reinterpret_cast<uint32_t*>(run + 2 * l) = lo[i];
-        } else if (l != 15) {
-          *reinterpret_cast<uint32_t*>(run + 2 * l + 1) = __byte_perm(lo[i], hi[i], 0x5432);
-        } else {
-          run[31] = uint16_t(lo[i] >> 16);
-          run[0] = uint16_t(hi[i]);
-        }
-      }
-      run += 2 * sk;
-    }
-  }
-}
-
 // [pixel][128 bytes of columns], swizzled, U units along columns; row r's element offset is lane r's y_off.
 template <typename U, int ES>
 __device__ __forceinline__ void strided_channels(char* out, uint32_t sbuf, int lane, int nc, uint32_t rows_ok, long long y_off) {
@@ -404,8 +327,9 @@ __device__ __forceinline__ void strided_channels(char* out, uint32_t sbuf, int l
   }
 }
 
-// The same for 16-bit rows that may start at odd elements: one row per store, as whole words and two ends (as in
-// strided_odd_pixels).
+// The same for 16-bit rows that may start at odd elements: one row per store, as whole words and two ends: word l
+// of a row that starts on a word boundary; else the halves either side of the boundary after it, and the last lane, whose
+// neighbour wraps to word 0, writes the first element.
 __device__ __forceinline__ void strided_odd_channels(char* out, uint32_t sbuf, int lane, int nc, uint32_t rows_ok, long long y_off) {
   uint16_t* y = reinterpret_cast<uint16_t*>(out);
   auto word = [&](int r, int w) { return sbuf + r * 128 + ((((w >> 2) ^ (r & 7)) << 4) | ((w & 3) << 2)); };
@@ -441,26 +365,11 @@ __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, i
   constexpr int kEs = int(sizeof(T));
   constexpr int kCols = 128 / kEs;                 // columns per group: 64 (16-bit) or 32 (fp32)
   constexpr int kLoads = kCols / 32;
-  constexpr int kColBytes = 32 * kEs;              // one column's 32 pixels
   int groups = (kout - n0 + kCols - 1) / kCols;
   if (groups > BN / kCols) groups = BN / kCols;
   if (groups <= 0) return;
   char* y = static_cast<char*>(o.y);
   const uint32_t rows_ok = __ballot_sync(0xffffffffu, o.row_ok);
-  // kYPixels: the unit of pixels this lane writes (the same one for every column)
-  const int unit_px = o.unit / kEs;
-  const int lanes_per_col = kColBytes / (o.unit >= 4 ? o.unit : 4);
-  const int my_unit = lane & (lanes_per_col - 1);
-  long long u_off = 0;
-  bool u_ok = false, whole = false;
-  if (o.mode == kYPixels) {
-    const int px = kEs == 2 && o.unit == 2 ? 0 : my_unit * unit_px;
-    const int m = o.m0 + px;
-    const int img = m / o.ohw;
-    u_ok = m < o.M;
-    u_off = img * o.sn + (m - img * o.ohw) + o.k_off;
-    whole = rows_ok == 0xffffffffu && (o.m0 + 31) / o.ohw == o.m0 / o.ohw;   // 32 pixels of one image
-  }
 #pragma unroll 1
   for (int g = 0; g < groups; ++g) {
     uint32_t raw[kLoads][32];
@@ -486,10 +395,10 @@ __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, i
       }
       if constexpr (RES) {
         if (o.res != nullptr && o.row_ok) {
-          const T* res = static_cast<const T*>(o.res) + o.y_off + (long long)(col0 + l * 32) * o.sk;
+          const T* res = static_cast<const T*>(o.res) + o.y_off + col0 + l * 32;
 #pragma unroll
           for (int j = 0; j < 32; ++j)
-            if (l * 32 + j < nc) v[j] += to_f32<T>(res[j * o.sk]);
+            if (l * 32 + j < nc) v[j] += to_f32<T>(res[j]);
         }
       }
       if (act > 1) {   // uniform; kept apart so that the common paths do not fetch 32 copies of erf and tanh
@@ -509,44 +418,21 @@ __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, i
     }
     const uint32_t sbuf = smem_u32(buf);
     if constexpr (NBUF == 1) __syncwarp();   // the group before has been read
-    if (o.mode == kYPixels) {
-      if constexpr (kEs == 4) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sts_u32(sbuf + j * 128 + lane * 4, row[j]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          sts_u16(sbuf + (2 * j) * 64 + lane * 2, uint16_t(row[j]));
-          sts_u16(sbuf + (2 * j + 1) * 64 + lane * 2, uint16_t(row[j] >> 16));
-        }
-      }
-      __syncwarp();
-      if (kEs == 2 && o.unit == 2) {
-        strided_odd_pixels(reinterpret_cast<uint16_t*>(y), sbuf, lane, nc, whole, o.row_ok, u_off + col0 * o.sk,
-                           o.y_off + col0 * o.sk, o.sk);
-      } else {
-        char* out = y + (u_off + col0 * o.sk) * kEs;
-        if (o.unit == 16) strided_pixels<uint4, kColBytes>(out, sbuf, lane, nc, u_ok, o.sk * kEs);
-        else if (o.unit == 8) strided_pixels<uint2, kColBytes>(out, sbuf, lane, nc, u_ok, o.sk * kEs);
-        else strided_pixels<uint32_t, kColBytes>(out, sbuf, lane, nc, u_ok, o.sk * kEs);
-      }
-    } else {   // kYChannels
-#pragma unroll
-      for (int q = 0; q < 8; ++q)   // 16-byte pieces swizzled by row, as for the TMA store
-        sts_v4(sbuf + lane * 128 + ((q ^ (lane & 7)) << 4), make_uint4(row[4 * q], row[4 * q + 1], row[4 * q + 2], row[4 * q + 3]));
-      __syncwarp();
-      char* out = y + (long long)col0 * kEs;
-      if (kEs == 2 && o.unit == 2) strided_odd_channels(out, sbuf, lane, nc, rows_ok, o.y_off);
-      else if (o.unit == 16) strided_channels<uint4, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
-      else if (o.unit == 8) strided_channels<uint2, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
-      else strided_channels<uint32_t, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
-    }
+    for (int q = 0; q < 8; ++q)   // 16-byte pieces swizzled by row, as for the TMA store
+      sts_v4(sbuf + lane * 128 + ((q ^ (lane & 7)) << 4), make_uint4(row[4 * q], row[4 * q + 1], row[4 * q + 2], row[4 * q + 3]));
+    __syncwarp();
+    char* out = y + (long long)col0 * kEs;
+    if (kEs == 2 && o.unit == 2) strided_odd_channels(out, sbuf, lane, nc, rows_ok, o.y_off);
+    else if (o.unit == 16) strided_channels<uint4, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
+    else if (o.unit == 8) strided_channels<uint2, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
+    else strided_channels<uint32_t, kEs>(out, sbuf, lane, nc, rows_ok, o.y_off);
   }
 }
 
-// Epilogue for 16-bit y along channels whose pixels start on 32-byte boundaries (a multiple of 16 channels, or views that
-// keep that): a lane writes its own pixel from the registers, 16 channels (one whole 32-byte sector) per store, without
-// staging.  y: the lane's pixel, first column of the warp's share; ok: the pixel exists.
+// Epilogue for y along channels whose pixels start on 32-byte boundaries (16-bit: a multiple of 16 channels, or views that
+// keep that): a lane writes its own pixel from the registers, 16 channels (fp32: 8; one whole 32-byte sector) per store,
+// without staging.  y: the lane's pixel, first column of the warp's share; ok: the pixel exists.
 // read_done() is called once, when the accumulator has been read and before its last columns are stored.
 template <typename T, int WC, typename Done>
 __device__ __forceinline__ void epilogue_store_sectors(uint32_t t_row, int n0, int kout, int act, const float* s_scale,
@@ -574,32 +460,39 @@ __device__ __forceinline__ void epilogue_store_sectors(uint32_t t_row, int n0, i
     }
     if (c + 1 < chunks) tmem_ld_32x32b_x32(t_row + (c + 1) * 32, raw);   // travels while this chunk is rounded and stored
     else read_done();
-    uint32_t row[16];
-    if (act == 1) {
+    if (act > 1) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) row[j] = round_pack2_relu<T>(v[2 * j], v[2 * j + 1]);
-    } else {
-      if (act) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = apply_activation(v[j], act);
-      }
-#pragma unroll
-      for (int j = 0; j < 16; ++j) row[j] = round_pack2<T>(v[2 * j], v[2 * j + 1]);
+      for (int j = 0; j < 32; ++j) v[j] = apply_activation(v[j], act);
     }
-    if (ok) {
-      if (n0 + c * 32 + 16 <= kout) stg_v8(y + c * 32, row);
-      if (n0 + c * 32 + 32 <= kout) stg_v8(y + c * 32 + 16, row + 8);
+    if constexpr (sizeof(T) == 4) {
+      uint32_t row[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) row[j] = __float_as_uint(act == 1 ? relu_keep_nan(v[j]) : v[j]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (ok && n0 + c * 32 + i * 8 + 8 <= kout) stg_v8(y + c * 32 + i * 8, row + i * 8);
+    } else {
+      uint32_t row[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) row[j] = act == 1 ? round_pack2_relu<T>(v[2 * j], v[2 * j + 1]) : round_pack2<T>(v[2 * j], v[2 * j + 1]);
+      if (ok) {
+        if (n0 + c * 32 + 16 <= kout) stg_v8(y + c * 32, row);
+        if (n0 + c * 32 + 32 <= kout) stg_v8(y + c * 32 + 16, row + 8);
+      }
     }
   }
 }
 
-// Epilogue for 16-bit y along pixels (NCHW) when some of the warp's 32 rows are no output: a lane writes its own pixel of
-// one channel after another, neighbouring lanes neighbouring pixels, straight from the registers.
-//   y: the lane's pixel, first column of the warp's share; sk: elements between channels
-template <typename T, int WC, typename Done>
+// Epilogue for y along pixels (NCHW): a lane writes its own pixel of one channel after another, neighbouring lanes
+// neighbouring pixels, straight from the registers.  A 64-byte run per store reaches 2.6 (any alignment) to 4 TB/s over the
+// chip; staging the rows to store wider units cost more in latency than it saved (64 -> 64 3x3 on 128 x 56 x 56, 16 bytes
+// per lane 60.1 us, 4 bytes 62.9, straight from the registers 38.0).
+//   y, res: the lane's pixel, first column of the warp's share (res: nullptr or a tensor with y's strides); sk: elements
+//   between channels; read_done() is called once, when the accumulator has been read and before its last columns are stored
+template <typename T, int WC, bool RES, typename Done>
 __device__ __forceinline__ void epilogue_store_pixels(uint32_t t_row, int n0, int kout, int act, const float* s_scale,
-                                                      const float* s_bias, bool use_scale, uint16_t* y, long long sk, bool ok,
-                                                      Done&& read_done) {
+                                                      const float* s_bias, bool use_scale, T* y, const T* res, long long sk,
+                                                      bool ok, Done&& read_done) {
   int chunks = (kout - n0 + 31) / 32;
   if (chunks > WC / 32) chunks = WC / 32;
   if (chunks <= 0) {
@@ -610,6 +503,16 @@ __device__ __forceinline__ void epilogue_store_pixels(uint32_t t_row, int n0, in
   tmem_ld_32x32b_x32(t_row, raw);
 #pragma unroll 1
   for (int c = 0; c < chunks; ++c) {
+    const int nc = kout - n0 - c * 32;
+    float r[RES ? 32 : 1];
+    if constexpr (RES) {
+      if (res != nullptr && ok) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (j < nc) r[j] = to_f32<T>(res[j * sk]);
+        res += 32 * sk;
+      }
+    }
     tmem_ld_wait();
     float v[32];
 #pragma unroll
@@ -623,35 +526,48 @@ __device__ __forceinline__ void epilogue_store_pixels(uint32_t t_row, int n0, in
     }
     if (c + 1 < chunks) tmem_ld_32x32b_x32(t_row + (c + 1) * 32, raw);   // travels while this chunk is rounded and stored
     else read_done();
-    uint32_t row[16];
-    if (act == 1) {
+    if constexpr (RES) {
+      if (res != nullptr && ok) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) row[j] = round_pack2_relu<T>(v[2 * j], v[2 * j + 1]);
-    } else {
-      if (act) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = apply_activation(v[j], act);
+        for (int j = 0; j < 32; ++j)
+          if (j < nc) v[j] += r[j];
       }
-#pragma unroll
-      for (int j = 0; j < 16; ++j) row[j] = round_pack2<T>(v[2 * j], v[2 * j + 1]);
     }
-    const int nc = kout - n0 - c * 32;
-    if (ok) {
-      if (nc >= 32) {
+    if (act > 1) {   // uniform; kept apart so that the common paths do not fetch 32 copies of erf and tanh
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          y[0] = uint16_t(row[j]);
-          y[sk] = uint16_t(row[j] >> 16);
-          y += 2 * sk;
-        }
-      } else {
+      for (int j = 0; j < 32; ++j) v[j] = apply_activation(v[j], act);
+    }
+    if constexpr (sizeof(T) == 4) {
+      if (ok) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (2 * j < nc) y[0] = uint16_t(row[j]);
-          if (2 * j + 1 < nc) y[sk] = uint16_t(row[j] >> 16);
-          y += 2 * sk;
+        for (int j = 0; j < 32; ++j) {
+          if (j < nc) *y = act == 1 ? relu_keep_nan(v[j]) : v[j];
+          y += sk;
         }
       }
+    } else {
+      uint32_t row[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) row[j] = act == 1 ? round_pack2_relu<T>(v[2 * j], v[2 * j + 1]) : round_pack2<T>(v[2 * j], v[2 * j + 1]);
+      uint16_t* y16 = reinterpret_cast<uint16_t*>(y);
+      if (ok) {
+        if (nc >= 32) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            y16[0] = uint16_t(row[j]);
+            y16[sk] = uint16_t(row[j] >> 16);
+            y16 += 2 * sk;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (2 * j < nc) y16[0] = uint16_t(row[j]);
+            if (2 * j + 1 < nc) y16[sk] = uint16_t(row[j] >> 16);
+            y16 += 2 * sk;
+          }
+        }
+      }
+      y = reinterpret_cast<T*>(y16);
     }
   }
 }

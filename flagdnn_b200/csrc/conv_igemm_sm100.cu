@@ -445,7 +445,6 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         m = st_row;
         m_end = p.M;
       }
-      const int m0 = m;
       m += lane;
       const bool row_ok = !(DENSE && p.lowc) && m < m_end;   // per-lane addresses: not needed for quads
       long long y_off = 0;
@@ -470,15 +469,16 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         epilogue_store_tile<T, WC, RES>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
                                    out_stage + (warp - kFirstEpiWarp) * 2 * 32 * kRowBytes, lane, &tmY, &tmA2, st_row,
                                    st_img, st_rows, store_seq, &rf, g_scale != nullptr);
-      } else if (p.y_mode != kYScattered) {
+      } else if (p.y_mode == kYPixels) {
+        const long long at = y_off + (long long)n0 * p.y_sk;
+        epilogue_store_pixels<T, WC, RES>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr, y + at,
+                                          RES && g_res != nullptr ? g_res + at : nullptr, p.y_sk, row_ok, []() {});
+      } else if (p.y_mode == kYChannels) {
         StridedOut so;
         so.y = p.y;
-        so.k_off = k0 * p.y_sk;
         so.res = g_res;
         so.y_off = y_off;
-        so.sn = p.y_sn; so.sk = p.y_sk;
-        so.mode = p.y_mode; so.unit = p.y_unit;
-        so.m0 = m0; so.M = m_end; so.ohw = ohw;
+        so.unit = p.y_unit;
         so.row_ok = row_ok;
         epilogue_store_strided<T, WC, RES>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
                                            out_stage + (warp - kFirstEpiWarp) * 2 * 32 * kRowBytes, lane, so, store_seq);

@@ -113,7 +113,7 @@ int igemm_pair_stages();
 int igemm_pair_threads();
 int igemm_pair_max_resident_steps();  // reductions this short (and one channel tile) keep the filter resident
 
-// CTA pairs with one activation copy per filter row (conv_rows_sm100.cu): 16-bit types, W-stride 1, y along channels.
+// CTA pairs with one activation copy per filter row (conv_rows_sm100.cu): W-stride 1, y along channels or pixels.
 constexpr int kRowsCopy = 136;   // walk rows of an activation copy: a tile's 128 and up to 8 for the taps to its right
 struct RowsParams {
   int M;                 // N * OH * P walk rows
@@ -122,9 +122,10 @@ struct RowsParams {
   int stride_h, pad_top, pad_left, dil_h, dil_w;
   int R, S;
   int s_pitch;           // taps per filter row in memory (S, or more where the filter lies packed for grouped pixels)
-  int c_blocks;          // 64-channel blocks of a reduction (1 with blk_groups > 1)
+  int c_blocks;          // 128-byte blocks of channels of a reduction (1 with blk_groups > 1)
+  int halves;            // 2 for fp32 (TF32 high and low halves of both operands), else 1
   int m_tiles, n_tiles;
-  int b_bytes;           // one CTA's filters of a tap and channel block
+  int b_bytes;           // one CTA's filters of a tap and channel block (all halves)
   int a_stages, b_stages, b_resident, b_taps, b_slot;   // rings (rows_stages): copies, slots, whole filter, a slot's taps and bytes
   int blk_groups;        // > 1: groups of a 64-channel block, of cg channels and kg filters each; column tiles are blocks
   int cg, kg;
@@ -141,8 +142,8 @@ struct RowsParams {
   int skip_copies;
 };
 void rows_stages(RowsParams* p);
-cudaError_t launch_rows(int dtype, int tile_n, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY,
-                        const RowsParams& p, int grid, cudaStream_t stream);
+cudaError_t launch_rows(int dtype, int tile_n, const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB,
+                        const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream);
 cudaError_t rows_prepare_device();
 
 // Direct convolution on CUDA cores (conv_direct.cu): any dtype, groups, strides.

@@ -74,16 +74,19 @@ constexpr int kStoreChannels = 1;   // along channels, any alignment
 constexpr int kStorePixels = 2;     // along pixels
 template <typename T, int BN, int BLK, int STORE>
 __global__ void __launch_bounds__(kThreads, 1)
-conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmY, const RowsParams p) {
+conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
+                 const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmY, const RowsParams p) {
   using C = Cfg<BN>;
-  constexpr uint32_t kFmt = std::is_same<T, __half>::value ? 0u : 1u;
+  constexpr bool kSplit = std::is_same<T, float>::value;
+  constexpr uint32_t kFmt = std::is_same<T, __half>::value ? 0u : kSplit ? 2u : 1u;
+  constexpr int kBlock = 128 / int(sizeof(T));      // channels per copy
+  constexpr int kAStage = (kSplit ? 2 : 1) * kABytes;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // activation ring, then the filter: a ring of one tap and channel block per slot, or all of them
   uint8_t* a_ring = smem;
-  uint8_t* b_ring = smem + p.a_stages * kABytes;
+  uint8_t* b_ring = smem + p.a_stages * kAStage;
   uint8_t* out_stage = smem + kRingBytes;
   float* epi_stage = reinterpret_cast<float*>(out_stage + kOutBytes);
   uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + kOutBytes + C::kEpiBytes);
@@ -120,6 +123,7 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     fence_barrier_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
+    if constexpr (kSplit) tma_prefetch_desc(&tmA2);
     if (p.y_rows) tma_prefetch_desc(&tmY);
   }
   if (warp == 1) {
@@ -157,6 +161,8 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const int group = n_tile * BLK + g;
             tma_load_3d_pair(dst + g * part, &tmB, bar, group * p.blk_c_step, group * p.kg + int(rank) * (p.kg / 2), tap);
           }
+        } else if constexpr (kSplit) {   // both halves, one behind the other
+          tma_load_4d_pair(dst, &tmB, bar, c0, n_tile * BN + int(rank) * (BN / 2), tap, 0);
         } else {
           tma_load_3d_pair(dst, &tmB, bar, c0, n_tile * BN + int(rank) * (BN / 2), tap);
         }
@@ -165,7 +171,7 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (rank == 0) mbar_arrive_expect_tx(&b_full[0], uint32_t(2 * steps * p.b_slot));
         uint8_t* dst = b_ring;
         for (int r = 0; r < p.R; ++r)
-          for (int cb = 0; cb < p.c_blocks; ++cb, dst += p.b_slot) copy_filter(dst, b_full0, 0, cb * 64, r * p.s_pitch);
+          for (int cb = 0; cb < p.c_blocks; ++cb, dst += p.b_slot) copy_filter(dst, b_full0, 0, cb * kBlock, r * p.s_pitch);
       }
       __syncwarp();
       for (int tile = pair_id; tile < total_tiles && alive; tile += num_pairs) {
@@ -183,11 +189,13 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             alive = false;
             break;
           }
-          const int c0 = BLK > 1 ? n_tile * 64 : cb * 64;
+          const int c0 = BLK > 1 ? n_tile * 64 : cb * kBlock;
           if (lead) {
-            if (rank == 0) mbar_arrive_expect_tx(&a_full[as], uint32_t(2 * kABytes));
-            tma_load_im2col_4d_pair(a_ring + as * kABytes, &tmA, a_full0 + as * 8, c0, w_base, h_base, img, 0,
-                                    static_cast<uint16_t>(r * p.dil_h));
+            if (rank == 0) mbar_arrive_expect_tx(&a_full[as], uint32_t(2 * kAStage));
+            uint8_t* dst = a_ring + as * kAStage;
+            const uint16_t off_h = static_cast<uint16_t>(r * p.dil_h);
+            tma_load_im2col_4d_pair(dst, &tmA, a_full0 + as * 8, c0, w_base, h_base, img, 0, off_h);
+            if constexpr (kSplit) tma_load_im2col_4d_pair(dst + kABytes, &tmA2, a_full0 + as * 8, c0, w_base, h_base, img, 0, off_h);
           }
           __syncwarp();
           if (++as == uint32_t(p.a_stages)) {
@@ -238,7 +246,7 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     constexpr uint32_t kIdesc = make_idesc(kFmt, 2 * kRows, BN);
     const uint32_t blk_idesc = make_idesc(kFmt, 2 * kRows, uint32_t(p.kg));
     const uint32_t tap_step = uint32_t(p.dil_w) * (128 / 16);    // descriptor units from one tap's rows to the next one's
-    const uint32_t b_step = uint32_t(p.b_slot / p.b_taps) / 16;  // ... and from its filters to the next one's
+    const uint32_t b_step = uint32_t(p.b_slot / p.b_taps) / (kSplit ? 32 : 16);   // ... and from its filters to the next one's
     // The loop holds the waits, the MMAs and the commits and little else: with a branch on the number of 16-channel slices
     // and 64-bit descriptors carried from tap to tap a step of four MMAs took 470 clocks whatever its width.
     auto walk = [&](auto res_tag, uint32_t d_tmem) {
@@ -260,6 +268,20 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
             acc = 1;
           }
+        } else if constexpr (kSplit) {
+          // fp32 as three products of TF32 halves, smallest first
+          constexpr uint32_t kALow = kABytes / 16;
+          const uint32_t b_low = uint32_t(p.b_slot) / 32;
+          uint32_t b_lo = sw128_desc_lo(b_addr);
+          for (int t = 0; t < n; ++t, a_lo += tap_step, b_lo += b_step) {
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k += 2) {
+              mma_tf32<true>(d_tmem, a_lo + kALow + k, b_lo + k, kIdesc, k == 0 ? acc : 1u);
+              mma_tf32<true>(d_tmem, a_lo + k, b_lo + b_low + k, kIdesc, 1u);
+              mma_tf32<true>(d_tmem, a_lo + k, b_lo + k, kIdesc, 1u);
+            }
+            acc = 1;
+          }
         } else {
           uint32_t b_lo = sw128_desc_lo(b_addr);
           for (int t = 0; t < n; ++t, a_lo += tap_step, b_lo += b_step) {
@@ -271,7 +293,7 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       for (int kit = 0; kit < steps; ++kit) {
         if (!mbar_wait_warp(&a_full[as], aphase, abort_flag, p.status, kIncidentMmaWaitFull, p.wait_limit)) return false;
         tc_fence_after();
-        const uint32_t a_lo = a0 + as * (kABytes / 16);
+        const uint32_t a_lo = a0 + as * (kAStage / 16);
         if constexpr (kRes) {
           if (lead) {
             taps(a_lo, b_at, p.S);
@@ -376,7 +398,7 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(tempty_leader + buf * 8);
       };
-      if (STORE == kStoreSectors && p.y_rows && __all_sync(0xffffffffu, row_ok)) {
+      if (STORE == kStoreSectors && !kSplit && p.y_rows && __all_sync(0xffffffffu, row_ok)) {
         // 32 pixels one after another: boxes through the TMA unit
         const int pixel = __shfl_sync(0xffffffffu, real, 0);
         epilogue_store_tile<T, WC, false, 1>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY, pixel, 0, 32,
@@ -386,15 +408,13 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         epilogue_store_sectors<T, WC>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr,
                                       static_cast<T*>(p.y) + y_off + n0, row_ok, read_done);
       } else if constexpr (STORE == kStorePixels) {
-        epilogue_store_pixels<T, WC>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr,
-                                     static_cast<uint16_t*>(p.y) + y_off + n0 * p.y_sk, p.y_sk, row_ok, read_done);
+        epilogue_store_pixels<T, WC, false>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr,
+                                            static_cast<T*>(p.y) + y_off + n0 * p.y_sk, nullptr, p.y_sk, row_ok, read_done);
       } else {
         StridedOut so = {};
         so.y = p.y;
         so.y_off = y_off;
-        so.sn = p.y_sn; so.sk = 1;
-        so.mode = kYChannels; so.unit = p.y_unit;
-        so.m0 = m0; so.M = p.M; so.ohw = p.OH * p.OW;
+        so.unit = p.y_unit;
         so.row_ok = row_ok;
         epilogue_store_strided<T, WC, false, 1>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, so, store_seq);
         read_done();
@@ -417,7 +437,7 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 // The kernels a layer may run on: 32-byte stores for all of them, the other stores for layers that are not grouped.
 template <typename T, int BN, int BLK, int STORE>
-cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
+cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
@@ -432,20 +452,22 @@ cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = launch_overlap_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, conv_rows_kernel<T, BN, BLK, STORE>, tmA, tmB, tmY, p);
+  return cudaLaunchKernelEx(&cfg, conv_rows_kernel<T, BN, BLK, STORE>, tmA, tmA2, tmB, tmY, p);
 }
 
 template <typename T, int BN>
-cudaError_t launch_bn(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
+cudaError_t launch_bn(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
   if (p.blk_groups == 1) {
-    if (p.y_sk != 1) return launch_one<T, BN, 1, kStorePixels>(tmA, tmB, tmY, p, grid, stream);
-    if (p.y_unit == 32) return launch_one<T, BN, 1, kStoreSectors>(tmA, tmB, tmY, p, grid, stream);
-    return launch_one<T, BN, 1, kStoreChannels>(tmA, tmB, tmY, p, grid, stream);
+    if (p.y_sk != 1) return launch_one<T, BN, 1, kStorePixels>(tmA, tmA2, tmB, tmY, p, grid, stream);
+    if (p.y_unit == 32) return launch_one<T, BN, 1, kStoreSectors>(tmA, tmA2, tmB, tmY, p, grid, stream);
+    return launch_one<T, BN, 1, kStoreChannels>(tmA, tmA2, tmB, tmY, p, grid, stream);
   }
-  if (p.y_sk != 1 || p.y_unit != 32) return cudaErrorInvalidValue;
-  if (p.blk_groups == 2) return launch_one<T, BN, 2, kStoreSectors>(tmA, tmB, tmY, p, grid, stream);
-  if constexpr (BN > 64) {   // four groups of 32 filters or more
-    if (p.blk_groups == 4) return launch_one<T, BN, 4, kStoreSectors>(tmA, tmB, tmY, p, grid, stream);
+  if constexpr (sizeof(T) == 2) {
+    if (p.y_sk != 1 || p.y_unit != 32) return cudaErrorInvalidValue;
+    if (p.blk_groups == 2) return launch_one<T, BN, 2, kStoreSectors>(tmA, tmA2, tmB, tmY, p, grid, stream);
+    if constexpr (BN > 64) {   // four groups of 32 filters or more
+      if (p.blk_groups == 4) return launch_one<T, BN, 4, kStoreSectors>(tmA, tmA2, tmB, tmY, p, grid, stream);
+    }
   }
   return cudaErrorInvalidValue;
 }
@@ -458,18 +480,22 @@ cudaError_t prepare_bn() {
   cudaError_t e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, kStoreSectors>));
   if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, kStoreChannels>));
   if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, kStorePixels>));
-  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 2, kStoreSectors>));
-  if constexpr (BN > 64) {
-    if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 4, kStoreSectors>));
+  if constexpr (sizeof(T) == 2) {
+    if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 2, kStoreSectors>));
+    if constexpr (BN > 64) {
+      if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 4, kStoreSectors>));
+    }
   }
   return e;
 }
 
 template <typename T>
-cudaError_t launch_t(int tile_n, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
-  if (tile_n == 64) return launch_bn<T, 64>(tmA, tmB, tmY, p, grid, stream);
-  if (tile_n == 128) return launch_bn<T, 128>(tmA, tmB, tmY, p, grid, stream);
-  if (tile_n == 256) return launch_bn<T, 256>(tmA, tmB, tmY, p, grid, stream);
+cudaError_t launch_t(int tile_n, const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
+  if (tile_n == 64) return launch_bn<T, 64>(tmA, tmA2, tmB, tmY, p, grid, stream);
+  if (tile_n == 128) return launch_bn<T, 128>(tmA, tmA2, tmB, tmY, p, grid, stream);
+  if constexpr (sizeof(T) == 2) {
+    if (tile_n == 256) return launch_bn<T, 256>(tmA, tmA2, tmB, tmY, p, grid, stream);
+  }
   return cudaErrorInvalidValue;
 }
 
@@ -482,6 +508,8 @@ cudaError_t rows_prepare_device() {
   if (e == cudaSuccess) e = prepare_bn<__nv_bfloat16, 64>();
   if (e == cudaSuccess) e = prepare_bn<__nv_bfloat16, 128>();
   if (e == cudaSuccess) e = prepare_bn<__nv_bfloat16, 256>();
+  if (e == cudaSuccess) e = prepare_bn<float, 64>();
+  if (e == cudaSuccess) e = prepare_bn<float, 128>();
   return e;
 }
 
@@ -489,30 +517,31 @@ cudaError_t rows_prepare_device() {
 // column tile, else two rings.  A filter slot holds the taps of a filter row where two of the rows' worth fit three times
 // over (one wait and one commit for twelve MMAs), else one tap.
 void rows_stages(RowsParams* p) {
-  const int row = p->S * p->b_bytes, filter = p->R * p->c_blocks * row;
-  p->b_resident = p->n_tiles == 1 && filter <= kRingBytes - 4 * kABytes ? 1 : 0;
+  const int copy = kABytes * p->halves, row = p->S * p->b_bytes, filter = p->R * p->c_blocks * row;
+  p->b_resident = p->n_tiles == 1 && filter <= kRingBytes - 4 * copy ? 1 : 0;
   if (p->b_resident) {
     p->b_taps = p->S;
     p->b_slot = row;
     p->b_stages = 0;
-    p->a_stages = (kRingBytes - filter) / kABytes;
+    p->a_stages = (kRingBytes - filter) / copy;
     if (p->a_stages > kMaxA) p->a_stages = kMaxA;
     return;
   }
-  p->b_taps = kRingBytes / (kABytes + row) >= 3 ? p->S : 1;
+  p->b_taps = kRingBytes / (copy + row) >= 3 ? p->S : 1;
   p->b_slot = p->b_taps * p->b_bytes;
   // the producer runs ahead by as many taps as the filter ring holds; activation copies cover as many, and one more
   for (p->a_stages = 2;; ++p->a_stages) {
-    p->b_stages = (kRingBytes - p->a_stages * kABytes) / p->b_slot;
+    p->b_stages = (kRingBytes - p->a_stages * copy) / p->b_slot;
     if (p->b_stages > kMaxB) p->b_stages = kMaxB;
     if (p->a_stages == kMaxA || (p->a_stages - 1) * p->S >= p->b_stages * p->b_taps) break;
   }
 }
 
-cudaError_t launch_rows(int dtype, int tile_n, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY,
-                        const RowsParams& p, int grid, cudaStream_t stream) {
-  if (dtype == FDNN_F16) return launch_t<__half>(tile_n, tmA, tmB, tmY, p, grid, stream);
-  if (dtype == FDNN_BF16) return launch_t<__nv_bfloat16>(tile_n, tmA, tmB, tmY, p, grid, stream);
+cudaError_t launch_rows(int dtype, int tile_n, const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB,
+                        const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
+  if (dtype == FDNN_F16) return launch_t<__half>(tile_n, tmA, tmA2, tmB, tmY, p, grid, stream);
+  if (dtype == FDNN_BF16) return launch_t<__nv_bfloat16>(tile_n, tmA, tmA2, tmB, tmY, p, grid, stream);
+  if (dtype == FDNN_F32) return launch_t<float>(tile_n, tmA, tmA2, tmB, tmY, p, grid, stream);
   return cudaErrorInvalidValue;
 }
 

@@ -546,20 +546,25 @@ __device__ __forceinline__ void mma_f16_pair_lo(uint32_t d_tmem, uint32_t a_lo, 
       : "memory");
 }
 
-// fp32 operands as TF32 (one CTA): low descriptor words of K-major rows in the 128-byte swizzle.
+// fp32 operands as TF32: low descriptor words of K-major rows in the 128-byte swizzle.  kPair: a CTA pair.
+template <bool kPair = false>
 __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      ".reg .b64 a, b;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 a, {%1, %3};\n\t"
-      "mov.b64 b, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], a, b, %4, p;\n\t"
-      "}\n"
-      :
-      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "n"(kSw128DescHi), "r"(idesc), "r"(acc)
-      : "memory");
+#define FDNN_MMA_TF32(GROUP)                                                                                      \
+  asm volatile(                                                                                                   \
+      "{\n\t"                                                                                                     \
+      ".reg .pred p;\n\t"                                                                                         \
+      ".reg .b64 a, b;\n\t"                                                                                       \
+      "setp.ne.b32 p, %5, 0;\n\t"                                                                                 \
+      "mov.b64 a, {%1, %3};\n\t"                                                                                  \
+      "mov.b64 b, {%2, %3};\n\t"                                                                                  \
+      "tcgen05.mma." GROUP ".kind::tf32 [%0], a, b, %4, p;\n\t"                                                   \
+      "}\n"                                                                                                       \
+      :                                                                                                           \
+      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "n"(kSw128DescHi), "r"(idesc), "r"(acc)                                \
+      : "memory")
+  if constexpr (kPair) FDNN_MMA_TF32("cta_group::2");
+  else FDNN_MMA_TF32("cta_group::1");
+#undef FDNN_MMA_TF32
 }
 
 // Instruction descriptor: fp32 accumulate, both operands K-major, dense.
