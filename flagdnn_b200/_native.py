@@ -40,6 +40,7 @@ EXPORTED_SYMBOLS = (
     "fdnn_conv2d_fwd",
     "fdnn_conv2d_fwd_residual",
     "fdnn_conv2d_fwd_ex",
+    "fdnn_conv2d_fwd_unpacked",
     "fdnn_max_pool2d_fwd",
     "fdnn_adaptive_avg_pool2d_fwd",
     "fdnn_conv2d_fwd_host",
@@ -141,6 +142,8 @@ def load() -> ctypes.CDLL:
     lib.fdnn_conv2d_fwd_residual.argtypes = [ctypes.POINTER(ConvDesc), vp, vp, vp, vp, vp, vp, i32, vp, vp, i64, vp]
     lib.fdnn_conv2d_fwd_ex.restype = i32
     lib.fdnn_conv2d_fwd_ex.argtypes = [ctypes.POINTER(ConvDesc), vp, vp, vp, vp, vp, vp, i32, vp, vp, i64, vp, i64, vp]
+    lib.fdnn_conv2d_fwd_unpacked.restype = i32
+    lib.fdnn_conv2d_fwd_unpacked.argtypes = [ctypes.POINTER(ConvDesc), vp, vp, vp, i64, vp, vp, vp, i32, vp, vp, i64, vp]
     lib.fdnn_conv2d_fwd_host.restype = i32
     lib.fdnn_conv2d_fwd_host.argtypes = [ctypes.POINTER(ConvDesc), vp, vp, vp, vp, i32, vp, vp, i64, vp]
     lib.fdnn_conv2d_host_arena_bytes.restype = i32

@@ -275,6 +275,7 @@ def _load_fast() -> Any:
                        (lib.fdnn_conv2d_query, lib.fdnn_conv2d_pack_weight, lib.fdnn_conv2d_fwd_ex)]
             _fastcall.bind(*address, _packed_for_native, lib.fdnn_abi_version(), ctypes.sizeof(nat.ConvDesc),
                            ctypes.sizeof(nat.ConvPlan))
+            _fastcall.bind_unpacked(ctypes.cast(lib.fdnn_conv2d_fwd_unpacked, ctypes.c_void_p).value)
             _fast = _fastcall
         except (ImportError, AttributeError, TypeError) as exc:   # not built, or built against something else
             warnings.warn(f"flagdnn_b200: the native host path is not used, calls take some 15 us longer ({exc}); "

@@ -882,13 +882,15 @@ struct MapSlot {
 constexpr int kMapSets = 128, kMapWays = 4;
 std::atomic<long long> g_map_hits{0}, g_map_misses{0};
 
+// Four chains side by side: one multiply after another over the whole key took a fifth of a microsecond per launch.
 inline uint64_t map_key_hash(const MapKey& k) {
-  uint64_t h = 0x9e3779b97f4a7c15ull;
-  for (uint64_t v : k.w) {
-    h ^= v + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
-    h *= 0xff51afd7ed558ccdull;
-  }
-  return h ^ (h >> 32);
+  constexpr int kWords = int(sizeof(k.w) / sizeof(k.w[0]));
+  uint64_t h[4] = {0x9e3779b97f4a7c15ull, 0xbf58476d1ce4e5b9ull, 0x94d049bb133111ebull, 0xff51afd7ed558ccdull};
+  for (int i = 0; i < kWords; ++i) h[i & 3] = (h[i & 3] ^ k.w[i]) * 0x9fb21c651e98df25ull;
+  uint64_t v = h[0] ^ (h[1] >> 31) ^ (h[2] << 17) ^ (h[3] >> 13);
+  v ^= v >> 32;
+  v *= 0xff51afd7ed558ccdull;
+  return v ^ (v >> 32);
 }
 
 template <typename Encode>
@@ -1492,7 +1494,8 @@ int fdnn_conv2d_pack_weight(const fdnn_conv_desc* desc, const void* w, const voi
 static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, const void* w_packed,
                     const void* bias, const void* scale, const void* residual, int activation, void* y,
                     void* workspace, int64_t workspace_bytes, void* stream_v, bool allow_group, int k_real,
-                    void* sk_scratch = nullptr, int64_t sk_bytes = 0, const GroupBatch* batch = nullptr);
+                    void* sk_scratch = nullptr, int64_t sk_bytes = 0, const GroupBatch* batch = nullptr,
+                    FilterPack* pack = nullptr);
 
 int fdnn_conv2d_fwd(const fdnn_conv_desc* desc, const void* x, const void* w, const void* w_packed,
                     const void* bias, const void* scale, int activation, void* y, void* workspace,
@@ -1525,6 +1528,34 @@ int fdnn_conv2d_fwd_ex(const fdnn_conv_desc* desc, const void* x, const void* w,
                   true, desc->k, streamk_scratch, streamk_bytes);
 }
 
+int fdnn_conv2d_fwd_unpacked(const fdnn_conv_desc* desc, const void* x, const void* w, void* packed, int64_t packed_bytes,
+                             const void* bias, const void* scale, const void* residual, int activation, void* y,
+                             void* workspace, int64_t workspace_bytes, void* stream_v) {
+  if (desc == nullptr) return fail(FDNN_BAD_PARAM, "descriptor is NULL");
+  if (residual != nullptr && (reinterpret_cast<uintptr_t>(residual) & 15u) != (reinterpret_cast<uintptr_t>(y) & 15u))
+    return fail(FDNN_NOT_SUPPORTED, "the residual must have y's alignment modulo 16 bytes");
+  fdnn_conv_plan plan;
+  int st = make_plan(desc, x, w, y, &plan);
+  if (st != FDNN_OK) return st;
+  FilterPack pack = {};
+  if (plan.algo != FDNN_ALGO_DIRECT && plan.w_packed) {
+    if (w == nullptr || packed == nullptr) return fail(FDNN_BAD_PARAM, "w and packed must not be NULL");
+    if (packed_bytes < plan.packed_weight_bytes) return fail(FDNN_WORKSPACE_TOO_SMALL, "packed filter buffer too small");
+    if (desc->groups > 1 || plan.low_channel || plan.pixel_group > 1) {
+      st = fdnn_conv2d_pack_weight(desc, w, y, packed, packed_bytes, stream_v);
+      if (st != FDNN_OK) return st;
+    } else {
+      pack = {w, {desc->w_strides[0], desc->w_strides[1], desc->w_strides[2], desc->w_strides[3]}, desc->k, desc->c, desc->r,
+              desc->s, plan.c_padded, packed, false};
+      remember_packed(packed, current_device_or_minus1(), packed_layout_of(*desc, plan));
+    }
+  } else {
+    packed = nullptr;
+  }
+  return fwd_impl(desc, x, w, packed, bias, scale, residual, activation, y, workspace, workspace_bytes, stream_v, true, desc->k,
+                  nullptr, 0, nullptr, pack.w != nullptr ? &pack : nullptr);
+}
+
 // One-time set-up of the current device for kernels that use tensor maps and bounded waits.
 static int prepare_device(int* device) {
   int dev = 0;
@@ -1548,14 +1579,23 @@ static int prepare_device(int* device) {
   return FDNN_OK;
 }
 
+static int pack_filter(int dtype, FilterPack* f, cudaStream_t stream) {
+  if (f == nullptr || f->done) return FDNN_OK;
+  f->done = true;
+  cudaError_t e = launch_pack_w(dtype, f->w, f->strides, f->K, f->C, f->R, f->S, f->c_pad, f->dst, (long long)f->K * f->R * f->S * f->c_pad,
+                                stream);
+  return e == cudaSuccess ? FDNN_OK : fail_cuda("pack_weight launch", e);
+}
+
 // Rewrites x into the scratch as dense NHWC where the plan says so, and says how the kernels see it.
 struct ActivationView {
   const void* base;
   int c;                       // channels that may be read
   long long sw, sh, sn, plane; // element strides; offset of the second plane (fp32)
 };
+// pack: the layer's filter, packed in the same launch where that is possible, else in one before it.
 static int relayout_x(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, bool by_groups, const void* x, void* workspace,
-                      int64_t workspace_bytes, cudaStream_t stream, ActivationView* a) {
+                      int64_t workspace_bytes, cudaStream_t stream, ActivationView* a, FilterPack* pack) {
   const int es = elem_size(d.dtype);
   // Extent-one dimensions get a harmless aligned stride (theirs may be anything).
   a->base = x;
@@ -1564,14 +1604,16 @@ static int relayout_x(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, bool 
   a->sh = d.h > 1 ? d.x_strides[2] : plan.c_padded;
   a->sn = d.n > 1 ? d.x_strides[0] : plan.c_padded;
   a->plane = 0;
-  if (!plan.x_repacked) return FDNN_OK;
+  if (!plan.x_repacked) return pack_filter(d.dtype, pack, stream);
   int x_pad = by_groups ? d.c : padded_x_channels(&d);   // groups side by side, 16-byte multiples each
   if (!by_groups && (long long)(d.dtype == FDNN_F32 ? 2 : 1) * d.n * d.h * d.w * x_pad * es > workspace_bytes)
     x_pad = round_up(d.c, 16 / es);
   a->plane = (long long)d.n * d.h * d.w * x_pad;
   cudaError_t e = launch_repack_x(d.dtype, x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w, x_pad,
-                                  workspace, a->plane, stream);
+                                  workspace, a->plane, stream, pack);
   if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
+  const int st = pack_filter(d.dtype, pack, stream);
+  if (st != FDNN_OK) return st;
   a->base = workspace;
   a->sw = x_pad;
   a->sh = (long long)d.w * x_pad;
@@ -1588,12 +1630,12 @@ struct FilterView {
 };
 
 static int fwd_rows(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, const RowsMode& rows, int dev, const void* x,
-                    const FilterView& f, const void* bias, const void* scale, int activation, void* y, void* workspace,
-                    int64_t workspace_bytes, cudaStream_t stream) {
+                    const FilterView& f, FilterPack* pack, const void* bias, const void* scale, int activation, void* y,
+                    void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
   ActivationView a;
   fdnn_conv_desc whole = d;    // a block of channels is copied whatever groups it holds
   whole.groups = 1;
-  int st = relayout_x(whole, plan, false, x, workspace, workspace_bytes, stream, &a);
+  int st = relayout_x(whole, plan, false, x, workspace, workspace_bytes, stream, &a, pack);
   if (st != FDNN_OK) return st;
   const int cg = d.c / d.groups, kg = d.k / d.groups, es = elem_size(d.dtype);
   alignas(64) CUtensorMap tmA, tmA2, tmB;
@@ -1664,7 +1706,7 @@ static int fwd_rows(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, const R
 static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, const void* w_packed,
                     const void* bias, const void* scale, const void* residual, int activation, void* y,
                     void* workspace, int64_t workspace_bytes, void* stream_v, bool allow_group, int k_real,
-                    void* sk_scratch, int64_t sk_bytes, const GroupBatch* batch) {
+                    void* sk_scratch, int64_t sk_bytes, const GroupBatch* batch, FilterPack* pack) {
   fdnn_conv_plan plan;
   // A caller that hands over a packed filter wants it used even when w itself
   // would qualify for in-place reads; plan accordingly.
@@ -1708,7 +1750,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
       int dev = 0;
       st = prepare_device(&dev);
       if (st != FDNN_OK) return st;
-      return fwd_rows(d, plan, rows, dev, x, f, bias, scale, activation, y, workspace, workspace_bytes, stream);
+      return fwd_rows(d, plan, rows, dev, x, f, nullptr, bias, scale, activation, y, workspace, workspace_bytes, stream);
     }
   }
   if (batch == nullptr && d.groups > 1 && plan.algo != FDNN_ALGO_DIRECT && allow_group) {
@@ -1855,7 +1897,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
         const int s_pitch = plan.pixel_group > 1 ? d.s + (plan.pixel_group - 1) * d.stride_w : d.s;
         f = {w_packed, c_pad, s_pitch, 0, c_pad, (long long)d.r * s_pitch * c_pad};
       }
-      return fwd_rows(d, plan, rows, dev, x, f, bias, scale, activation, y, workspace, workspace_bytes, stream);
+      return fwd_rows(d, plan, rows, dev, x, f, pack, bias, scale, activation, y, workspace, workspace_bytes, stream);
     }
   }
   if (plan.pixel_group > 1) {
@@ -1882,9 +1924,11 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     e = launch_repack_x_windows(x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w, d.pad_left,
                                 windows.w_pad, workspace, stream);
     if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
+    st = pack_filter(d.dtype, pack, stream);
+    if (st != FDNN_OK) return st;
     a.base = workspace;
   } else {
-    st = relayout_x(d, plan, batch != nullptr, x, workspace, workspace_bytes, stream, &a);
+    st = relayout_x(d, plan, batch != nullptr, x, workspace, workspace_bytes, stream, &a, pack);
     if (st != FDNN_OK) return st;
   }
   const bool b_mn = !plan.w_packed && filter_mn_major(&d, w);

@@ -193,9 +193,17 @@ cudaError_t launch_adaptive_avg_pool2d(int dtype, const PoolParams& p, cudaStrea
 // x[N,C,H,W] (any strides) -> dense NHWC with C padded to c_pad (zeros).  For
 // f32 two planes are written: TF32-rounded high halves at dst, the rounded
 // remainders at dst + plane_elems.
+// pack: a filter to pack to [K, R, S, c_pad] in the same launch if its kernel can (pack->done then), or nullptr.
+struct FilterPack {
+  const void* w;
+  long long strides[4];
+  int K, C, R, S, c_pad;
+  void* dst;
+  bool done;
+};
 cudaError_t launch_repack_x(int dtype, const void* x, const long long x_s[4], int N, int C, int H,
                             int W, int c_pad, void* dst, long long plane_elems,
-                            cudaStream_t stream);
+                            cudaStream_t stream, FilterPack* pack = nullptr);
 // Low-channel relayouts (C <= 4, 16-bit types):
 // x -> [N][H][w_pad][4]: `pad_left` zero pixels, the image row, zeros up to w_pad; channel 4 is zero.
 cudaError_t launch_repack_x_lowc(int dtype, const void* x, const long long x_s[4], int N, int C, int H,

@@ -9,7 +9,8 @@
 // padding, empty results, a residual that cannot be fused); the Python implementation then runs, raises the
 // documented errors, or takes the slow route.  Nothing is remembered about tensors: plans are kept by geometry,
 // strides and alignment (at most kMaxPlans of them), and filters that need packing are either packed into a buffer of
-// this call or looked up by the Python-side cache through the callback given to bind().
+// this call (small ones of NCHW layers, by the launch that relays x out) or looked up by the Python-side cache through the
+// callback given to bind().
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -27,12 +28,13 @@
 namespace {
 
 using QueryFn = int (*)(const fdnn_conv_desc*, const void*, const void*, const void*, fdnn_conv_plan*);
-using PackFn = int (*)(const fdnn_conv_desc*, const void*, const void*, void*, int64_t, void*);
 using FwdFn = int (*)(const fdnn_conv_desc*, const void*, const void*, const void*, const void*, const void*, const void*,
                       int, void*, void*, int64_t, void*, int64_t, void*);
 QueryFn g_query = nullptr;
-PackFn g_pack = nullptr;
 FwdFn g_fwd = nullptr;
+using FwdUnpackedFn = int (*)(const fdnn_conv_desc*, const void*, const void*, void*, int64_t, const void*, const void*, const void*,
+                              int, void*, void*, int64_t, void*);
+FwdUnpackedFn g_fwd_unpacked = nullptr;
 PyObject* g_packed_weight = nullptr;   // (weight, address of desc, address of plan, stream, y address) -> packed tensor
 
 // The descriptor (all plain integers), the alignment of x, w and y, and the device.
@@ -52,6 +54,9 @@ struct PlanHash {
 };
 static_assert(sizeof(fdnn_conv_desc) % 4 == 0 && sizeof(PlanKey) % 4 == 0, "hashed and compared by words");
 constexpr size_t kMaxPlans = 1024;
+// Packing a filter of up to a megabyte in the launch that relays an NCHW x out anyway costs less than the look-up of a kept
+// one, which is Python code (64 -> 64 3x3 on one 14 x 14 image, f16, a call: XX us with the look-up, YY so).
+constexpr int64_t kPackAlways = 1 << 20;
 std::unordered_map<PlanKey, fdnn_conv_plan, PlanHash>& plans() {   // used with the GIL held
   static auto* m = new std::unordered_map<PlanKey, fdnn_conv_plan, PlanHash>();
   return *m;
@@ -146,23 +151,25 @@ int launch(const fdnn_conv_desc& d, const at::Tensor& x, const at::Tensor& w, Py
   }
   const fdnn_conv_plan plan = it->second;   // a copy: the callback below may run other Python code
   void* stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
-  at::Tensor packed, scratch;
+  at::Tensor scratch;
   PyObject* held = nullptr;
   const void* packed_ptr = nullptr;
   if (plan.algo != FDNN_ALGO_DIRECT && plan.w_packed) {
-    if (weight_obj != nullptr) {
-      held = PyObject_CallFunction(g_packed_weight, "OKKKK", weight_obj, (unsigned long long)(uintptr_t)&d,
-                                   (unsigned long long)(uintptr_t)&plan, (unsigned long long)(uintptr_t)stream,
-                                   (unsigned long long)(uintptr_t)yp);
-      if (held == nullptr) return -1;
-      packed_ptr = THPVariable_Unpack(held).const_data_ptr();
-    } else {
+    const bool in_relayout = plan.x_repacked && d.groups == 1 && plan.low_channel == 0 && plan.pixel_group <= 1 && d.c >= 8 &&
+                             d.x_strides[3] == 1 && d.x_strides[1] != 1 && d.w > 1 && plan.packed_weight_bytes <= kPackAlways;
+    if (weight_obj == nullptr || in_relayout) {
       WithoutGil free;
-      packed = at::empty({plan.packed_weight_bytes}, x.options().dtype(at::kByte));
-      const int st = g_pack(&d, wp, yp, packed.mutable_data_ptr(), plan.packed_weight_bytes, stream);
-      if (st != FDNN_OK) return st;
-      packed_ptr = packed.const_data_ptr();
+      const int64_t ws_bytes = (plan.workspace_bytes + 255) / 256 * 256;
+      scratch = at::empty({ws_bytes + plan.packed_weight_bytes}, x.options().dtype(at::kByte));
+      char* base = static_cast<char*>(scratch.mutable_data_ptr());
+      return g_fwd_unpacked(&d, xp, wp, base + ws_bytes, plan.packed_weight_bytes, bias, scale, residual, act, yp,
+                            plan.workspace_bytes > 0 ? base : nullptr, plan.workspace_bytes, stream);
     }
+    held = PyObject_CallFunction(g_packed_weight, "OKKKK", weight_obj, (unsigned long long)(uintptr_t)&d,
+                                 (unsigned long long)(uintptr_t)&plan, (unsigned long long)(uintptr_t)stream,
+                                 (unsigned long long)(uintptr_t)yp);
+    if (held == nullptr) return -1;
+    packed_ptr = THPVariable_Unpack(held).const_data_ptr();
   }
   int st;
   try {
@@ -191,7 +198,7 @@ PyObject* finish(int status, at::Tensor&& y) {
 // conv(input, weight, bias, scale, residual, stride, padding, dilation, groups, algo, activation)
 PyObject* fast_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS   // C++ exceptions leave as the Python types torch gives them (torch.OutOfMemoryError among them)
-  if (n != 11 || g_fwd == nullptr) return none();
+  if (n != 11 || g_fwd_unpacked == nullptr) return none();
     const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
     if (x == nullptr || w == nullptr || x->dim() != 4 || w->dim() != 4) return none();
     const int dtype = dtype_code(x->scalar_type());
@@ -254,7 +261,7 @@ PyObject* fast_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // conv1d(input [N, C, L], weight, bias, stride, padding, dilation, groups, algo): the 2-D call with H = R = 1
 PyObject* fast_conv1d(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS   // C++ exceptions leave as the Python types torch gives them (torch.OutOfMemoryError among them)
-  if (n != 8 || g_fwd == nullptr) return none();
+  if (n != 8 || g_fwd_unpacked == nullptr) return none();
     const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
     if (x == nullptr || w == nullptr || x->dim() != 3 || w->dim() != 3) return none();
     const int dtype = dtype_code(x->scalar_type());
@@ -315,7 +322,7 @@ PyObject* fast_conv1d(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // mm(a [M, K], b [K, N], algo): a 1x1 convolution over one row of M pixels whose filter is b transposed
 PyObject* fast_mm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS   // C++ exceptions leave as the Python types torch gives them (torch.OutOfMemoryError among them)
-  if (n != 3 || g_fwd == nullptr) return none();
+  if (n != 3 || g_fwd_unpacked == nullptr) return none();
     const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
     if (x == nullptr || w == nullptr || x->dim() != 2 || w->dim() != 2) return none();
     const int dtype = dtype_code(x->scalar_type());
@@ -366,9 +373,17 @@ PyObject* bind(PyObject*, PyObject* args) {
   Py_INCREF(cb);
   Py_XDECREF(g_packed_weight);
   g_packed_weight = cb;
+  (void)p;   // fdnn_conv2d_pack_weight: the packed-filter callback calls it
   g_query = reinterpret_cast<QueryFn>(uintptr_t(q));
-  g_pack = reinterpret_cast<PackFn>(uintptr_t(p));
   g_fwd = reinterpret_cast<FwdFn>(uintptr_t(f));
+  return none();
+}
+
+// bind_unpacked(address of fdnn_conv2d_fwd_unpacked), after bind()
+PyObject* bind_unpacked(PyObject*, PyObject* arg) {
+  const unsigned long long f = PyLong_AsUnsignedLongLong(arg);
+  if (PyErr_Occurred()) return nullptr;
+  g_fwd_unpacked = reinterpret_cast<FwdUnpackedFn>(uintptr_t(f));
   return none();
 }
 
@@ -377,6 +392,7 @@ PyMethodDef kMethods[] = {
     {"conv1d", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fast_conv1d)), METH_FASTCALL, nullptr},
     {"mm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fast_mm)), METH_FASTCALL, nullptr},
     {"bind", bind, METH_VARARGS, nullptr},
+    {"bind_unpacked", bind_unpacked, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_fastcall", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

@@ -177,6 +177,13 @@ int fdnn_conv2d_fwd(const fdnn_conv_desc* desc, const void* x, const void* w,
                     int activation, void* y, void* workspace,
                     int64_t workspace_bytes, void* stream);
 
+/* fdnn_conv2d_fwd_residual for a filter that is not kept packed: where the plan needs one, w is packed into
+ * `packed` (plan.packed_weight_bytes, 16-byte aligned) first, in the launch that relays x out where that is
+ * possible.  For layers whose filter is small beside x, or new on every call. */
+int fdnn_conv2d_fwd_unpacked(const fdnn_conv_desc* desc, const void* x, const void* w, void* packed,
+                             int64_t packed_bytes, const void* bias, const void* scale, const void* residual,
+                             int activation, void* y, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* y = act( conv(x, w) * scale[k] + bias[k] + residual ): fdnn_conv2d_fwd with a
  * residual tensor added in fp32 before the activation and the single rounding
  * (a ResNet block's third convolution, its shortcut add and the ReLU in one
