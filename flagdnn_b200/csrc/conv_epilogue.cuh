@@ -53,6 +53,17 @@ __device__ __forceinline__ float apply_activation(float v, int act) {
   return v;
 }
 
+// The same for kernels that exist once with GELU and once without (GELU = false: none or ReLU).  erf and tanh, inlined for
+// every value of an unrolled epilogue, are 110 KB of a tensor-core kernel's 180 KB of code; spread between the instructions
+// of the other activations they made the drain loop miss the instruction cache, most of all where layers of different
+// kernels alternate (in a ResNet-50 of 128 images: 64 -> 256 1x1 at 56 x 56 60.4 -> 51.0 us, 64 -> 64 3x3 37.9 -> 35.3;
+// an 8192 x 4096 x 4096 product 177.1 -> 173.2).
+template <bool GELU>
+__device__ __forceinline__ float activate(float v, int act) {
+  if constexpr (GELU) return apply_activation(v, act);
+  return act == 1 ? relu_keep_nan(v) : v;
+}
+
 template <typename T>
 __device__ __forceinline__ uint32_t round_pack2(float a, float b);
 template <>
@@ -116,7 +127,7 @@ struct ResidualFetch {
 //                    reduction splitting: the accumulator holds only the tile's last reduction steps; add the
 //                    fp32 partial sums of sk_count other CTAs first (slots sk_slot0, sk_slot0 - sk_slot_stride,
 //                    ... in that order; this lane's row sk_row, this warp's first 16-byte piece sk_pc0)
-template <typename T, int BN, bool RES = false, int NBUF = 2>
+template <typename T, int BN, bool RES, int NBUF, bool GELU>
 __device__ __forceinline__ void epilogue_store_tile(uint32_t t_row, int n0, int kout, int act,
                                                     const float* s_scale, const float* s_bias,
                                                     uint8_t* my_out, int lane, const CUtensorMap* tm_full,
@@ -215,12 +226,10 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_row, int n0, int 
           }
         }
         if constexpr (std::is_same<T, float>::value) {
-          if (act) {  // uniform across the launch
-            v0 = apply_activation(v0, act);
-            v1 = apply_activation(v1, act);
-            v2 = apply_activation(v2, act);
-            v3 = apply_activation(v3, act);
-          }
+          v0 = activate<GELU>(v0, act);   // uniform across the launch
+          v1 = activate<GELU>(v1, act);
+          v2 = activate<GELU>(v2, act);
+          v3 = activate<GELU>(v3, act);
           row[4 * j4 + 0] = __float_as_uint(v0);
           row[4 * j4 + 1] = __float_as_uint(v1);
           row[4 * j4 + 2] = __float_as_uint(v2);
@@ -229,7 +238,7 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_row, int n0, int 
           row[l * 16 + 2 * j4 + 0] = round_pack2_relu<T>(v0, v1);
           row[l * 16 + 2 * j4 + 1] = round_pack2_relu<T>(v2, v3);
         } else {
-          if (act) {
+          if constexpr (GELU) {
             v0 = apply_activation(v0, act);
             v1 = apply_activation(v1, act);
             v2 = apply_activation(v2, act);
@@ -358,7 +367,7 @@ __device__ __forceinline__ void strided_odd_channels(char* out, uint32_t sbuf, i
 }
 
 // NBUF staging buffers of 4 KB per warp.
-template <typename T, int BN, bool RES, int NBUF = 2>
+template <typename T, int BN, bool RES, int NBUF, bool GELU>
 __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, int kout, int act, const float* s_scale,
                                                        const float* s_bias, uint8_t* my_out, int lane,
                                                        const StridedOut& o, uint32_t& store_seq) {
@@ -401,7 +410,7 @@ __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, i
             if (l * 32 + j < nc) v[j] += to_f32<T>(res[j]);
         }
       }
-      if (act > 1) {   // uniform; kept apart so that the common paths do not fetch 32 copies of erf and tanh
+      if constexpr (GELU) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = apply_activation(v[j], act);
       }
@@ -434,7 +443,7 @@ __device__ __forceinline__ void epilogue_store_strided(uint32_t t_row, int n0, i
 // keep that): a lane writes its own pixel from the registers, 16 channels (fp32: 8; one whole 32-byte sector) per store,
 // without staging.  y: the lane's pixel, first column of the warp's share; ok: the pixel exists.
 // read_done() is called once, when the accumulator has been read and before its last columns are stored.
-template <typename T, int WC, typename Done>
+template <typename T, int WC, bool GELU, typename Done>
 __device__ __forceinline__ void epilogue_store_sectors(uint32_t t_row, int n0, int kout, int act, const float* s_scale,
                                                        const float* s_bias, bool use_scale, T* y, bool ok, Done&& read_done) {
   int chunks = (kout - n0 + 31) / 32;
@@ -460,7 +469,7 @@ __device__ __forceinline__ void epilogue_store_sectors(uint32_t t_row, int n0, i
     }
     if (c + 1 < chunks) tmem_ld_32x32b_x32(t_row + (c + 1) * 32, raw);   // travels while this chunk is rounded and stored
     else read_done();
-    if (act > 1) {
+    if constexpr (GELU) {
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] = apply_activation(v[j], act);
     }
@@ -489,7 +498,7 @@ __device__ __forceinline__ void epilogue_store_sectors(uint32_t t_row, int n0, i
 // per lane 60.1 us, 4 bytes 62.9, straight from the registers 38.0).
 //   y, res: the lane's pixel, first column of the warp's share (res: nullptr or a tensor with y's strides); sk: elements
 //   between channels; read_done() is called once, when the accumulator has been read and before its last columns are stored
-template <typename T, int WC, bool RES, typename Done>
+template <typename T, int WC, bool RES, bool GELU, typename Done>
 __device__ __forceinline__ void epilogue_store_pixels(uint32_t t_row, int n0, int kout, int act, const float* s_scale,
                                                       const float* s_bias, bool use_scale, T* y, const T* res, long long sk,
                                                       bool ok, Done&& read_done) {
@@ -533,7 +542,7 @@ __device__ __forceinline__ void epilogue_store_pixels(uint32_t t_row, int n0, in
           if (j < nc) v[j] += r[j];
       }
     }
-    if (act > 1) {   // uniform; kept apart so that the common paths do not fetch 32 copies of erf and tanh
+    if constexpr (GELU) {
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] = apply_activation(v[j], act);
     }

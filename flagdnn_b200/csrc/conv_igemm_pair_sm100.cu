@@ -80,7 +80,8 @@ static_assert(kStages * kStageBytes <= kRingBytes, "streaming ring must fit");
 constexpr uint32_t kTmemColsPair = 512;              // two 256-column accumulators
 static_assert(kSmemPair <= 227 * 1024, "shared memory budget");
 
-template <typename T, bool RES>
+// GELU: the activation is one of the GELU forms (p.act > 1).
+template <typename T, bool RES, bool GELU>
 __global__ void __launch_bounds__(kThreadsPair, 1)
 conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmY2,
@@ -640,7 +641,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         st_rows = 32;
       }
       const float* sk_slot0 = sk_count > 0 ? p.sk_slots + (long long)(2 * (pair_id - 1) + int(rank)) * kSkSlotFloats : nullptr;
-      epilogue_store_tile<T, kWarpCols, RES, kOutBufs>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY2,
+      epilogue_store_tile<T, kWarpCols, RES, kOutBufs, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY2,
                                      st_row, st_img, st_rows, store_seq, &rf, g_scale != nullptr,
                                      sk_slot0, sk_count, 2LL * kSkSlotFloats, sk_row, sk_pc0);
       if (sk_count > 0) {
@@ -691,24 +692,29 @@ cudaError_t launch_pair_t(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = launch_overlap_enabled() ? 2 : 1;
-  if (p.residual != nullptr) return cudaLaunchKernelEx(&cfg, conv_igemm_pair_kernel<T, true>, tmA, tmB, tmY, tmY2, tmR, tmRbox, p);
-  return cudaLaunchKernelEx(&cfg, conv_igemm_pair_kernel<T, false>, tmA, tmB, tmY, tmY2, tmR, tmRbox, p);
+  const bool gelu = p.act > 1;
+  auto* kernel = p.residual != nullptr ? (gelu ? conv_igemm_pair_kernel<T, true, true> : conv_igemm_pair_kernel<T, true, false>)
+                                       : (gelu ? conv_igemm_pair_kernel<T, false, true> : conv_igemm_pair_kernel<T, false, false>);
+  return cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, tmY, tmY2, tmR, tmRbox, p);
 }
 
 }  // namespace
 
+template <typename T>
+static cudaError_t prepare_t() {
+  auto opt_in = [](const void* kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPair);
+  };
+  cudaError_t e = opt_in(reinterpret_cast<const void*>(conv_igemm_pair_kernel<T, false, false>));
+  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_pair_kernel<T, true, false>));
+  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_pair_kernel<T, false, true>));
+  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_pair_kernel<T, true, true>));
+  return e;
+}
+
 cudaError_t igemm_pair_prepare_device() {
-  cudaError_t e = cudaFuncSetAttribute(conv_igemm_pair_kernel<__half, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPair);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(conv_igemm_pair_kernel<__half, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kSmemPair);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(conv_igemm_pair_kernel<__nv_bfloat16, false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPair);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(conv_igemm_pair_kernel<__nv_bfloat16, true>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPair);
+  cudaError_t e = prepare_t<__half>();
+  if (e == cudaSuccess) e = prepare_t<__nv_bfloat16>();
   return e;
 }
 

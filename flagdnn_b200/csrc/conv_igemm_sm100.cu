@@ -65,7 +65,6 @@ template <typename T, int BN>
 struct TileCfg {
   static constexpr bool kSplit = std::is_same<T, float>::value;
   static constexpr int kKB = kRowBytes / int(sizeof(T));  // reduction elements per stage
-  static constexpr int kUK = 32 / int(sizeof(T));         // reduction elements per MMA
   static constexpr int kABytes = kBM * kRowBytes;
   static constexpr int kBBytes = BN * kRowBytes;
   static constexpr int kStageBytes = (kSplit ? 2 : 1) * (kABytes + kBBytes);
@@ -99,7 +98,8 @@ __device__ __forceinline__ void store32_contig(float* dst, const float (&v)[32])
 
 // DENSE: y goes through the TMA unit (p.tma_store); otherwise through the warps' own stores, whose registers would push
 // the dense path's loop state to local memory if both lived in one kernel.
-template <typename T, int BN, bool RES, bool DENSE>
+// GELU: the activation is one of the GELU forms (p.act > 1).
+template <typename T, int BN, bool RES, bool DENSE, bool GELU>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
                   const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmB2,
@@ -466,12 +466,12 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if constexpr (DENSE) {
         // a tile's last warp may own fewer than 32 valid rows: tmA2 then holds a second
         // output map whose box is exactly that short (low-channel mode, 16-bit only)
-        epilogue_store_tile<T, WC, RES>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
+        epilogue_store_tile<T, WC, RES, 2, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
                                    out_stage + (warp - kFirstEpiWarp) * 2 * 32 * kRowBytes, lane, &tmY, &tmA2, st_row,
                                    st_img, st_rows, store_seq, &rf, g_scale != nullptr);
       } else if (p.y_mode == kYPixels) {
         const long long at = y_off + (long long)n0 * p.y_sk;
-        epilogue_store_pixels<T, WC, RES>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr, y + at,
+        epilogue_store_pixels<T, WC, RES, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr, y + at,
                                           RES && g_res != nullptr ? g_res + at : nullptr, p.y_sk, row_ok, []() {});
       } else if (p.y_mode == kYChannels) {
         StridedOut so;
@@ -480,7 +480,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         so.y_off = y_off;
         so.unit = p.y_unit;
         so.row_ok = row_ok;
-        epilogue_store_strided<T, WC, RES>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
+        epilogue_store_strided<T, WC, RES, 2, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
                                            out_stage + (warp - kFirstEpiWarp) * 2 * 32 * kRowBytes, lane, so, store_seq);
       } else {
 #pragma unroll 1
@@ -497,7 +497,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           a = fmaf(a, s_scale[chunk * 32 + j], s_bias[chunk * 32 + j]);
           if (RES && g_res != nullptr && row_ok && col0 + j < p.Kout)
             a += to_f32<T>(g_res[y_off + (long long)(col0 + j) * p.y_sk]);
-          if (p.act) a = apply_activation(a, p.act);
+          a = activate<GELU>(a, p.act);
           v[j] = a;
         }
         if (row_ok && p.out_f32) {
@@ -555,8 +555,12 @@ cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CU
   cfg.attrs = attr;
   cfg.numAttrs = launch_overlap_enabled() ? 1 : 0;
   const bool res = p.residual != nullptr, dense = p.tma_store != 0;
-  auto* kernel = res ? (dense ? conv_igemm_kernel<T, BN, true, true> : conv_igemm_kernel<T, BN, true, false>)
-                     : (dense ? conv_igemm_kernel<T, BN, false, true> : conv_igemm_kernel<T, BN, false, false>);
+  auto pick = [&](auto gelu) {
+    constexpr bool G = decltype(gelu)::value;
+    return res ? (dense ? conv_igemm_kernel<T, BN, true, true, G> : conv_igemm_kernel<T, BN, true, false, G>)
+               : (dense ? conv_igemm_kernel<T, BN, false, true, G> : conv_igemm_kernel<T, BN, false, false, G>);
+  };
+  auto* kernel = p.act > 1 ? pick(std::true_type{}) : pick(std::false_type{});
   return cudaLaunchKernelEx(&cfg, kernel, tmA, tmA2, tmB, tmB2, tmY, tmR, tmRbox, p);
 }
 
@@ -566,10 +570,16 @@ cudaError_t prepare_one() {
   auto opt_in = [](const void* kernel) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   };
-  cudaError_t e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, false, true>));
-  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, true, true>));
-  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, false, false>));
-  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, true, false>));
+  auto all = [&](auto gelu) {
+    constexpr bool G = decltype(gelu)::value;
+    cudaError_t e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, false, true, G>));
+    if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, true, true, G>));
+    if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, false, false, G>));
+    if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_igemm_kernel<T, BN, true, false, G>));
+    return e;
+  };
+  cudaError_t e = all(std::false_type{});
+  if (e == cudaSuccess) e = all(std::true_type{});
   return e;
 }
 

@@ -72,7 +72,8 @@ struct Cfg {
 constexpr int kStoreSectors = 0;    // along channels, whole 32-byte sectors per lane
 constexpr int kStoreChannels = 1;   // along channels, any alignment
 constexpr int kStorePixels = 2;     // along pixels
-template <typename T, int BN, int BLK, int STORE>
+// GELU: the activation is one of the GELU forms (p.act > 1).
+template <typename T, int BN, int BLK, int STORE, bool GELU>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
                  const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmY, const RowsParams p) {
@@ -401,14 +402,14 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (STORE == kStoreSectors && !kSplit && p.y_rows && __all_sync(0xffffffffu, row_ok)) {
         // 32 pixels one after another: boxes through the TMA unit
         const int pixel = __shfl_sync(0xffffffffu, real, 0);
-        epilogue_store_tile<T, WC, false, 1>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY, pixel, 0, 32,
+        epilogue_store_tile<T, WC, false, 1, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY, pixel, 0, 32,
                                              store_seq, nullptr, g_scale != nullptr);
         read_done();
       } else if constexpr (STORE == kStoreSectors) {
-        epilogue_store_sectors<T, WC>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr,
+        epilogue_store_sectors<T, WC, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr,
                                       static_cast<T*>(p.y) + y_off + n0, row_ok, read_done);
       } else if constexpr (STORE == kStorePixels) {
-        epilogue_store_pixels<T, WC, false>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr,
+        epilogue_store_pixels<T, WC, false, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr,
                                             static_cast<T*>(p.y) + y_off + n0 * p.y_sk, nullptr, p.y_sk, row_ok, read_done);
       } else {
         StridedOut so = {};
@@ -416,7 +417,7 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         so.y_off = y_off;
         so.unit = p.y_unit;
         so.row_ok = row_ok;
-        epilogue_store_strided<T, WC, false, 1>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, so, store_seq);
+        epilogue_store_strided<T, WC, false, 1, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, so, store_seq);
         read_done();
       }
     }
@@ -452,7 +453,8 @@ cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CU
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = launch_overlap_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, conv_rows_kernel<T, BN, BLK, STORE>, tmA, tmA2, tmB, tmY, p);
+  auto* kernel = p.act > 1 ? conv_rows_kernel<T, BN, BLK, STORE, true> : conv_rows_kernel<T, BN, BLK, STORE, false>;
+  return cudaLaunchKernelEx(&cfg, kernel, tmA, tmA2, tmB, tmY, p);
 }
 
 template <typename T, int BN>
@@ -474,16 +476,20 @@ cudaError_t launch_bn(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUt
 
 template <typename T, int BN>
 cudaError_t prepare_bn() {
-  auto opt_in = [](const void* kernel) {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem);
+  auto opt_in = [](auto blk, auto store) {
+    auto* plain = conv_rows_kernel<T, BN, decltype(blk)::value, decltype(store)::value, false>;
+    auto* gelu = conv_rows_kernel<T, BN, decltype(blk)::value, decltype(store)::value, true>;
+    cudaError_t e = cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gelu, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem);
+    return e;
   };
-  cudaError_t e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, kStoreSectors>));
-  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, kStoreChannels>));
-  if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 1, kStorePixels>));
+  cudaError_t e = opt_in(std::integral_constant<int, 1>{}, std::integral_constant<int, kStoreSectors>{});
+  if (e == cudaSuccess) e = opt_in(std::integral_constant<int, 1>{}, std::integral_constant<int, kStoreChannels>{});
+  if (e == cudaSuccess) e = opt_in(std::integral_constant<int, 1>{}, std::integral_constant<int, kStorePixels>{});
   if constexpr (sizeof(T) == 2) {
-    if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 2, kStoreSectors>));
+    if (e == cudaSuccess) e = opt_in(std::integral_constant<int, 2>{}, std::integral_constant<int, kStoreSectors>{});
     if constexpr (BN > 64) {
-      if (e == cudaSuccess) e = opt_in(reinterpret_cast<const void*>(conv_rows_kernel<T, BN, 4, kStoreSectors>));
+      if (e == cudaSuccess) e = opt_in(std::integral_constant<int, 4>{}, std::integral_constant<int, kStoreSectors>{});
     }
   }
   return e;

