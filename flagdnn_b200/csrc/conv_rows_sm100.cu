@@ -133,7 +133,6 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
   tc_fence_before();
   __syncthreads();
-  griddep_wait();      // from here on global memory is consumed: the launch before this one must be complete
   cluster_sync_all();  // both CTAs' barriers exist before anyone signals across
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
@@ -148,6 +147,7 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     const bool lead = elect_one();
+    griddep_wait();      // from here on global memory is read: the launch before this one must be complete
     if (!p.skip_copies) {
       bool alive = true;
       uint32_t as = 0, aphase = 0, bs = 0, bphase = 0;
@@ -359,13 +359,17 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int ohp = p.OH * p.P;
     int staged_n_tile = -1;
     uint32_t tcount = 0, store_seq = 0;
+    // The first pass is a rehearsal that stores nothing: it brings the drain loop's instructions in while the launch before
+    // this one still runs, instead of after the first accumulator is complete (0.5 to 1 us of a launch: one 128 x 28 x 28
+    // image 6.6 -> 6.1 us, 128 -> 128 3x3 in a ResNet-50 of 128 images 27.6 -> 26.1).
+    bool rehearsal = true;
     for (int tile = pair_id; tile < total_tiles; tile += num_pairs, ++tcount) {
-      if (C::kSets == 2 && (tcount & 1u) != uint32_t(half)) continue;
+      if (C::kSets == 2 && !rehearsal && (tcount & 1u) != uint32_t(half)) continue;
       const int m_pair = tile / p.n_tiles;
       const int n_tile = tile - m_pair * p.n_tiles;
       const int n0 = n_tile * BN + col_off;
       const uint32_t buf = tcount & 1u;
-      if (n_tile != staged_n_tile) {
+      if (!rehearsal && n_tile != staged_n_tile) {
         __syncwarp();
         for (int j = lane; j < WC; j += 32) {
           const int col = n0 + j;
@@ -389,20 +393,24 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         real = (img * p.OH + oh) * p.OW + ow;
         y_off = img * p.y_sn + oh * p.y_sh + ow * p.y_sw;
       }
-      bool ok = mbar_wait_bounded(&tmem_full[buf], (tcount >> 1) & 1u, abort_flag, p.status, kIncidentEpilogueWait, p.wait_limit);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
+      if (!rehearsal) {
+        bool ok = mbar_wait_bounded(&tmem_full[buf], (tcount >> 1) & 1u, abort_flag, p.status, kIncidentEpilogueWait, p.wait_limit);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+      }
+      const bool boxes = STORE == kStoreSectors && !kSplit && p.y_rows && __all_sync(0xffffffffu, row_ok);
+      row_ok = row_ok && !rehearsal;
       const uint32_t t_row = tmem_base + (uint32_t(ew * 32) << 16) + buf * BN + col_off;
       auto read_done = [&]() {   // one arrival per warp, before the last stores and without waiting for the earlier ones
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_remote(tempty_leader + buf * 8);
+        if (lane == 0 && !rehearsal) mbar_arrive_remote(tempty_leader + buf * 8);
       };
-      if (STORE == kStoreSectors && !kSplit && p.y_rows && __all_sync(0xffffffffu, row_ok)) {
+      if (boxes) {
         // 32 pixels one after another: boxes through the TMA unit
         const int pixel = __shfl_sync(0xffffffffu, real, 0);
-        epilogue_store_tile<T, WC, false, 1, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY, pixel, 0, 32,
+        epilogue_store_tile<T, WC, false, 1, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY, pixel, 0, rehearsal ? 0 : 32,
                                              store_seq, nullptr, g_scale != nullptr);
         read_done();
       } else if constexpr (STORE == kStoreSectors) {
@@ -419,6 +427,12 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         so.row_ok = row_ok;
         epilogue_store_strided<T, WC, false, 1, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, so, store_seq);
         read_done();
+      }
+      if (rehearsal) {
+        rehearsal = false;
+        griddep_wait();   // from here on global memory is read and written
+        tile -= num_pairs;
+        --tcount;
       }
     }
     if (STORE == kStoreSectors && p.y_rows && lane == 0) bulk_wait_group0();   // stores must be done before the CTA retires
