@@ -159,7 +159,6 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   }
   tc_fence_before();
   __syncthreads();
-  griddep_wait();      // from here on global memory is consumed: the launch before this one must be complete
   cluster_sync_all();  // both CTAs' barriers exist before anyone signals across
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
@@ -179,6 +178,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (lane == 0 && !p.skip_copies) {
+      griddep_wait();      // from here on global memory is read: the launch before this one must be complete
       uint32_t stage = 0, phase = 0;
       bool alive = true;
       long long prof_wait = 0, prof_issue = 0, prof_iters = 0, prof_t0 = p.prof ? clock64() : 0;
@@ -405,6 +405,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     // (nothing passes through registers), the finished image leaves by one bulk copy to the CTA's slot in
     // global memory, where it stays in L2 for the window copies of the producer.
     if (warp == 2) {
+      griddep_wait();
       const int row_bytes = p.row_chunks * 16;
       const int lead_bytes = p.lead_chunks * 16;
       int data_bytes = p.x_row_chunks * 16;
@@ -476,6 +477,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     // A tile reads raw_rows input rows of its image.  Each goes into the CTA's scratch slot as row_chunks
     // 16-byte pieces: lead_chunks zero pieces (the left padding, rounded so that windows start on 16 bytes),
     // the row's x_row_chunks pieces, zeros to the end; rows above or below the image are all zeros.
+    griddep_wait();
     const int t = (warp - 2) * 32 + lane;
     const int per_tile = p.raw_rows * p.row_chunks;
     const uint4* x16 = static_cast<const uint4*>(p.x3);
@@ -566,15 +568,20 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     const int my_warp = warp - kFirstEpiWarpPair;
     const int sk_row = ew * 32 + lane;                   // this lane's row in the CTA's slot
     const int sk_pc0 = chalf * (kWarpCols / 4);          // this warp's first 16-byte piece of a slot row
-    for (; walk_next(walk); ++tcount) {
-      const int tile = walk.tile;
+    // The first pass is a rehearsal that stores nothing: it brings the drain loop's instructions in while the launch before
+    // this one still runs, instead of after the first accumulator is complete (see conv_rows_sm100.cu, and
+    // conv_igemm_sm100.cu for when not).
+    bool rehearsal = k_iters >= 8 || total_tiles > 2 * num_pairs;
+    if (!rehearsal) griddep_wait();
+    while (rehearsal || walk_next(walk)) {
+      const int tile = rehearsal ? pair_id : walk.tile;
       const int m_pair = tile / n_tiles;
       const int n_tile = tile - m_pair * n_tiles;
       const int n0 = n_tile * kPairN + chalf * kWarpCols;  // first column this warp owns
       const uint32_t buf = tcount & 1u;
       const uint32_t bphase = (tcount >> 1) & 1u;
-      const bool finishes = walk.ke == k_iters;            // this pair computes the tile's last reduction steps
-      if (finishes && n_tile != staged_n_tile) {
+      const bool finishes = rehearsal || walk.ke == k_iters;            // this pair computes the tile's last reduction steps
+      if (finishes && !rehearsal && n_tile != staged_n_tile) {
         __syncwarp();
         for (int j = lane; j < kWarpCols; j += 32) {
           const int col = n0 + j;
@@ -585,12 +592,15 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         staged_n_tile = n_tile;
       }
       const int m_tile = 2 * m_pair + int(rank);
-      const long long et0 = p.prof ? clock64() : 0;
-      bool ok = mbar_wait_bounded(&tmem_full[buf], bphase, abort_flag, p.status, kIncidentEpilogueWait, p.wait_limit);
-      ok = __all_sync(0xffffffffu, ok);
-      if (p.prof) prof_ewait += clock64() - et0;
-      if (!ok) break;
-      tc_fence_after();
+      bool ok = true;
+      if (!rehearsal) {
+        const long long et0 = p.prof ? clock64() : 0;
+        ok = mbar_wait_bounded(&tmem_full[buf], bphase, abort_flag, p.status, kIncidentEpilogueWait, p.wait_limit);
+        ok = __all_sync(0xffffffffu, ok);
+        if (p.prof) prof_ewait += clock64() - et0;
+        if (!ok) break;
+        tc_fence_after();
+      }
       const uint32_t t_row = tmem_base + (uint32_t(ew * 32) << 16) + buf * kPairN + chalf * kWarpCols;
       if (!finishes) {
         // contributor: the tile's first reduction steps; the raw sums go to this CTA's slot
@@ -602,10 +612,11 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(tempty_leader + buf * 8);
+        ++tcount;
         continue;
       }
       int sk_count = 0;
-      if (walk.kb > 0) {
+      if (!rehearsal && walk.kb > 0) {
         // owner of a split tile: pairs pair_id-1, pair_id-2, ... hold its earlier steps, each as the first
         // thing it computed; wait for this warp's counterpart in each of them
         const long long L = (long long)total_tiles * k_iters;
@@ -640,6 +651,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         st_row = m_tile * kRows + ew * 32;
         st_rows = 32;
       }
+      if (rehearsal) st_rows = 0;
       const float* sk_slot0 = sk_count > 0 ? p.sk_slots + (long long)(2 * (pair_id - 1) + int(rank)) * kSkSlotFloats : nullptr;
       epilogue_store_tile<T, kWarpCols, RES, kOutBufs, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY2,
                                      st_row, st_img, st_rows, store_seq, &rf, g_scale != nullptr,
@@ -651,9 +663,15 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           for (int c = 0; c < sk_count; ++c)
             p.sk_flags[(2 * (pair_id - 1 - c) + int(rank)) * kSkFlagsPerCta + my_warp] = 0u;
       }
+      if (rehearsal) {
+        rehearsal = false;
+        griddep_wait();   // from here on global memory is read and written
+        continue;
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(tempty_leader + buf * 8);
+      ++tcount;
     }
     if (lane == 0) bulk_wait_group0();
     if (p.prof && blockIdx.x == 0 && threadIdx.x == 32 * kFirstEpiWarpPair) {  // first epilogue warp of the first leader
