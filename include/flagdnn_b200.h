@@ -144,7 +144,9 @@ const char* fdnn_last_error(void);
  * src/flag_dnn/ops/conv2d.py:90-135) and fills `plan`.  Needs no GPU except to
  * read the current device's SM count for the grid size (148 assumed if no
  * device is visible).  `x`, `w`, `y` may be NULL; when given, their alignment
- * decides whether the tensors can be consumed in place by TMA. */
+ * decides whether the tensors can be consumed in place by TMA.  The tiles are those of the plan's kernel; a
+ * layer of W stride 1 with several filter columns may run on other ones, with the same scratch, packed filter
+ * and results. */
 int fdnn_conv2d_query(const fdnn_conv_desc* desc, const void* x, const void* w,
                       const void* y, fdnn_conv_plan* plan);
 
