@@ -1845,16 +1845,17 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     p.x = x; p.w = w; p.bias = bias; p.scale = scale; p.residual = residual; p.y = y;
     p.act = activation;
     int dw = (d.algo & 0xff) == FDNN_ALGO_AUTO ? depthwise_kind(d.dtype, p) : 0;  // a forced "direct" stays direct
-    if (dw == 6) {
+    if (dw == 6 || dw == 9) {
       int dev = 0;
       if (prepare_device(&dev) == FDNN_OK && g_status_ptr[dev] != nullptr) {
-        const long long limit = g_wait_limit.load(std::memory_order_relaxed);
-        cudaError_t e = launch_depthwise_tma(d.dtype, p, g_status_ptr[dev], limit > 0 ? limit : default_wait_limit_cycles(), stream);
+        const long long set = g_wait_limit.load(std::memory_order_relaxed), limit = set > 0 ? set : default_wait_limit_cycles();
+        cudaError_t e = dw == 9 ? launch_depthwise_ring(d.dtype, p, g_status_ptr[dev], limit, stream)
+                                : launch_depthwise_tma(d.dtype, p, g_status_ptr[dev], limit, stream);
         if (e == cudaSuccess) return FDNN_OK;
         if (e != cudaErrorInvalidValue) return fail_cuda("depthwise launch", e);
         cudaGetLastError();
       }
-      dw = 1;   // no tensor map over this x: the kernel that reads it with plain loads
+      dw = dw == 9 ? 2 : 1;   // no tensor map over this x: the kernel that reads it with plain loads
     }
     cudaError_t e = dw != 0 ? launch_depthwise(d.dtype, p, dw, stream) : launch_direct(d.dtype, p, stream);
     if (e != cudaSuccess) return fail_cuda("direct conv launch", e);

@@ -819,7 +819,8 @@ cudaError_t go(const DirectParams& p, int channels_last, cudaStream_t stream) { 
 
 // 0: not a case for these kernels (the caller uses the direct kernel); 1: channels-last kernel; 2: plane kernel;
 // 3 / 4 / 5: row-vector kernel (NCHW) on 16- / 8- / 4-byte vectors; 6: a case of kernel 1 that the staged kernel
-// (conv_depthwise_tma.cu) takes; 7: several dense planes per block; 8: channels-last, channel by channel.
+// (conv_depthwise_tma.cu) takes; 7: several dense planes per block; 8: channels-last, channel by channel; 9: dense planes
+// through a ring (conv_depthwise_ring.cu).
 int depthwise_kind(int dtype, const DirectParams& p) {
   if (p.groups != p.C || p.K != p.C || p.C < 1) return 0;
   if (dtype != FDNN_F16 && dtype != FDNN_BF16 && dtype != FDNN_F32) return 0;
@@ -841,6 +842,7 @@ int depthwise_kind(int dtype, const DirectParams& p) {
   if (unrolled && p.C >= 8 && p.x_s[1] == 1 && p.y_s[1] == 1 && p.x_s[3] != 1 &&
       (long long)p.N * p.C * p.OH * ((p.OW + 3) / 4) < 2147483647LL * 128)
     return 8;
+  if (unrolled && depthwise_ring_ok(dtype, p)) return 9;
   if (unrolled && p.pad_left == p.S / 2 && p.x_s[3] == 1 && p.y_s[3] == 1) {
     for (int vb = 16; vb >= 4; vb /= 2) {
       const int vv = vb / es;

@@ -168,12 +168,16 @@ cudaError_t launch_direct(int dtype, const DirectParams& p, cudaStream_t stream)
 //   6  channels-last, input rows staged by the TMA unit (conv_depthwise_tma.cu); 1 where no map can be made of x
 //   7  NCHW, several whole planes per block
 //   8  channels-last, one channel per thread (channel counts and pitches that fill no 16-byte pieces)
+//   9  NCHW, whole dense planes through a ring in shared memory (conv_depthwise_ring.cu)
 int depthwise_kind(int dtype, const DirectParams& p);
 // Whether a problem of kind 1 is one of kind 6.
 bool depthwise_tma_ok(const DirectParams& p);
 cudaError_t launch_depthwise_tma(int dtype, const DirectParams& p, uint32_t* status, long long wait_limit, cudaStream_t stream);
 // Tensor map over a channels-last x for it: boxes of `chunk` channels x `span` pixels x `rows` rows.  False: not encodable.
 bool encode_depthwise_map(CUtensorMap* tm, int dtype, const DirectParams& p, int chunk, int span, int rows);
+// Whether a layer is one of kind 9.
+bool depthwise_ring_ok(int dtype, const DirectParams& p);
+cudaError_t launch_depthwise_ring(int dtype, const DirectParams& d, uint32_t* status, long long wait_limit, cudaStream_t stream);
 int current_sm_count();   // of the current device (148 when none is visible)
 cudaError_t launch_depthwise(int dtype, const DirectParams& p, int kind, cudaStream_t stream);
 
