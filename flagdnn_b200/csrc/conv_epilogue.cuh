@@ -108,12 +108,17 @@ struct ResidualFetch {
   volatile uint32_t* abort_flag;  // bounded waits, as everywhere in the kernels
   uint32_t* status_word;
   long long wait_limit;
+  // With three staging buffers a box is on its way one group ahead, across tiles as well: `requested` counts the boxes asked
+  // for (as store_seq counts the boxes staged); the warp's next tile, if it has one with columns of its own.
+  uint32_t requested;
+  bool next;
+  int next_n0, next_row, next_img;
 };
 
 // t_row     tensor-memory address of this warp's lane quarter, first column of the tile
 // n0        first GEMM column of the tile; kout: number of valid GEMM columns overall
 // s_scale / s_bias  this warp's fp32 copies for columns n0 .. n0+BN-1
-// my_out    this warp's NBUF 4 KB staging buffers (1024-byte aligned; two are used in rotation so
+// my_out    this warp's NBUF 4 KB staging buffers (1024-byte aligned; two or three are used in rotation so
 //           that a box can still be leaving through the TMA unit while the next one is staged;
 //           with one, the other warp of the lane quarter fills that gap)
 // tm_full / tm_tail  output maps with a 32-row box and a box of the tile's ragged last rows
@@ -133,7 +138,7 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_row, int n0, int 
                                                     uint8_t* my_out, int lane, const CUtensorMap* tm_full,
                                                     const CUtensorMap* tm_tail, int st_row, int st_img,
                                                     int st_rows, uint32_t& store_seq,
-                                                    const ResidualFetch* rf = nullptr, bool use_scale = true,
+                                                    ResidualFetch* rf = nullptr, bool use_scale = true,
                                                     const float* sk_slot0 = nullptr, int sk_count = 0,
                                                     long long sk_slot_stride = 0, int sk_row = 0, int sk_pc0 = 0) {
   constexpr int kPerStore = 128 / int(sizeof(T));  // channels per staged row: 64 (16-bit) or 32 (fp32)
@@ -146,9 +151,40 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_row, int n0, int 
   for (int l = 0; l < kLoads; ++l) tmem_ld_32x32b_x32(t_row + l * 32, raw[l]);
 #pragma unroll 1
   for (int g = 0; g < groups; ++g) {
-    uint8_t* buf = my_out + (NBUF == 2 ? (store_seq & 1u) * (32 * 128) : 0u);  // alternates across groups AND tiles
+    const uint32_t slot = NBUF == 1 ? 0u : store_seq % uint32_t(NBUF);   // alternates across groups AND tiles
+    uint8_t* buf = my_out + slot * (32 * 128);
     ++store_seq;
-    if constexpr (RES) {
+    if constexpr (RES && NBUF == 3) {
+      const bool have = rf != nullptr && rf->tm != nullptr && st_rows > 0;   // uniform across the warp
+      if (have) {
+        auto request = [&](uint32_t to, int col, int row, int img) {
+          mbar_arrive_expect_tx(&rf->bars[to], 32 * 128);
+          tma_load_3d(my_out + to * (32 * 128), rf->tm, &rf->bars[to], col, row, img);
+        };
+        const bool first = rf->requested != store_seq;     // not asked for during the group before
+        const bool more = g + 1 < groups || rf->next;
+        if (lane == 0) {
+          if (first) {
+            bulk_wait_group_read0();
+            request(slot, n0 + g * kPerStore, st_row, st_img);
+          } else {
+            bulk_wait_group_read1();   // the box staged two groups ago has left the buffer asked for here
+          }
+          if (more) {
+            const bool here = g + 1 < groups;
+            request(slot == 2 ? 0u : slot + 1u, here ? n0 + (g + 1) * kPerStore : rf->next_n0, here ? st_row : rf->next_row,
+                    here ? st_img : rf->next_img);
+          }
+        }
+        rf->requested = store_seq + (more ? 1u : 0u);
+        __syncwarp();
+        mbar_wait_bounded(&rf->bars[slot], (*rf->phases >> slot) & 1u, rf->abort_flag, rf->status_word, kIncidentResidualWait,
+                          rf->wait_limit);
+        *rf->phases ^= 1u << slot;
+      } else if (lane == 0) {
+        bulk_wait_group_read1();
+      }
+    } else if constexpr (RES) {
       const bool have = rf != nullptr && rf->tm != nullptr && st_rows > 0;   // uniform across the warp
       const uint32_t b = NBUF == 2 ? ((store_seq - 1u) & 1u) : 0u;
       if (lane == 0) {

@@ -61,7 +61,8 @@ constexpr int kRegsEpilogue = kEpiWarps == 8 ? 200 : 232;  // 128 * 104 + 256 * 
 static_assert(128 * kRegsLean + 32 * kEpiWarps * kRegsEpilogue <= kThreads * (65536 / kThreads / 8 * 8),
               "register reallocation exceeds the launch allocation");
 
-template <typename T, int BN>
+// BUFS: output staging buffers per epilogue warp.
+template <typename T, int BN, int BUFS = 2>
 struct TileCfg {
   static constexpr bool kSplit = std::is_same<T, float>::value;
   static constexpr int kKB = kRowBytes / int(sizeof(T));  // reduction elements per stage
@@ -77,13 +78,13 @@ struct TileCfg {
   static constexpr int kColSplit = (kEpiWarps == 8 && BN / kOutCols >= 4) ? 2 : 1;
   static constexpr int kWarpCols = BN / kColSplit;             // columns one epilogue warp drains
   static constexpr int kActiveEpiWarps = 4 * kColSplit;
-  static constexpr int kOutBytes = kActiveEpiWarps * 2 * 32 * kRowBytes;  // two 4 KB buffers per warp
+  static constexpr int kOutBytes = kActiveEpiWarps * BUFS * 32 * kRowBytes;  // 4 KB buffers
   static constexpr int kEpiBytes = kActiveEpiWarps * 2 * kWarpCols * int(sizeof(float));
   // operand ring: what is left of the 227 KB; 3 x 48 KB for the widest 16-bit tile
   static constexpr int kMaxStages = 16;
-  static constexpr int kRingBudget = 227 * 1024 - kOutBytes - kEpiBytes - (2 * kMaxStages + 8) * 8 - 1024;
+  static constexpr int kRingBudget = 227 * 1024 - kOutBytes - kEpiBytes - (2 * kMaxStages + 32) * 8 - 1024;
   static constexpr int kStages = kRingBudget / kStageBytes < kMaxStages ? kRingBudget / kStageBytes : kMaxStages;
-  static constexpr int kBarBytes = (2 * kStages + 4 + 1 + 1 + 16) * 8 + 16;   // ring, accumulators, drain, slot words, residual boxes
+  static constexpr int kBarBytes = (2 * kStages + 4 + 1 + 1 + 24) * 8 + 16;   // ring, accumulators, drain, slot words, residual boxes
   static constexpr int kSmemBytes = kStages * kStageBytes + kOutBytes + kEpiBytes + kBarBytes + 1024;
   static_assert(kStages >= 2, "pipeline needs at least two stages");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
@@ -99,13 +100,13 @@ __device__ __forceinline__ void store32_contig(float* dst, const float (&v)[32])
 // DENSE: y goes through the TMA unit (p.tma_store); otherwise through the warps' own stores, whose registers would push
 // the dense path's loop state to local memory if both lived in one kernel.
 // GELU: the activation is one of the GELU forms (p.act > 1).
-template <typename T, int BN, bool RES, bool DENSE, bool GELU>
+template <typename T, int BN, bool RES, bool DENSE, bool GELU, int BUFS = 2>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
                   const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmB2,
                   const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmR,
                   const __grid_constant__ CUtensorMap tmRbox, const IgemmParams p) {
-  using Cfg = TileCfg<T, BN>;
+  using Cfg = TileCfg<T, BN, BUFS>;
   constexpr int kStages = Cfg::kStages;
   constexpr uint32_t kFmt = std::is_same<T, __half>::value ? 0u : (std::is_same<T, __nv_bfloat16>::value ? 1u : 2u);
   constexpr uint32_t kIdesc = make_idesc(kFmt, kBM, BN);
@@ -123,7 +124,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint64_t* drain_bar = bars + 2 * kStages + 4;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 5);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  uint64_t* res_bar = bars + 2 * kStages + 6;     // [8 epilogue warps][2 staging buffers]
+  uint64_t* res_bar = bars + 2 * kStages + 6;     // [8 epilogue warps][staging buffers]
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -140,7 +141,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     mbar_init(&tmem_empty[1], Cfg::kActiveEpiWarps);
     mbar_init(drain_bar, 1);
     if constexpr (RES) {
-      for (int i = 0; i < 16; ++i) mbar_init(&res_bar[i], 1);
+      for (int i = 0; i < 8 * BUFS; ++i) mbar_init(&res_bar[i], 1);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -402,7 +403,9 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     uint32_t res_phases = 0;
     ResidualFetch rf;
     rf.tm = (DENSE && g_res != nullptr) ? &tmRbox : nullptr;
-    rf.bars = res_bar + (warp - kFirstEpiWarp) * 2;
+    rf.bars = res_bar + (warp - kFirstEpiWarp) * BUFS;
+    rf.requested = 0;
+    rf.next = false;
     rf.phases = &res_phases;
     rf.abort_flag = abort_flag;
     rf.status_word = p.status;
@@ -473,11 +476,20 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
 
       const uint32_t t_row = tmem_base + (uint32_t(ew * 32) << 16) + buf * BN + chalf * WC;
+      if constexpr (RES && DENSE && BUFS == 3) {   // where this warp's next box lies (dense y: one "image", or groups)
+        const int after = tile + int(gridDim.x);
+        const int nm = after / p.n_tiles, nn = after - nm * p.n_tiles;
+        const int ng = p.groups > 1 ? nn / p.group_n_tiles : 0;
+        rf.next_n0 = (nn - ng * p.group_n_tiles) * BN + chalf * WC;
+        rf.next_row = nm * kBM + ew * 32;
+        rf.next_img = ng;
+        rf.next = after < total_tiles && rf.next_n0 < p.Kout;
+      }
       if constexpr (DENSE) {
         // a tile's last warp may own fewer than 32 valid rows: tmA2 then holds a second
         // output map whose box is exactly that short (low-channel mode, 16-bit only)
-        epilogue_store_tile<T, WC, RES, 2, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
-                                   out_stage + (warp - kFirstEpiWarp) * 2 * 32 * kRowBytes, lane, &tmY, &tmA2, st_row,
+        epilogue_store_tile<T, WC, RES, BUFS, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias,
+                                   out_stage + (warp - kFirstEpiWarp) * BUFS * 32 * kRowBytes, lane, &tmY, &tmA2, st_row,
                                    st_img, st_rows, store_seq, &rf, g_scale != nullptr);
       } else if (p.y_mode == kYPixels) {
         const long long at = y_off + (long long)n0 * p.y_sk;
@@ -531,6 +543,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
       if (rehearsal) {
         rehearsal = false;
+        rf.requested = store_seq;
         griddep_wait();   // from here on global memory is read and written
         tile -= gridDim.x;
         --tcount;
@@ -539,6 +552,12 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[buf]);   // one arrival per warp
+    }
+    if constexpr (RES && DENSE && BUFS == 3) {   // after a failed wait: the box asked for ahead lands before the CTA retires
+      uint32_t never = 0;
+      const uint32_t slot = store_seq % 3u;
+      if (rf.requested == store_seq + 1)
+        mbar_wait_bounded(&rf.bars[slot], (res_phases >> slot) & 1u, &never, p.status, kIncidentDrainWait, kWaitLimitCycles / 16);
     }
     if (DENSE && lane == 0) bulk_wait_group0();  // stores must be done before the CTA retires
     if (p.prof && blockIdx.x == 0 && threadIdx.x == 32 * kFirstEpiWarp) {  // first epilogue warp
@@ -553,6 +572,16 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tc_fence_after();
     tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
+}
+
+// Whether a launch takes the variant with three staging buffers and two pipeline stages: a shortcut added to 256-column
+// tiles of a short reduction, where a tile waits for its residual boxes and not for its operands.
+// Measured with and without (kernels of the 53-layer stack at 128 images, us): 128 -> 512 on 28 x 28 50.2 and 53.3, 256 -> 1024 on
+// 14 x 14 31.0 and 32.3, 64 -> 256 on 56 x 56 102.9 and 104.1; 512 -> 2048 on 7 x 7 has eight steps and waits for its operands.
+template <typename T, int BN>
+bool three_buffers(const IgemmParams& p) {
+  return sizeof(T) == 2 && BN == 256 && p.residual != nullptr && p.tma_store != 0 && !p.lowc && p.act <= 1 &&
+         p.R * p.S * p.c_blocks <= 4;
 }
 
 template <typename T, int BN>
@@ -578,6 +607,12 @@ cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CU
                : (dense ? conv_igemm_kernel<T, BN, false, true, G> : conv_igemm_kernel<T, BN, false, false, G>);
   };
   auto* kernel = p.act > 1 ? pick(std::true_type{}) : pick(std::false_type{});
+  if constexpr (sizeof(T) == 2 && BN == 256) {
+    if (three_buffers<T, BN>(p)) {
+      kernel = conv_igemm_kernel<T, BN, true, true, false, 3>;
+      cfg.dynamicSmemBytes = TileCfg<T, BN, 3>::kSmemBytes;
+    }
+  }
   return cudaLaunchKernelEx(&cfg, kernel, tmA, tmA2, tmB, tmB2, tmY, tmR, tmRbox, p);
 }
 
@@ -597,6 +632,11 @@ cudaError_t prepare_one() {
   };
   cudaError_t e = all(std::false_type{});
   if (e == cudaSuccess) e = all(std::true_type{});
+  if constexpr (sizeof(T) == 2 && BN == 256) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(conv_igemm_kernel<T, BN, true, true, false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               TileCfg<T, BN, 3>::kSmemBytes);
+  }
   return e;
 }
 
