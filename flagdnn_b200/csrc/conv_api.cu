@@ -1496,6 +1496,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
                     void* workspace, int64_t workspace_bytes, void* stream_v, bool allow_group, int k_real,
                     void* sk_scratch = nullptr, int64_t sk_bytes = 0, const GroupBatch* batch = nullptr,
                     FilterPack* pack = nullptr);
+static int pack_filter(int dtype, FilterPack* f, cudaStream_t stream);
 
 int fdnn_conv2d_fwd(const fdnn_conv_desc* desc, const void* x, const void* w, const void* w_packed,
                     const void* bias, const void* scale, int activation, void* y, void* workspace,
@@ -1537,23 +1538,23 @@ int fdnn_conv2d_fwd_unpacked(const fdnn_conv_desc* desc, const void* x, const vo
   fdnn_conv_plan plan;
   int st = make_plan(desc, x, w, y, &plan);
   if (st != FDNN_OK) return st;
-  FilterPack pack = {};
-  if (plan.algo != FDNN_ALGO_DIRECT && plan.w_packed) {
-    if (w == nullptr || packed == nullptr) return fail(FDNN_BAD_PARAM, "w and packed must not be NULL");
-    if (packed_bytes < plan.packed_weight_bytes) return fail(FDNN_WORKSPACE_TOO_SMALL, "packed filter buffer too small");
-    if (desc->groups > 1 || plan.low_channel || plan.pixel_group > 1) {
-      st = fdnn_conv2d_pack_weight(desc, w, y, packed, packed_bytes, stream_v);
-      if (st != FDNN_OK) return st;
-    } else {
-      pack = {w, {desc->w_strides[0], desc->w_strides[1], desc->w_strides[2], desc->w_strides[3]}, desc->k, desc->c, desc->r,
-              desc->s, plan.c_padded, packed, false};
-      remember_packed(packed, current_device_or_minus1(), packed_layout_of(*desc, plan));
-    }
-  } else {
-    packed = nullptr;
+  if (plan.algo == FDNN_ALGO_DIRECT || !plan.w_packed)
+    return fwd_impl(desc, x, w, nullptr, bias, scale, residual, activation, y, workspace, workspace_bytes, stream_v, true, desc->k);
+  if (w == nullptr || packed == nullptr) return fail(FDNN_BAD_PARAM, "w and packed must not be NULL");
+  if (packed_bytes < plan.packed_weight_bytes) return fail(FDNN_WORKSPACE_TOO_SMALL, "packed filter buffer too small");
+  if (desc->groups > 1 || plan.low_channel || plan.pixel_group > 1) {
+    st = fdnn_conv2d_pack_weight(desc, w, y, packed, packed_bytes, stream_v);
+    if (st != FDNN_OK) return st;
+    return fwd_impl(desc, x, w, packed, bias, scale, residual, activation, y, workspace, workspace_bytes, stream_v, true, desc->k);
   }
-  return fwd_impl(desc, x, w, packed, bias, scale, residual, activation, y, workspace, workspace_bytes, stream_v, true, desc->k,
-                  nullptr, 0, nullptr, pack.w != nullptr ? &pack : nullptr);
+  FilterPack pack = {w, {desc->w_strides[0], desc->w_strides[1], desc->w_strides[2], desc->w_strides[3]}, desc->k, desc->c, desc->r,
+                     desc->s, plan.c_padded, packed, false};
+  st = fwd_impl(desc, x, w, packed, bias, scale, residual, activation, y, workspace, workspace_bytes, stream_v, true, desc->k,
+                nullptr, 0, nullptr, &pack);
+  // a small layer that ran without it (no scratch, or few channels and a residual) has it packed all the same, for later calls
+  if (st == FDNN_OK && aligned16(packed)) st = pack_filter(desc->dtype, &pack, static_cast<cudaStream_t>(stream_v));
+  if (pack.done) remember_packed(packed, current_device_or_minus1(), packed_layout_of(*desc, plan));
+  return st;
 }
 
 // One-time set-up of the current device for kernels that use tensor maps and bounded waits.
@@ -1581,10 +1582,10 @@ static int prepare_device(int* device) {
 
 static int pack_filter(int dtype, FilterPack* f, cudaStream_t stream) {
   if (f == nullptr || f->done) return FDNN_OK;
-  f->done = true;
-  cudaError_t e = launch_pack_w(dtype, f->w, f->strides, f->K, f->C, f->R, f->S, f->c_pad, f->dst, (long long)f->K * f->R * f->S * f->c_pad,
-                                stream);
-  return e == cudaSuccess ? FDNN_OK : fail_cuda("pack_weight launch", e);
+  const cudaError_t e = launch_pack_w(dtype, f->w, f->strides, f->K, f->C, f->R, f->S, f->c_pad, f->dst,
+                                      (long long)f->K * f->R * f->S * f->c_pad, stream);
+  f->done = e == cudaSuccess;
+  return f->done ? FDNN_OK : fail_cuda("pack_weight launch", e);
 }
 
 // Rewrites x into the scratch as dense NHWC where the plan says so, and says how the kernels see it.
@@ -1879,9 +1880,9 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   }
   if (plan.w_packed && (reinterpret_cast<uintptr_t>(w_packed) & 15u) != 0)
     return fail(FDNN_BAD_PARAM, "packed filter must be 16-byte aligned");
-  if (plan.w_packed && allow_group) {
+  if (plan.w_packed && allow_group && pack == nullptr) {
     // the buffer must hold the layout this plan reads (allow_group is false only for the inner call of
-    // a pixel-grouped layer, whose buffer was checked by the outer one)
+    // a pixel-grouped layer, whose buffer was checked by the outer one; with `pack` this call writes it)
     PackedLayout have;
     const PackedLayout want = packed_layout_of(d, plan);
     if (find_packed(w_packed, dev, &have) && !(have == want)) return fail_layout(have, want);

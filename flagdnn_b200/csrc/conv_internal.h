@@ -203,7 +203,7 @@ struct FilterPack {
   long long strides[4];
   int K, C, R, S, c_pad;
   void* dst;
-  bool done;
+  bool done;         // the launch that packs it has been queued
 };
 cudaError_t launch_repack_x(int dtype, const void* x, const long long x_s[4], int N, int C, int H,
                             int W, int c_pad, void* dst, long long plane_elems,

@@ -457,7 +457,6 @@ int grid_for(long long work_items, int per_block) {
   return int(blocks);
 }
 
-// Transposition of `mats` matrices: matrix i starts at (i / mats2) * ms + (i % mats2) * ms2.
 template <typename T>
 PackJob<T> pack_job(const FilterPack& f) {
   PackJob<T> j = {static_cast<const T*>(f.w), f.strides[0], f.strides[1], f.strides[2], f.strides[3], f.K, f.C, f.R, f.S, f.c_pad,
@@ -466,6 +465,7 @@ PackJob<T> pack_job(const FilterPack& f) {
   return j;
 }
 
+// Transposition of `mats` matrices: matrix i starts at (i / mats2) * ms + (i % mats2) * ms2.
 template <typename T>
 cudaError_t transpose_t(const T* x, long long ms, long long ms2, int mats2, long long sc, int mats, int C, int P,
                         int c_pad, T* dst, long long plane, cudaStream_t stream, FilterPack* pack = nullptr) {
@@ -475,14 +475,13 @@ cudaError_t transpose_t(const T* x, long long ms, long long ms2, int mats2, long
                    mult(mats2, ms2);
   const long long tiles = (long long)mats * ((P + 63) / 64) * ((c_pad + 128 / int(sizeof(T)) - 1) / (128 / int(sizeof(T))));
   PackJob<T> job = {};
-  if (pack != nullptr) {
-    job = pack_job<T>(*pack);
-    pack->done = true;
-  }
+  if (pack != nullptr) job = pack_job<T>(*pack);
   auto* kernel = pack != nullptr ? (vec ? transpose_repack<T, true, true> : transpose_repack<T, false, true>)
                                  : (vec ? transpose_repack<T, true, false> : transpose_repack<T, false, false>);
   launch_chained(kernel, dim3(grid_for(tiles, 1) + job.blocks), 256, stream, x, ms, ms2, mats2, sc, mats, C, P, c_pad, dst, plane, job);
-  return cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
+  if (pack != nullptr) pack->done = e == cudaSuccess;
+  return e;
 }
 
 // Rows of channels: `pixels` pixels `sw` elements apart.
