@@ -1400,8 +1400,9 @@ int fdnn_conv2d_query(const fdnn_conv_desc* desc, const void* x, const void* w, 
   return make_plan(desc, x, w, y, plan);
 }
 
-int fdnn_conv2d_pack_weight(const fdnn_conv_desc* desc, const void* w, const void* y, void* packed,
-                            int64_t packed_bytes, void* stream) {
+// note: whether the buffer outlives the call and its layout is remembered
+static int pack_weight(const fdnn_conv_desc* desc, const void* w, const void* y, void* packed, int64_t packed_bytes, void* stream,
+                       bool note) {
   fdnn_conv_desc d;
   if (desc == nullptr) return fail(FDNN_BAD_PARAM, "descriptor is NULL");
   if (validate(desc) == FDNN_OK && group_dense_ok(desc)) {
@@ -1423,7 +1424,7 @@ int fdnn_conv2d_pack_weight(const fdnn_conv_desc* desc, const void* w, const voi
       if (pv.w_packed) {
         // the dense plan wants its own layout (pixel groups, padded channels): packed behind the dense filter
         const long long off = dense_filter_bytes(desc);
-        return fdnn_conv2d_pack_weight(&v, packed, y, static_cast<char*>(packed) + off, packed_bytes - off, stream);
+        return pack_weight(&v, packed, y, static_cast<char*>(packed) + off, packed_bytes - off, stream, note);
       }
       return FDNN_OK;
     }
@@ -1442,7 +1443,7 @@ int fdnn_conv2d_pack_weight(const fdnn_conv_desc* desc, const void* w, const voi
       for (int g = 0; g < desc->groups; ++g) {
         const char* wg = static_cast<const char*>(w) + (long long)g * sub.k * desc->w_strides[0] * es;
         const char* yg = y == nullptr ? nullptr : static_cast<const char*>(y) + (long long)g * sub.k * desc->y_strides[1] * es;
-        gst = fdnn_conv2d_pack_weight(&sub, wg, yg, static_cast<char*>(packed) + g * per_group, per_group, stream);
+        gst = pack_weight(&sub, wg, yg, static_cast<char*>(packed) + g * per_group, per_group, stream, note);
         if (gst != FDNN_OK) return gst;
       }
       return FDNN_OK;
@@ -1462,7 +1463,7 @@ int fdnn_conv2d_pack_weight(const fdnn_conv_desc* desc, const void* w, const voi
   }
   if (st != FDNN_OK) return st;
   // a grouped filter [K, C / groups, R, S] is packed group by group or made dense above, never as one of C channels
-  if (d.groups > 1 && d.algo != desc->algo) return fdnn_conv2d_pack_weight(&d, w, y, packed, packed_bytes, stream);
+  if (d.groups > 1 && d.algo != desc->algo) return pack_weight(&d, w, y, packed, packed_bytes, stream, note);
   if (d.groups > 1) return fail(FDNN_NOT_SUPPORTED, "no packed layout for this grouped filter");
   if (w == nullptr || packed == nullptr) return fail(FDNN_BAD_PARAM, "w and packed must not be NULL");
   if (packed_bytes < plan.packed_weight_bytes)
@@ -1487,8 +1488,13 @@ int fdnn_conv2d_pack_weight(const fdnn_conv_desc* desc, const void* w, const voi
                       plan.c_padded, packed, plane, static_cast<cudaStream_t>(stream));
   }
   if (e != cudaSuccess) return fail_cuda(what, e);
-  remember_packed(packed, current_device_or_minus1(), packed_layout_of(d, plan));
+  if (note) remember_packed(packed, current_device_or_minus1(), packed_layout_of(d, plan));
   return FDNN_OK;
+}
+
+int fdnn_conv2d_pack_weight(const fdnn_conv_desc* desc, const void* w, const void* y, void* packed,
+                            int64_t packed_bytes, void* stream) {
+  return pack_weight(desc, w, y, packed, packed_bytes, stream, true);
 }
 
 static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, const void* w_packed,
@@ -1542,16 +1548,23 @@ int fdnn_conv2d_fwd_unpacked(const fdnn_conv_desc* desc, const void* x, const vo
     return fwd_impl(desc, x, w, nullptr, bias, scale, residual, activation, y, workspace, workspace_bytes, stream_v, true, desc->k);
   if (w == nullptr || packed == nullptr) return fail(FDNN_BAD_PARAM, "w and packed must not be NULL");
   if (packed_bytes < plan.packed_weight_bytes) return fail(FDNN_WORKSPACE_TOO_SMALL, "packed filter buffer too small");
-  if (desc->groups > 1 || plan.low_channel || plan.pixel_group > 1) {
-    st = fdnn_conv2d_pack_weight(desc, w, y, packed, packed_bytes, stream_v);
-    if (st != FDNN_OK) return st;
-    return fwd_impl(desc, x, w, packed, bias, scale, residual, activation, y, workspace, workspace_bytes, stream_v, true, desc->k);
-  }
+  // a buffer inside the workspace is scratch like the rest of it: the workspace ends where it begins, nothing is remembered
+  const uintptr_t base = reinterpret_cast<uintptr_t>(workspace), at = reinterpret_cast<uintptr_t>(packed);
+  const bool kept = workspace == nullptr || at < base || at - base >= uintptr_t(workspace_bytes > 0 ? workspace_bytes : 0);
+  if (!kept) workspace_bytes = int64_t(at - base);
   FilterPack pack = {w, {desc->w_strides[0], desc->w_strides[1], desc->w_strides[2], desc->w_strides[3]}, desc->k, desc->c, desc->r,
                      desc->s, plan.c_padded, packed, false};
+  if (desc->groups > 1 || plan.low_channel || plan.pixel_group > 1) {
+    st = pack_weight(desc, w, y, packed, packed_bytes, stream_v, kept);
+    if (st != FDNN_OK) return st;
+    pack.done = true;
+    return fwd_impl(desc, x, w, packed, bias, scale, residual, activation, y, workspace, workspace_bytes, stream_v, true, desc->k,
+                    nullptr, 0, nullptr, kept ? nullptr : &pack);
+  }
   st = fwd_impl(desc, x, w, packed, bias, scale, residual, activation, y, workspace, workspace_bytes, stream_v, true, desc->k,
                 nullptr, 0, nullptr, &pack);
   // a small layer that ran without it (no scratch, or few channels and a residual) has it packed all the same, for later calls
+  if (!kept) return st;
   if (st == FDNN_OK && aligned16(packed)) st = pack_filter(desc->dtype, &pack, static_cast<cudaStream_t>(stream_v));
   if (pack.done) remember_packed(packed, current_device_or_minus1(), packed_layout_of(*desc, plan));
   return st;
@@ -1611,7 +1624,7 @@ static int relayout_x(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, bool 
     x_pad = round_up(d.c, 16 / es);
   a->plane = (long long)d.n * d.h * d.w * x_pad;
   cudaError_t e = launch_repack_x(d.dtype, x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w, x_pad,
-                                  workspace, a->plane, stream, pack);
+                                  workspace, a->plane, stream, pack != nullptr && !pack->done ? pack : nullptr);
   if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
   const int st = pack_filter(d.dtype, pack, stream);
   if (st != FDNN_OK) return st;
@@ -1703,7 +1716,7 @@ static int fwd_rows(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, const R
 }
 
 // k_real: length of bias / scale (differs from desc->k only for the equivalent convolution of a
-// pixel-grouped layer, whose GEMM column j uses entry j % k_real).
+// pixel-grouped layer, whose GEMM column j uses entry j % k_real).  pack: this call writes w_packed itself, or has (done).
 static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, const void* w_packed,
                     const void* bias, const void* scale, const void* residual, int activation, void* y,
                     void* workspace, int64_t workspace_bytes, void* stream_v, bool allow_group, int k_real,
@@ -1771,7 +1784,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
       fdnn_conv_desc part = d;
       const long long cg = d.c / d.groups, kg = d.k / d.groups;
       const long long filter_bytes = kg * d.r * d.s * own.one.c_padded * es;
-      if (from_packed) {
+      if (from_packed && pack == nullptr) {
         PackedLayout have;
         const PackedLayout want = packed_layout_of(one_group_desc(&d), own.one);
         if (find_other_layout(w_packed, filter_bytes, d.groups, current_device_or_minus1(), want, &have))
@@ -1808,7 +1821,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     if (st != FDNN_OK) return st;
     const void* inner = pv.w_packed ? static_cast<const char*>(w_packed) + dense_filter_bytes(&d) : nullptr;
     return fwd_impl(&v, x, w_packed, inner, bias, scale, residual, activation, y, workspace, workspace_bytes, stream_v,
-                    allow_group, k_real, sk_scratch, sk_bytes);
+                    allow_group, k_real, sk_scratch, sk_bytes, nullptr, pack);
   }
   if (batch == nullptr && d.groups > 1 && plan.algo != FDNN_ALGO_DIRECT) {
     // one launch per group on views of the tensors (see group_loop_ok); the groups share the scratch, which the
@@ -1825,7 +1838,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
                     w_packed == nullptr ? nullptr : static_cast<const char*>(w_packed) + g * per_group,
                     at(bias, k0), at(scale, k0), at(residual, k0 * d.y_strides[1]), activation,
                     const_cast<void*>(at(y, k0 * d.y_strides[1])), workspace, workspace_bytes, stream_v, allow_group,
-                    sub.k, sk_scratch, sk_bytes);
+                    sub.k, sk_scratch, sk_bytes, nullptr, pack);
       if (st != FDNN_OK) return st;
     }
     return FDNN_OK;

@@ -159,11 +159,10 @@ int launch(const fdnn_conv_desc& d, const at::Tensor& x, const at::Tensor& w, Py
                              d.x_strides[3] == 1 && d.x_strides[1] != 1 && d.w > 1 && plan.packed_weight_bytes <= kPackAlways;
     if (weight_obj == nullptr || in_relayout) {
       WithoutGil free;
-      const int64_t ws_bytes = (plan.workspace_bytes + 255) / 256 * 256;
-      scratch = at::empty({ws_bytes + plan.packed_weight_bytes}, x.options().dtype(at::kByte));
+      const int64_t ws_bytes = (plan.workspace_bytes + 255) / 256 * 256, bytes = ws_bytes + plan.packed_weight_bytes;
+      scratch = at::empty({bytes}, x.options().dtype(at::kByte));
       char* base = static_cast<char*>(scratch.mutable_data_ptr());
-      return g_fwd_unpacked(&d, xp, wp, base + ws_bytes, plan.packed_weight_bytes, bias, scale, residual, act, yp,
-                            plan.workspace_bytes > 0 ? base : nullptr, plan.workspace_bytes, stream);
+      return g_fwd_unpacked(&d, xp, wp, base + ws_bytes, plan.packed_weight_bytes, bias, scale, residual, act, yp, base, bytes, stream);
     }
     held = PyObject_CallFunction(g_packed_weight, "OKKKK", weight_obj, (unsigned long long)(uintptr_t)&d,
                                  (unsigned long long)(uintptr_t)&plan, (unsigned long long)(uintptr_t)stream,

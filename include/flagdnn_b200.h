@@ -182,7 +182,8 @@ int fdnn_conv2d_fwd(const fdnn_conv_desc* desc, const void* x, const void* w,
 /* fdnn_conv2d_fwd_residual for a filter that is not kept packed: where the plan needs one, w is packed into
  * `packed` (plan.packed_weight_bytes, 16-byte aligned) first, in the launch that relays x out where that is
  * possible.  After FDNN_OK the buffer holds what fdnn_conv2d_pack_weight writes and is remembered as such, also
- * where this call itself ran without it.  For layers whose filter is small beside x, or new on every call. */
+ * where this call itself ran without it.  A `packed` inside [workspace, workspace + workspace_bytes) is part of
+ * the scratch: the workspace ends where it begins, and nothing is remembered of it.  For layers whose filter is small beside x, or new on every call. */
 int fdnn_conv2d_fwd_unpacked(const fdnn_conv_desc* desc, const void* x, const void* w, void* packed,
                              int64_t packed_bytes, const void* bias, const void* scale, const void* residual,
                              int activation, void* y, void* workspace, int64_t workspace_bytes, void* stream);

@@ -156,3 +156,39 @@ def test_the_record_follows_what_the_buffer_holds(native_lib):
     assert a.unpacked(packed, scratch=False) == nat.FDNN_WORKSPACE_TOO_SMALL
     nat.check(b.packed_call(packed))
     b.check()
+
+
+@pytest.mark.parametrize("name", LAYERS)
+def test_a_buffer_inside_the_workspace_is_scratch(native_lib, name):
+    """Nothing is remembered of it: afterwards it may hold any layer's packed filter."""
+    layer, other = Layer(**LAYERS[name]), Layer(BF16, 3, 64, 20, 20, 64, 3, 3)
+    begin, nbytes = -(-layer.plan.workspace_bytes // 256) * 256, layer.plan.packed_weight_bytes
+    arena = torch.full((begin + max(nbytes, other.plan.packed_weight_bytes) + 256,), 0x2A, dtype=torch.uint8, device="cuda")
+    layer.scratch = arena[:begin + nbytes]
+    nat.check(layer.unpacked(arena.data_ptr() + begin))
+    layer.check()
+    assert bool((arena[begin + nbytes:] == 0x2A).all())
+    region = arena[begin:begin + other.plan.packed_weight_bytes]
+    region.copy_(other.pack(other.buffer()))
+    nat.check(other.packed_call(region))
+    other.check()
+
+
+def test_calls_that_pack_on_the_way_leave_the_records_alone(native_lib):
+    """More of them than there are records, each with scratch of its own: a buffer packed for another layer is refused still."""
+    import flagdnn_b200 as fd
+
+    a, b = Layer(F16, 3, 40, 20, 20, 64, 3, 3), Layer(F16, 3, 64, 20, 20, 64, 3, 3)
+    packed = a.pack(a.buffer())
+    x, w = torch.randn(1, 64, 50, device="cuda").half(), torch.randn(64, 64, 3, device="cuda").half()
+    x2, w2 = torch.randn(1, 64, 14, 14, device="cuda").half(), torch.randn(64, 64, 3, 3, device="cuda").half()
+    held = []
+    for _ in range(300):
+        before = torch.cuda.memory_allocated()
+        fd.conv1d(x, w, padding=1)
+        fd.conv2d(x2, w2, padding=1)
+        assert torch.cuda.memory_allocated() == before
+        held.append([torch.empty(n, dtype=torch.uint8, device="cuda") for n in (32 << 10, 128 << 10)])   # where the scratch was
+    assert b.packed_call(packed) == nat.FDNN_BAD_PARAM
+    nat.check(a.packed_call(packed))
+    a.check()
