@@ -416,16 +416,37 @@ cudaError_t launch_ring_t(const DirectParams& d, uint32_t* status, long long lim
   return d.stride_w == 1 ? launch_ring_vb<T, 5, 1>(d, status, limit, stream) : launch_ring_vb<T, 5, 2>(d, status, limit, stream);
 }
 
+// Bytes of x from which this kernel is ahead of the other NCHW kernels, or none.  A ring starts later than a kernel that reads
+// where it stands, and has nothing to overlap while a block has a group or two; what there is to gain depends on how wide the
+// others can read (rows on 16, 8 or fewer bytes) and on the multiplications per input.  2200 layers of 7 to 112 columns and 1 to
+// 136 MiB were timed on both: with these lines 26 take over 5 % longer than on the other (1.36 times at most), with one line of a megabyte 420 did (up to 1.9).  The others
+// and this one, us, 3x3 bf16 unless said otherwise:
+//   stride 1  rows off 8 bytes     6 x 512 x 14 x 14 5.4 and 5.0, 34 x 100 x 25 x 25 13.0 and 8.3, 168 x 512 x 14 x 14 62.4 and 34.9
+//             rows on 8 bytes      3 x 256 x 28 x 28 3.8 and 5.0, 11 x 256 x 28 x 28 9.3 and 7.8
+//             rows on 16 bytes     81 x 384 x 24 x 24 31.6 and 36.0, 162 x 384 x 24 x 24 71.7 and 60.8; 45 x 256 x 56 x 56 56.1 and
+//                                  57.9, 89 x 256 x 56 x 56 105.9 and 103.9; 5x5 on 144 x 32 x 56 x 56 45.5 and 47.3
+//             fp32                 3 x 512 x 14 x 14 3.6 and 4.5, 12 x 256 x 27 x 27 12.3 and 8.0; rows on 16 bytes 115 and 127
+//   stride 2  16 bits              3 x 240 x 28 x 28 3.0 and 4.0, 45 x 240 x 28 x 28 12.7 and 11.0; 5x5 with rows on 16 bytes
+//                                  32 x 512 x 16 x 16 7.8 and 10.0, 41 x 128 x 40 x 40 18.5 and 13.1
+//             fp32                 7 x 96 x 57 x 57 6.6 and 9.6; 5x5 on 15 x 192 x 27 x 27 8.4 and 6.7
+constexpr long long kNever = 1LL << 62, kMiB = 1 << 20;
+long long ring_least_bytes(const DirectParams& p, int es) {
+  const int row = p.W * es, area = p.H * p.W;
+  if (p.stride_w == 1) {
+    if (row % 16 == 0) return es == 4 || p.R == 5 ? kNever : area > 576 ? 96 * kMiB : row == 32 ? 24 * kMiB : 44 * kMiB;
+    return es == 4 ? 19 * kMiB / 10 : row % 8 == 0 ? 3 * kMiB : kMiB;
+  }
+  if (p.W < 8) return kNever;
+  if (row % 16 == 0) return p.R == 3 || row < 48 ? kNever : es == 2 && area <= 3136 ? 11 * kMiB / 2 : 7 * kMiB;
+  if (es == 2) return row % 8 != 0 ? 3 * kMiB : p.R == 3 ? 15 * kMiB / 4 : 14 * kMiB / 5;
+  if (p.R == 5) return area <= 2500 ? 11 * kMiB / 2 : kNever;
+  return area > 2025 || (row % 8 == 0 && area > 400) ? 48 * kMiB : 13 * kMiB / 2;
+}
+
 }  // namespace
 
 // Dense NCHW planes one after another, "same" padding of an unrolled filter, two groups of planes in shared memory, and a
-// layer this is ahead on.  Kernels, the other NCHW kernels and this one (us, 3x3 bf16 unless said otherwise):
-//   rows off 16 bytes       512 x 64 x 28 x 28 58.9 and 48.0, 14 x 14 27.3 and 18.1; 109 x 100 x 37 x 37 67.6 and 40.0;
-//                           77 x 50 x 110 x 110 159 and 86.8; 617 x 197 x 13 x 13 stride 2 42.3 and 27.3;
-//                           333 x 10 x 55 x 55 5x5 fp32 67.1 and 45.1
-//   16-byte rows            64 x 256 x 56 x 56 78.5 and 74.6, but fp32 115 and 127, 96 x 128 x 112 x 112 stride 2 91.2 and 92.3,
-//                           144 x 32 x 56 x 56 5x5 45.5 and 47.3; 200 x 30 x 40 x 40 5x5 stride 2 fp32 28.7 and 22.8
-//   under a megabyte of x   64 x 2 x 56 x 56 3.2 and 5.2, 32 x 3 x 9 x 9 5x5 stride 2 3.9 and 4.5: a ring has nothing to overlap
+// layer this is ahead on.
 bool depthwise_ring_ok(int dtype, const DirectParams& p) {
   const int es = dtype == FDNN_F32 ? 4 : 2;
   if (p.dil_h != 1 || p.dil_w != 1 || p.stride_h != p.stride_w || p.R != p.S || (p.R != 3 && p.R != 5) ||
@@ -439,19 +460,19 @@ bool depthwise_ring_ok(int dtype, const DirectParams& p) {
   // every strip's own columns begin inside the row: what lies past its end is padding
   if (p.OW > (p.W + p.stride_w - 1) / p.stride_w || p.OH > (p.H + p.stride_h - 1) / p.stride_h) return false;
   if ((long long)p.H * p.W > (1 << 20)) return false;
-  const long long bytes = (long long)p.N * p.C * p.H * p.W * es;
-  int per_sm = 1;
-  if (bytes < (1 << 20)) return false;
-  if (p.W * es % 16 == 0) {
-    if (es == 2 && p.R == 3 && p.stride_w == 1) {
-      if (bytes < (16 << 20)) return false;
-      per_sm = 2;
-    } else if (p.R != 5 || p.stride_w != 2) {
-      return false;
-    }
+  const long long planes = (long long)p.N * p.C, unit = group_unit(p, es);
+  if (planes * p.H * p.W * es < ring_least_bytes(p, es)) return false;
+  // Planes that start off 16 bytes come in groups of up to eight, of which an SM holds two or three where planes are large:
+  // too few groups leave SMs idle, and a second round that is nearly empty costs as much as the first.
+  const long long groups = (planes + unit - 1) / unit, sms = current_sm_count(), rounds = (groups + sms - 1) / sms;
+  if (p.stride_w == 2 || (es == 4 && p.R == 3)) {
+    if (100 * groups < 57 * rounds * sms) return false;
+  } else if (10 * groups < (es == 4 ? 5 : 3) * sms) {
+    return false;
   }
-  const long long unit = group_unit(p, es);
-  return 2 * slot_bytes(p, es, unit, false) + slot_bytes(p, es, unit, true) + kFixedBytes <= smem_of(per_sm);
+  const int per_sm = es == 2 && p.R == 3 && p.stride_w == 1 && p.W * es % 16 == 0 ? 2 : 1;
+  const int slots = p.stride_w == 2 && p.R == 3 ? 3 : 2;   // (186 x 64 x 75 x 75, two slots: 1.37 times as long)
+  return slots * slot_bytes(p, es, unit, false) + slot_bytes(p, es, unit, true) + kFixedBytes <= smem_of(per_sm);
 }
 
 cudaError_t launch_depthwise_ring(int dtype, const DirectParams& d, uint32_t* status, long long wait_limit, cudaStream_t stream) {
