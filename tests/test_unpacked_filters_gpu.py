@@ -1,5 +1,6 @@
 """fdnn_conv2d_fwd_unpacked: the filter is packed on the way, and the buffer then serves fdnn_conv2d_fwd."""
 import ctypes
+import gc
 
 import pytest
 import torch
@@ -165,10 +166,12 @@ def test_a_buffer_inside_the_workspace_is_scratch(native_lib, name):
     begin, nbytes = -(-layer.plan.workspace_bytes // 256) * 256, layer.plan.packed_weight_bytes
     arena = torch.full((begin + max(nbytes, other.plan.packed_weight_bytes) + 256,), 0x2A, dtype=torch.uint8, device="cuda")
     layer.scratch = arena[:begin + nbytes]
+    region = arena[begin:begin + other.plan.packed_weight_bytes]
+    other.pack(region)     # whatever lay at this address before is forgotten
+    arena.fill_(0x2A)
     nat.check(layer.unpacked(arena.data_ptr() + begin))
     layer.check()
     assert bool((arena[begin + nbytes:] == 0x2A).all())
-    region = arena[begin:begin + other.plan.packed_weight_bytes]
     region.copy_(other.pack(other.buffer()))
     nat.check(other.packed_call(region))
     other.check()
@@ -183,6 +186,7 @@ def test_calls_that_pack_on_the_way_leave_the_records_alone(native_lib):
     x, w = torch.randn(1, 64, 50, device="cuda").half(), torch.randn(64, 64, 3, device="cuda").half()
     x2, w2 = torch.randn(1, 64, 14, 14, device="cuda").half(), torch.randn(64, 64, 3, 3, device="cuda").half()
     held = []
+    gc.collect()     # what other tests left for it is not freed in between
     for _ in range(300):
         before = torch.cuda.memory_allocated()
         fd.conv1d(x, w, padding=1)
