@@ -81,10 +81,11 @@ repack_x_generic(const T* __restrict__ x, long long sn, long long sc, long long 
   }
 }
 
-// A filter [K, C, R, S] (any strides) as [K, R, S, c_pad]: a thread takes ten taps (a 3x3 filter's at once) of one input
-// channel of one filter, so that a warp reads PyTorch's [K][C][R][S] by contiguous stretches and writes 32 channels of a tap
-// at a time.  (Threads that walked all taps of their channel left a filter of few channels and many taps to a few warps:
-// 16 -> 16 31x31 63 us, a call on 2 x 64 x 64 NCHW 246 us and now 189; conv1d 64 -> 64 of 31 taps on 16 x 2000 28.9 and 20.7.)
+// A filter [K, C, R, S] (any strides) as [K, R, S, c_pad]: a thread takes a run of TAPS taps of one input channel of one
+// filter, so that a warp reads PyTorch's [K][C][R][S] by contiguous stretches and writes 32 channels of a tap at a time.
+// Ten at a time by itself (a 3x3 filter's at once), five in the launch that relays x out.  (Threads that walked all taps of
+// their channel left a filter of few channels and many taps to a few warps: 16 -> 16 31x31 63 us, a call on 2 x 64 x 64 NCHW
+// 246 us and now 189; conv1d 64 -> 64 of 31 taps on 16 x 2000 28.9 and 20.7.)
 template <typename T>
 struct PackJob {
   const T* w;
@@ -94,20 +95,20 @@ struct PackJob {
   long long plane;
   int blocks;          // of 256 threads
 };
-constexpr int kPackTaps = 10;
-template <typename T>
+constexpr int kPackTaps = 10, kPackTapsRelayout = 5;
+template <typename T, int TAPS>
 __device__ __forceinline__ void pack_taps(const PackJob<T>& j, int block) {
-  const int taps = j.R * j.S, runs = (taps + kPackTaps - 1) / kPackTaps;
+  const int taps = j.R * j.S, runs = (taps + TAPS - 1) / TAPS;
   const long long total = (long long)j.K * runs * j.c_pad;
   for (long long i = block * 256LL + threadIdx.x; i < total; i += j.blocks * 256LL) {
     const long long i2 = i / j.c_pad;
-    const int c = int(i - i2 * j.c_pad), k = int(i2 / runs), t0 = int(i2 - (long long)k * runs) * kPackTaps;
+    const int c = int(i - i2 * j.c_pad), k = int(i2 / runs), t0 = int(i2 - (long long)k * runs) * TAPS;
     const T* src = j.w + k * j.sk + c * j.sc;
     const long long at = ((long long)k * taps + t0) * j.c_pad + c;
     int r = t0 / j.S, s = t0 - r * j.S;
-    T v[kPackTaps];
+    T v[TAPS];
 #pragma unroll
-    for (int u = 0; u < kPackTaps; ++u) {
+    for (int u = 0; u < TAPS; ++u) {
       v[u] = (t0 + u < taps && c < j.C) ? src[r * j.sr + s * j.ss] : T(0.0f);
       if (++s == j.S) {
         s = 0;
@@ -115,7 +116,7 @@ __device__ __forceinline__ void pack_taps(const PackJob<T>& j, int block) {
       }
     }
 #pragma unroll
-    for (int u = 0; u < kPackTaps; ++u)
+    for (int u = 0; u < TAPS; ++u)
       if (t0 + u < taps) put<T>(j.dst, j.plane, at + (long long)u * j.c_pad, v[u]);
   }
 }
@@ -134,15 +135,19 @@ __device__ __forceinline__ void pack_taps(const PackJob<T>& j, int block) {
 // of two channels and joins them, the writer reads four neighbouring words.
 // PACK: the launch's first blocks pack the layer's filter instead (one launch for both where a call brings a filter that is
 // not kept packed; as the last blocks they ended 0.8 us after the others, 128 -> 128 3x3 on 32 x 28 x 28).
+// The tiles wait for memory, so that blocks per SM count: eight where the transposition itself lets them in, six for reads by
+// element.  With ten taps in flight in the packing blocks every block held 44 to 62 registers, and an SM four or five blocks:
+// 64 -> 64 1x1 on 32 x 56 x 56 fp32 23.9 us, now 18.6 (17.1 without a filter to pack), 64 channels of 8 x 112 x 112 39.6 and 34.2
+// (33.2), bf16 14.5 and 13.2 (11.7).
 template <typename T, bool VEC, bool PACK>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, VEC ? 8 : 6)
 transpose_repack(const T* __restrict__ x, long long mat_stride, long long mat_stride2, int mats2, long long sc, int mats,
                  int C, int P, int c_pad, T* __restrict__ dst, long long plane, const PackJob<T> pack) {
   chain_launches();
   const int first = PACK ? pack.blocks : 0, blocks = int(gridDim.x) - first;
   if constexpr (PACK) {
     if (int(blockIdx.x) < first) {
-      pack_taps<T>(pack, int(blockIdx.x));
+      pack_taps<T, kPackTapsRelayout>(pack, int(blockIdx.x));
       return;
     }
   }
@@ -313,7 +318,7 @@ repack_rows(const T* __restrict__ x, long long sw, long long pixels, int C, int 
 template <typename T>
 __global__ void __launch_bounds__(256) pack_w_kernel(const PackJob<T> job) {
   chain_launches();
-  pack_taps<T>(job, int(blockIdx.x));
+  pack_taps<T, kPackTaps>(job, int(blockIdx.x));
 }
 
 // Low-channel input relayout: one thread per stored pixel (4 channels = 8 bytes).
@@ -460,10 +465,10 @@ int grid_for(long long work_items, int per_block) {
 }
 
 template <typename T>
-PackJob<T> pack_job(const FilterPack& f) {
+PackJob<T> pack_job(const FilterPack& f, int run) {
   PackJob<T> j = {static_cast<const T*>(f.w), f.strides[0], f.strides[1], f.strides[2], f.strides[3], f.K, f.C, f.R, f.S, f.c_pad,
                   static_cast<T*>(f.dst), (long long)f.K * f.R * f.S * f.c_pad, 0};
-  j.blocks = grid_for((long long)f.K * f.c_pad * ((f.R * f.S + kPackTaps - 1) / kPackTaps), 256);
+  j.blocks = grid_for((long long)f.K * f.c_pad * ((f.R * f.S + run - 1) / run), 256);
   return j;
 }
 
@@ -477,7 +482,7 @@ cudaError_t transpose_t(const T* x, long long ms, long long ms2, int mats2, long
                    mult(mats2, ms2);
   const long long tiles = (long long)mats * ((P + 63) / 64) * ((c_pad + 128 / int(sizeof(T)) - 1) / (128 / int(sizeof(T))));
   PackJob<T> job = {};
-  if (pack != nullptr) job = pack_job<T>(*pack);
+  if (pack != nullptr) job = pack_job<T>(*pack, kPackTapsRelayout);
   auto* kernel = pack != nullptr ? (vec ? transpose_repack<T, true, true> : transpose_repack<T, false, true>)
                                  : (vec ? transpose_repack<T, true, false> : transpose_repack<T, false, false>);
   launch_chained(kernel, dim3(grid_for(tiles, 1) + job.blocks), 256, stream, x, ms, ms2, mats2, sc, mats, C, P, c_pad, dst, plane, job);
@@ -542,7 +547,7 @@ cudaError_t pack_w_t(const void* w, const long long s[4], int K, int C, int R, i
   if (R * S == 1 && s[0] == 1 && K > 1 && s[1] != 1)
     return transpose_t<T>(src, 0, 0, 1, s[1], 1, C, K, c_pad, out, plane, stream);
   FilterPack f = {w, {s[0], s[1], s[2], s[3]}, K, C, R, S, c_pad, dst, false};
-  const PackJob<T> job = pack_job<T>(f);
+  const PackJob<T> job = pack_job<T>(f, kPackTaps);
   launch_chained(pack_w_kernel<T>, dim3(job.blocks), 256, stream, job);
   return cudaGetLastError();
 }
