@@ -242,8 +242,9 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         int s_ = walk.kb - row * p.S;
         int r = row / p.c_blocks;
         int cb = row - r * p.c_blocks;
-        auto copy_steps = [&](auto prof_tag) {
+        auto copy_steps = [&](auto prof_tag, auto mn_tag) {
           constexpr bool kProf = decltype(prof_tag)::value;
+          constexpr bool kMn = decltype(mn_tag)::value;   // filter with K contiguous: boxes of 64 filters x 64 channels
           for (int kit = walk.kb; kit < walk.ke; ++kit) {
             long long pt0 = 0, pt1 = 0;
             if constexpr (kProf) pt0 = clock64();
@@ -267,7 +268,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
               tma_load_im2col_4d_pair(st, &tmA, bar, c0, w_base, h_base, img, static_cast<uint16_t>(s_ * p.dil_w),
                                       static_cast<uint16_t>(r * p.dil_h));
             }
-            if (p.b_mn) {   // filter with K contiguous: boxes of 64 filters x 64 channels
+            if constexpr (kMn) {
               tma_load_3d_pair(st + kABytes, &tmB, bar, b_row0, c0, 0);
               tma_load_3d_pair(st + kABytes + kMnBoxBytes, &tmB, bar, b_row0 + int(kMnBoxElems), c0, 0);
             } else if (!b_resident) {
@@ -287,7 +288,13 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             }
           }
         };
-        if (p.prof == nullptr) copy_steps(std::false_type{}); else copy_steps(std::true_type{});
+        if (p.b_mn) {
+          copy_steps(std::false_type{}, std::true_type{});
+        } else if (p.prof == nullptr) {
+          copy_steps(std::false_type{}, std::false_type{});
+        } else {
+          copy_steps(std::true_type{}, std::false_type{});
+        }
       }
       if (p.prof && blockIdx.x == 0) {
         p.prof[0] = prof_wait; p.prof[1] = prof_issue; p.prof[2] = clock64() - prof_t0; p.prof[3] = prof_iters;
@@ -334,7 +341,9 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         // put together in place, one commit for both CTAs, a first look at the barrier without the suspend-time hint and
         // one hand-over of the accumulator per epilogue warp instead of per thread took 1024 -> 2048 1x1 stride 2 on
         // 128 x 14 x 14 from 27.1 to 25.8 us, 32 x 1024 rows of a 4096 x 4096 product from 179.7 to 177.1):
-        // it exists once with four MMAs per step and once with a runtime count for the 3-channel mode.
+        // it exists once with four MMAs per step and once with three for the 3-channel mode (a count known only at run time,
+        // and a branch on the second operand's layout in the producer's loop, took the stem of 256 x 224 x 224 from 206.5 to
+        // 209.5 us a call; without them 206.9).
         auto reduce = [&](auto four_tag, auto prof_tag, auto mn_tag) {
           constexpr bool kMn = decltype(mn_tag)::value;   // the filter lies MN-major in its stages
           constexpr bool kFour = decltype(four_tag)::value;
@@ -358,7 +367,8 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             } else if constexpr (kFour) {
               mma4_f16_pair(d_tmem, a_lo, b_lo, kIdesc, acc);
             } else {
-              for (uint32_t k = 0; k < uint32_t(k16); ++k)
+#pragma unroll
+              for (uint32_t k = 0; k < 3; ++k)
                 mma_f16_pair_lo<kSw128DescHi, kSw128DescHi>(d_tmem, a_lo + 2 * k, b_lo + 2 * k, kIdesc, k == 0 ? acc : 1u);
             }
             tc_commit_both(empty_own + stage * 8);
