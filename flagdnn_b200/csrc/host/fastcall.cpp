@@ -54,9 +54,14 @@ struct PlanHash {
 };
 static_assert(sizeof(fdnn_conv_desc) % 4 == 0 && sizeof(PlanKey) % 4 == 0, "hashed and compared by words");
 constexpr size_t kMaxPlans = 1024;
-// Packing a filter of up to a megabyte in the launch that relays an NCHW x out anyway costs less than the look-up of a kept
-// one, which is Python code (64 -> 64 3x3 on one 14 x 14 image, f16, a call: 14.4 us with the look-up, 12.0 so).
+// Packing a filter of up to a megabyte in the launch that relays an NCHW x out costs less than the look-up of a kept one, which
+// is Python code, as long as the GPU is done before the host: calls of 64 -> 64 3x3 bf16 on one 14 x 14 image 8.6 us against
+// 10.5, on 4 x 56 x 56 8.7 and 10.6.  Beyond some 9 us of GPU time the look-up is hidden and the packing is not: 128 -> 128 on
+// 8 x 28 x 28 11.6 and 10.4, on 32 x 28 x 28 16.5 and 15.5, fp32 64 -> 64 on 8 x 56 x 56 21.9 and 20.9.
 constexpr int64_t kPackAlways = 1 << 20;
+bool sooner_than_a_look_up(const fdnn_conv_plan& plan, int dtype) {
+  return plan.packed_weight_bytes <= kPackAlways && plan.bytes <= 6e6 && plan.flops <= (dtype == FDNN_F32 ? 2e8 : 1.5e9);
+}
 std::unordered_map<PlanKey, fdnn_conv_plan, PlanHash>& plans() {   // used with the GIL held
   static auto* m = new std::unordered_map<PlanKey, fdnn_conv_plan, PlanHash>();
   return *m;
@@ -156,7 +161,7 @@ int launch(const fdnn_conv_desc& d, const at::Tensor& x, const at::Tensor& w, Py
   const void* packed_ptr = nullptr;
   if (plan.algo != FDNN_ALGO_DIRECT && plan.w_packed) {
     const bool in_relayout = plan.x_repacked && d.groups == 1 && plan.low_channel == 0 && plan.pixel_group <= 1 && d.c >= 8 &&
-                             d.x_strides[3] == 1 && d.x_strides[1] != 1 && d.w > 1 && plan.packed_weight_bytes <= kPackAlways;
+                             d.x_strides[3] == 1 && d.x_strides[1] != 1 && d.w > 1 && sooner_than_a_look_up(plan, d.dtype);
     if (weight_obj == nullptr || in_relayout) {
       WithoutGil free;
       const int64_t ws_bytes = (plan.workspace_bytes + 255) / 256 * 256, bytes = ws_bytes + plan.packed_weight_bytes;
