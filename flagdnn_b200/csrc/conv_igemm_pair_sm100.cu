@@ -581,7 +581,7 @@ conv_igemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     // The first pass is a rehearsal that stores nothing: it brings the drain loop's instructions in while the launch before
     // this one still runs, instead of after the first accumulator is complete (see conv_rows_sm100.cu, and
     // conv_igemm_sm100.cu for when not).
-    bool rehearsal = k_iters >= 8 || total_tiles > 2 * num_pairs;
+    bool rehearsal = !GELU && (k_iters >= 8 || total_tiles > 2 * num_pairs);
     if (!rehearsal) griddep_wait();
     while (rehearsal || walk_next(walk)) {
       const int tile = rehearsal ? pair_id : walk.tile;

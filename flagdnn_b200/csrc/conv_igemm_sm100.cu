@@ -416,7 +416,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // this one still runs, instead of after the first accumulator is complete (see conv_rows_sm100.cu).  Not for one or two
     // tiles of a short reduction, whose accumulator is complete before the rehearsal is (128 -> 512 1x1 with a shortcut on
     // 10 x 28 x 28 10.5 us, rehearsed 12.4; on 128 images 55.4 and 53.4).
-    bool rehearsal = k_iters >= 8 || total_tiles > 2 * int(gridDim.x);
+    bool rehearsal = !GELU && (k_iters >= 8 || total_tiles > 2 * int(gridDim.x));
     if (!rehearsal) griddep_wait();
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++tcount) {
       const int m_tile = tile / p.n_tiles;
