@@ -718,12 +718,21 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
 // 128 -> 128 on 128 x 28 x 28 34.7 and 25.1; 512 -> 512 on 128 x 7 x 7, an eighth of the walk rows no output, 30.5 and 27.6;
 // 104 -> 152 on 24 x 45 x 37 40.6 and 25.7; NCHW 64 -> 64 on 128 x 56 x 56 60.1 and 38.0; two groups 64 -> 128 on
 // 256 x 56 x 56 (block-diagonal before) 122 and 72; sixteen groups of 32 on 16 x 28 x 28 27.9 and 15.0.
-//   Where it loses: fewer pair tiles than pairs and nine steps in all (64 -> 128 on 8 x 28 x 28 5.5 and 5.9: smaller tiles
-// start sooner), and where pair tiles fill a round and a bit (200 -> 200 5x5 on 20 x 31 x 29 NCHW: 141 tiles of 128 x 256
-// in one round against 152 in three, 42 and 50).  So both sides are counted in clocks of the busiest SM, with what a step
-// of four MMAs was measured to take: 380 / 520 / 780 for 64 / 128 / 256 columns and 640 on pairs with a copy per tap,
-// 230 / 310 / 570 here (fp32, twelve MMAs: 800 / 1100 and 600 / 830), 1500 more for a launch, and 1350 per copy where pixels straddle 128-byte lines (24 -> 24 on
-// 112 x 112 10.4 and 7.0).
+//   Where it loses: few steps in all (64 -> 128 on 8 x 28 x 28 5.5 and 5.9: smaller tiles start sooner); where pair tiles fill a
+// round and a bit (200 -> 200 5x5 on 20 x 31 x 29 NCHW: 141 tiles of 128 x 256 in one round against 152 in three, 42 and 50);
+// and where the taps of a filter row do not fit a slot of the filter ring, so that every tap is waited for by itself
+// (86 columns, 7x7 on 81 x 28 x 28 x 201 183 and 219).  So both sides are counted in clocks of the busiest SM: rounds of tiles,
+// each as long as its steps of four MMAs (fp32: twelve) or as its drain, whichever is longer, and 1700 for the launch.
+//                              a copy per tap                          here
+//   step, columns 64/128/256   365 / 510 / 650, pairs 690              225 / 290 / 600; a tap by itself 600
+//   fp32                       800 / 1100                              600 / 830
+//   drain                      1500 / 3000 / 5000 through the TMA      2000 / 3000 / 4400 by sectors of 32 bytes
+//                              unit, else 6500 / 10000 / 11500         2700 / 5300 / 9200 along channels, 1500 / 2800 / 4000 pixels
+//   pixels off 128-byte lines  1100 per copy up to 192 bytes, wider    1100 per copy up to 192 bytes
+//                              ones 1.05 (64 columns) or 1.15 times
+// The constants are fitted to 1200 layers timed on the copy per tap and on all three widths here: 34 are over 4 % slower than on
+// the copy per tap (by 1.3 times at most), against 75 with one step time for all and 1350 for any pixel off a line
+// (34 x 66 x 8 x 824 -> 288 80 and 105, 87 x 14 x 14 x 440 -> 184 5x5 65 and 81).
 struct RowsMode {
   int tile_n;          // 0: no
   int pitch;           // walk rows per image row
@@ -764,26 +773,43 @@ RowsMode rows_mode(const fdnn_conv_desc* d, const fdnn_conv_plan& plan, const vo
     g.tile_n = bn;
     g.n_tiles = d->c / 64;
   } else {
-    // clocks of the busiest SM: rounds of tiles x steps x what a step takes
-    const long long pitch = es * d->x_strides[3];
-    const bool straddles = !plan.x_repacked && d->w > 1 && pitch % 128 != 0 && pitch != 16 && pitch != 32 && pitch != 64;
+    // clocks of the busiest SM (see above)
+    const long long pixel = es * (plan.x_repacked ? padded_x_channels(d) : d->x_strides[3]);
+    const bool off_lines = d->w > 1 && pixel % 128 != 0 && pixel != 64;
+    const double copy = off_lines && pixel <= 192 ? 1100 : 0;
     const double steps = double(d->r) * ((d->c * es + 127) / 128);
     const int q = plan.pixel_group > 1 ? plan.pixel_group : 1;
     const bool pair = plan.algo == FDNN_ALGO_IGEMM_PAIR;
+    auto column_class = [](int columns) { return columns == 64 ? 0 : columns == 128 ? 1 : 2; };
+    auto rounds = [](long long tiles, int units) { return double((tiles + units - 1) / units); };
+    auto longer = [](double x, double z) { return x > z ? x : z; };
+    static constexpr double kStep[3] = {365, 510, 650}, kDrainTma[3] = {1500, 3000, 5000}, kDrainOther[3] = {6500, 10000, 11500};
+    static constexpr double kTap[3] = {225, 290, 600}, kSectors[3] = {2000, 3000, 4400}, kChannels[3] = {2700, 5300, 9200},
+                            kPixels[3] = {1500, 2800, 4000};
+    const int now_class = column_class(plan.tile_n);
+    double step = pair ? 690 : es == 4 ? (now_class == 0 ? 800 : 1100) : kStep[now_class];
+    step = longer(step, copy);
+    if (off_lines && pixel > 192) step *= !pair && now_class == 0 ? 1.05 : 1.15;
     const long long m_now = ((long long)d->n * oh * ow / q + plan.tile_m - 1) / plan.tile_m;
     const long long tiles_now = m_now * (((long long)q * d->k + plan.tile_n - 1) / plan.tile_n);
-    const int units = pair ? sms / 2 : sms;
-    double step = pair ? 640 : plan.tile_n == 64 ? 380 : plan.tile_n == 128 ? 520 : 780;
-    if (es == 4) step = plan.tile_n == 64 ? 800 : 1100;   // twelve MMAs
-    if (straddles && step < 1350) step = 1350;
-    const double now = double((tiles_now + units - 1) / units) * steps * (d->s + (q - 1) * d->stride_w) * step;
-    double best_cost = now;
+    double best_cost = rounds(tiles_now, pair ? sms / 2 : sms) *
+                       longer(steps * (d->s + (q - 1) * d->stride_w) * step, (y_is_dense_nhwc(d, oh, ow, y) ? kDrainTma : kDrainOther)[now_class]);
+    const double* drain = d->y_strides[1] != 1 ? kPixels : sector_aligned(*d, oh, ow, y) ? kSectors : kChannels;
     for (int bn = 64; bn <= (es == 2 ? 256 : 128); bn *= 2) {
       if (bn > 64 && bn / 2 >= d->k) break;
-      const long long tiles = (long long)((g.m_tiles + 1) / 2) * ((d->k + bn - 1) / bn);
-      double tap = es == 4 ? (bn == 64 ? 600 : 830) : bn == 64 ? 230 : bn == 128 ? 310 : 570;
-      if (straddles && tap * d->s < 1350) tap = 1350.0 / d->s;
-      const double cost = 1500 + double((tiles + sms / 2 - 1) / (sms / 2)) * steps * d->s * tap;
+      RowsParams ring = {};
+      ring.R = d->r;
+      ring.S = d->s;
+      ring.halves = es == 4 ? 2 : 1;
+      ring.c_blocks = int((d->c * es + 127) / 128);
+      ring.n_tiles = (d->k + bn - 1) / bn;
+      ring.b_bytes = ring.halves * (bn / 2) * 128;
+      rows_stages(&ring);
+      const long long tiles = (long long)((g.m_tiles + 1) / 2) * ring.n_tiles;
+      double tap = es == 4 ? (bn == 64 ? 600 : 830) : kTap[column_class(bn)];
+      if (ring.b_taps != d->s) tap = longer(tap, 600);
+      tap = longer(tap, copy / d->s);
+      const double cost = 1700 + rounds(tiles, sms / 2) * longer(steps * d->s * tap, drain[column_class(bn)]);
       if (cost < best_cost) {
         best_cost = cost;
         g.tile_n = bn;
