@@ -766,7 +766,9 @@ RowsMode rows_mode(const fdnn_conv_desc* d, const fdnn_conv_plan& plan, const vo
   g.m_tiles = int((walk + 127) / 128);
   g.blk_groups = 1;
   if (d->groups > 1) {
-    if (es != 2 || (cg != 16 && cg != 32) || d->c % 64 != 0 || kg % 32 != 0 || d->y_strides[1] != 1 || !sector_aligned(*d, oh, ow, y)) return g;
+    if (es != 2 || (cg != 16 && cg != 32) || d->c % 64 != 0 || kg % 32 != 0 || d->y_strides[1] != 1 ||
+        !sector_aligned(*d, oh, ow, y))
+      return g;
     g.blk_groups = 64 / cg;
     const int bn = g.blk_groups * kg;
     if (bn != 64 && bn != 128 && bn != 256) return g;
@@ -1652,8 +1654,6 @@ static int relayout_x(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, bool 
   cudaError_t e = launch_repack_x(d.dtype, x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w, x_pad,
                                   workspace, a->plane, stream, pack != nullptr && !pack->done ? pack : nullptr);
   if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
-  const int st = pack_filter(d.dtype, pack, stream);
-  if (st != FDNN_OK) return st;
   a->base = workspace;
   a->sw = x_pad;
   a->sh = (long long)d.w * x_pad;
@@ -1962,11 +1962,11 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
   if (windows.scratch > workspace_bytes) windows.ok = false;
   ActivationView a = {};
   if (windows.ok) {
+    st = pack_filter(d.dtype, pack, stream);
+    if (st != FDNN_OK) return st;
     e = launch_repack_x_windows(x, reinterpret_cast<const long long*>(d.x_strides), d.n, d.c, d.h, d.w, d.pad_left,
                                 windows.w_pad, workspace, stream);
     if (e != cudaSuccess) return fail_cuda("repack_x launch", e);
-    st = pack_filter(d.dtype, pack, stream);
-    if (st != FDNN_OK) return st;
     a.base = workspace;
   } else {
     st = relayout_x(d, plan, batch != nullptr, x, workspace, workspace_bytes, stream, &a, pack);

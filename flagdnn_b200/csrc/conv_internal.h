@@ -197,7 +197,7 @@ cudaError_t launch_adaptive_avg_pool2d(int dtype, const PoolParams& p, cudaStrea
 // x[N,C,H,W] (any strides) -> dense NHWC with C padded to c_pad (zeros).  For
 // f32 two planes are written: TF32-rounded high halves at dst, the rounded
 // remainders at dst + plane_elems.
-// pack: a filter to pack to [K, R, S, c_pad] in the same launch if its kernel can (pack->done then), or nullptr.
+// pack: a filter to pack to [K, R, S, c_pad] too, in the same launch if its kernel can, else in one before it; or nullptr.
 struct FilterPack {
   const void* w;
   long long strides[4];

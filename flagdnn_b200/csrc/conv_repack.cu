@@ -510,6 +510,9 @@ cudaError_t rows_t(const T* x, long long sw, long long pixels, int C, int c_pad,
 // else row by row) -> transposition; channels contiguous and pixels evenly spaced -> rows; anything else -> the
 // element-wise gather.  Extents of one carry no stride.
 template <typename T>
+cudaError_t pack_w_t(const void* w, const long long s[4], int K, int C, int R, int S, int c_pad, void* dst, long long plane,
+                     cudaStream_t stream);
+template <typename T>
 cudaError_t repack_x_t(const void* x, const long long x_s[4], int N, int C, int H, int W, int c_pad,
                        void* dst, long long plane, cudaStream_t stream, FilterPack* pack) {
   long long s[4] = {x_s[0], x_s[1], x_s[2], x_s[3]};
@@ -525,6 +528,12 @@ cudaError_t repack_x_t(const void* x, const long long x_s[4], int N, int C, int 
       return transpose_t<T>(src, s[0], 0, 1, s[1], N, C, H * W, c_pad, out, plane, stream, pack);
     if ((long long)N * H < (1LL << 30))
       return transpose_t<T>(src, s[0], s[2], H, s[1], N * H, C, W, c_pad, out, plane, stream, pack);
+  }
+  if (pack != nullptr) {   // a launch of its own, and the first one: the shorter of the two is not left for the end
+    const cudaError_t e = pack_w_t<T>(pack->w, pack->strides, pack->K, pack->C, pack->R, pack->S, pack->c_pad, pack->dst,
+                                      (long long)pack->K * pack->R * pack->S * pack->c_pad, stream);
+    if (e != cudaSuccess) return e;
+    pack->done = true;
   }
   if ((s[1] == 1 || C == 1) && !(C == 1 && s[3] == 1)) {
     const long long sw = W > 1 ? s[3] : (H > 1 ? s[2] : s[0]);
