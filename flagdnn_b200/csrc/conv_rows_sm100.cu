@@ -400,7 +400,9 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (!ok) break;
         tc_fence_after();
       }
-      const bool boxes = STORE == kStoreSectors && !kSplit && p.y_rows && __all_sync(0xffffffffu, row_ok);
+      // With GELU every drain takes the same way out: two copies of erf and tanh for all values, by turns, outgrow the instruction
+      // cache (64 -> 64 3x3 on 32 x 56 x 56 27.3 us by turns, 16.3 so; four groups 128 -> 256 on 85 x 56 x 56 192 and 105).
+      const bool boxes = STORE == kStoreSectors && !kSplit && !GELU && p.y_rows && __all_sync(0xffffffffu, row_ok);
       row_ok = row_ok && !rehearsal;
       const uint32_t t_row = tmem_base + (uint32_t(ew * 32) << 16) + buf * BN + col_off;
       auto read_done = [&]() {   // one arrival per warp, before the last stores and without waiting for the earlier ones
