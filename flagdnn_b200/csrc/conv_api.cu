@@ -724,7 +724,8 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
 // (86 columns, 7x7 on 81 x 28 x 28 x 201 183 and 219).  So both sides are counted in clocks of the busiest SM: rounds of tiles,
 // each as long as its steps of four MMAs (fp32: twelve) or as its drain, whichever is longer, and 1700 for the launch.
 //                              a copy per tap                          here
-//   step, columns 64/128/256   365 / 510 / 650, pairs 690              225 / 290 / 600; a tap by itself 600
+//   step, columns 64/128/256   365 / 510 / 650, pairs 690              225 / 290 / 600 (570 where there are
+//                                                                      more rounds); a tap by itself 600
 //   fp32                       800 / 1100                              600 / 830
 //   drain                      1500 / 3000 / 5000 through the TMA      2000 / 3000 / 4400 by sectors of 32 bytes
 //                              unit, else 6500 / 10000 / 11500         2700 / 5300 / 9200 along channels, 1500 / 2800 / 4000 pixels
@@ -808,10 +809,11 @@ RowsMode rows_mode(const fdnn_conv_desc* d, const fdnn_conv_plan& plan, const vo
       ring.b_bytes = ring.halves * (bn / 2) * 128;
       rows_stages(&ring);
       const long long tiles = (long long)((g.m_tiles + 1) / 2) * ring.n_tiles;
-      double tap = es == 4 ? (bn == 64 ? 600 : 830) : kTap[column_class(bn)];
-      if (ring.b_taps != d->s) tap = longer(tap, 600);
+      const double all_rounds = rounds(tiles, sms / 2);
+      double tap = es == 4 ? (bn == 64 ? 600 : 830) : bn == 256 && all_rounds > 1 ? 570 : kTap[column_class(bn)];
+      if (ring.b_taps != d->s && bn < 256) tap = longer(tap, 600);
       tap = longer(tap, copy / d->s);
-      const double cost = 1700 + rounds(tiles, sms / 2) * longer(steps * d->s * tap, drain[column_class(bn)]);
+      const double cost = 1700 + all_rounds * longer(steps * d->s * tap, drain[column_class(bn)]);
       if (cost < best_cost) {
         best_cost = cost;
         g.tile_n = bn;
