@@ -46,9 +46,9 @@ WORKLOADS = {
                stride=1, pad=1, dtype="float32", layout="nchw", dist="normal", bound="tensor"),
 }
 
-# dram__bytes_read.sum + dram__bytes_write.sum per launch of the implicit-GEMM
-# kernel, from the ncu captures summarised under profiles/ (None = not captured).
-NCU_TRAFFIC_BYTES = {"c3": 26.98e6, "c2": 495.9e6, "c4": 435.0e6, "c1": None}
+# dram__bytes_read.sum + dram__bytes_write.sum per launch of the main kernel, from the ncu captures summarised under
+# profiles/, with the kernel they were taken of.
+NCU_TRAFFIC_BYTES = {"c3": ("conv_rows_kernel", 27.01e6), "c2": ("conv_igemm_kernel", 495.9e6), "c4": ("conv_igemm_pair_kernel", 435.0e6)}
 
 # the arithmetic type as the JSON line names it (fp32 tensors run as 3xTF32 with fp32 accumulation)
 SHORT_DTYPE = {"bfloat16": "bf16", "float16": "f16", "float32": "f32"}
@@ -341,6 +341,7 @@ def run_ours(args):
     node_types = [n.op_type for n in compiled.graph.nodes]
     plan = fd.conv2d_plan(xs[0], w, stride=wl["stride"], padding=wl["pad"])
     launches_per_step = plan["launches"]
+    kernel = main_kernel(xs[0], w, compiled.run(xs[0], w, b), wl)
 
     # first calls through the eager API (pack the filter, set kernel attributes); not the counted warm-up
     for i in range(3):
@@ -526,7 +527,7 @@ def run_ours(args):
     status_word = fd.device_status()
     if rank == 0:
         _report(args, world, wl, nums, peaks, peak_src, ms_per_step, value, steps, warmup, n_sets, per_set, node_types,
-                plan, launches_per_step, clocks, status_word, e2e, concurrent, sustained, eager, cpu, parity_ranks, stack)
+                plan, kernel, launches_per_step, clocks, status_word, e2e, concurrent, sustained, eager, cpu, parity_ranks, stack)
     if dist is not None:
         dist.barrier()
         dist.destroy_process_group()
@@ -602,24 +603,43 @@ def _e2e_leg(args, torch, dist, device, compiled, xs, outs, w, b, nums, world, b
     return result
 
 
-def _c_abi_host_call_ms(torch, x_dev, x_host, w, b, y_host, wl, repeats=5):
-    import ctypes
-
+def descriptor(x, w, y, wl):
     from flagdnn_b200 import _native as nat
 
-    lib = nat.load()
     d = nat.ConvDesc()
     d.dtype = {"bfloat16": nat.BF16, "float16": nat.F16, "float32": nat.F32}[wl["dtype"]]
-    d.n, d.c, d.h, d.w = x_dev.shape
+    d.n, d.c, d.h, d.w = x.shape
     d.k, _, d.r, d.s = w.shape
     d.stride_h = d.stride_w = wl["stride"]
     d.pad_top = d.pad_bottom = d.pad_left = d.pad_right = wl["pad"]
     d.dil_h = d.dil_w = 1
     d.groups = 1
     d.algo = nat.ALGO_AUTO
-    w_host, b_host = w.cpu().pin_memory(), b.cpu().pin_memory()
     for i in range(4):
-        d.x_strides[i], d.w_strides[i], d.y_strides[i] = x_host.stride(i), w_host.stride(i), y_host.stride(i)
+        d.x_strides[i], d.w_strides[i], d.y_strides[i] = x.stride(i), w.stride(i), y.stride(i)
+    return d
+
+
+def main_kernel(x, w, y, wl):
+    """Name, tile and grid of the kernel that computes y: what the library launches for these tensors."""
+    import ctypes
+
+    from flagdnn_b200 import _native as nat
+
+    k = nat.ConvKernel()
+    nat.check(nat.load().fdnn_conv2d_main_kernel(ctypes.byref(descriptor(x, w, y, wl)), x.data_ptr(), w.data_ptr(), y.data_ptr(),
+                                                 ctypes.byref(k)))
+    return {"name": nat.KERNEL_NAMES[k.kernel], "tile": [k.tile_m, k.tile_n], "grid": k.grid}
+
+
+def _c_abi_host_call_ms(torch, x_dev, x_host, w, b, y_host, wl, repeats=5):
+    import ctypes
+
+    from flagdnn_b200 import _native as nat
+
+    lib = nat.load()
+    w_host, b_host = w.cpu().pin_memory(), b.cpu().pin_memory()
+    d = descriptor(x_host, w_host, y_host, wl)
     need = ctypes.c_int64(0)
     nat.check(lib.fdnn_conv2d_host_arena_bytes(ctypes.byref(d), ctypes.byref(need)))
     arena = torch.empty(need.value, dtype=torch.uint8, device=x_dev.device)
@@ -636,7 +656,7 @@ def _c_abi_host_call_ms(torch, x_dev, x_host, w, b, y_host, wl, repeats=5):
 
 
 def _report(args, world, wl, nums, peaks, peak_src, ms_per_step, value, steps, warmup, n_sets, per_set, node_types,
-            plan, launches_per_step, clocks, status_word, e2e, concurrent, sustained, eager, cpu, parity_ranks, stack):
+            plan, kernel, launches_per_step, clocks, status_word, e2e, concurrent, sustained, eager, cpu, parity_ranks, stack):
     # ---- roofline of the dominant kernel (the implicit-GEMM kernel; one launch per step)
     if wl["bound"] == "tensor":
         achieved = nums["flops"] / (ms_per_step * 1e-3) / 1e12
@@ -646,9 +666,10 @@ def _report(args, world, wl, nums, peaks, peak_src, ms_per_step, value, steps, w
         achieved = nums["bytes"] / (ms_per_step * 1e-3) / 1e9
         peak, unit = peaks["hbm_gbs"], "GB/s"
         extra = {}
+    traffic_of, traffic = NCU_TRAFFIC_BYTES.get(args.workload, (None, None))
     roofline = {"bound": wl["bound"], "achieved": achieved, "peak": peak, "unit": unit, "frac": achieved / peak,
-                "traffic": NCU_TRAFFIC_BYTES.get(args.workload), "peak_source": f"of {peak_src}",
-                "kernel": "conv_igemm_pair_kernel" if plan["algo"] == 3 else "conv_igemm_kernel",
+                "traffic": traffic if traffic_of == kernel["name"] else None, "peak_source": f"of {peak_src}",
+                "kernel": kernel["name"],
                 "algorithmic_flops_per_launch": nums["flops"], "algorithmic_bytes_per_launch": nums["bytes"], **extra}
     if stack is not None:
         roofline["c5_strong"] = stack
@@ -666,8 +687,7 @@ def _report(args, world, wl, nums, peaks, peak_src, ms_per_step, value, steps, w
                    "timing": "CUDA events on the launching stream around exactly the counted steps; a 150 us spin kernel "
                              "ahead of the first event lets the CPU queue the region's launches before the GPU reaches it",
                    "per_gpu_batch": wl["n"], "parallelism": f"batch-sharded replicas x{world}, no collective",
-                   "tile": [plan["tile_m"], plan["tile_n"], plan["tile_k"]], "stages": plan["stages"],
-                   "grid": plan["grid"], "parity_checked_ranks": parity_ranks},
+                   "tile": kernel["tile"] + [plan["tile_k"]], "grid": kernel["grid"], "parity_checked_ranks": parity_ranks},
         "pct_of_bf16_peak": 100.0 * (value / world) / peaks["bf16_tflops"],
         "roofline": roofline, "cpu_baseline": cpu,
         "e2e": e2e,

@@ -36,6 +36,7 @@ EXPORTED_SYMBOLS = (
     "fdnn_status_string",
     "fdnn_last_error",
     "fdnn_conv2d_query",
+    "fdnn_conv2d_main_kernel",
     "fdnn_conv2d_pack_weight",
     "fdnn_conv2d_fwd",
     "fdnn_conv2d_fwd_residual",
@@ -98,6 +99,13 @@ class ConvPlan(ctypes.Structure):
         return {name: getattr(self, name) for name, _ in self._fields_}
 
 
+KERNEL_NAMES = ("CUDA cores", "conv_igemm_kernel", "conv_igemm_pair_kernel", "conv_rows_kernel")   # by ConvKernel.kernel
+
+
+class ConvKernel(ctypes.Structure):
+    _fields_ = [(name, ctypes.c_int32) for name in ("kernel", "tile_m", "tile_n", "grid")]
+
+
 class PoolDesc(ctypes.Structure):
     _fields_ = [(name, ctypes.c_int32) for name in
                 ("dtype", "n", "c", "h", "w", "oh", "ow", "kernel_h", "kernel_w", "stride_h", "stride_w",
@@ -130,6 +138,8 @@ def load() -> ctypes.CDLL:
     lib.fdnn_last_error.restype = ctypes.c_char_p
     lib.fdnn_conv2d_query.restype = i32
     lib.fdnn_conv2d_query.argtypes = [ctypes.POINTER(ConvDesc), vp, vp, vp, ctypes.POINTER(ConvPlan)]
+    lib.fdnn_conv2d_main_kernel.restype = i32
+    lib.fdnn_conv2d_main_kernel.argtypes = [ctypes.POINTER(ConvDesc), vp, vp, vp, ctypes.POINTER(ConvKernel)]
     lib.fdnn_conv2d_pack_weight.restype = i32
     lib.fdnn_conv2d_pack_weight.argtypes = [ctypes.POINTER(ConvDesc), vp, vp, vp, i64, vp]
     lib.fdnn_conv2d_fwd.restype = i32

@@ -827,6 +827,29 @@ RowsMode rows_mode(const fdnn_conv_desc* d, const fdnn_conv_plan& plan, const vo
   return g;
 }
 
+// ... of a layer without groups, or of one with them and its filters where rows_filter finds them.
+bool rows_layer_ok(const fdnn_conv_desc& d, const fdnn_conv_plan& plan) {
+  return plan.algo != FDNN_ALGO_DIRECT && plan.low_channel == 0 && !(plan.x_repacked && d.c < 8);
+}
+
+// The filter as the kernels of conv_rows_sm100.cu read it.
+struct FilterView {
+  const void* base;
+  int c, s_pitch, c_step;      // channels per tap, taps per filter row, first channel of group g: g * c_step
+  long long s_tap, s_k;
+};
+// A grouped layer's filters: in place, or in the dense filter in front of the packed one.  False: neither.
+bool rows_group_filter(const fdnn_conv_desc& d, const void* w, const void* w_packed, FilterView* f) {
+  const int cg = d.c / d.groups;
+  if (w != nullptr && filter_in_place(&d, w)) {
+    *f = {w, cg, d.s, 0, d.s > 1 ? d.w_strides[3] : d.w_strides[2], d.w_strides[0]};
+    return true;
+  }
+  if (!group_dense_ok(&d) || w_packed == nullptr || !aligned16(w_packed)) return false;
+  *f = {w_packed, d.c, d.s, cg, d.c, (long long)d.r * d.s * d.c};
+  return true;
+}
+
 // Several groups of a grouped 16-bit layer in one launch of the single-CTA kernel (see IgemmParams::groups), where that
 // beats the route its plan names.  `group_batch` fills `one` with the plan of a single group on that kernel and
 // answers how many column tiles of which width the launch would have, or 0 tiles when it does not apply:
@@ -1430,6 +1453,26 @@ int fdnn_conv2d_query(const fdnn_conv_desc* desc, const void* x, const void* w, 
   return make_plan(desc, x, w, y, plan);
 }
 
+int fdnn_conv2d_main_kernel(const fdnn_conv_desc* desc, const void* x, const void* w, const void* y, fdnn_conv_kernel* kernel) {
+  if (kernel == nullptr) return fail(FDNN_BAD_PARAM, "kernel is NULL");
+  fdnn_conv_plan plan;
+  const int st = make_plan(desc, x, w, y, &plan);
+  if (st != FDNN_OK) return st;
+  *kernel = {};
+  if (plan.algo == FDNN_ALGO_DIRECT) return FDNN_OK;
+  const RowsMode rows = rows_mode(desc, plan, y);
+  FilterView f;
+  // a packed filter is 16-byte aligned wherever it lies
+  const bool have = desc->groups > 1 ? rows_group_filter(*desc, w, reinterpret_cast<const void*>(uintptr_t(256)), &f)
+                                     : rows_layer_ok(*desc, plan);
+  if (rows.tile_n != 0 && have) {
+    *kernel = {FDNN_KERNEL_ROWS, 256, rows.tile_n, rows.grid};
+  } else {
+    *kernel = {plan.algo == FDNN_ALGO_IGEMM_PAIR ? FDNN_KERNEL_PAIR : FDNN_KERNEL_IGEMM, plan.tile_m, plan.tile_n, plan.grid};
+  }
+  return FDNN_OK;
+}
+
 // note: whether the buffer outlives the call and its layout is remembered
 static int pack_weight(const fdnn_conv_desc* desc, const void* w, const void* y, void* packed, int64_t packed_bytes, void* stream,
                        bool note) {
@@ -1664,13 +1707,6 @@ static int relayout_x(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, bool 
   return FDNN_OK;
 }
 
-// The filter as the kernels of conv_rows_sm100.cu read it.
-struct FilterView {
-  const void* base;
-  int c, s_pitch, c_step;      // channels per tap, taps per filter row, first channel of group g: g * c_step
-  long long s_tap, s_k;
-};
-
 static int fwd_rows(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, const RowsMode& rows, int dev, const void* x,
                     const FilterView& f, FilterPack* pack, const void* bias, const void* scale, int activation, void* y,
                     void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
@@ -1703,7 +1739,7 @@ static int fwd_rows(const fdnn_conv_desc& d, const fdnn_conv_plan& plan, const R
   p.m_tiles = rows.m_tiles;
   p.n_tiles = rows.n_tiles;
   p.blk_groups = rows.blk_groups;
-  p.cg = cg; p.kg = kg;
+  p.kg = kg;
   p.blk_c_step = f.c_step;
   p.b_bytes = blk ? rows.blk_groups * (kg / 2) * cg * 2 : p.halves * (rows.tile_n / 2) * 128;
   rows_stages(&p);
@@ -1780,14 +1816,8 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
 
   if (batch == nullptr && d.groups > 1 && plan.algo != FDNN_ALGO_DIRECT && allow_group && residual == nullptr) {
     const RowsMode rows = rows_mode(&d, plan, y);
-    const int cg = d.c / d.groups;
-    FilterView f = {w, cg, d.s, 0, d.s > 1 ? d.w_strides[3] : d.w_strides[2], d.w_strides[0]};
-    bool have = w != nullptr && filter_in_place(&d, w);
-    if (!have && group_dense_ok(&d) && w_packed != nullptr && aligned16(w_packed)) {
-      f = {w_packed, d.c, d.s, cg, d.c, (long long)d.r * d.s * d.c};   // the dense filter in front of the packed one
-      have = true;
-    }
-    if (rows.tile_n != 0 && have && (plan.x_repacked == 0 || (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 &&
+    FilterView f = {};
+    if (rows.tile_n != 0 && rows_group_filter(d, w, w_packed, &f) && (plan.x_repacked == 0 || (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 &&
         workspace_bytes >= tight_x_bytes(&d)))) {
       int dev = 0;
       st = prepare_device(&dev);
@@ -1929,8 +1959,7 @@ static int fwd_impl(const fdnn_conv_desc* desc, const void* x, const void* w, co
     if (find_packed(w_packed, dev, &have) && !(have == want)) return fail_layout(have, want);
   }
 
-  if (batch == nullptr && residual == nullptr && allow_group && k_real == d.k && plan.low_channel == 0 &&
-      !(plan.x_repacked && d.c < 8)) {
+  if (batch == nullptr && residual == nullptr && allow_group && k_real == d.k && rows_layer_ok(d, plan)) {
     const RowsMode rows = rows_mode(&d, plan, y);
     if (rows.tile_n != 0) {
       const int c_pad = plan.c_padded;

@@ -419,8 +419,8 @@ cudaError_t launch_ring_t(const DirectParams& d, uint32_t* status, long long lim
 // Bytes of x from which this kernel is ahead of the other NCHW kernels, or none.  A ring starts later than a kernel that reads
 // where it stands, and has nothing to overlap while a block has a group or two; what there is to gain depends on how wide the
 // others can read (rows on 16, 8 or fewer bytes) and on the multiplications per input.  2200 layers of 7 to 112 columns and 1 to
-// 136 MiB were timed on both: with these lines 26 take over 5 % longer than on the other (1.36 times at most), with one line of a megabyte 420 did (up to 1.9).  The others
-// and this one, us, 3x3 bf16 unless said otherwise:
+// 136 MiB were timed on both: with these lines 26 take over 5 % longer than on the other (1.36 times at most); with one line at
+// a megabyte 420 did (up to 1.9).  The others and this one, us, 3x3 bf16 unless said otherwise:
 //   stride 1  rows off 8 bytes     6 x 512 x 14 x 14 5.4 and 5.0, 34 x 100 x 25 x 25 13.0 and 8.3, 168 x 512 x 14 x 14 62.4 and 34.9
 //             rows on 8 bytes      3 x 256 x 28 x 28 3.8 and 5.0, 11 x 256 x 28 x 28 9.3 and 7.8
 //             rows on 16 bytes     81 x 384 x 24 x 24 31.6 and 36.0, 162 x 384 x 24 x 24 71.7 and 60.8; 45 x 256 x 56 x 56 56.1 and

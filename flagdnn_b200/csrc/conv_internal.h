@@ -128,7 +128,7 @@ struct RowsParams {
   int b_bytes;           // one CTA's filters of a tap and channel block (all halves)
   int a_stages, b_stages, b_resident, b_taps, b_slot;   // rings (rows_stages): copies, slots, whole filter, a slot's taps and bytes
   int blk_groups;        // > 1: groups of a 64-channel block, of cg channels and kg filters each; column tiles are blocks
-  int cg, kg;
+  int kg;
   int blk_c_step;        // first channel of group g in the filter map: g * blk_c_step
   long long y_sn, y_sk, y_sh, y_sw;
   int y_unit;            // bytes per lane and store: 32 where every pixel starts on 32 bytes (grouped layers: always)

@@ -413,8 +413,8 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (boxes) {
         // 32 pixels one after another: boxes through the TMA unit
         const int pixel = __shfl_sync(0xffffffffu, real, 0);
-        epilogue_store_tile<T, WC, false, 1, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY, pixel, 0, rehearsal ? 0 : 32,
-                                             store_seq, nullptr, g_scale != nullptr);
+        epilogue_store_tile<T, WC, false, 1, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, my_out, lane, &tmY, &tmY, pixel, 0,
+                                                   rehearsal ? 0 : 32, store_seq, nullptr, g_scale != nullptr);
         read_done();
       } else if constexpr (STORE == kStoreSectors) {
         epilogue_store_sectors<T, WC, GELU>(t_row, n0, p.Kout, p.act, s_scale, s_bias, g_scale != nullptr,
@@ -455,7 +455,8 @@ conv_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 // The kernels a layer may run on: 32-byte stores for all of them, the other stores for layers that are not grouped.
 template <typename T, int BN, int BLK, int STORE>
-cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
+cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB, const CUtensorMap& tmY,
+                       const RowsParams& p, int grid, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
@@ -475,7 +476,8 @@ cudaError_t launch_one(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CU
 }
 
 template <typename T, int BN>
-cudaError_t launch_bn(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
+cudaError_t launch_bn(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB, const CUtensorMap& tmY,
+                      const RowsParams& p, int grid, cudaStream_t stream) {
   if (p.blk_groups == 1) {
     if (p.y_sk != 1) return launch_one<T, BN, 1, kStorePixels>(tmA, tmA2, tmB, tmY, p, grid, stream);
     if (p.y_unit == 32) return launch_one<T, BN, 1, kStoreSectors>(tmA, tmA2, tmB, tmY, p, grid, stream);
@@ -513,7 +515,8 @@ cudaError_t prepare_bn() {
 }
 
 template <typename T>
-cudaError_t launch_t(int tile_n, const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB, const CUtensorMap& tmY, const RowsParams& p, int grid, cudaStream_t stream) {
+cudaError_t launch_t(int tile_n, const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB, const CUtensorMap& tmY,
+                     const RowsParams& p, int grid, cudaStream_t stream) {
   if (tile_n == 64) return launch_bn<T, 64>(tmA, tmA2, tmB, tmY, p, grid, stream);
   if (tile_n == 128) return launch_bn<T, 128>(tmA, tmA2, tmB, tmY, p, grid, stream);
   if constexpr (sizeof(T) == 2) {

@@ -146,9 +146,23 @@ const char* fdnn_last_error(void);
  * device is visible).  `x`, `w`, `y` may be NULL; when given, their alignment
  * decides whether the tensors can be consumed in place by TMA.  The tiles are those of the plan's kernel; a
  * layer of W stride 1 with several filter columns may run on other ones, with the same scratch, packed filter
- * and results. */
+ * and results: fdnn_conv2d_main_kernel tells. */
 int fdnn_conv2d_query(const fdnn_conv_desc* desc, const void* x, const void* w,
                       const void* y, fdnn_conv_plan* plan);
+
+/* The kernel that fdnn_conv2d_fwd does the main work of a problem with, given the scratch and the packed filter of
+ * its plan (a grouped layer: w in place or packed, as the plan asks). */
+#define FDNN_KERNEL_DIRECT 0  /* CUDA cores: direct and depthwise kernels, no tiles */
+#define FDNN_KERNEL_IGEMM 1   /* conv_igemm_kernel, one CTA per tile */
+#define FDNN_KERNEL_PAIR 2    /* conv_igemm_pair_kernel, a CTA pair per tile */
+#define FDNN_KERNEL_ROWS 3    /* conv_rows_kernel, CTA pairs, one activation copy per filter row */
+typedef struct fdnn_conv_kernel {
+  int32_t kernel;               /* FDNN_KERNEL_* */
+  int32_t tile_m, tile_n;       /* rows and columns of a tile (0 for FDNN_KERNEL_DIRECT) */
+  int32_t grid;                 /* CTAs (0 for FDNN_KERNEL_DIRECT) */
+} fdnn_conv_kernel;
+int fdnn_conv2d_main_kernel(const fdnn_conv_desc* desc, const void* x, const void* w, const void* y,
+                            fdnn_conv_kernel* kernel);
 
 /* One-time filter relayout, the counterpart of the reference's packers
  * (src/flag_dnn/ops/conv2d.py:193-276): w[K,C/g,R,S] (any strides) ->
