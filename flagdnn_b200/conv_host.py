@@ -47,7 +47,8 @@ def set_stream_k(enabled: bool) -> bool:
     Off (the default), every tile is computed whole by one pair, and an image's result does not depend on the
     batch it is computed in down to the last bit.  On, layers whose tiles do not fill whole rounds of the GPU's
     pairs share the reduction steps evenly; on B200 that measured no faster (the layers are bound by operand
-    traffic from L2, which the split does not reduce), which is why it is off."""
+    traffic from L2, which the split does not reduce), which is why it is off.  While it is on, layers of W stride 1
+    with several filter columns stay on the kernels that copy their activations per tap."""
     global _STREAM_K
     prev, _STREAM_K = _STREAM_K, bool(enabled)
     return prev
