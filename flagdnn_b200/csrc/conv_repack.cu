@@ -135,12 +135,13 @@ __device__ __forceinline__ void pack_taps(const PackJob<T>& j, int block) {
 // of two channels and joins them, the writer reads four neighbouring words.
 // PACK: the launch's first blocks pack the layer's filter instead (one launch for both where a call brings a filter that is
 // not kept packed; as the last blocks they ended 0.8 us after the others, 128 -> 128 3x3 on 32 x 28 x 28).
-// The tiles wait for memory, so that blocks per SM count: eight where the transposition itself lets them in, six for reads by
-// element.  With ten taps in flight in the packing blocks every block held 44 to 62 registers, and an SM four or five blocks:
-// 64 -> 64 1x1 on 32 x 56 x 56 fp32 23.9 us, now 18.6 (17.1 without a filter to pack), 64 channels of 8 x 112 x 112 39.6 and 34.2
-// (33.2), bf16 14.5 and 13.2 (11.7).
-template <typename T, bool VEC, bool PACK>
-__global__ void __launch_bounds__(256, VEC ? 8 : 6)
+// The tiles wait for memory, so that blocks per SM count where there are many: eight where the transposition itself lets them
+// in, six for reads by element.  Unbounded, every block holds the 50 to 67 registers of the packing ones: 64 -> 64 1x1 on
+// 32 x 56 x 56 fp32 23.9 us, now 18.6 (17.1 without a filter to pack), 64 channels of 8 x 112 x 112 39.6 and 34.2 (33.2), bf16 14.5
+// and 13.2 (11.7).  FEW: with up to four blocks per SM those registers are loads in flight instead (calls of conv1d 136 -> 327
+// of 5 taps on 3 x 1265 11.1 us, bounded 12.9; 56 -> 24 5x5 on 94 x 8 x 21 11.0 and 12.3).
+template <typename T, bool VEC, bool PACK, bool FEW>
+__global__ void __launch_bounds__(256, FEW ? 1 : VEC ? 8 : 6)
 transpose_repack(const T* __restrict__ x, long long mat_stride, long long mat_stride2, int mats2, long long sc, int mats,
                  int C, int P, int c_pad, T* __restrict__ dst, long long plane, const PackJob<T> pack) {
   chain_launches();
@@ -483,9 +484,14 @@ cudaError_t transpose_t(const T* x, long long ms, long long ms2, int mats2, long
   const long long tiles = (long long)mats * ((P + 63) / 64) * ((c_pad + 128 / int(sizeof(T)) - 1) / (128 / int(sizeof(T))));
   PackJob<T> job = {};
   if (pack != nullptr) job = pack_job<T>(*pack, kPackTapsRelayout);
-  auto* kernel = pack != nullptr ? (vec ? transpose_repack<T, true, true> : transpose_repack<T, false, true>)
-                                 : (vec ? transpose_repack<T, true, false> : transpose_repack<T, false, false>);
-  launch_chained(kernel, dim3(grid_for(tiles, 1) + job.blocks), 256, stream, x, ms, ms2, mats2, sc, mats, C, P, c_pad, dst, plane, job);
+  const int grid = grid_for(tiles, 1) + job.blocks;
+  auto pick = [vec](auto packing, auto few) {
+    constexpr bool P = decltype(packing)::value, F = decltype(few)::value;
+    return vec ? transpose_repack<T, true, P, F> : transpose_repack<T, false, P, F>;
+  };
+  auto* kernel = pack == nullptr ? pick(std::false_type{}, std::false_type{})
+                 : grid <= 4 * current_sm_count() ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{});
+  launch_chained(kernel, dim3(grid), 256, stream, x, ms, ms2, mats2, sc, mats, C, P, c_pad, dst, plane, job);
   const cudaError_t e = cudaGetLastError();
   if (pack != nullptr) pack->done = e == cudaSuccess;
   return e;
@@ -506,12 +512,13 @@ cudaError_t rows_t(const T* x, long long sw, long long pixels, int C, int c_pad,
   return cudaGetLastError();
 }
 
-// Which kernel relays a tensor out: pixels contiguous in memory (W innermost; whole planes when rows are not padded,
-// else row by row) -> transposition; channels contiguous and pixels evenly spaced -> rows; anything else -> the
-// element-wise gather.  Extents of one carry no stride.
 template <typename T>
 cudaError_t pack_w_t(const void* w, const long long s[4], int K, int C, int R, int S, int c_pad, void* dst, long long plane,
                      cudaStream_t stream);
+
+// Which kernel relays a tensor out: pixels contiguous in memory (W innermost; whole planes when rows are not padded,
+// else row by row) -> transposition; channels contiguous and pixels evenly spaced -> rows; anything else -> the
+// element-wise gather.  Extents of one carry no stride.
 template <typename T>
 cudaError_t repack_x_t(const void* x, const long long x_s[4], int N, int C, int H, int W, int c_pad,
                        void* dst, long long plane, cudaStream_t stream, FilterPack* pack) {
