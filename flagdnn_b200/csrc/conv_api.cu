@@ -728,11 +728,13 @@ int make_plan(const fdnn_conv_desc* d, const void* x, const void* w, const void*
 //                                                                      more rounds); a tap by itself 600
 //   fp32                       800 / 1100                              600 / 830
 //   drain                      1500 / 3000 / 5000 through the TMA      2000 / 3000 / 4400 by sectors of 32 bytes
-//                              unit, else 6500 / 10000 / 11500         2700 / 5300 / 9200 along channels, 1500 / 2800 / 4000 pixels
+//                              unit, 6500 / 10000 / 11500 along        2700 / 5300 / 9200 along channels
+//                              channels, 2000 / 3500 / 5500 pixels     1500 / 2800 / 4000 pixels
 //   pixels off 128-byte lines  1100 per copy up to 192 bytes, wider    1100 per copy up to 192 bytes
-//                              ones 1.05 (64 columns) or 1.15 times
-// The constants are fitted to 1200 layers timed on the copy per tap and on all three widths here: 34 are over 4 % slower than on
-// the copy per tap (by 1.3 times at most), against 75 with one step time for all and 1350 for any pixel off a line
+//                              ones 1.05 (64 columns) or 1.15 times;
+//                              64-byte ones 1100 from three rounds on
+// The constants are fitted to 1600 layers timed on the copy per tap and on all three widths here: 29 are over 4 % slower than on
+// the copy per tap (by 1.3 times at most); with one step time for all and 1350 for any pixel off a line it was 75 of 1200
 // (34 x 66 x 8 x 824 -> 288 80 and 105, 87 x 14 x 14 x 440 -> 184 5x5 65 and 81).
 struct RowsMode {
   int tile_n;          // 0: no
@@ -786,17 +788,18 @@ RowsMode rows_mode(const fdnn_conv_desc* d, const fdnn_conv_plan& plan, const vo
     auto column_class = [](int columns) { return columns == 64 ? 0 : columns == 128 ? 1 : 2; };
     auto rounds = [](long long tiles, int units) { return double((tiles + units - 1) / units); };
     auto longer = [](double x, double z) { return x > z ? x : z; };
-    static constexpr double kStep[3] = {365, 510, 650}, kDrainTma[3] = {1500, 3000, 5000}, kDrainOther[3] = {6500, 10000, 11500};
+    static constexpr double kStep[3] = {365, 510, 650}, kDrainTma[3] = {1500, 3000, 5000}, kDrainOther[3] = {6500, 10000, 11500}, kDrainPixels[3] = {2000, 3500, 5500};
     static constexpr double kTap[3] = {225, 290, 600}, kSectors[3] = {2000, 3000, 4400}, kChannels[3] = {2700, 5300, 9200},
                             kPixels[3] = {1500, 2800, 4000};
     const int now_class = column_class(plan.tile_n);
-    double step = pair ? 690 : es == 4 ? (now_class == 0 ? 800 : 1100) : kStep[now_class];
-    step = longer(step, copy);
-    if (off_lines && pixel > 192) step *= !pair && now_class == 0 ? 1.05 : 1.15;
     const long long m_now = ((long long)d->n * oh * ow / q + plan.tile_m - 1) / plan.tile_m;
     const long long tiles_now = m_now * (((long long)q * d->k + plan.tile_n - 1) / plan.tile_n);
-    double best_cost = rounds(tiles_now, pair ? sms / 2 : sms) *
-                       longer(steps * (d->s + (q - 1) * d->stride_w) * step, (y_is_dense_nhwc(d, oh, ow, y) ? kDrainTma : kDrainOther)[now_class]);
+    const double rounds_now = rounds(tiles_now, pair ? sms / 2 : sms);
+    double step = pair ? 690 : es == 4 ? (now_class == 0 ? 800 : 1100) : kStep[now_class];
+    step = longer(step, pixel == 64 && d->w > 1 && q == 1 && rounds_now >= 3 ? 1100 : copy);
+    if (off_lines && pixel > 192) step *= !pair && now_class == 0 ? 1.05 : 1.15;
+    const double* drain_now = y_is_dense_nhwc(d, oh, ow, y) ? kDrainTma : d->y_strides[1] != 1 ? kDrainPixels : kDrainOther;
+    double best_cost = rounds_now * longer(steps * (d->s + (q - 1) * d->stride_w) * step, drain_now[now_class]);
     const double* drain = d->y_strides[1] != 1 ? kPixels : sector_aligned(*d, oh, ow, y) ? kSectors : kChannels;
     for (int bn = 64; bn <= (es == 2 ? 256 : 128); bn *= 2) {
       if (bn > 64 && bn / 2 >= d->k) break;
