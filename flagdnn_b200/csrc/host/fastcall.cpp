@@ -15,6 +15,7 @@
 
 #include <ATen/ATen.h>
 #include <c10/core/DeviceGuard.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -59,8 +60,11 @@ constexpr size_t kMaxPlans = 1024;
 // 10.5, on 4 x 56 x 56 8.7 and 10.6.  Beyond some 9 us of GPU time the look-up is hidden and the packing is not: 128 -> 128 on
 // 8 x 28 x 28 11.6 and 10.4, on 32 x 28 x 28 16.5 and 15.5, fp32 64 -> 64 on 8 x 56 x 56 21.9 and 20.9.
 constexpr int64_t kPackAlways = 1 << 20;
-bool sooner_than_a_look_up(const fdnn_conv_plan& plan, int dtype) {
-  return plan.packed_weight_bytes <= kPackAlways && plan.bytes <= 6e6 && plan.flops <= (dtype == FDNN_F32 ? 2e8 : 1.5e9);
+// Under capture they are packed on the way at any size: replays then read the filter as it is, not as it was.
+bool pack_on_the_way(const fdnn_conv_plan& plan, int dtype) {
+  if (plan.packed_weight_bytes > kPackAlways) return false;
+  return (plan.bytes <= 6e6 && plan.flops <= (dtype == FDNN_F32 ? 2e8 : 1.5e9)) ||
+         c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
 }
 std::unordered_map<PlanKey, fdnn_conv_plan, PlanHash>& plans() {   // used with the GIL held
   static auto* m = new std::unordered_map<PlanKey, fdnn_conv_plan, PlanHash>();
@@ -161,7 +165,7 @@ int launch(const fdnn_conv_desc& d, const at::Tensor& x, const at::Tensor& w, Py
   const void* packed_ptr = nullptr;
   if (plan.algo != FDNN_ALGO_DIRECT && plan.w_packed) {
     const bool in_relayout = plan.x_repacked && d.groups == 1 && plan.low_channel == 0 && plan.pixel_group <= 1 && d.c >= 8 &&
-                             d.x_strides[3] == 1 && d.x_strides[1] != 1 && d.w > 1 && sooner_than_a_look_up(plan, d.dtype);
+                             d.x_strides[3] == 1 && d.x_strides[1] != 1 && d.w > 1 && pack_on_the_way(plan, d.dtype);
     if (weight_obj == nullptr || in_relayout) {
       WithoutGil free;
       const int64_t ws_bytes = (plan.workspace_bytes + 255) / 256 * 256, bytes = ws_bytes + plan.packed_weight_bytes;
