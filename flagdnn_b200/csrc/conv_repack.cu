@@ -138,8 +138,9 @@ __device__ __forceinline__ void pack_taps(const PackJob<T>& j, int block) {
 // The tiles wait for memory, so that blocks per SM count where there are many: eight where the transposition itself lets them
 // in, six for reads by element.  Unbounded, every block holds the 50 to 67 registers of the packing ones: 64 -> 64 1x1 on
 // 32 x 56 x 56 fp32 23.9 us, now 18.6 (17.1 without a filter to pack), 64 channels of 8 x 112 x 112 39.6 and 34.2 (33.2), bf16 14.5
-// and 13.2 (11.7).  FEW: with up to four blocks per SM those registers are loads in flight instead (calls of conv1d 136 -> 327
-// of 5 taps on 3 x 1265 11.1 us, bounded 12.9; 56 -> 24 5x5 on 94 x 8 x 21 11.0 and 12.3).
+// and 13.2 (11.7).  FEW: with up to four blocks per SM registers are loads in flight instead (calls of conv1d 136 -> 327 of 5
+// taps on 3 x 1265 11.1 us, bounded 12.9; 56 -> 24 5x5 on 94 x 8 x 21 11.0 and 12.3; 256 -> 512 1x1 on 64 x 7 x 7, nothing to pack,
+// 9.0 and 10.5).
 template <typename T, bool VEC, bool PACK, bool FEW>
 __global__ void __launch_bounds__(256, FEW ? 1 : VEC ? 8 : 6)
 transpose_repack(const T* __restrict__ x, long long mat_stride, long long mat_stride2, int mats2, long long sc, int mats,
@@ -489,8 +490,9 @@ cudaError_t transpose_t(const T* x, long long ms, long long ms2, int mats2, long
     constexpr bool P = decltype(packing)::value, F = decltype(few)::value;
     return vec ? transpose_repack<T, true, P, F> : transpose_repack<T, false, P, F>;
   };
-  auto* kernel = pack == nullptr ? pick(std::false_type{}, std::false_type{})
-                 : grid <= 4 * current_sm_count() ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{});
+  const bool few = grid <= 4 * current_sm_count();
+  auto* kernel = pack == nullptr ? (few ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{}))
+                                 : (few ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{}));
   launch_chained(kernel, dim3(grid), 256, stream, x, ms, ms2, mats2, sc, mats, C, P, c_pad, dst, plane, job);
   const cudaError_t e = cudaGetLastError();
   if (pack != nullptr) pack->done = e == cudaSuccess;
