@@ -57,13 +57,14 @@ static_assert(sizeof(fdnn_conv_desc) % 4 == 0 && sizeof(PlanKey) % 4 == 0, "hash
 constexpr size_t kMaxPlans = 1024;
 // Packing a filter of up to a megabyte in the launch that relays an NCHW x out costs less than the look-up of a kept one, which
 // is Python code, as long as the GPU is done before the host: calls of 64 -> 64 3x3 bf16 on one 14 x 14 image 8.6 us against
-// 10.5, on 4 x 56 x 56 8.7 and 10.6.  Beyond some 9 us of GPU time the look-up is hidden and the packing is not: 128 -> 128 on
-// 8 x 28 x 28 11.6 and 10.4, on 32 x 28 x 28 16.5 and 15.5, fp32 64 -> 64 on 8 x 56 x 56 21.9 and 20.9.
+// 10.5, on 4 x 56 x 56 8.7 and 10.6, 128 -> 128 on 8 x 28 x 28 10.4 and 11.4, fp32 64 -> 64 on 4 x 56 x 56 through a graph 13.7 and 15.8.
+// Beyond some 12 us of GPU time the look-up is hidden and the packing is not: 128 -> 128 on 32 x 28 x 28 16.5 and 15.5, fp32
+// 64 -> 64 on 8 x 56 x 56 21.9 and 20.9.
 constexpr int64_t kPackAlways = 1 << 20;
 // Under capture they are packed on the way at any size: replays then read the filter as it is, not as it was.
 bool pack_on_the_way(const fdnn_conv_plan& plan, int dtype) {
   if (plan.packed_weight_bytes > kPackAlways) return false;
-  return (plan.bytes <= 6e6 && plan.flops <= (dtype == FDNN_F32 ? 2e8 : 1.5e9)) ||
+  return (plan.bytes <= 1e7 && plan.flops <= (dtype == FDNN_F32 ? 1e9 : 3e9)) ||
          c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
 }
 std::unordered_map<PlanKey, fdnn_conv_plan, PlanHash>& plans() {   // used with the GIL held
